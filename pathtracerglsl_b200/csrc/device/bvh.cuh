@@ -447,14 +447,14 @@ __device__ __forceinline__ bool inst_mesh_flat(const DevScene& S, const DevBatch
 #define PTR_FLAT_INST 1
 #endif
 __device__ __forceinline__ bool inst_mesh_flat_ok(const DevScene& S, const DevBatch& b) {
-    return PTR_FLAT_INST && b.proto_shape == PTR_SHAPE_MESH && S.accel == PTR_ACCEL_CWBVH &&
+    return kHasMesh && PTR_FLAT_INST && b.proto_shape == PTR_SHAPE_MESH && S.accel == PTR_ACCEL_CWBVH &&
            !(S.inst_accel == PTR_ACCEL_CWBVH && b.tlas_w) && S.meshes[b.proto_mesh].cwbvh != nullptr;
 }
 
 // ---- region arms ------------------------------------------------------------------------
 __device__ __forceinline__ void accel_closest(const DevScene& S, const ptr_region& g, int region, const Ray& r, HitRec& h,
                                               Work* w = nullptr) {
-    if (g.shape == PTR_SHAPE_MESH) {
+    if (kHasMesh && g.shape == PTR_SHAPE_MESH) {
         const DevMesh& m = S.meshes[g.ref];
         int prim = -1;
         float t = h.t;
@@ -480,7 +480,7 @@ __device__ __forceinline__ void accel_closest(const DevScene& S, const ptr_regio
     auto wins_tie = [&](int i) { return h.region == region && __ldg(inst_id + i) < __ldg(inst_id + h.element); };
     // one instance: the params-tier sphere, or the mesh prototype in the placement's frame
     auto instance = [&](int i) {
-        if (b.proto_shape == PTR_SHAPE_SPHERE) {
+        if (!kHasMesh || b.proto_shape == PTR_SHAPE_SPHERE) {
             float4 rec = __ldg(place + 2 * i);
             float t;
             if (sphere_intersect(r, xyz(rec), rec.w, t) && (t < t_near || (t == t_near && wins_tie(i)))) {
@@ -511,7 +511,7 @@ __device__ __forceinline__ void accel_closest(const DevScene& S, const ptr_regio
 
 __device__ __forceinline__ bool accel_any(const DevScene& S, const ptr_region& g, const Ray& r, float max_dist,
                                           Work* w = nullptr) {
-    if (g.shape == PTR_SHAPE_MESH) return mesh_any(S, S.meshes[g.ref], r.o, r.d, max_dist, w);
+    if (kHasMesh && g.shape == PTR_SHAPE_MESH) return mesh_any(S, S.meshes[g.ref], r.o, r.d, max_dist, w);
     const DevBatch& b = S.batches[g.ref];
     if (inst_mesh_flat_ok(S, b)) {
         HitRec unused;
@@ -520,7 +520,7 @@ __device__ __forceinline__ bool accel_any(const DevScene& S, const ptr_region& g
     const bool wide = S.inst_accel == PTR_ACCEL_CWBVH && b.tlas_w;
     const float4* place = wide ? b.place_w : b.place;
     auto instance = [&](int i) -> bool {
-        if (b.proto_shape == PTR_SHAPE_SPHERE) {
+        if (!kHasMesh || b.proto_shape == PTR_SHAPE_SPHERE) {
             float4 rec = __ldg(place + 2 * i);
             float t;
             return sphere_intersect(r, xyz(rec), rec.w, t) && t < max_dist;
@@ -580,7 +580,7 @@ __device__ __forceinline__ f3 accel_hit_normal(const DevScene& S, const ptr_regi
         const DevBatch& b = S.batches[g.ref];
         // hr.element indexes the placements of the TLAS the hit was found with
         const float4* place = (S.inst_accel == PTR_ACCEL_CWBVH && b.tlas_w) ? b.place_w : b.place;
-        if (b.proto_shape == PTR_SHAPE_SPHERE) {
+        if (!kHasMesh || b.proto_shape == PTR_SHAPE_SPHERE) {
             float4 rec = __ldg(place + 2 * hr.element);
             f3 n = normalize(h.p - xyz(rec));
             ng = n;   // a primitive's normal is its true surface normal (set from frame.n)

@@ -16,12 +16,15 @@ namespace ptx {
 // build with PTR_WIDE_MATH (ptr_specialize with that define) evaluates them in double and
 // rounds once, the same functions as the oracle's wide twin, so that samples can be
 // compared without the two libms' last-ulp differences.
+#ifndef PTR_MINL
+#define PTR_MINL __noinline__
+#endif
 #ifdef PTR_WIDE_MATH
 #define PTR_M1(name, fn) __device__ __forceinline__ float name(float x) { return (float)fn((double)x); }
 #define PTR_M2(name, fn) __device__ __forceinline__ float name(float x, float y) { return (float)fn((double)x, (double)y); }
 #else
-#define PTR_M1(name, fn) __device__ __forceinline__ float name(float x) { return fn##f(x); }
-#define PTR_M2(name, fn) __device__ __forceinline__ float name(float x, float y) { return fn##f(x, y); }
+#define PTR_M1(name, fn) __device__ PTR_MINL float name(float x) { return fn##f(x); }
+#define PTR_M2(name, fn) __device__ PTR_MINL float name(float x, float y) { return fn##f(x, y); }
 #endif
 PTR_M1(m_exp, exp) PTR_M1(m_log, log) PTR_M1(m_sin, sin) PTR_M1(m_cos, cos) PTR_M1(m_tan, tan)
 PTR_M1(m_tanh, tanh) PTR_M1(m_atanh, atanh) PTR_M1(m_cosh, cosh) PTR_M2(m_atan2, atan2) PTR_M2(m_pow, pow)
@@ -49,6 +52,12 @@ PTR_M1(m_tanh, tanh) PTR_M1(m_atanh, atanh) PTR_M1(m_cosh, cosh) PTR_M2(m_atan2,
 #ifndef PTR_SPEC_TREE
 #define PTR_SPEC_TREE 1         // 0: the build never selects lights with the light tree
 #endif
+#ifndef PTR_SPEC_HET
+#define PTR_SPEC_HET 1          // 0: no medium of the build has a coefficient field
+#endif
+#ifndef PTR_SPEC_MESH
+#define PTR_SPEC_MESH 1         // 0: the build holds no triangle meshes (mesh regions or instanced meshes)
+#endif
 #ifndef PTR_SPEC_NREGIONS
 #define PTR_SPEC_NREGIONS 0     // 1..16: the region count and PTR_SPEC_SHAPE_CODE (the region BVH unused)
 #endif
@@ -56,6 +65,9 @@ __host__ __device__ constexpr bool has_mat(int m) { return ((PTR_SPEC_MATS) >> m
 __host__ __device__ constexpr bool has_light(int k) { return ((PTR_SPEC_LIGHTS) >> k) & 1u; }
 __host__ __device__ constexpr bool has_env(int k) { return ((PTR_SPEC_ENVS) >> k) & 1u; }
 __host__ __device__ constexpr bool has_shape(int k) { return ((PTR_SPEC_SHAPES) >> k) & 1u; }
+constexpr bool kHasMesh = PTR_SPEC_MESH;
+// regions walked through acceleration structures (meshes, instanced batches)
+__host__ __device__ constexpr bool has_accel() { return kHasMesh || has_shape(PTR_SHAPE_INSTANCES); }
 // (material models and light kinds are dispatched through their registries, occupant.cuh)
 #if PTR_SPEC_NREGIONS > 0
 static_assert(PTR_SPEC_NREGIONS <= 16, "the shape code holds 16 regions");
@@ -182,9 +194,8 @@ struct Frame { f3 t, b, n; };
 __device__ __forceinline__ float fp_uncertainty(f3 p) {
     return gmax(kFpAbs, kFpRel * gmax(fabsf(p.x), gmax(fabsf(p.y), fabsf(p.z))));
 }
-// Shading frame from a normal (the Euclidean ambient_frame, euclidean.glsl:6-33).
-__device__ __forceinline__ Frame ambient_frame(f3 n) {
-    f3 nn = normalize(n);
+// Shading frame from a normalised normal (the Euclidean ambient_frame, euclidean.glsl:6-33).
+__device__ __forceinline__ Frame unit_frame(f3 nn) {
     f3 t = fabsf(nn.x) < 0.9f ? f3(1.f, 0.f, 0.f) : f3(0.f, 1.f, 0.f);
     t = normalize(t - dot(t, nn) * nn);
     Frame f;

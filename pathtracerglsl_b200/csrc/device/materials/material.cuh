@@ -10,6 +10,7 @@
 //   kNonDelta     it has a non-delta lobe: NEE and MIS evaluate eval() / pdf() toward lights
 //   kSphereQuery  light selection queries a sphere of directions around the point (a
 //                 transmissive non-delta lobe sees lights on both sides)
+//   kUsesIor      it reads the IORs of the surface's two sides (MatSite::n_from / n_to)
 //   aov(m)        the first-hit albedo picture's colour
 //   sample(...)   the continuation lobe: direction, weight f cos / pdf, pdf, lobe flags
 //   eval / pdf    the non-delta lobe toward a light direction (kNonDelta models only)
@@ -45,6 +46,7 @@ struct NeeGrad {
 struct MaterialModel {
     static constexpr bool kNonDelta = false;
     static constexpr bool kSphereQuery = false;
+    static constexpr bool kUsesIor = false;
     __device__ static f3 aov(const ptr_material& m) { return ld3(m.transmittance); }
     __device__ static void nee_grad(const MatSite<f3>&, f3, f3, NeeGrad&) {}
     __device__ static void cont_grad(const MatSite<f3>&, const ISample<f3>&, f3, const GradAcc&, f3, bool, NeeGrad&) {}
@@ -54,6 +56,7 @@ struct MaterialModel {
 // it has a non-delta lobe / queries lights over the sphere.
 template <class M> struct MatPresent { static constexpr bool value = has_mat(M::kId); };
 template <class M> struct MatNonDelta { static constexpr bool value = has_mat(M::kId) && M::kNonDelta; };
+template <class M> struct MatUsesIor { static constexpr bool value = has_mat(M::kId) && M::kUsesIor; };
 template <class M> struct MatSphereQuery { static constexpr bool value = has_mat(M::kId) && M::kSphereQuery; };
 
 }  // namespace ptx

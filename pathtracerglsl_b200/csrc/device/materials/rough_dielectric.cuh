@@ -97,6 +97,7 @@ struct RoughDielectric : MaterialModel {
     static constexpr int kId = PTR_MAT_ROUGH_DIELECTRIC;
     static constexpr bool kNonDelta = true;
     static constexpr bool kSphereQuery = true;
+    static constexpr bool kUsesIor = true;
     template <class Col>
     __device__ static ISample<Col> sample(const MatSite<Col>& s, f3 wo, float uc, float u0, float u1) {
         return rough_dielectric_sample(wo, s.hit, Colors<Col>::tint(s.S, s.mat, s.wl), s.alpha, s.n_from, s.n_to, uc, u0, u1);

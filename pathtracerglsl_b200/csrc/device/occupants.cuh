@@ -18,16 +18,16 @@ namespace ptx {
 // (color/spectral/lookup.glsl:38-59, spectra/blackbody/blackbody.glsl:4-10).
 struct Wl { float4 lambda; };
 
-__device__ __forceinline__ float4 spectral_curves(const DevScene& S, float lambda) {
+__device__ __forceinline__ float4 spectral_curves(const float4* curves, float lambda) {
     float x = (lambda - 360.0f) / 5.0f;
     int i = (int)x;
     i = i < 93 ? i : 93;
-    float4 a = __ldg(S.spec_curves + i), b = __ldg(S.spec_curves + i + 1);
+    float4 a = __ldg(curves + i), b = __ldg(curves + i + 1);
     float f = x - (float)i;
     return make_float4(a.x * (1.0f - f) + b.x * f, a.y * (1.0f - f) + b.y * f, a.z * (1.0f - f) + b.z * f,
                        a.w * (1.0f - f) + b.w * f);
 }
-__device__ __forceinline__ float spec_lane(const DevScene& S, const ptr_spectrum& sp, float lambda) {
+__device__ __forceinline__ float spec_lane(const float4* curves, const ptr_spectrum& sp, float lambda) {
     float v;
     if (sp.kind == PTR_SPEC_LIFTED) {
         float t = (lambda - 360.0f) / 470.0f;
@@ -43,12 +43,16 @@ __device__ __forceinline__ float spec_lane(const DevScene& S, const ptr_spectrum
     } else {
         v = sp.scale;
     }
-    if (sp.d65) v = v * spectral_curves(S, lambda).w;
+    if (sp.d65) v = v * spectral_curves(curves, lambda).w;
     return v;
 }
+__device__ __noinline__ float4 spec_lanes(const float4* curves, const ptr_spectrum* sp, float4 l) {
+    const ptr_spectrum s = *sp;
+    return make_float4(spec_lane(curves, s, l.x), spec_lane(curves, s, l.y), spec_lane(curves, s, l.z), spec_lane(curves, s, l.w));
+}
 __device__ __forceinline__ s4 spec_eval(const DevScene& S, const ptr_spectrum& sp, const Wl& wl) {
-    return s4(spec_lane(S, sp, wl.lambda.x), spec_lane(S, sp, wl.lambda.y), spec_lane(S, sp, wl.lambda.z),
-              spec_lane(S, sp, wl.lambda.w));
+    const float4 v = spec_lanes(S.spec_curves, &sp, wl.lambda);
+    return s4(v.x, v.y, v.z, v.w);
 }
 
 template <class Col> struct Colors;
@@ -70,7 +74,7 @@ template <> struct Colors<s4> {
     __device__ static s4 sigma_a(const DevScene& S, int mi, const Wl& w) { return spec_eval(S, S.spec_mats[mi].sigma_a, w); }
     __device__ static s4 sigma_s(const DevScene& S, int mi, const Wl& w) { return spec_eval(S, S.spec_mats[mi].sigma_s, w); }
     __device__ static s4 light(const DevScene& S, int li, const Wl& w) { return spec_eval(S, S.spec_lights[li], w); }
-    __device__ static s4 env_color(const DevScene& S, const Wl& w) { return spec_eval(S, S.spec_env, w); }
+    __device__ static s4 env_color(const DevScene& S, const Wl& w) { const ptr_spectrum e = S.spec_env; return spec_eval(S, e, w); }
 };
 
 // ---- surface material models: one header each under materials/ (registry.cuh) ---------
@@ -347,62 +351,42 @@ __device__ __forceinline__ float light_tree_pmf(const DevScene& S, const LightQu
     }
     return pmf;
 }
+// A light direction: the two-stage env-vs-finite draw (lighting.ts generateLightSampling), the
+// finite stage by the power CDF with the rescaled coordinate (lighting.ts:546-637) or by
+// the light tree's descent (lighting.ts:830-900).  The stages only choose the light and its
+// coordinate, so every light kind's code is met once.
 template <class Col>
-__device__ LightSample<Col> lighting_sample_tree(const DevScene& S, const LightQuery& q, float x0, float x1, Rng& rng,
-                                                 const Wl& wl) {
+__device__ __forceinline__ LightSample<Col> lighting_sample(const DevScene& S, const LightQuery& q, float x0, float x1, Rng& rng,
+                                                            bool tree, const Wl& wl) {
     LightSample<Col> ls;
-    float sel;
-    int id = light_tree_pick(S, q, x0, rng, sel);
-    if (id < 0) { ls.pdf = 0.0f; return ls; }   // dead descent: a zero-contribution event
-    float lx = rng.next();
-    ls = light_sample_one(S, S.lights[id], Colors<Col>::light(S, id, wl), q.p, lx, x1);
+    ls.pdf = 0.0f;
+    const bool live = S.env_select_live;
+    const float pe = S.env_select_prob;
+    if (S.n_lights == 0 ? S.env_samplable : (live && x0 < pe)) {
+        ls = env_sample<Col>(S, S.n_lights == 0 ? x0 : clampf(x0 / pe, 0.0f, 0.9999999f), x1, wl);
+        if (S.n_lights != 0) ls.pdf *= pe;
+        return ls;
+    }
+    if (S.n_lights == 0) return ls;
+    if (live) x0 = clampf((x0 - pe) / (1.0f - pe), 0.0f, 0.9999999f);
+    int id = 0;
+    float sel = 1.0f;
+    if (PTR_SPEC_TREE && tree) {
+        id = light_tree_pick(S, q, x0, rng, sel);
+        if (id < 0) return ls;   // dead descent: a zero-contribution event
+        x0 = rng.next();
+    } else if (S.n_lights > 1) {
+        id = S.n_lights - 1;
+        for (int i = 0; i < S.n_lights - 1; ++i)
+            if (x0 < S.lights[i].select_cdf) { id = i; break; }
+        const float lo = id == 0 ? 0.0f : S.lights[id - 1].select_cdf;
+        sel = S.lights[id].select_pdf;
+        x0 = clampf((x0 - lo) / sel, 0.0f, 0.9999999f);
+    }
+    ls = light_sample_one(S, S.lights[id], Colors<Col>::light(S, id, wl), q.p, x0, x1);
     ls.light_id = id;
     ls.pdf *= sel;
-    return ls;
-}
-
-// Finite-light selection by the power CDF with the rescaled coordinate (lighting.ts:546-637).
-template <class Col>
-__device__ LightSample<Col> lighting_sample_finite(const DevScene& S, f3 p, float x0, float x1, const Wl& wl) {
-    if (S.n_lights == 1) {
-        LightSample<Col> ls = light_sample_one(S, S.lights[0], Colors<Col>::light(S, 0, wl), p, x0, x1);
-        ls.light_id = 0;
-        return ls;
-    }
-    int id = S.n_lights - 1;
-    for (int i = 0; i < S.n_lights - 1; ++i)
-        if (x0 < S.lights[i].select_cdf) { id = i; break; }
-    float lo = id == 0 ? 0.0f : S.lights[id - 1].select_cdf;
-    float sel = S.lights[id].select_pdf;
-    float xr = (x0 - lo) / sel;
-    LightSample<Col> ls = light_sample_one(S, S.lights[id], Colors<Col>::light(S, id, wl), p, clampf(xr, 0.0f, 0.9999999f), x1);
-    ls.light_id = id;
-    ls.pdf *= sel;
-    return ls;
-}
-// Two-stage env-vs-finite draw (lighting.ts generateLightSampling).
-// (tree: the light-tree walk replaces the finite stage, lighting.ts:830-900)
-template <class Col>
-__device__ LightSample<Col> lighting_sample(const DevScene& S, const LightQuery& q, float x0, float x1, Rng& rng,
-                                            bool tree, const Wl& wl) {
-    if (S.n_lights == 0) {
-        if (S.env_samplable) return env_sample<Col>(S, x0, x1, wl);
-        LightSample<Col> ls;
-        ls.pdf = 0.0f;
-        return ls;
-    }
-    tree = PTR_SPEC_TREE && tree;
-    if (!S.env_select_live)
-        return tree ? lighting_sample_tree<Col>(S, q, x0, x1, rng, wl) : lighting_sample_finite<Col>(S, q.p, x0, x1, wl);
-    float pe = S.env_select_prob;
-    if (x0 < pe) {
-        LightSample<Col> ls = env_sample<Col>(S, clampf(x0 / pe, 0.0f, 0.9999999f), x1, wl);
-        ls.pdf *= pe;
-        return ls;
-    }
-    float fx = clampf((x0 - pe) / (1.0f - pe), 0.0f, 0.9999999f);
-    LightSample<Col> ls = tree ? lighting_sample_tree<Col>(S, q, fx, x1, rng, wl) : lighting_sample_finite<Col>(S, q.p, fx, x1, wl);
-    ls.pdf *= (1.0f - pe);
+    if (live) ls.pdf *= (1.0f - pe);
     return ls;
 }
 // q: the selection context stored when the path left the previous vertex
@@ -435,7 +419,9 @@ template <class Col> struct MediumSample { bool scattered; Col weight; f3 exit_p
 // A coefficient field: the stack program of a GLSL expression of p (validated at upload:
 // known opcodes, stack depth within PTR_FIELD_MAX_STACK, END inside the table).
 __device__ __forceinline__ float fract_(float x) { return x - floorf(x); }
-__device__ f3 field_eval(const uint32_t* code, f3 p) {
+// One copy of the interpreter serves every tracking loop (inlined, its copies crowd the
+// instruction cache: the walk's kernels stall on instruction fetch first).
+__device__ __noinline__ f3 field_eval(const uint32_t* code, f3 p) {
     f3 st[PTR_FIELD_MAX_STACK];
     int sp = 0;
     for (int pc = 0;;) {
@@ -463,9 +449,9 @@ __device__ f3 field_eval(const uint32_t* code, f3 p) {
         }
         if (op >= PTR_FOP_NEG && op <= PTR_FOP_FRACT) {
             f3 a = st[sp - 1];
-            float r[3] = {a.x, a.y, a.z};
-            for (int k = 0; k < 3; ++k) {
-                float x = r[k];
+#pragma unroll 1
+            for (int k = 0; k < 3; ++k) {   // lane by lane, rotating: one copy of each function
+                float x = a.x;
                 switch (op) {
                     case PTR_FOP_NEG: x = -x; break;
                     case PTR_FOP_EXP: x = m_exp(x); break;
@@ -477,16 +463,16 @@ __device__ f3 field_eval(const uint32_t* code, f3 p) {
                     case PTR_FOP_FLOOR: x = floorf(x); break;
                     default: x = fract_(x); break;
                 }
-                r[k] = x;
+                a = f3(a.y, a.z, x);
             }
-            st[sp - 1] = f3(r[0], r[1], r[2]);
+            st[sp - 1] = a;
             continue;
         }
         if (op >= PTR_FOP_POW && op <= PTR_FOP_STEP) {
             f3 b = st[--sp], a = st[sp - 1];
-            float ra[3] = {a.x, a.y, a.z}, rb[3] = {b.x, b.y, b.z};
+#pragma unroll 1
             for (int k = 0; k < 3; ++k) {
-                float x = ra[k], y = rb[k];
+                float x = a.x, y = b.x;
                 switch (op) {
                     case PTR_FOP_POW: x = m_pow(x, y); break;
                     case PTR_FOP_MIN: x = y < x ? y : x; break;
@@ -494,9 +480,10 @@ __device__ f3 field_eval(const uint32_t* code, f3 p) {
                     case PTR_FOP_MOD: x = x - y * floorf(x / y); break;
                     default: x = y < x ? 0.0f : 1.0f; break;   // step(edge = a, x = b)
                 }
-                ra[k] = x;
+                a = f3(a.y, a.z, x);
+                b = f3(b.y, b.z, b.x);
             }
-            st[sp - 1] = f3(ra[0], ra[1], ra[2]);
+            st[sp - 1] = a;
             continue;
         }
         if (op >= PTR_FOP_CLAMP && op <= PTR_FOP_SMOOTHSTEP) {
@@ -536,7 +523,7 @@ __device__ f3 field_eval(const uint32_t* code, f3 p) {
     }
     return st[0];
 }
-__device__ __forceinline__ bool mat_is_het(const ptr_material& m) { return (m.field_a | m.field_s) != 0; }
+__device__ __forceinline__ bool mat_is_het(const ptr_material& m) { return PTR_SPEC_HET && (m.field_a | m.field_s) != 0; }
 // The rendered medium at p: the fields (or constants), scaled down proportionally where the
 // maximum extinction exceeds the majorant (the D1 ceiling of the generated lookup).
 struct HetProps { f3 sa, ss; };

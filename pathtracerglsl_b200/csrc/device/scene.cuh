@@ -63,6 +63,10 @@ struct DevScene {
     // Without a region BVH: the region list as runs of one shape, (shape, first, count, 0)
     // in region order, so the scan dispatches once per run (NULL: per region)
     const int4* region_runs;
+    // One float4 per region for the run scans and the unrolled arms of a per-scene build: a
+    // sphere's (centre, radius^2 widened by kScanPad); a quad's edge dot products (e1.e1,
+    // e2.e2, e1.e2) and their determinant, the values quad_intersect would compute
+    const float4* region_scan;
     int n_linear, n_region_nodes, n_runs, pad_r1;
     int n_regions, n_materials, n_lights, ambient_material;
     int has_media, accel, n_meshes, n_batches;
@@ -118,6 +122,31 @@ __device__ __forceinline__ bool plane_intersect(const Ray& r, f3 n, float off, f
     t = -(dot(r.o, n) + off) / denom;
     return t > 0.0f;
 }
+// A cheap necessary condition of sphere_intersect for rays of unit direction: scan = (centre,
+// widened radius^2).  It rejects spheres whose line distance exceeds the radius and spheres
+// wholly behind the origin.  kScanPad covers the rounding of both forms: with |d|^2 = 1 +-
+// 1e-3 (RayScan) the exact |perp|^2 differs from |oc|^2 - b^2 (2 - |d|^2) by less than
+// 1e-6 (|oc|^2 + r^2), and b > 0 with b^2 > 1.01 r^2 leaves both exact roots negative.
+// FMA is free to use here: the verdict only selects who runs the exact test.
+constexpr float kScanPad = 4.0e-6f;
+struct RayScan {
+    float k;      // 2 - |d|^2
+    bool unit;    // the condition holds for this direction; else every sphere is a candidate
+    __device__ __forceinline__ explicit RayScan(const Ray& r) {
+        const float dd = dot(r.d, r.d);
+        k = 2.0f - dd;
+        unit = fabsf(dd - 1.0f) < 1.0e-3f;
+    }
+    __device__ __forceinline__ bool sphere(const Ray& r, float4 scan) const {
+        const float x = r.o.x - scan.x, y = r.o.y - scan.y, z = r.o.z - scan.z;
+        const float b = __fmaf_rn(z, r.d.z, __fmaf_rn(y, r.d.y, x * r.d.x));
+        const float oc2 = __fmaf_rn(z, z, __fmaf_rn(y, y, x * x));
+        const float bb = b * b;
+        const bool miss = __fmaf_rn(-bb, k, oc2 * (1.0f - kScanPad)) > scan.w;
+        const bool behind = b > 0.0f && bb > 1.01f * scan.w;
+        return !(miss || behind) || !unit;
+    }
+};
 // Quad: plane root + inside test through the 2x2 Gram system (quad.glsl:9-22).
 __device__ __forceinline__ bool quad_intersect(const Ray& r, f3 corner, f3 e1, f3 e2, f3 n, float& t) {
     float denom = dot(r.d, n);
@@ -130,6 +159,19 @@ __device__ __forceinline__ bool quad_intersect(const Ray& r, f3 corner, f3 e1, f
     float det = e11 * e22 - e12 * e12;
     float u = (d1 * e22 - d2 * e12) / det;
     float v = (d2 * e11 - d1 * e12) / det;
+    return u >= 0.0f && u <= 1.0f && v >= 0.0f && v <= 1.0f;
+}
+// The same with the edge products given (region_scan) and hits beyond limit left out before the
+// inside test.
+__device__ __forceinline__ bool quad_intersect_scan(const Ray& r, f3 corner, f3 e1, f3 e2, f3 n, float4 g, float limit, float& t) {
+    float denom = dot(r.d, n);
+    if (fabsf(denom) < 1e-8f) return false;
+    t = dot(corner - r.o, n) / denom;
+    if (!(t > 0.0f && t < limit)) return false;
+    f3 local = r.o + r.d * t - corner;
+    float d1 = dot(local, e1), d2 = dot(local, e2);
+    float u = (d1 * g.y - d2 * g.z) / g.w;
+    float v = (d2 * g.x - d1 * g.z) / g.w;
     return u >= 0.0f && u <= 1.0f && v >= 0.0f && v <= 1.0f;
 }
 // Box: slab method with inside-test root selection (box.glsl).

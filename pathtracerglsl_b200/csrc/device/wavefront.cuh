@@ -70,7 +70,6 @@ struct PathPool {
     unsigned int* cnt; // [0],[1] queue counts, [2] shadow count, [3] error flags, [4] slot-2 shadow count
     unsigned long long* stats; // [0] closest queries, [1] shadow queries, [2] paths
     long long* wave;   // [0] first global path index of the wave, [1] wave size
-    int* job;          // batched renders: the job (scene x program x frame) of each path
     // adjoint replay only (NULL otherwise)
     float4* l_rem;     // radiance the path has still to gather (forward total minus what it gathered)
     float4* dl;        // adjoint radiance of the path: dLoss/dI of its pixel / spp
@@ -167,6 +166,7 @@ struct FrameParams {
     ptr_camera cam;
     int wavelengths;   // PTR_WAVELENGTHS_* (spectral programs)
     float lambda_min, lambda_max;
+    int fresh;         // 1: the film starts from zero at each pixel's first sample of this frame
 };
 
 struct ProgParams {
@@ -213,10 +213,10 @@ struct WaveJobs {
     long long base = 0;
     int single = 0;   // >= 0: every slot of the wave belongs to this job
     WaveJobs() = default;
-    __device__ __forceinline__ WaveJobs(const PathPool& pool, const BatchTables& bt) {
-        base = pool.wave[0];
+    __device__ __forceinline__ WaveJobs(const PathPool& pool, const BatchTables& bt) : WaveJobs(pool.wave[0], pool.wave[1], bt) {}
+    __device__ __forceinline__ WaveJobs(long long base_, long long n, const BatchTables& bt) : base(base_) {
         const int j = job_of(bt, base);
-        single = bt.offsets[j + 1] >= base + pool.wave[1] ? j : -1;
+        single = bt.offsets[j + 1] >= base + n ? j : -1;
     }
     __device__ __forceinline__ int of(const BatchTables& bt, int slot) const {
         return single >= 0 ? single : job_of(bt, base + slot);
@@ -267,26 +267,49 @@ __device__ __forceinline__ void for_region_runs(const DevScene& S, F&& f) {
     }
 }
 
-// The root of region i inside a run of one analytic shape, its parameters fetched as
-// aligned float4s: an uploaded region table is 256-byte aligned and its records 80 bytes,
-// so a record's bytes 16..79 are four float4s (ior, p[0..2]), (p[3..6]), (p[7..10]),
-// (p[11..14]).  Same operands as analytic_root_shape, fewer load instructions.
+// The root of region i of one analytic shape below limit, its parameters fetched as aligned
+// float4s: an uploaded region table is 256-byte aligned and its records 80 bytes, so a
+// record's bytes 16..79 are four float4s (ior, p[0..2]), (p[3..6]), (p[7..10]), (p[11..14]).
+// Same operands as analytic_root_shape, fewer load instructions.
 template <int SH>
-__device__ __forceinline__ bool run_root(const DevScene& S, int i, const Ray& r, float& t) {
+__device__ __forceinline__ bool run_root(const DevScene& S, int i, const Ray& r, float limit, float& t) {
     const float4* g4 = reinterpret_cast<const float4*>(S.regions + i);
     if constexpr (SH == PTR_SHAPE_SPHERE) {
         const float4 a = __ldg(g4 + 1), b = __ldg(g4 + 2);
-        return sphere_intersect(r, f3(a.y, a.z, a.w), b.x, t);
-    } else if constexpr (SH == PTR_SHAPE_QUAD) {
-        const float4 a = __ldg(g4 + 1), b = __ldg(g4 + 2), c = __ldg(g4 + 3), d = __ldg(g4 + 4);
-        return quad_intersect(r, f3(a.y, a.z, a.w), f3(b.x, b.y, b.z), f3(b.w, c.x, c.y), f3(c.z, c.w, d.x), t);
+        return sphere_intersect(r, f3(a.y, a.z, a.w), b.x, t) && t < limit;
     } else {
-        return analytic_root(S.regions[i], r, t);
+        static_assert(SH == PTR_SHAPE_QUAD, "a run of spheres or quads");
+        const float4 a = __ldg(g4 + 1), b = __ldg(g4 + 2), c = __ldg(g4 + 3), d = __ldg(g4 + 4);
+        return quad_intersect_scan(r, f3(a.y, a.z, a.w), f3(b.x, b.y, b.z), f3(b.w, c.x, c.y), f3(c.z, c.w, d.x),
+                                   __ldg(S.region_scan + i), limit, t);
     }
 }
 #ifndef __CUDACC_RTC__   // (NVRTC has no offsetof; the library build checks the layout)
 static_assert(sizeof(ptr_region) == 80 && __builtin_offsetof(ptr_region, p) == 20, "run_root's float4 view of a region record");
 #endif
+
+// Calls hit(i) for the spheres [a, b) that may meet the ray, in ascending order, until it
+// returns true.  A run is scanned 32 spheres at a time in two passes: the cheap condition
+// marks the candidates of every lane (all lanes busy), then each lane runs the exact test of
+// its own few.  In one pass a warp runs the root's square root and division at almost every
+// sphere, for the one or two lanes that need it.
+template <class F>
+__device__ __forceinline__ bool for_sphere_candidates(const DevScene& S, const Ray& r, int a, int b, F&& hit) {
+    const RayScan scan(r);
+    for (int base = a; base < b; base += 32) {
+        const int cnt = min(32, b - base);
+        unsigned mask = 0u;
+#pragma unroll 4
+        for (int k = 0; k < cnt; ++k)
+            if (scan.sphere(r, __ldg(S.region_scan + base + k))) mask |= 1u << k;
+        while (mask) {
+            const int k = __ffs(mask) - 1;
+            mask &= mask - 1u;
+            if (hit(base + k)) return true;
+        }
+    }
+    return false;
+}
 
 __device__ __forceinline__ HitRec scene_closest(const DevScene& S, const Ray& r, Work* w = nullptr) {
     HitRec h;
@@ -295,18 +318,19 @@ __device__ __forceinline__ HitRec scene_closest(const DevScene& S, const Ray& r,
     h.region = -1;
     h.element = 0;
     h.prim = -1;
+    auto take = [&](int i, float t) {
+        h.t = t;
+        h.region = i;
+        h.element = 0;
+        h.prim = -1;
+    };
     auto arm = [&](int i, const ptr_region& g, int shape) {
-        if (shape >= PTR_SHAPE_MESH) {
+        if (has_accel() && shape >= PTR_SHAPE_MESH) {
             accel_closest(S, g, i, r, h, w);
             return;
         }
         float t;
-        if (analytic_root_shape(shape, g, r, t) && t < h.t) {
-            h.t = t;
-            h.region = i;
-            h.element = 0;
-            h.prim = -1;
-        }
+        if (analytic_root_shape(shape, g, r, t) && t < h.t) take(i, t);
     };
 #if PTR_SPEC_NREGIONS > 0
     constexpr bool tabled = false;
@@ -315,32 +339,29 @@ __device__ __forceinline__ HitRec scene_closest(const DevScene& S, const Ray& r,
         const int sh = spec_shape(k);   // folds to a constant in each unrolled arm
         float t;
         bool hit = false;
-        if (sh == PTR_SHAPE_SPHERE) hit = run_root<PTR_SHAPE_SPHERE>(S, k, r, t);
-        else if (sh == PTR_SHAPE_QUAD) hit = run_root<PTR_SHAPE_QUAD>(S, k, r, t);
+        if (sh == PTR_SHAPE_SPHERE) hit = run_root<PTR_SHAPE_SPHERE>(S, k, r, h.t, t);
+        else if (sh == PTR_SHAPE_QUAD) hit = run_root<PTR_SHAPE_QUAD>(S, k, r, h.t, t);
         else arm(k, S.regions[k], sh);
-        if (hit && t < h.t) {
-            h.t = t;
-            h.region = k;
-            h.element = 0;
-            h.prim = -1;
-        }
+        if (hit) take(k, t);
     }
 #else
     const bool tabled = S.region_bvh != nullptr;
     if (!tabled && S.region_runs) {
         for_region_runs(S, [&](auto sc, int a, int b) {
             constexpr int SH = decltype(sc)::value;
-            for (int i = a; i < b; ++i) {
-                if constexpr (SH >= 0) {
-                    float t;
-                    if (run_root<SH>(S, i, r, t) && t < h.t) {
-                        h.t = t;
-                        h.region = i;
-                        h.element = 0;
-                        h.prim = -1;
+            float t;
+            if constexpr (SH == PTR_SHAPE_SPHERE) {
+                for_sphere_candidates(S, r, a, b, [&](int i) {
+                    if (run_root<SH>(S, i, r, h.t, t)) take(i, t);
+                    return false;
+                });
+            } else {
+                for (int i = a; i < b; ++i) {
+                    if constexpr (SH == PTR_SHAPE_QUAD) {
+                        if (run_root<SH>(S, i, r, h.t, t)) take(i, t);
+                    } else {
+                        arm(i, S.regions[i], S.regions[i].shape);
                     }
-                } else {
-                    arm(i, S.regions[i], S.regions[i].shape);
                 }
             }
         });
@@ -362,10 +383,7 @@ __device__ __forceinline__ HitRec scene_closest(const DevScene& S, const Ray& r,
                 // unrolled arms) keeps the hit
                 if (analytic_root(S.regions[i], r, t) && (t < tb || (t == tb && h.region > i))) {
                     tb = t;
-                    h.t = t;
-                    h.region = i;
-                    h.element = 0;
-                    h.prim = -1;
+                    take(i, t);
                 }
             }
             return false;
@@ -376,7 +394,7 @@ __device__ __forceinline__ HitRec scene_closest(const DevScene& S, const Ray& r,
 
 __device__ __forceinline__ bool scene_any(const DevScene& S, const Ray& r, float max_dist, Work* w = nullptr) {
     auto arm = [&](const ptr_region& g, int shape) -> bool {
-        if (shape >= PTR_SHAPE_MESH) return accel_any(S, g, r, max_dist, w);
+        if (has_accel() && shape >= PTR_SHAPE_MESH) return accel_any(S, g, r, max_dist, w);
         float t;
         return analytic_root_shape(shape, g, r, t) && t < max_dist;
     };
@@ -387,9 +405,9 @@ __device__ __forceinline__ bool scene_any(const DevScene& S, const Ray& r, float
         const int sh = spec_shape(k);   // folds to a constant in each unrolled arm
         float t;
         if (sh == PTR_SHAPE_SPHERE) {
-            if (run_root<PTR_SHAPE_SPHERE>(S, k, r, t) && t < max_dist) return true;
+            if (run_root<PTR_SHAPE_SPHERE>(S, k, r, max_dist, t)) return true;
         } else if (sh == PTR_SHAPE_QUAD) {
-            if (run_root<PTR_SHAPE_QUAD>(S, k, r, t) && t < max_dist) return true;
+            if (run_root<PTR_SHAPE_QUAD>(S, k, r, max_dist, t)) return true;
         } else if (arm(S.regions[k], sh)) {
             return true;
         }
@@ -403,9 +421,9 @@ __device__ __forceinline__ bool scene_any(const DevScene& S, const Ray& r, float
             const int a = run.y, b = run.y + run.z;
             float t;
             if (has_shape(PTR_SHAPE_SPHERE) && run.x == PTR_SHAPE_SPHERE) {
-                for (int i = a; i < b && !hit; ++i) hit = run_root<PTR_SHAPE_SPHERE>(S, i, r, t) && t < max_dist;
+                hit = for_sphere_candidates(S, r, a, b, [&](int i) { return run_root<PTR_SHAPE_SPHERE>(S, i, r, max_dist, t); });
             } else if (has_shape(PTR_SHAPE_QUAD) && run.x == PTR_SHAPE_QUAD) {
-                for (int i = a; i < b && !hit; ++i) hit = run_root<PTR_SHAPE_QUAD>(S, i, r, t) && t < max_dist;
+                for (int i = a; i < b && !hit; ++i) hit = run_root<PTR_SHAPE_QUAD>(S, i, r, max_dist, t);
             } else {
                 for (int i = a; i < b && !hit; ++i) hit = arm(S.regions[i], S.regions[i].shape);
             }
@@ -437,7 +455,7 @@ __device__ __forceinline__ int scene_region_at(const DevScene& S, f3 p) {
     int region = -1;
     float best = -1.0e20f;
     auto arm = [&](int i, const ptr_region& g, int shape) {
-        float d = shape == PTR_SHAPE_INSTANCES ? accel_region_sdf(S, g, p) : analytic_sdf_shape(shape, g, p);
+        float d = has_shape(PTR_SHAPE_INSTANCES) && shape == PTR_SHAPE_INSTANCES ? accel_region_sdf(S, g, p) : analytic_sdf_shape(shape, g, p);
         if (d < 0.0f && (d > best || (d == best && i < region))) { best = d; region = i; }
     };
 #if PTR_SPEC_NREGIONS > 0
@@ -450,7 +468,12 @@ __device__ __forceinline__ int scene_region_at(const DevScene& S, f3 p) {
         for_region_runs(S, [&](auto sc, int a, int b) {
             constexpr int SH = decltype(sc)::value;
             for (int i = a; i < b; ++i) {
-                if constexpr (SH == PTR_SHAPE_SPHERE) {   // the sphere's centre and radius as two float4 loads
+                if constexpr (SH == PTR_SHAPE_SPHERE) {
+                    // inside only if |p - c|^2 is below the widened radius^2: the exact distance
+                    // (a square root) is taken for the few that pass
+                    const float4 scan = __ldg(S.region_scan + i);
+                    const float x = p.x - scan.x, y = p.y - scan.y, z = p.z - scan.z;
+                    if (!(__fmaf_rn(z, z, __fmaf_rn(y, y, x * x)) < scan.w)) continue;
                     const float4* g4 = reinterpret_cast<const float4*>(S.regions + i);
                     const float4 c = __ldg(g4 + 1), rr = __ldg(g4 + 2);
                     const float d = length(p - f3(c.y, c.z, c.w)) - rr.x;
@@ -495,41 +518,49 @@ __device__ __forceinline__ int scene_region_at(const DevScene& S, f3 p) {
 
 // Complete the hit record: point, uncertainty, frame, and the region classification of
 // scene_intersect (intersection.ts:1665-1713).
-__device__ __forceinline__ void fill_hit(const DevScene& S, const Ray& r, const HitRec& hr, Hit& h) {
+// need_from / need_to: whether the caller reads region_from / region_to; a side nobody reads is
+// not classified (its point scan over every region is the costliest part) and holds -1 or the
+// hit region.
+__device__ __forceinline__ void fill_hit(const DevScene& S, const Ray& r, const HitRec& hr, Hit& h, bool need_from, bool need_to) {
     h.t = hr.t;
     h.p = r.o + r.d * hr.t;
     h.region_owner = hr.region;
     h.element = hr.element;
     h.alpha = -1.0f;
     const ptr_region& g = S.regions[hr.region];
-    if (g.shape == PTR_SHAPE_MESH || (g.shape == PTR_SHAPE_INSTANCES && S.batches[g.ref].proto_shape == PTR_SHAPE_MESH)) {
+    f3 n;
+    bool mesh = false;
+    if (kHasMesh && (g.shape == PTR_SHAPE_MESH || (g.shape == PTR_SHAPE_INSTANCES && S.batches[g.ref].proto_shape == PTR_SHAPE_MESH))) {
         // mesh hits: frame from the (normalised) shading normal, ng the triangle's plane normal
-        f3 ngv;
-        f3 n = accel_hit_normal(S, g, hr, r, h, ngv);
-        h.frame = ambient_frame(n);
-        h.ng = ngv;
+        n = accel_hit_normal(S, g, hr, r, h, h.ng);
+        mesh = true;
+    } else if (has_shape(PTR_SHAPE_INSTANCES) && g.shape == PTR_SHAPE_INSTANCES) {
+        f3 unused;
+        n = accel_hit_normal(S, g, hr, r, h, unused);
     } else {
-        f3 n;
-        if (g.shape == PTR_SHAPE_INSTANCES) {
-            f3 unused;
-            n = accel_hit_normal(S, g, hr, r, h, unused);
-        } else {
-            n = analytic_normal(g, h.p);
-            h.eps = fp_uncertainty(h.p);
-        }
-        h.frame = ambient_frame(n);
-        h.ng = h.frame.n;   // a primitive's normal is its true surface normal
+        n = analytic_normal(g, h.p);
+        h.eps = fp_uncertainty(h.p);
     }
-    int outside = scene_region_at(S, h.p + h.ng * kEpsInterface);
-    if (dot(r.d, h.ng) < 0.0f) {
-        h.region_from = outside;
-        h.region_to = hr.region;
-    } else {
-        h.region_from = g.thin ? scene_region_at(S, h.p + h.ng * (-kEpsInterface)) : hr.region;
-        h.region_to = outside;
-        h.frame = ambient_frame(-h.frame.n);
+    n = normalize(n);
+    if (!mesh) h.ng = n;   // a primitive's normal is its true surface normal
+    // the classification probes a caller needs: the outer side, and for a thin owner met from
+    // behind its inner side too (one scan's code for both)
+    const bool front = dot(r.d, h.ng) < 0.0f;
+    int inside = hr.region, outside = -1;
+    const int first = (front ? need_from : need_to) ? 0 : 1, last = !front && g.thin && need_from ? 2 : 1;
+#pragma unroll 1
+    for (int k = first; k < last; ++k) {
+        const int at = scene_region_at(S, h.p + h.ng * (k == 0 ? kEpsInterface : -kEpsInterface));
+        if (k == 0) outside = at; else inside = at;
+    }
+    h.region_from = front ? outside : inside;
+    h.region_to = front ? hr.region : outside;
+    if (!front) {
+        n = -n;
         h.ng = -h.ng;
+        n = normalize(n);
     }
+    h.frame = unit_frame(n);
 }
 
 __device__ __forceinline__ int material_of(const DevScene& S, int region) {
@@ -554,24 +585,30 @@ __device__ __forceinline__ Col medium_transmittance(const DevScene& S, const Pro
 // wavelengths_sample (color/spectral/spectral.glsl:1-10): one number, four cyclic
 // quarter-interval offsets in CDF space, each lane with its own marginal density; the
 // visible density is the normalised sech^2 (visible.glsl:3-13), or uniform (uniform.glsl).
-__device__ __forceinline__ void wavelengths_sample(const FrameParams& F, float u, float4& lam, float4& pdf) {
-    float l[4], p[4];
+__device__ __forceinline__ float wavelength_pdf(const FrameParams& F, float lambda) {
+    if (F.wavelengths == PTR_WAVELENGTHS_UNIFORM) return 1.0f / (F.lambda_max - F.lambda_min);
+    float a = m_tanh(0.0072f * (F.lambda_min - 538.0f));
+    float b = m_tanh(0.0072f * (F.lambda_max - 538.0f));
+    float c = m_cosh(0.0072f * (lambda - 538.0f));
+    return 0.0072f / ((b - a) * c * c);
+}
+__device__ __forceinline__ float4 wavelength_pdfs(const FrameParams& F, float4 l) {
+    return make_float4(wavelength_pdf(F, l.x), wavelength_pdf(F, l.y), wavelength_pdf(F, l.z), wavelength_pdf(F, l.w));
+}
+__device__ __forceinline__ float4 wavelengths_sample(const FrameParams& F, float u) {
+    float l[4];
     for (int k = 0; k < 4; ++k) {
         float v = u + 0.25f * (float)k;
         v = v - floorf(v);
         if (F.wavelengths == PTR_WAVELENGTHS_UNIFORM) {
             l[k] = F.lambda_min + (F.lambda_max - F.lambda_min) * v;
-            p[k] = 1.0f / (F.lambda_max - F.lambda_min);
         } else {
             float a = m_tanh(0.0072f * (F.lambda_min - 538.0f));
             float b = m_tanh(0.0072f * (F.lambda_max - 538.0f));
             l[k] = 538.0f + m_atanh(a * (1.0f - v) + b * v) / 0.0072f;
-            float c = m_cosh(0.0072f * (l[k] - 538.0f));
-            p[k] = 0.0072f / ((b - a) * c * c);
         }
     }
-    lam = make_float4(l[0], l[1], l[2], l[3]);
-    pdf = make_float4(p[0], p[1], p[2], p[3]);
+    return make_float4(l[0], l[1], l[2], l[3]);
 }
 
 // color_to_pixel (spectral.glsl:27-33) with the CIE 1931 sensor (sensor/cie1931/cie1931.glsl:3-5):
@@ -580,7 +617,7 @@ __device__ __forceinline__ f3 color_to_pixel(const DevScene& S, float4 L, float4
     const float Ls[4] = {L.x, L.y, L.z, L.w}, ls[4] = {lam.x, lam.y, lam.z, lam.w}, ps[4] = {pdf.x, pdf.y, pdf.z, pdf.w};
     f3 pixel(0.0f);
     for (int k = 0; k < 4; ++k) {
-        float4 c = spectral_curves(S, ls[k]);
+        float4 c = spectral_curves(S.spec_curves, ls[k]);
         f3 rgb(S.spec_m[0] * c.x + S.spec_m[1] * c.y + S.spec_m[2] * c.z,
                S.spec_m[3] * c.x + S.spec_m[4] * c.y + S.spec_m[5] * c.z,
                S.spec_m[6] * c.x + S.spec_m[7] * c.y + S.spec_m[8] * c.z);
@@ -591,7 +628,52 @@ __device__ __forceinline__ f3 color_to_pixel(const DevScene& S, float4 L, float4
 
 // ---- kernels ---------------------------------------------------------------------------
 
-// Camera rays for one wave (accumulation.ts:14-26 cameraSample; pinhole.glsl:4-18).
+// Pixel and sample of a frame's path index (samples are the outer dimension).
+__device__ __forceinline__ void split_path(long long g, unsigned npix, int& pix, int& sample) {
+    if ((unsigned long long)g >> 32) {
+        pix = (int)(g % npix);
+        sample = (int)(g / npix);
+    } else {   // the 32-bit division is several times cheaper
+        const unsigned k = (unsigned)g, q = k / npix;
+        pix = (int)(k - q * npix);
+        sample = (int)q;
+    }
+}
+// The camera ray of one sample of pixel pix and its random stream (accumulation.ts:14-26
+// cameraSample; pinhole.glsl:4-18); spectral programs also draw their wavelengths.
+template <bool SPECTRAL>
+__device__ __forceinline__ void camera_path(const FrameParams& F, int pix, int sample, Rng& rng, Ray& r, float4& lambda) {
+    int x = (int)((unsigned)pix % (unsigned)F.width), y = (int)((unsigned)pix / (unsigned)F.width);
+    rng.init((uint32_t)(x + F.px_off), (uint32_t)(y + F.py_off), (uint32_t)(F.first_sample + sample), F.salt);
+    float pxf = (float)x + 0.5f + (float)F.px_off;
+    float pyf = (float)y + 0.5f + (float)F.py_off;
+    float a0 = rng.next();
+    float a1 = rng.next();
+    float fx = pxf + (a0 - 0.5f), fy = pyf + (a1 - 0.5f);
+    if (SPECTRAL) lambda = wavelengths_sample(F, rng.next());   // between the film point and the camera ray
+    rng.next();   // the lens draw (a pinhole has no aperture)
+    rng.next();
+    float ndcx = (2.0f * fx / (float)F.img_w) - 1.0f;
+    float ndcy = (2.0f * fy / (float)F.img_h) - 1.0f;
+    ndcx *= F.cam.aspect;
+    r.d = normalize(ld3(F.cam.forward) + ndcx * F.cam.tan_fov * ld3(F.cam.right) +
+                    ndcy * F.cam.tan_fov * ld3(F.cam.up));
+    r.o = ld3(F.cam.position);
+}
+// path_state_init of path slot i.
+__device__ __forceinline__ void init_slot(const DevScene& S, const PathPool& pool, long long i, const Rng& rng, const Ray& r) {
+    int medium = S.has_media ? scene_region_at(S, r.o) : -1;
+    pool.ray_o[i] = f4(r.o, 0.0f);
+    pool.ray_d[i] = f4(r.d, 1.0f);
+    pool.thr[i] = make_float4(1.f, 1.f, 1.f, 1.f);   // the spectral model's fourth lane included
+    pool.rad[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    pool.prev_q[i] = f4(r.o, 0.0f);
+    pool.st[i] = make_int4(0, medium, 0, 1);
+    pool.rng[i] = make_uint2(rng.base, rng.dim);
+    pool.q[0][i] = (int)i;
+}
+
+// Camera rays for one wave.
 template <bool ADJ = false, bool SPECTRAL = false>
 __global__ void k_generate(DevScene S, PathPool pool, const FrameParams* fp, AdjParams adj = AdjParams{}) {
     const FrameParams F = *fp;
@@ -604,48 +686,25 @@ __global__ void k_generate(DevScene S, PathPool pool, const FrameParams* fp, Adj
         pool.stats[2] += (unsigned long long)n;
         if (pool.fetch) pool.fetch[0] = 0u;
     }
-    const long long npix = (long long)F.width * F.height;
+    const unsigned npix = (unsigned)F.width * (unsigned)F.height;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        long long g = base + i;
-        int pix = (int)(g % npix);
-        int sample = (int)(g / npix);
-        int x = pix % F.width, y = pix / F.width;
+        int pix, sample;
+        split_path(base + i, npix, pix, sample);
         Rng rng;
-        rng.init((uint32_t)(x + F.px_off), (uint32_t)(y + F.py_off), (uint32_t)(F.first_sample + sample), F.salt);
-        float pxf = (float)x + 0.5f + (float)F.px_off;
-        float pyf = (float)y + 0.5f + (float)F.py_off;
-        float a0 = rng.next();
-        float a1 = rng.next();
-        float fx = pxf + (a0 - 0.5f), fy = pyf + (a1 - 0.5f);
-        if (SPECTRAL) {   // wavelengths_sample, between the film point and the camera ray
-            float4 lam, pdf;
-            wavelengths_sample(F, rng.next(), lam, pdf);
-            pool.wl[i] = lam;
-            pool.wl_pdf[i] = pdf;
+        Ray r;
+        float4 lambda;
+        camera_path<SPECTRAL>(F, pix, sample, rng, r, lambda);
+        if (SPECTRAL) {
+            pool.wl[i] = lambda;
+            pool.wl_pdf[i] = wavelength_pdfs(F, lambda);
         }
-        rng.next();   // the lens draw (a pinhole has no aperture)
-        rng.next();
-        float ndcx = (2.0f * fx / (float)F.img_w) - 1.0f;
-        float ndcy = (2.0f * fy / (float)F.img_h) - 1.0f;
-        ndcx *= F.cam.aspect;
-        f3 dir = normalize(ld3(F.cam.forward) + ndcx * F.cam.tan_fov * ld3(F.cam.right) +
-                           ndcy * F.cam.tan_fov * ld3(F.cam.up));
-        f3 o = ld3(F.cam.position);
-        int medium = S.has_media ? scene_region_at(S, o) : -1;
         if (ADJ) {   // replay: the forward pass left this path's total radiance in rad
             pool.l_rem[i] = pool.rad[i];
             const float* g = adj.dl_image + 3 * (size_t)pix;
             pool.dl[i] = make_float4(g[0] * adj.inv_spp, g[1] * adj.inv_spp, g[2] * adj.inv_spp, 0.f);
         }
-        pool.ray_o[i] = f4(o, 0.0f);
-        pool.ray_d[i] = f4(dir, 1.0f);
-        pool.thr[i] = make_float4(1.f, 1.f, 1.f, 1.f);   // the spectral model's fourth lane included
-        pool.rad[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-        pool.prev_q[i] = f4(o, 0.0f);
-        pool.st[i] = make_int4(0, medium, 0, 1);
-        pool.rng[i] = make_uint2(rng.base, rng.dim);
+        init_slot(S, pool, i, rng, r);
         if (pool.aov) { pool.aov[2 * i] = make_float4(0.f, 0.f, 0.f, 0.f); pool.aov[2 * i + 1] = make_float4(0.f, 0.f, 0.f, 0.f); }
-        pool.q[0][i] = (int)i;
     }
 }
 
@@ -1001,6 +1060,340 @@ __device__ __forceinline__ const int* closest_queue(const PathPool& pool, int in
     return pool.ray_in ? sorted_queue(pool.q_ray, pool.q[in], pool.cnt[in]) : pool.q[in];
 }
 
+// What one walk iteration carries of a path: k_shade loads it from the pool and stores it
+// back, k_walk keeps it in registers for the whole walk.
+template <class Col>
+struct WalkState {
+    Ray r;
+    float prev_bsdf_pdf, eta_scale;
+    Col thr, rad;
+    f3 prev_qp;              // the stored light-query point
+    Wl wl;                   // spectral only
+    int bounce, cur_med, nulls;
+    bool prev_delta;
+    Rng rng;
+    Col lrem;                // adjoint replay only: the radiance still to come
+};
+
+// One walk iteration of a path whose segment's closest hit is hr: the medium segment, null
+// pass-through, emitter scoring, NEE sampling (its queries go to the sink), the
+// continuation lobe and roulette.  Returns true while the path goes on.
+// Sink: segment_query / vertex_query take the iteration's shadow queries (slots 1 and 0),
+// seed() the sampler dimension of a heterogeneous medium's query, put_prev_n / get_prev_n
+// the stored query normal of light-tree programs, aov() the path's two first-hit samples
+// (null when the program has none).
+// ADJ: also scatters the gradient terms through ga and leaves the slot-0 query's vertex
+// material and lobe derivative in sh_mat / sg.
+// live: this lane has a path; phase() is called by every lane between the parts of the iteration.
+template <class Col, int DIRECT, bool MEDIA, bool ADJ, class Sink, class Phase>
+__device__ __forceinline__ bool walk_iteration(const DevScene& S, const ProgParams& P, WalkState<Col>& ws, const HitRec& hr,
+                                               Sink& sink, const GradAcc& ga, int& sh_mat, NeeGrad& sg, bool live, Phase phase) {
+    constexpr bool SPECTRAL = sizeof(Col) == sizeof(s4);
+    using CM = Colors<Col>;
+    const bool nee = DIRECT != PTR_DIRECT_NONE;
+    const bool mis = DIRECT == PTR_DIRECT_MIS;
+    const bool tree = PTR_SPEC_TREE && P.light_tree;
+    Ray& r = ws.r;
+    float& prev_bsdf_pdf = ws.prev_bsdf_pdf;
+    float& eta_scale = ws.eta_scale;
+    Col& thr = ws.thr;
+    Col& rad = ws.rad;
+    f3& prev_qp = ws.prev_qp;
+    const Wl& wl = ws.wl;
+    int &bounce = ws.bounce, &cur_med = ws.cur_med, &nulls = ws.nulls;
+    bool& prev_delta = ws.prev_delta;
+    Rng& rng = ws.rng;
+    Col& lrem = ws.lrem;
+    bool alive = false, shadow = false;
+    const bool boundary = hr.region >= 0;
+    const int N = P.max_bounces;
+
+    // -- the volumetric call site: one segment (features/materials.ts:675-746).  event: the
+    // segment scattered at p_evt in the medium of material mat
+    bool event = false, het = false;
+    int mat = 0;
+    f3 p_evt;
+    if (MEDIA && live) {
+        const int med_mat = material_of(S, cur_med);
+        if (mat_has_medium(S, med_mat)) {
+            const ptr_material& mm = S.materials[med_mat];
+            // the per-segment equiangular site precedes the transmittance sample
+            // (pt.ts:322-328) and rides the second shadow slot
+            if (P.equiangular && bounce < N) {
+                EquiangularQuery<Col> eq;
+                if (equiangular_site<Col>(S, med_mat, r, boundary ? hr.t : kMaxDist, rng, thr, wl, eq))
+                    sink.segment_query(eq.p_evt, eq.wi, P.max_null - nulls, eq.light_pos, eq.contrib, eq.denom);
+            }
+            float x0 = rng.next();
+            float x1 = rng.next();
+            float t_max = boundary ? hr.t : kMaxDist;
+            // heterogeneous media take the tracking arms (delta_tracking.glsl)
+            het = !SPECTRAL && PTR_SPEC_HET && S.has_het && mat_is_het(mm);
+            if (!scatter_live(S, P, med_mat) && !het) {
+                thr = thr * vexp(-CM::sigma_a(S, med_mat, wl) * t_max);
+                if constexpr (ADJ) {   // w = exp(-(1-a) st t)
+                    GreyMedium gm = grey_medium(mm);
+                    ga.scl(med_mat, PTR_GRAD_SIGMA_T, lrem, -(1.0f - gm.a) * t_max);
+                    ga.scl(med_mat, PTR_GRAD_MEDIUM_ALBEDO, lrem, gm.st * t_max);
+                }
+            } else {
+                MediumSample<Col> ms;
+                bool tracked = false;
+                if constexpr (!SPECTRAL && PTR_SPEC_HET) {
+                    if (het && scatter_live(S, P, med_mat)) {
+                        ms = medium_sample_delta(S, mm, r, t_max, x0, x1, rng);
+                        tracked = true;
+                    } else if (het) {   // absorbing only: the ratio-tracked pass-through
+                        ms.scattered = false;
+                        ms.weight = medium_ratio_track(S, mm, r, t_max, rng, false);
+                        tracked = true;
+                    }
+                }
+                if (!tracked)
+                    ms = medium_sample_analytic<Col>(CM::sigma_a(S, med_mat, wl), CM::sigma_s(S, med_mat, wl), r, t_max, x0, x1);
+                thr = thr * ms.weight;
+                if constexpr (ADJ) {   // scattered at t: w = a st exp(-st t)/pdf; passed: exp(-st t_max)/P
+                    GreyMedium gm = grey_medium(mm);
+                    if (ms.scattered) {
+                        float t_evt = dot(ms.exit_p - r.o, r.d);
+                        ga.scl(med_mat, PTR_GRAD_SIGMA_T, lrem, 1.0f / gm.st - t_evt);
+                        ga.scl(med_mat, PTR_GRAD_MEDIUM_ALBEDO, lrem, 1.0f / gm.a);
+                    } else {
+                        ga.scl(med_mat, PTR_GRAD_SIGMA_T, lrem, -t_max);
+                    }
+                }
+                event = ms.scattered;
+                p_evt = ms.exit_p;
+                mat = med_mat;
+            }
+        }
+    }
+
+    // -- the segment's end: a miss, a null interface, or a surface vertex.  vertex: the walk
+    // scatters here (medium event or surface) and the bounce budget allows it
+    bool vertex = event && bounce != N;
+    Hit hit;
+    if (MEDIA) phase();
+    if (!live) {
+    } else if (!event && !boundary) {   // kernel_score_miss (kernel.glsl:11-14)
+        float w = 1.0f;
+        if (nee && S.env_samplable && !prev_delta) {
+            if (!mis) w = 0.0f;
+            else {
+                float pe = S.env_select_live ? S.env_select_prob : 1.0f;
+                w = power_heuristic(prev_bsdf_pdf, pe * env_pdf(S, r.d));
+            }
+        }
+        Col e = thr * w * env_radiance<Col>(S, r.d, wl);
+        rad = rad + e;
+        if constexpr (ADJ) lrem = lrem - e;
+    } else if (!event) {
+        mat = material_of(S, hr.region);
+        // the incident side: the current medium, or the IOR of a model that refracts
+        fill_hit(S, r, hr, hit, MEDIA || material_in<MatUsesIor>(S.materials[mat].model), true);
+        if (MEDIA && hit.region_from != cur_med) cur_med = hit.region_from;
+        const ptr_material& m = S.materials[mat];
+        if (MEDIA && m.model == PTR_MAT_NONE) {   // null pass-through (pt.ts:404-417)
+            cur_med = hit.region_to;
+            r = ray_spawn(hit, r.d);
+            nulls += 1;
+            alive = nulls <= P.max_null;
+        } else {
+            const f3 wo = -r.d;
+            // the AOV capture (pt.ts:422-433): the first non-null surface before
+            // any event, weighted by the arrival throughput
+            if constexpr (!SPECTRAL) {
+                if (bounce == 0 && sink.aov()) {
+                    f3 fact = ld3(m.transmittance);
+                    auto aov = [&](auto M) { fact = decltype(M)::aov(m); };
+                    dispatch_material<MatPresent>(m.model, aov);
+                    fact = vmin(vmax(fact, f3(0.0f)), f3(1.0f));
+                    f3 nf = dot(hit.frame.n, wo) < 0.0f ? -hit.frame.n : hit.frame.n;
+                    sink.aov()[0] = f4(fact * thr, 0.0f);
+                    sink.aov()[1] = f4(nf * spectrum_average(thr), 0.0f);
+                }
+            }
+            // kernel_score_emitter_hit (kernel.glsl:16-25; combiner.ts:27-46)
+            int mat_emit = material_of(S, hit.region_to);
+            if (mat_emit >= 0 && (S.materials[mat_emit].flags & PTR_MATF_EMISSIVE)) {
+                float w = 1.0f;
+                if (nee) {
+                    int lid = hit.region_to >= 0 ? emitter_light(S, hit) : -1;
+                    if (lid >= 0 && !prev_delta) {
+                        if (!mis) w = 0.0f;
+                        else {
+                            // the stored selection context (its normal and sidedness
+                            // only under light-tree selection)
+                            LightQuery pq{prev_qp, f3(0.0f), false};
+                            if (tree) {
+                                float4 pqn = sink.get_prev_n();
+                                pq.n = xyz(pqn);
+                                pq.two_sided = pqn.w != 0.0f;
+                            }
+                            w = power_heuristic(prev_bsdf_pdf, lighting_pdf(S, pq, r.d, lid, hit.p, hit.ng, tree));
+                        }
+                    }
+                }
+                Col e = thr * w * CM::emission(S, mat_emit, wl);
+                rad = rad + e;
+                if constexpr (ADJ) lrem = lrem - e;
+            }
+            vertex = bounce != N;
+        }
+    }
+    phase();
+
+    // -- the vertex: next-event estimation, then the continuation.  Medium events and
+    // surfaces meet one light-sampling site (one copy of its code, their lanes together).
+    const ptr_material& m = S.materials[mat];
+    const f3 wo = -r.d;
+    const float alpha = !event && hit.alpha >= 0.0f ? hit.alpha : m.alpha;
+    // light queries with sphere support (a transmissive non-delta lobe)
+    const bool rough = vertex && !event && material_in<MatSphereQuery>(m.model);
+    const bool surface = vertex && !event;
+    const float n_from = surface ? ior_of(S, hit.region_from) : 1.0f, n_to = surface ? ior_of(S, hit.region_to) : 1.0f;
+    const MatSite<Col> site{S, mat, m, hit, wl, alpha, n_from, n_to};
+    const f3 vp = event ? p_evt : hit.p;
+    if (vertex && nee && (event ? !P.equiangular : material_in<MatNonDelta>(m.model))) {
+        // light_sample_direct (light.glsl:8-28), light_sample_direct_medium (light_medium.glsl:7-18)
+        float y0 = rng.next();
+        float y1 = rng.next();
+        // no orientation at a medium event; rough glass: sphere support
+        LightQuery lq{vp, event ? f3(0.0f) : hit.frame.n, rough};
+        LightSample<Col> ls = lighting_sample<Col>(S, lq, y0, y1, rng, tree, wl);
+        if (MEDIA && PTR_SPEC_HET && S.has_het) sink.seed(rng.dim);
+        if (ls.pdf > 0.0f) {
+            const f3 light_p = vp + ls.wi * ls.distance;
+            const bool want_pdf = mis && !(ls.flags & kLightDelta);
+            Ray sr{vp, ls.wi};
+            float maxd = 0.0f, bp = 0.0f;
+            Col contrib;
+            if (event) {
+                const float ph = hg_eval(ls.wi, wo, m.phase_g);
+                contrib = thr * ls.radiance * Col(ph);
+                if (want_pdf) bp = spectrum_average(Col(ph));
+                if constexpr (ADJ) {
+                    sg.kind = kGradKindPhase;
+                    sg.dnee = f3(hg_dlog_g(ls.wi, wo, m.phase_g), 0.0f, 0.0f);
+                }
+            } else {
+                sr = ray_spawn(hit, ls.wi);
+                sr.d = normalize(light_p - sr.o);
+                Col f(0.0f);
+                auto lobe = [&](auto M) {
+                    f = decltype(M)::eval(site, ls.wi, wo);
+                    if (want_pdf) bp = decltype(M)::pdf(site, ls.wi, wo);
+                };
+                dispatch_material<MatNonDelta, true>(m.model, lobe);   // the model has a non-delta lobe here
+                const float cos_i = fabsf(dot(ls.wi, hit.frame.n));
+                maxd = length(light_p - sr.o) - kShadowBackoff;
+                contrib = thr * ls.radiance * f * cos_i;
+                if constexpr (ADJ) {
+                    auto ng = [&](auto M) { decltype(M)::nee_grad(site, ls.wi, wo, sg); };
+                    dispatch_material<MatNonDelta, true>(m.model, ng);
+                }
+            }
+            sh_mat = mat;
+            const float w = want_pdf ? power_heuristic(ls.pdf, bp) : 1.0f;
+            sink.vertex_query(sr.o, maxd, sr.d, P.max_null - nulls, light_p, w, contrib, ls.pdf);
+            shadow = true;
+        }
+    }
+    phase();
+    if (!vertex) return alive;
+    bool survive = true;
+    if (event) {
+        float z0 = rng.next();
+        float z1 = rng.next();
+        ISample<Col> ps = hg_sample<Col>(wo, m.phase_g, z0, z1);
+        thr = thr * ps.weight;
+        if constexpr (ADJ) {   // phase continuation: w = p_HG / pdf_detached
+            float dg = hg_dlog_g(ps.wi, wo, m.phase_g);
+            ga.scl(mat, PTR_GRAD_HG_G, lrem, dg);
+            if (shadow) sg.dnee.x -= dg;
+        }
+        prev_delta = false;
+        prev_bsdf_pdf = ps.pdf;
+        prev_qp = p_evt;
+        if (tree) sink.put_prev_n(make_float4(0.f, 0.f, 0.f, 0.f));   // no orientation
+        r.o = p_evt;
+        r.d = ps.wi;
+        // roulette_interior (pt.ts:230-283); nothing is owed after a
+        // tracking arm, whose lottery settled absorption already
+        if (P.rr_start >= 0 && bounce >= P.rr_start && !het) {
+            Col ss = CM::sigma_s(S, mat, wl), sa = CM::sigma_a(S, mat, wl);
+            Col surv = ss / vmax(ss + sa, Col(1e-9f));
+            float p_survive = spectrum_max(surv);
+            if (p_survive <= 0.0f) survive = false;
+            else if (rng.next() > p_survive) survive = false;
+            else thr = thr / p_survive;
+        }
+    } else {
+        // kernel_sample_continuation (kernel.glsl:27-34)
+        float uc = rng.next();
+        float u0 = rng.next();
+        float u1 = rng.next();
+        ISample<Col> bs;
+        bs.weight = Col(0.0f);   // stays black only in a build without the scene's models
+        auto cont = [&](auto M) { bs = decltype(M)::sample(site, wo, uc, u0, u1); };
+        dispatch_material<MatPresent>(m.model, cont);
+        if (spectrum_is_black(bs.weight)) return false;
+        thr = thr * bs.weight;
+        if constexpr (ADJ) {   // the continuation lobe: d log w_cont
+            auto cg = [&](auto M) { decltype(M)::cont_grad(site, bs, wo, ga, lrem, shadow, sg); };
+            dispatch_material<MatPresent>(m.model, cg);
+        }
+        prev_delta = (bs.flags & kLobeDelta) != 0u;
+        prev_bsdf_pdf = bs.pdf;
+        prev_qp = hit.p;
+        if (tree) sink.put_prev_n(f4(hit.frame.n, rough ? 1.0f : 0.0f));
+        if (bs.flags & kLobeTransmission) {
+            if (MEDIA) cur_med = hit.region_to;
+            float rr = n_to / n_from;
+            eta_scale *= rr * rr;
+        }
+        // roulette (pt.ts:204-222)
+        if (P.rr_start >= 0 && bounce >= P.rr_start) {
+            float p_survive = gmin(P.rr_max_survival, spectrum_max(thr) * eta_scale);
+            if (p_survive <= 0.0f) survive = false;
+            else if (rng.next() > p_survive) survive = false;
+            else thr = thr / p_survive;
+        }
+        if (survive) r = ray_spawn(hit, bs.wi);
+    }
+    if (survive) bounce += 1;
+    return survive;
+}
+
+// k_shade's sink: queries and stored normals go to the path's pool records at once.
+template <class Col>
+struct PoolSink {
+    const PathPool& pool;
+    const int i;
+    bool shadow = false, shadow2 = false;
+    __device__ __forceinline__ PoolSink(const PathPool& p, int slot) : pool(p), i(slot) {}
+    __device__ __forceinline__ void segment_query(f3 o, f3 d, int crossings, f3 light_p, Col contrib, float pdf) {
+        pool.sh2_o[i] = f4(o, 0.0f);
+        pool.sh2_d[i] = f4(d, __int_as_float(crossings));
+        pool.sh2_lp[i] = f4(light_p, 1.0f);
+        pool.sh2_c[i] = col_st(contrib, pdf);
+        if constexpr (sizeof(Col) == sizeof(s4)) pool.sh2_pdf[i] = pdf;
+        shadow2 = true;
+    }
+    __device__ __forceinline__ void vertex_query(f3 o, float max_dist, f3 d, int crossings, f3 light_p, float w, Col contrib, float pdf) {
+        pool.sh_o[i] = f4(o, max_dist);
+        pool.sh_d[i] = f4(d, __int_as_float(crossings));
+        pool.sh_lp[i] = f4(light_p, w);
+        pool.sh_c[i] = col_st(contrib, pdf);
+        if constexpr (sizeof(Col) == sizeof(s4)) pool.sh_pdf[i] = pdf;
+        shadow = true;
+    }
+    __device__ __forceinline__ void seed(unsigned dim) { pool.sh_seed[i] = dim; }
+    __device__ __forceinline__ void put_prev_n(float4 n) { pool.prev_n[i] = n; }
+    __device__ __forceinline__ float4 get_prev_n() const { return pool.prev_n[i]; }
+    __device__ __forceinline__ float4* aov() const { return pool.aov ? pool.aov + 2 * i : nullptr; }
+};
+
 // One walk iteration for every live path.
 #ifndef PTR_SHADE_MIN_BLOCKS
 #define PTR_SHADE_MIN_BLOCKS 3
@@ -1014,7 +1407,6 @@ __global__ void __launch_bounds__(256, PTR_SHADE_MIN_BLOCKS) k_shade(DevScene S0
                                                                      AdjParams adj = AdjParams{}) {
     constexpr bool SPECTRAL = sizeof(Col) == sizeof(s4);
     static_assert(!(ADJ && SPECTRAL), "the adjoint replay is RGB only");
-    using CM = Colors<Col>;
     extern __shared__ double s_grad[];
     if constexpr (ADJ) grad_block_init(s_grad, PTR_GRAD_SLOTS * S0.n_materials);
     const unsigned n = pool.cnt[in];
@@ -1022,8 +1414,6 @@ __global__ void __launch_bounds__(256, PTR_SHADE_MIN_BLOCKS) k_shade(DevScene S0
     // ascending, so the pool's SoA reads and writes stay coalesced
     const int* q = pool.sort_buckets > 1 ? sorted_queue(pool.q_sorted, pool.q[in], n) : pool.q[in];
     int* qout = pool.q[in ^ 1];
-    const bool nee = DIRECT != PTR_DIRECT_NONE;
-    const bool mis = DIRECT == PTR_DIRECT_MIS;
     if (blockIdx.x == 0 && threadIdx.x == 0 && pool.fetch) pool.fetch[0] = 0u;   // the next k_closest's ticket
     const WaveJobs wj = BATCH ? WaveJobs(pool, bt) : WaveJobs{};
     QueueCursor cur(n, pool.fetch ? pool.fetch + 3 : nullptr);
@@ -1038,32 +1428,30 @@ __global__ void __launch_bounds__(256, PTR_SHADE_MIN_BLOCKS) k_shade(DevScene S0
             const DevScene& S = BATCH ? bt.scenes[job] : S0;
             const ProgParams& P = BATCH ? bt.progs[job] : P0;
             float4 ro = pool.ray_o[i], rd = pool.ray_d[i];
-            Ray r;
-            r.o = xyz(ro);
-            r.d = xyz(rd);
-            float prev_bsdf_pdf = ro.w;
-            float eta_scale = rd.w;
-            Col thr = col_ld<Col>(pool.thr[i]);
-            Col rad = col_ld<Col>(pool.rad[i]);
-            f3 prev_qp = xyz(pool.prev_q[i]);
-            Wl wl;
-            const bool tree = PTR_SPEC_TREE && P.light_tree;
-            if constexpr (SPECTRAL) wl.lambda = pool.wl[i];
+            WalkState<Col> ws;
+            ws.r.o = xyz(ro);
+            ws.r.d = xyz(rd);
+            ws.prev_bsdf_pdf = ro.w;
+            ws.eta_scale = rd.w;
+            ws.thr = col_ld<Col>(pool.thr[i]);
+            ws.rad = col_ld<Col>(pool.rad[i]);
+            ws.prev_qp = xyz(pool.prev_q[i]);
+            if constexpr (SPECTRAL) ws.wl.lambda = pool.wl[i];
             int4 st = pool.st[i];
-            int bounce = st.x, cur_med = st.y, nulls = st.z;
-            bool prev_delta = st.w != 0;
+            ws.bounce = st.x;
+            ws.cur_med = st.y;
+            ws.nulls = st.z;
+            ws.prev_delta = st.w != 0;
             uint2 rs = pool.rng[i];
-            Rng rng;
-            rng.base = rs.x;
-            rng.dim = rs.y;
-            Col lrem(0.0f);
+            ws.rng.base = rs.x;
+            ws.rng.dim = rs.y;
             GradAcc ga;
             int sh_mat = 0;
             // the NEE query's lobe derivative: dlog f toward the light (per channel) and its
             // scalar part (GGX alpha beside the per-channel F0 part)
             NeeGrad sg{kGradKindNone, f3(0.0f), 0.0f};
             if constexpr (ADJ) {
-                lrem = xyz(pool.l_rem[i]);
+                ws.lrem = xyz(pool.l_rem[i]);
                 ga.s = s_grad;
                 ga.dl = xyz(pool.dl[i]);
             }
@@ -1072,311 +1460,32 @@ __global__ void __launch_bounds__(256, PTR_SHADE_MIN_BLOCKS) k_shade(DevScene S0
             HitRec hr;
             hr.t = hf.x; hr.u = hf.y; hr.v = hf.z;
             hr.region = hi.x; hr.element = hi.y; hr.prim = hi.z;
-            const bool boundary = hr.region >= 0;
-            const int N = P.max_bounces;
-            Hit hit;
-            if (boundary) fill_hit(S, r, hr, hit);
-            bool done = false, handled = false;
-
-            // -- the volumetric call site: one segment (features/materials.ts:675-746)
-            if (MEDIA) {
-                int med_mat = material_of(S, cur_med);
-                if (mat_has_medium(S, med_mat)) {
-                    const ptr_material& mm = S.materials[med_mat];
-                    // the per-segment equiangular site precedes the transmittance sample
-                    // (pt.ts:322-328) and rides the second shadow slot
-                    if (P.equiangular && bounce < N) {
-                        EquiangularQuery<Col> eq;
-                        if (equiangular_site<Col>(S, med_mat, r, boundary ? hr.t : kMaxDist, rng, thr, wl, eq)) {
-                            pool.sh2_o[i] = f4(eq.p_evt, 0.0f);
-                            pool.sh2_d[i] = f4(eq.wi, __int_as_float(P.max_null - nulls));
-                            pool.sh2_lp[i] = f4(eq.light_pos, 1.0f);
-                            pool.sh2_c[i] = col_st(eq.contrib, eq.denom);
-                            if constexpr (SPECTRAL) pool.sh2_pdf[i] = eq.denom;
-                            shadow2 = true;
-                        }
-                    }
-                    float x0 = rng.next();
-                    float x1 = rng.next();
-                    float t_max = boundary ? hr.t : kMaxDist;
-                    // heterogeneous media take the tracking arms (delta_tracking.glsl)
-                    const bool het = !SPECTRAL && S.has_het && mat_is_het(mm);
-                    if (!scatter_live(S, P, med_mat) && !het) {
-                        thr = thr * vexp(-CM::sigma_a(S, med_mat, wl) * t_max);
-                        if constexpr (ADJ) {   // w = exp(-(1-a) st t)
-                            GreyMedium gm = grey_medium(mm);
-                            ga.scl(med_mat, PTR_GRAD_SIGMA_T, lrem, -(1.0f - gm.a) * t_max);
-                            ga.scl(med_mat, PTR_GRAD_MEDIUM_ALBEDO, lrem, gm.st * t_max);
-                        }
-                    } else {
-                        MediumSample<Col> ms;
-                        if constexpr (!SPECTRAL) {
-                            if (het && scatter_live(S, P, med_mat)) {
-                                ms = medium_sample_delta(S, mm, r, t_max, x0, x1, rng);
-                            } else if (het) {   // absorbing only: the ratio-tracked pass-through
-                                ms.scattered = false;
-                                ms.weight = medium_ratio_track(S, mm, r, t_max, rng, false);
-                            } else {
-                                ms = medium_sample_analytic<Col>(CM::sigma_a(S, med_mat, wl), CM::sigma_s(S, med_mat, wl),
-                                                                 r, t_max, x0, x1);
-                            }
-                        } else {
-                            ms = medium_sample_analytic<Col>(CM::sigma_a(S, med_mat, wl), CM::sigma_s(S, med_mat, wl),
-                                                             r, t_max, x0, x1);
-                        }
-                        thr = thr * ms.weight;
-                        if constexpr (ADJ) {   // scattered at t: w = a st exp(-st t)/pdf; passed: exp(-st t_max)/P
-                            GreyMedium gm = grey_medium(mm);
-                            if (ms.scattered) {
-                                float t_evt = dot(ms.exit_p - r.o, r.d);
-                                ga.scl(med_mat, PTR_GRAD_SIGMA_T, lrem, 1.0f / gm.st - t_evt);
-                                ga.scl(med_mat, PTR_GRAD_MEDIUM_ALBEDO, lrem, 1.0f / gm.a);
-                            } else {
-                                ga.scl(med_mat, PTR_GRAD_SIGMA_T, lrem, -t_max);
-                            }
-                        }
-                        if (ms.scattered) {
-                            handled = true;
-                            if (bounce == N) {
-                                done = true;
-                            } else {
-                                f3 p_evt = ms.exit_p;
-                                f3 wo_med = -ms.exit_dir;
-                                if (nee && !P.equiangular) {   // light_sample_direct_medium (light_medium.glsl:7-18)
-                                    float y0 = rng.next();
-                                    float y1 = rng.next();
-                                    LightQuery lq{p_evt, f3(0.0f), false};   // no orientation at a medium event
-                                    LightSample<Col> ls = lighting_sample<Col>(S, lq, y0, y1, rng, tree, wl);
-                                    if (S.has_het) pool.sh_seed[i] = rng.dim;
-                                    if (ls.pdf > 0.0f) {
-                                        f3 light_p = p_evt + ls.wi * ls.distance;
-                                        float ph = hg_eval(ls.wi, wo_med, mm.phase_g);
-                                        float w = 1.0f;
-                                        if (mis && !(ls.flags & kLightDelta)) w = power_heuristic(ls.pdf, spectrum_average(Col(ph)));
-                                        pool.sh_o[i] = f4(p_evt, 0.0f);
-                                        pool.sh_d[i] = f4(ls.wi, __int_as_float(P.max_null - nulls));
-                                        pool.sh_lp[i] = f4(light_p, w);
-                                        pool.sh_c[i] = col_st(thr * ls.radiance * Col(ph), ls.pdf);
-                                        if constexpr (SPECTRAL) pool.sh_pdf[i] = ls.pdf;
-                                        shadow = true;
-                                        if constexpr (ADJ) {
-                                            sg.kind = kGradKindPhase;
-                                            sh_mat = med_mat;
-                                            sg.dnee = f3(hg_dlog_g(ls.wi, wo_med, mm.phase_g), 0.0f, 0.0f);
-                                        }
-                                    }
-                                }
-                                float z0 = rng.next();
-                                float z1 = rng.next();
-                                ISample<Col> ps = hg_sample<Col>(wo_med, mm.phase_g, z0, z1);
-                                thr = thr * ps.weight;
-                                if constexpr (ADJ) {   // phase continuation: w = p_HG / pdf_detached
-                                    float dg = hg_dlog_g(ps.wi, wo_med, mm.phase_g);
-                                    ga.scl(med_mat, PTR_GRAD_HG_G, lrem, dg);
-                                    if (shadow) sg.dnee.x -= dg;
-                                }
-                                prev_delta = false;
-                                prev_bsdf_pdf = ps.pdf;
-                                prev_qp = p_evt;
-                                if (tree) pool.prev_n[i] = make_float4(0.f, 0.f, 0.f, 0.f);   // no orientation
-                                r.o = p_evt;
-                                r.d = ps.wi;
-                                // roulette_interior (pt.ts:230-283); nothing is owed after a
-                                // tracking arm, whose lottery settled absorption already
-                                bool survive = true;
-                                if (P.rr_start >= 0 && bounce >= P.rr_start && !het) {
-                                    Col ss = CM::sigma_s(S, med_mat, wl), sa = CM::sigma_a(S, med_mat, wl);
-                                    Col surv = ss / vmax(ss + sa, Col(1e-9f));
-                                    float p_survive = spectrum_max(surv);
-                                    if (p_survive <= 0.0f) survive = false;
-                                    else if (rng.next() > p_survive) survive = false;
-                                    else thr = thr / p_survive;
-                                }
-                                if (survive) { bounce += 1; alive = true; }
-                                else done = true;
-                            }
-                        }
-                    }
-                }
-            }
-            if (!handled) {
-                if (!boundary) {   // kernel_score_miss (kernel.glsl:11-14)
-                    float w = 1.0f;
-                    if (nee && S.env_samplable && !prev_delta) {
-                        if (!mis) w = 0.0f;
-                        else {
-                            float pe = S.env_select_live ? S.env_select_prob : 1.0f;
-                            w = power_heuristic(prev_bsdf_pdf, pe * env_pdf(S, r.d));
-                        }
-                    }
-                    Col e = thr * w * env_radiance<Col>(S, r.d, wl);
-                    rad = rad + e;
-                    if constexpr (ADJ) lrem = lrem - e;
-                    done = true;
-                } else {
-                    if (MEDIA && hit.region_from != cur_med) cur_med = hit.region_from;
-                    int mat = material_of(S, hit.region_owner);
-                    const ptr_material& m = S.materials[mat];
-                    if (MEDIA && m.model == PTR_MAT_NONE) {   // null pass-through (pt.ts:404-417)
-                        cur_med = hit.region_to;
-                        Ray nr = ray_spawn(hit, r.d);
-                        r = nr;
-                        nulls += 1;
-                        if (nulls > P.max_null) done = true;
-                        else alive = true;
-                    } else {
-                        f3 wo = -r.d;
-                        // the AOV capture (pt.ts:422-433): the first non-null surface before
-                        // any event, weighted by the arrival throughput
-                        if constexpr (!SPECTRAL) {
-                            if (bounce == 0 && pool.aov) {
-                                f3 fact = ld3(m.transmittance);
-                                auto aov = [&](auto M) { fact = decltype(M)::aov(m); };
-                                dispatch_material<MatPresent>(m.model, aov);
-                                fact = vmin(vmax(fact, f3(0.0f)), f3(1.0f));
-                                f3 nf = dot(hit.frame.n, wo) < 0.0f ? -hit.frame.n : hit.frame.n;
-                                pool.aov[2 * i] = f4(fact * thr, 0.0f);
-                                pool.aov[2 * i + 1] = f4(nf * spectrum_average(thr), 0.0f);
-                            }
-                        }
-                        // kernel_score_emitter_hit (kernel.glsl:16-25; combiner.ts:27-46)
-                        int mat_emit = material_of(S, hit.region_to);
-                        if (mat_emit >= 0 && (S.materials[mat_emit].flags & PTR_MATF_EMISSIVE)) {
-                            float w = 1.0f;
-                            if (nee) {
-                                int lid = hit.region_to >= 0 ? emitter_light(S, hit) : -1;
-                                if (lid >= 0 && !prev_delta) {
-                                    if (!mis) w = 0.0f;
-                                    else {
-                                        // the stored selection context (its normal and sidedness
-                                        // only under light-tree selection)
-                                        LightQuery pq{prev_qp, f3(0.0f), false};
-                                        if (tree) {
-                                            float4 pqn = pool.prev_n[i];
-                                            pq.n = xyz(pqn);
-                                            pq.two_sided = pqn.w != 0.0f;
-                                        }
-                                        w = power_heuristic(prev_bsdf_pdf, lighting_pdf(S, pq, r.d, lid, hit.p, hit.ng, tree));
-                                    }
-                                }
-                            }
-                            Col e = thr * w * CM::emission(S, mat_emit, wl);
-                            rad = rad + e;
-                            if constexpr (ADJ) lrem = lrem - e;
-                        }
-                        if (bounce == N) {
-                            done = true;
-                        } else {
-                            const float alpha = hit.alpha >= 0.0f ? hit.alpha : m.alpha;
-                            // light queries with sphere support (a transmissive non-delta lobe)
-                            const bool rough = material_in<MatSphereQuery>(m.model);
-                            const bool nondelta = material_in<MatNonDelta>(m.model);
-                            const float n_from = ior_of(S, hit.region_from), n_to = ior_of(S, hit.region_to);
-                            const MatSite<Col> site{S, mat, m, hit, wl, alpha, n_from, n_to};
-                            // light_sample_direct (light.glsl:8-28)
-                            if (nee && nondelta) {
-                                float y0 = rng.next();
-                                float y1 = rng.next();
-                                LightQuery lq{hit.p, hit.frame.n, rough};   // rough glass: sphere support
-                                LightSample<Col> ls = lighting_sample<Col>(S, lq, y0, y1, rng, tree, wl);
-                                if (MEDIA && S.has_het) pool.sh_seed[i] = rng.dim;
-                                if (ls.pdf > 0.0f) {
-                                    f3 light_p = hit.p + ls.wi * ls.distance;
-                                    Ray sr = ray_spawn(hit, ls.wi);
-                                    sr.d = normalize(light_p - sr.o);
-                                    Col f(0.0f);
-                                    float bp = 0.0f;
-                                    const bool want_pdf = mis && !(ls.flags & kLightDelta);
-                                    auto lobe = [&](auto M) {
-                                        f = decltype(M)::eval(site, ls.wi, wo);
-                                        if (want_pdf) bp = decltype(M)::pdf(site, ls.wi, wo);
-                                    };
-                                    dispatch_material<MatNonDelta, true>(m.model, lobe);   // nondelta holds here
-                                    float cos_i = fabsf(dot(ls.wi, hit.frame.n));
-                                    float w = 1.0f;
-                                    if (want_pdf) w = power_heuristic(ls.pdf, bp);
-                                    float maxd = length(light_p - sr.o) - kShadowBackoff;
-                                    pool.sh_o[i] = f4(sr.o, maxd);
-                                    pool.sh_d[i] = f4(sr.d, __int_as_float(P.max_null - nulls));
-                                    pool.sh_lp[i] = f4(light_p, w);
-                                    pool.sh_c[i] = col_st(thr * ls.radiance * f * cos_i, ls.pdf);
-                                    if constexpr (SPECTRAL) pool.sh_pdf[i] = ls.pdf;
-                                    shadow = true;
-                                    if constexpr (ADJ) {
-                                        sh_mat = mat;
-                                        auto ng = [&](auto M) { decltype(M)::nee_grad(site, ls.wi, wo, sg); };
-                                        dispatch_material<MatNonDelta, true>(m.model, ng);
-                                    }
-                                }
-                            }
-                            // kernel_sample_continuation (kernel.glsl:27-34)
-                            float uc = rng.next();
-                            float u0 = rng.next();
-                            float u1 = rng.next();
-                            ISample<Col> bs;
-                            bs.weight = Col(0.0f);   // stays black only in a build without the scene's models
-                            auto cont = [&](auto M) { bs = decltype(M)::sample(site, wo, uc, u0, u1); };
-                            dispatch_material<MatPresent>(m.model, cont);
-                            if (spectrum_is_black(bs.weight)) {
-                                done = true;
-                            } else {
-                                thr = thr * bs.weight;
-                                if constexpr (ADJ) {   // the continuation lobe: d log w_cont
-                                    auto cg = [&](auto M) { decltype(M)::cont_grad(site, bs, wo, ga, lrem, shadow, sg); };
-                                    dispatch_material<MatPresent>(m.model, cg);
-                                }
-                                prev_delta = (bs.flags & kLobeDelta) != 0u;
-                                prev_bsdf_pdf = bs.pdf;
-                                prev_qp = hit.p;
-                                if (tree) pool.prev_n[i] = f4(hit.frame.n, rough ? 1.0f : 0.0f);
-                                if (bs.flags & kLobeTransmission) {
-                                    if (MEDIA) cur_med = hit.region_to;
-                                    float rr = ior_of(S, hit.region_to) / ior_of(S, hit.region_from);
-                                    eta_scale *= rr * rr;
-                                }
-                                // roulette (pt.ts:204-222)
-                                bool survive = true;
-                                if (P.rr_start >= 0 && bounce >= P.rr_start) {
-                                    float p_survive = gmin(P.rr_max_survival, spectrum_max(thr) * eta_scale);
-                                    if (p_survive <= 0.0f) survive = false;
-                                    else if (rng.next() > p_survive) survive = false;
-                                    else thr = thr / p_survive;
-                                }
-                                if (survive) {
-                                    r = ray_spawn(hit, bs.wi);
-                                    bounce += 1;
-                                    alive = true;
-                                } else {
-                                    done = true;
-                                }
-                            }
-                        }
-                    }
-                }
-            }
-            (void)done;
+            PoolSink<Col> sink(pool, i);
+            alive = walk_iteration<Col, DIRECT, MEDIA, ADJ>(S, P, ws, hr, sink, ga, sh_mat, sg, true, [] {});
+            shadow = sink.shadow;
+            shadow2 = sink.shadow2;
             if (pool.ray_sort) {
-                if (alive) rk = ray_key(S, r.o, r.d);
+                if (alive) rk = ray_key(S, ws.r.o, ws.r.d);
                 if (shadow) {
                     float4 so = pool.sh_o[i], sd = pool.sh_d[i];
                     sk = ray_key(S, xyz(so), xyz(sd));
                 }
             }
-            pool.rad[i] = col_st(rad, 0.0f);
-            pool.thr[i] = col_st(thr, 0.0f);   // with rad: the whole record, for a dying path too
+            pool.rad[i] = col_st(ws.rad, 0.0f);
+            pool.thr[i] = col_st(ws.thr, 0.0f);   // with rad: the whole record, for a dying path too
             if constexpr (ADJ) {
-                pool.l_rem[i] = f4(lrem, 0.0f);
+                pool.l_rem[i] = f4(ws.lrem, 0.0f);
                 if (shadow) {
                     pool.sh_g[i] = f4(sg.dnee, sg.dw);
                     pool.sh_gm[i] = sh_mat | (sg.kind << 16);
                 }
             }
             if (alive) {
-                pool.ray_o[i] = f4(r.o, prev_bsdf_pdf);
-                pool.ray_d[i] = f4(r.d, eta_scale);
-                pool.prev_q[i] = f4(prev_qp, 0.0f);
-                pool.st[i] = make_int4(bounce, cur_med, nulls, prev_delta ? 1 : 0);
-                pool.rng[i] = make_uint2(rng.base, rng.dim);
+                pool.ray_o[i] = f4(ws.r.o, ws.prev_bsdf_pdf);
+                pool.ray_d[i] = f4(ws.r.d, ws.eta_scale);
+                pool.prev_q[i] = f4(ws.prev_qp, 0.0f);
+                pool.st[i] = make_int4(ws.bounce, ws.cur_med, ws.nulls, ws.prev_delta ? 1 : 0);
+                pool.rng[i] = make_uint2(ws.rng.base, ws.rng.dim);
             }
         }
         int slot = warp_append(&pool.cnt[in ^ 1], alive);
@@ -1405,6 +1514,107 @@ __global__ void __launch_bounds__(256, PTR_SHADE_MIN_BLOCKS) k_shade(DevScene S0
 // its vertex and d log T / d theta of every medium segment the shadow ray crossed.
 constexpr int kAdjMaxMedia = 4;            // distinct media one adjoint shadow query may cross
 constexpr unsigned kErrAdjMedia = 8u;      // ... more were crossed (their terms were dropped)
+// The distinct media a shadow query crossed and its length in each (the adjoint's terms).
+struct ShadowMedia {
+    int id[kAdjMaxMedia];
+    float len[kAdjMaxMedia];
+    int n = 0;
+};
+// What one shadow query lets through: opaque visibility (shadow/opaque/opaque.glsl:16-19) or
+// the media segment walker (shadow/media/media.glsl:29-62).  seed_of() starts the query's own
+// stream, called only where a heterogeneous medium asks for it.  collect: note the media
+// crossed in mm; flag_more: raise the adjoint's guard where they exceed it (a recording
+// walk logs a negative count there instead).
+template <class Col, bool MEDIA, class SeedOf>
+__device__ __forceinline__ Col shadow_visibility(const DevScene& S, const ProgParams& P, const Ray& sr, float max_dist, f3 light_p,
+                                                 int crossings_left, const Wl& wl, SeedOf seed_of, bool collect, bool flag_more,
+                                                 ShadowMedia& mm, Work* work) {
+    constexpr bool SPECTRAL = sizeof(Col) == sizeof(s4);
+    if (!MEDIA) return scene_any(S, sr, max_dist, work) ? Col(0.0f) : Col(1.0f);
+    Col T(1.0f);
+    Rng srng;
+    bool srng_live = false;
+    int medium = scene_region_at(S, sr.o);
+    Ray seg = sr;
+    for (int crossed = 0; crossed <= crossings_left; crossed++) {
+        float remaining = length(light_p - seg.o) - kShadowBackoff;
+        if (remaining <= 0.0f) return T;
+        HitRec hr = scene_closest(S, seg, work);
+        bool hit_boundary = hr.region >= 0 && hr.t < remaining;
+        float seg_len = hit_boundary ? hr.t : remaining;
+        int med_mat = material_of(S, medium);
+        if (mat_has_medium(S, med_mat)) {
+            bool het = false;
+            if constexpr (!SPECTRAL) {
+                const ptr_material& smm = S.materials[med_mat];
+                if ((PTR_SPEC_HET && S.has_het) && mat_is_het(smm)) {   // ratio tracking on the query's own stream
+                    het = true;
+                    if (!srng_live) { srng = seed_of(); srng_live = true; }
+                    T = T * medium_ratio_track(S, smm, seg, seg_len, srng, scatter_live(S, P, med_mat));
+                }
+            }
+            if (!het) T = T * medium_transmittance<Col>(S, P, med_mat, seg_len, wl);
+            if (collect) {
+                int e = 0;
+                while (e < mm.n && mm.id[e] != med_mat) e++;
+                if (e < mm.n) mm.len[e] += seg_len;
+                else if (mm.n < kAdjMaxMedia) { mm.id[mm.n] = med_mat; mm.len[mm.n] = seg_len; mm.n++; }
+                else if (flag_more) flag_error(S, kErrAdjMedia);
+            }
+        }
+        if (!hit_boundary) return T;
+        // an optical surface blocks the query: decided from the hit region alone,
+        // before the hit's frame and its region classification
+        const int om = material_of(S, hr.region);
+        if (!(om >= 0 && S.materials[om].model == PTR_MAT_NONE)) return Col(0.0f);
+        Hit h;
+        fill_hit(S, seg, hr, h, false, true);
+        medium = h.region_to;
+        seg = ray_spawn(h, seg.d);
+        seg.d = normalize(light_p - seg.o);
+    }
+    return Col(0.0f);
+}
+// The walk log's shadow record (PathPool::hit_log): visibility rgb and the media count, then
+// up to two (medium, length) pairs; a count of -1 marks a query the replay walks again.
+__device__ __forceinline__ void shadow_log_write(float4* rec, f3 vis, const ShadowMedia& mm) {
+    rec[0] = make_float4(vis.x, vis.y, vis.z, __int_as_float(mm.n <= 2 ? mm.n : -1));
+    rec[1] = make_float4(__int_as_float(mm.n > 0 ? mm.id[0] : -1), mm.n > 0 ? mm.len[0] : 0.0f,
+                         __int_as_float(mm.n > 1 ? mm.id[1] : -1), mm.n > 1 ? mm.len[1] : 0.0f);
+}
+__device__ __forceinline__ bool shadow_log_read(const float4* rec, f3& vis, ShadowMedia& mm) {
+    const float4 a = rec[0], b = rec[1];
+    const int n = __float_as_int(a.w);
+    if (n < 0) return false;
+    vis = f3(a.x, a.y, a.z);
+    mm.n = n;
+    mm.id[0] = __float_as_int(b.x);
+    mm.len[0] = b.y;
+    mm.id[1] = __float_as_int(b.z);
+    mm.len[1] = b.w;
+    return true;
+}
+// The replay's gradient terms of one shadow query whose contribution is add: its vertex's lobe
+// derivative and d log T / d theta of every medium it crossed.
+__device__ __forceinline__ void shadow_grads(const DevScene& S, const ProgParams& P, const GradAcc& ga, f3 add, int vmat, int kind,
+                                             f3 D, float dw, const ShadowMedia& mm) {
+    if (kind == kGradKindAlbedo) ga.vec(vmat, PTR_GRAD_COLOR_R, add, D);
+    else if (kind == kGradKindGGX) {
+        ga.vec(vmat, PTR_GRAD_COLOR_R, add, D);
+        ga.scl(vmat, PTR_GRAD_ALPHA, add, dw);
+    }
+    else if (kind == kGradKindPhase) ga.scl(vmat, PTR_GRAD_HG_G, add, D.x);
+    for (int e = 0; e < mm.n; ++e) {   // T = exp(-st len) (scattering) or exp(-(1-a) st len)
+        GreyMedium g = grey_medium(S.materials[mm.id[e]]);
+        if (scatter_live(S, P, mm.id[e])) {
+            ga.scl(mm.id[e], PTR_GRAD_SIGMA_T, add, -mm.len[e]);
+        } else {
+            ga.scl(mm.id[e], PTR_GRAD_SIGMA_T, add, -(1.0f - g.a) * mm.len[e]);
+            ga.scl(mm.id[e], PTR_GRAD_MEDIUM_ALBEDO, add, g.st * mm.len[e]);
+        }
+    }
+}
+
 // Opaque shadow queries over the same scene form, with the same per-lane refill: the
 // regions before the instanced one, the flat any-hit walk, then the regions after it (the
 // order of scene_any); an unoccluded query adds its stored contribution as k_shadow does.
@@ -1532,84 +1742,17 @@ __global__ void __launch_bounds__(256, PTR_TRACE_MIN_BLOCKS) k_shadow(DevScene S
         sr.o = xyz(so);
         sr.d = xyz(sd);
         Col vis;
-        int mm_id[kAdjMaxMedia];
-        float mm_len[kAdjMaxMedia];
-        int n_mm = 0;
+        ShadowMedia mm;
         bool logged = false;
         if constexpr (ADJ) {
-            if (rep) {   // the forward walk's visibility and media of this same query
-                const float4 a = slog[4 * (size_t)i], b = slog[4 * (size_t)i + 1];
-                n_mm = __float_as_int(a.w);
-                logged = n_mm >= 0;
-                if (logged) {
-                    vis = Col(a.x, a.y, a.z);
-                    mm_id[0] = __float_as_int(b.x);
-                    mm_len[0] = b.y;
-                    mm_id[1] = __float_as_int(b.z);
-                    mm_len[1] = b.w;
-                } else {
-                    n_mm = 0;
-                }
-            }
+            if (rep) logged = shadow_log_read(slog + 4 * (size_t)i, vis, mm);
         }
-        if (logged) {
-        } else if (!MEDIA) {
-            vis = scene_any(S, sr, so.w, COUNT ? &wk : nullptr) ? Col(0.0f) : Col(1.0f);
-        } else {
-            f3 light_p = xyz(lp);
-            int crossings_left = __float_as_int(sd.w);
-            Col T(1.0f);
-            Rng srng;
-            bool srng_live = false;
-            int medium = scene_region_at(S, sr.o);
-            Ray seg = sr;
-            bool finished = false;
-            for (int crossed = 0; crossed <= crossings_left; crossed++) {
-                float remaining = length(light_p - seg.o) - kShadowBackoff;
-                if (remaining <= 0.0f) { finished = true; break; }
-                HitRec hr = scene_closest(S, seg, COUNT ? &wk : nullptr);
-                bool hit_boundary = hr.region >= 0 && hr.t < remaining;
-                float seg_len = hit_boundary ? hr.t : remaining;
-                int med_mat = material_of(S, medium);
-                if (mat_has_medium(S, med_mat)) {
-                    bool het = false;
-                    if constexpr (!SPECTRAL) {
-                        const ptr_material& smm = S.materials[med_mat];
-                        if (S.has_het && mat_is_het(smm)) {   // ratio tracking on the query's own stream
-                            het = true;
-                            if (!srng_live) { srng = shadow_rng(pool.rng[i].x, pool.sh_seed[i]); srng_live = true; }
-                            T = T * medium_ratio_track(S, smm, seg, seg_len, srng, scatter_live(S, P, med_mat));
-                        }
-                    }
-                    if (!het) T = T * medium_transmittance<Col>(S, P, med_mat, seg_len, wl);
-                    if (ADJ || rec) {
-                        int e = 0;
-                        while (e < n_mm && mm_id[e] != med_mat) e++;
-                        if (e < n_mm) mm_len[e] += seg_len;
-                        else if (n_mm < kAdjMaxMedia) { mm_id[n_mm] = med_mat; mm_len[n_mm] = seg_len; n_mm++; }
-                        else if (ADJ) flag_error(S, kErrAdjMedia);   // (a recording walk logs -1 here)
-                    }
-                }
-                if (!hit_boundary) { finished = true; break; }
-                // an optical surface blocks the query: decided from the hit region alone,
-                // before the hit's frame and its region classification
-                const int om = material_of(S, hr.region);
-                if (!(om >= 0 && S.materials[om].model == PTR_MAT_NONE)) { T = Col(0.0f); finished = true; break; }
-                Hit h;
-                fill_hit(S, seg, hr, h);
-                medium = h.region_to;
-                seg = ray_spawn(h, seg.d);
-                seg.d = normalize(light_p - seg.o);
-            }
-            vis = finished ? T : Col(0.0f);
-        }
+        if (!logged)
+            vis = shadow_visibility<Col, MEDIA>(S, P, sr, so.w, xyz(lp), __float_as_int(sd.w), wl,
+                                                [&] { return shadow_rng(pool.rng[i].x, pool.sh_seed[i]); }, ADJ || rec, ADJ, mm,
+                                                COUNT ? &wk : nullptr);
         if constexpr (!ADJ && !SPECTRAL) {
-            if (rec) {
-                const bool fits = n_mm <= 2;
-                slog[4 * (size_t)i] = make_float4(vis.x, vis.y, vis.z, __int_as_float(fits ? n_mm : -1));
-                slog[4 * (size_t)i + 1] = make_float4(__int_as_float(n_mm > 0 ? mm_id[0] : -1), n_mm > 0 ? mm_len[0] : 0.0f,
-                                                      __int_as_float(n_mm > 1 ? mm_id[1] : -1), n_mm > 1 ? mm_len[1] : 0.0f);
-            }
+            if (rec) shadow_log_write(slog + 4 * (size_t)i, vis, mm);
         }
         if (!spectrum_is_black(vis)) {
             float w = lp.w;
@@ -1622,24 +1765,8 @@ __global__ void __launch_bounds__(256, PTR_TRACE_MIN_BLOCKS) k_shadow(DevScene S
                 float4 lr = pool.l_rem[i];
                 pool.l_rem[i] = make_float4(lr.x - add.x, lr.y - add.y, lr.z - add.z, 0.f);
                 const int gm = pool.sh_gm[i];
-                const int kind = gm >> 16, vmat = gm & 0xFFFF;
                 const float4 Dg = pool.sh_g[i];
-                const f3 D = xyz(Dg);
-                if (kind == kGradKindAlbedo) ga.vec(vmat, PTR_GRAD_COLOR_R, add, D);
-                else if (kind == kGradKindGGX) {
-                    ga.vec(vmat, PTR_GRAD_COLOR_R, add, D);
-                    ga.scl(vmat, PTR_GRAD_ALPHA, add, Dg.w);
-                }
-                else if (kind == kGradKindPhase) ga.scl(vmat, PTR_GRAD_HG_G, add, D.x);
-                for (int e = 0; e < n_mm; ++e) {   // T = exp(-st len) (scattering) or exp(-(1-a) st len)
-                    GreyMedium g = grey_medium(S.materials[mm_id[e]]);
-                    if (scatter_live(S, P, mm_id[e])) {
-                        ga.scl(mm_id[e], PTR_GRAD_SIGMA_T, add, -mm_len[e]);
-                    } else {
-                        ga.scl(mm_id[e], PTR_GRAD_SIGMA_T, add, -(1.0f - g.a) * mm_len[e]);
-                        ga.scl(mm_id[e], PTR_GRAD_MEDIUM_ALBEDO, add, g.st * mm_len[e]);
-                    }
-                }
+                shadow_grads(S, P, ga, add, gm & 0xFFFF, gm >> 16, xyz(Dg), Dg.w, mm);
             }
         }
     }
@@ -1647,42 +1774,257 @@ __global__ void __launch_bounds__(256, PTR_TRACE_MIN_BLOCKS) k_shadow(DevScene S
     if constexpr (ADJ) grad_block_flush(s_grad, PTR_GRAD_SLOTS * S0.n_materials, adj.grads);
 }
 
-// Fold the wave's per-path radiance into the film, per pixel in sample order; then
-// advance the wave cursor.
-// SPECTRAL: each sample's four lanes are projected to linear sRGB first (color_to_pixel).
-template <bool SPECTRAL = false>
-__global__ void k_film(PathPool pool, const FrameParams* fp, double* sum, double* sumsq, float* samples_out,
-                       DevScene S = DevScene{}) {
-    const FrameParams F = *fp;
-    const long long base = pool.wave[0];
-    const long long n = pool.wave[1];
-    const long long npix = (long long)F.width * F.height;
-    const long long nslot = n < npix ? n : npix;
-    for (long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x; j < nslot; j += (long long)gridDim.x * blockDim.x) {
-        int pix = (int)((base + j) % npix);
-        double s0 = sum[3 * pix + 0], s1 = sum[3 * pix + 1], s2 = sum[3 * pix + 2];
-        double q0 = sumsq[3 * pix + 0], q1 = sumsq[3 * pix + 1], q2 = sumsq[3 * pix + 2];
-        for (long long i = j; i < n; i += npix) {
-            float4 L = pool.rad[i];
-            if (SPECTRAL) {
-                f3 px = color_to_pixel(S, L, pool.wl[i], pool.wl_pdf[i]);
-                L = make_float4(px.x, px.y, px.z, 0.0f);
-            }
-            s0 += (double)L.x; s1 += (double)L.y; s2 += (double)L.z;
-            q0 += (double)L.x * (double)L.x; q1 += (double)L.y * (double)L.y; q2 += (double)L.z * (double)L.z;
-            if (samples_out) {
-                long long g = base + i;
-                samples_out[3 * g + 0] = L.x; samples_out[3 * g + 1] = L.y; samples_out[3 * g + 2] = L.z;
+// ---- the whole walk in one kernel ------------------------------------------------------
+// k_walk runs every iteration of a path in one thread, its state in registers: no path
+// record, queue or shadow query travels through memory, only 16 bytes of radiance per path
+// go to the film pass.  A lane whose path has ended takes the next one (warp-aggregated
+// tickets), so lanes stay busy whatever the paths' lengths, and a wave is one launch instead
+// of three per iteration.  The arithmetic and the order of the random numbers and radiance
+// sums are walk_iteration's and shadow_visibility's, so samples are bit-identical to the
+// wavefront kernels'.
+struct WalkArgs {
+    float4* film;                 // radiance of path base + i at [i]
+    float4* aov;                  // first-hit samples, two per path (null: none)
+    unsigned* ticket;             // zero at the launch
+    unsigned long long* stats;    // [0] closest queries, [1] shadow queries, [2] paths
+    long long base;               // the wave's paths: [base, base + n) of the frame or job space
+    unsigned n;
+    int iters;                    // walk iterations at most
+    int lockstep;                 // the block's warps run each part of an iteration together
+    float4* hit_log;              // PathPool::hit_log of the adjoint (null: none)
+    long long hit_log_stride;
+    int hit_log_iters;
+};
+
+// k_walk's sink: an iteration's queries stay in registers until the walk resolves them.
+template <class Col>
+struct WalkQuery {
+    Ray r;
+    float max_dist;
+    int crossings;
+    f3 light_p;
+    float w;
+    Col contrib;
+    float pdf;
+    bool live;
+};
+template <class Col>
+struct WalkSink {
+    WalkQuery<Col> seg, vtx;
+    unsigned dim;
+    float4 prev_n;
+    float4* aov_p;
+    __device__ __forceinline__ void segment_query(f3 o, f3 d, int crossings, f3 light_p, Col contrib, float pdf) {
+        seg = WalkQuery<Col>{Ray{o, d}, 0.0f, crossings, light_p, 1.0f, contrib, pdf, true};
+    }
+    __device__ __forceinline__ void vertex_query(f3 o, float max_dist, f3 d, int crossings, f3 light_p, float w, Col contrib, float pdf) {
+        vtx = WalkQuery<Col>{Ray{o, d}, max_dist, crossings, light_p, w, contrib, pdf, true};
+    }
+    __device__ __forceinline__ void seed(unsigned d) { dim = d; }
+    __device__ __forceinline__ void put_prev_n(float4 n) { prev_n = n; }
+    __device__ __forceinline__ float4 get_prev_n() const { return prev_n; }
+    __device__ __forceinline__ float4* aov() const { return aov_p; }
+};
+
+#ifndef PTR_WALK_MIN_BLOCKS
+#define PTR_WALK_MIN_BLOCKS 3
+#endif
+#ifndef PTR_WALK_REFILL
+#define PTR_WALK_REFILL 1
+#endif
+template <class Col, int DIRECT, bool MEDIA, bool BATCH, bool ADJ = false>
+__global__ void __launch_bounds__(256, PTR_WALK_MIN_BLOCKS) k_walk(DevScene S0, ProgParams P0, FrameParams F0, BatchTables bt,
+                                                                   WalkArgs wa, AdjParams adj = AdjParams{}) {
+    constexpr bool SPECTRAL = sizeof(Col) == sizeof(s4);
+    static_assert(!(ADJ && SPECTRAL), "the adjoint replay is RGB only");
+    extern __shared__ double s_grad[];
+    if constexpr (ADJ) grad_block_init(s_grad, PTR_GRAD_SLOTS * S0.n_materials);
+    if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&wa.stats[2], (unsigned long long)wa.n);
+    const WaveJobs wj = BATCH ? WaveJobs(wa.base, (long long)wa.n, bt) : WaveJobs{};
+    unsigned n_closest = 0u, n_shadow = 0u;
+    WalkState<Col> ws;
+    WalkSink<Col> sink;
+    GradAcc ga;
+    ga.s = s_grad;
+    int i = -1, job = 0, it = 0;
+    bool active = false, exhausted = false;
+    auto phase = [&] { if (wa.lockstep) __syncthreads(); else __syncwarp(); };
+    for (;;) {
+        const unsigned idle = __ballot_sync(0xffffffffu, !active);
+        if (!exhausted && __popc(idle) >= PTR_WALK_REFILL) {
+            unsigned first = 0u;
+            if ((threadIdx.x & 31u) == 0u) first = atomicAdd(wa.ticket, (unsigned)__popc(idle));
+            first = __shfl_sync(0xffffffffu, first, 0);
+            exhausted = first + (unsigned)__popc(idle) >= wa.n;
+            const unsigned k = first + __popc(idle & lanemask_lt());
+            if (!active && k < wa.n) {
+                active = true;
+                i = (int)k;
+                it = 0;
+                if (BATCH) job = wj.of(bt, i);
+                const DevScene& S = BATCH ? bt.scenes[job] : S0;
+                const FrameParams& F = BATCH ? bt.jobs[job].frame : F0;
+                int pix, sample;
+                split_path(wa.base + i - (BATCH ? bt.offsets[job] : 0ll), (unsigned)F.width * (unsigned)F.height, pix, sample);
+                float4 lambda;
+                camera_path<SPECTRAL>(F, pix, sample, ws.rng, ws.r, lambda);
+                if constexpr (SPECTRAL) ws.wl.lambda = lambda;
+                ws.prev_bsdf_pdf = 0.0f;
+                ws.eta_scale = 1.0f;
+                ws.thr = Col(1.0f);
+                ws.rad = Col(0.0f);
+                ws.prev_qp = ws.r.o;
+                ws.bounce = 0;
+                ws.cur_med = S.has_media ? scene_region_at(S, ws.r.o) : -1;
+                ws.nulls = 0;
+                ws.prev_delta = true;
+                if constexpr (ADJ) {   // the forward walk left this path's total radiance
+                    ws.lrem = xyz(wa.film[i]);
+                    const float* g = adj.dl_image + 3 * (size_t)pix;
+                    ga.dl = f3(g[0] * adj.inv_spp, g[1] * adj.inv_spp, g[2] * adj.inv_spp);
+                }
+                sink.aov_p = nullptr;
+                if (wa.aov) {
+                    sink.aov_p = wa.aov + 2 * (size_t)i;
+                    sink.aov_p[0] = make_float4(0.f, 0.f, 0.f, 0.f);
+                    sink.aov_p[1] = make_float4(0.f, 0.f, 0.f, 0.f);
+                }
             }
         }
-        sum[3 * pix + 0] = s0; sum[3 * pix + 1] = s1; sum[3 * pix + 2] = s2;
-        sumsq[3 * pix + 0] = q0; sumsq[3 * pix + 1] = q1; sumsq[3 * pix + 2] = q2;
-        if (pool.aov_sum) {   // the first-hit pictures, in the same sample order
-            double* as = pool.aov_sum + 3 * (size_t)pix;
-            double* ns = pool.aov_sum + 3 * ((size_t)npix + pix);
-            double a0 = as[0], a1 = as[1], a2 = as[2], n0 = ns[0], n1 = ns[1], n2 = ns[2];
+        if (wa.lockstep ? !__syncthreads_or(active) : !__any_sync(0xffffffffu, active)) break;
+        const DevScene& S = BATCH ? bt.scenes[job] : S0;
+        const ProgParams& P = BATCH ? bt.progs[job] : P0;
+        // this iteration's record of the adjoint's walk log: the closest hit, then the query
+        float4* rec = (!BATCH && !SPECTRAL && active && wa.hit_log && it < wa.hit_log_iters)
+                          ? wa.hit_log + 4 * ((size_t)it * (size_t)wa.hit_log_stride + (size_t)i) : nullptr;
+        HitRec hr;
+        if (active) {
+            if (ADJ && rec) {
+                const float4 hf = rec[0];
+                const int4 hi = float4_as_int4(rec[1]);
+                hr.t = hf.x; hr.u = hf.y; hr.v = hf.z;
+                hr.region = hi.x; hr.element = hi.y; hr.prim = hi.z;
+            } else {
+                hr = scene_closest(S, ws.r);
+                if (!ADJ && rec) {
+                    rec[0] = make_float4(hr.t, hr.u, hr.v, 0.f);
+                    rec[1] = int4_as_float4(make_int4(hr.region, hr.element, hr.prim, 0));
+                }
+            }
+            n_closest++;
+        }
+        phase();
+        bool alive = false;
+        int sh_mat = 0;
+        NeeGrad sg{kGradKindNone, f3(0.0f), 0.0f};
+        sink.seg.live = sink.vtx.live = false;
+        alive = walk_iteration<Col, DIRECT, MEDIA, ADJ>(S, P, ws, hr, sink, ga, sh_mat, sg, active, phase);
+        phase();
+        if constexpr (MEDIA && DIRECT == PTR_DIRECT_NEE && !ADJ) {   // the equiangular segment query comes first
+            if (sink.seg.live) {
+                ShadowMedia none;
+                n_shadow++;
+                const Col vis = shadow_visibility<Col, MEDIA>(S, P, sink.seg.r, 0.0f, sink.seg.light_p, sink.seg.crossings, ws.wl,
+                                                              [&] { return shadow_rng(ws.rng.base, sink.dim); }, false, false, none, nullptr);
+                if (!spectrum_is_black(vis)) ws.rad = ws.rad + sink.seg.contrib * vis * sink.seg.w / sink.seg.pdf;
+            }
+            phase();
+        }
+        if constexpr (DIRECT != PTR_DIRECT_NONE) {
+            if (sink.vtx.live) {
+                const WalkQuery<Col>& q = sink.vtx;
+                ShadowMedia mm;
+                Col vis;
+                bool logged = false;
+                n_shadow++;
+                if constexpr (ADJ) {
+                    if (rec) logged = shadow_log_read(rec + 2, vis, mm);
+                }
+                if (!logged)
+                    vis = shadow_visibility<Col, MEDIA>(S, P, q.r, q.max_dist, q.light_p, q.crossings, ws.wl,
+                                                        [&] { return shadow_rng(ws.rng.base, sink.dim); }, ADJ || rec, ADJ, mm, nullptr);
+                if constexpr (!ADJ && !SPECTRAL) {
+                    if (rec) shadow_log_write(rec + 2, vis, mm);
+                }
+                if (!spectrum_is_black(vis)) {
+                    const Col add = q.contrib * vis * q.w / q.pdf;
+                    ws.rad = ws.rad + add;
+                    if constexpr (ADJ) {
+                        ws.lrem = ws.lrem - add;
+                        shadow_grads(S, P, ga, add, sh_mat, sg.kind, sg.dnee, sg.dw, mm);
+                    }
+                }
+            }
+            phase();
+        }
+        if (active && (!alive || ++it >= wa.iters)) {
+            active = false;
+            if constexpr (SPECTRAL) {
+                const f3 px = color_to_pixel(S, col_st(ws.rad, 0.0f), ws.wl.lambda, wavelength_pdfs(BATCH ? bt.jobs[job].frame : F0, ws.wl.lambda));
+                wa.film[i] = f4(px, 0.0f);
+            } else if constexpr (!ADJ) {
+                wa.film[i] = f4(ws.rad, 0.0f);
+            }
+        }
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        n_closest += __shfl_xor_sync(0xffffffffu, n_closest, o);
+        n_shadow += __shfl_xor_sync(0xffffffffu, n_shadow, o);
+    }
+    if ((threadIdx.x & 31u) == 0u && n_closest) {
+        atomicAdd(&wa.stats[0], (unsigned long long)n_closest);
+        atomicAdd(&wa.stats[1], (unsigned long long)n_shadow);
+    }
+    if constexpr (ADJ) grad_block_flush(s_grad, PTR_GRAD_SLOTS * S0.n_materials, adj.grads);
+}
+
+// Adds one pixel's samples of a wave, paths i, i + npix, ... below n, to its film sums in
+// sample order; first: the film starts from zero here.  The samples are fetched four ahead of
+// the serial FP64 sums, so a pixel keeps several loads in flight.
+template <class Get>
+__device__ __forceinline__ void film_pixel(double* su, double* sq, bool first, long long i, long long n, long long npix, Get get) {
+    double s0 = 0.0, s1 = 0.0, s2 = 0.0, q0 = 0.0, q1 = 0.0, q2 = 0.0;
+    if (!first) { s0 = su[0]; s1 = su[1]; s2 = su[2]; q0 = sq[0]; q1 = sq[1]; q2 = sq[2]; }
+    auto add = [&](float4 L) {
+        s0 += (double)L.x; s1 += (double)L.y; s2 += (double)L.z;
+        q0 += (double)L.x * (double)L.x; q1 += (double)L.y * (double)L.y; q2 += (double)L.z * (double)L.z;
+    };
+    for (; i + 3 * npix < n; i += 4 * npix) {
+        const float4 a = get(i), b = get(i + npix), c = get(i + 2 * npix), d = get(i + 3 * npix);
+        add(a); add(b); add(c); add(d);
+    }
+    for (; i < n; i += npix) add(get(i));
+    su[0] = s0; su[1] = s1; su[2] = s2;
+    sq[0] = q0; sq[1] = q1; sq[2] = q2;
+}
+// Fold a wave's radiance (paths [base, base + n) of the frame, path base + i at
+// rad[i * stride]) into the film, per pixel in sample order, and its first-hit samples into
+// theirs.  color(i, L): the pixel colour of path i's radiance.
+template <class Color>
+__device__ __forceinline__ void film_wave(const FrameParams& F, const float4* rad, int stride, const float4* aov, double* aov_sum,
+                                          long long base, long long n, double* sum, double* sumsq, float* samples_out, Color color) {
+    const long long npix = (long long)F.width * F.height;
+    const long long nslot = n < npix ? n : npix;
+    const unsigned pix0 = (unsigned)(base % npix);
+    for (long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x; j < nslot; j += (long long)gridDim.x * blockDim.x) {
+        const long long p1 = (long long)pix0 + j;
+        const size_t pix = (size_t)(p1 < npix ? p1 : p1 - npix);
+        const bool first = F.fresh && base + j < npix;
+        film_pixel(sum + 3 * pix, sumsq + 3 * pix, first, j, n, npix, [&](long long i) {
+            const float4 L = color(i, rad[i * stride]);
+            if (samples_out) {
+                float* o = samples_out + 3 * (base + i);
+                o[0] = L.x; o[1] = L.y; o[2] = L.z;
+            }
+            return L;
+        });
+        if (aov_sum) {   // the first-hit pictures, in the same sample order
+            double* as = aov_sum + 3 * pix;
+            double* ns = aov_sum + 3 * ((size_t)npix + pix);
+            double a0 = 0.0, a1 = 0.0, a2 = 0.0, n0 = 0.0, n1 = 0.0, n2 = 0.0;
+            if (!first) { a0 = as[0]; a1 = as[1]; a2 = as[2]; n0 = ns[0]; n1 = ns[1]; n2 = ns[2]; }
             for (long long i = j; i < n; i += npix) {
-                float4 a = pool.aov[2 * i], b = pool.aov[2 * i + 1];
+                float4 a = aov[2 * i], b = aov[2 * i + 1];
                 a0 += (double)a.x; a1 += (double)a.y; a2 += (double)a.z;
                 n0 += (double)b.x; n1 += (double)b.y; n2 += (double)b.z;
             }
@@ -1690,6 +2032,24 @@ __global__ void k_film(PathPool pool, const FrameParams* fp, double* sum, double
             ns[0] = n0; ns[1] = n1; ns[2] = n2;
         }
     }
+}
+// SPECTRAL: each sample's four lanes are projected to linear sRGB first (color_to_pixel).
+template <bool SPECTRAL = false>
+__global__ void k_film(PathPool pool, const FrameParams* fp, double* sum, double* sumsq, float* samples_out,
+                       DevScene S = DevScene{}) {
+    const FrameParams F = *fp;
+    film_wave(F, pool.rad.p, 2, pool.aov, pool.aov_sum, pool.wave[0], pool.wave[1], sum, sumsq, samples_out, [&](long long i, float4 L) {
+        if (!SPECTRAL) return L;
+        const f3 px = color_to_pixel(S, L, pool.wl[i], pool.wl_pdf[i]);
+        return f4(px, 0.0f);
+    });
+}
+
+// The film pass after k_walk (its radiance is already the pixel colour), which also clears the
+// tickets for the next wave's walk.
+__global__ void k_film_walk(FrameParams F, WalkArgs wa, double* aov_sum, double* sum, double* sumsq, float* samples_out) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) *wa.ticket = 0u;
+    film_wave(F, wa.film, 1, wa.aov, aov_sum, wa.base, wa.n, sum, sumsq, samples_out, [](long long, float4 L) { return L; });
 }
 
 // ---- batched renders ------------------------------------------------------------------
@@ -1706,73 +2066,48 @@ __global__ void k_generate_batch(PathPool pool, BatchTables bt) {
         if (pool.fetch) pool.fetch[0] = 0u;
     }
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        long long g = base + i;
-        int j = job_of(bt, g);
+        const int j = job_of(bt, base + i);
         const FrameParams& F = bt.jobs[j].frame;
-        const DevScene& S = bt.scenes[j];
-        long long local = g - bt.offsets[j];
-        const long long npix = (long long)F.width * F.height;
-        int pix = (int)(local % npix);
-        int sample = (int)(local / npix);
-        int x = pix % F.width, y = pix / F.width;
+        int pix, sample;
+        split_path(base + i - bt.offsets[j], (unsigned)F.width * (unsigned)F.height, pix, sample);
         Rng rng;
-        rng.init((uint32_t)(x + F.px_off), (uint32_t)(y + F.py_off), (uint32_t)(F.first_sample + sample), F.salt);
-        float pxf = (float)x + 0.5f + (float)F.px_off;
-        float pyf = (float)y + 0.5f + (float)F.py_off;
-        float a0 = rng.next();
-        float a1 = rng.next();
-        float fx = pxf + (a0 - 0.5f), fy = pyf + (a1 - 0.5f);
-        rng.next();
-        rng.next();
-        float ndcx = (2.0f * fx / (float)F.img_w) - 1.0f;
-        float ndcy = (2.0f * fy / (float)F.img_h) - 1.0f;
-        ndcx *= F.cam.aspect;
-        f3 dir = normalize(ld3(F.cam.forward) + ndcx * F.cam.tan_fov * ld3(F.cam.right) +
-                           ndcy * F.cam.tan_fov * ld3(F.cam.up));
-        f3 o = ld3(F.cam.position);
-        int medium = S.has_media ? scene_region_at(S, o) : -1;
-        pool.ray_o[i] = f4(o, 0.0f);
-        pool.ray_d[i] = f4(dir, 1.0f);
-        pool.thr[i] = make_float4(1.f, 1.f, 1.f, 0.f);
-        pool.rad[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-        pool.prev_q[i] = f4(o, 0.0f);
-        pool.st[i] = make_int4(0, medium, 0, 1);
-        pool.rng[i] = make_uint2(rng.base, rng.dim);
-        pool.job[i] = j;
-        pool.q[0][i] = (int)i;
+        Ray r;
+        float4 unused;
+        camera_path<false>(F, pix, sample, rng, r, unused);
+        init_slot(bt.scenes[j], pool, i, rng, r);
     }
 }
 
-// Fold the wave's radiance into each job's film.  Within a wave the paths of job j are the
-// contiguous range [s, e) of the concatenated index space, and one pixel's samples lie npix
-// apart in it.  The first npix paths of the range (one per pixel the wave touches) each add
-// their pixel's samples to the film in sample order, like k_film: the film is the sequential
-// FP64 sum of every pixel's samples in sample order, so a batched film equals the job's plain
-// film bit for bit, however the waves split the jobs.
-__global__ void k_film_batch(PathPool pool, BatchTables bt) {
-    const long long base = pool.wave[0];
-    const long long n = pool.wave[1];
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        const int j = pool.job[i];
+// Fold the wave [base, base + n) of the concatenated job space into each job's film.  The
+// wave's paths of job j are one contiguous range of the index space, and one pixel's samples
+// lie npix apart in it.  The first npix paths of the range (one per pixel the wave touches)
+// each add their pixel's samples to the film in sample order, like k_film: the film is the
+// sequential FP64 sum of every pixel's samples in sample order, so a batched film equals the
+// job's plain film bit for bit, however the waves split the jobs.  The grid walks the wave's
+// jobs one after another, so no path looks its job up.
+__device__ __forceinline__ void film_batch(const BatchTables& bt, const float4* rad, int stride, long long base, long long n) {
+    const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x, nthr = (long long)gridDim.x * blockDim.x;
+    for (int j = job_of(bt, base); j < bt.n_jobs && bt.offsets[j] < base + n; ++j) {
         const BatchJob& J = bt.jobs[j];
         const long long npix = (long long)J.frame.width * J.frame.height;
-        const long long off = bt.offsets[j];
-        const long long g = base + i;
-        if (g - (off > base ? off : base) >= npix) continue;   // not the first visit of its pixel in this wave
-        const long long job_end = j + 1 < bt.n_jobs ? bt.offsets[j + 1] : bt.total;
-        const long long end = job_end < base + n ? job_end : base + n;
-        const long long pix = (g - off) % npix;
-        double* su = J.sum + 3 * pix;
-        double* sq = J.sumsq + 3 * pix;
-        double s0 = su[0], s1 = su[1], s2 = su[2], q0 = sq[0], q1 = sq[1], q2 = sq[2];
-        for (long long k = g; k < end; k += npix) {
-            const float4 L = pool.rad[k - base];
-            s0 += (double)L.x; s1 += (double)L.y; s2 += (double)L.z;
-            q0 += (double)L.x * (double)L.x; q1 += (double)L.y * (double)L.y; q2 += (double)L.z * (double)L.z;
+        const long long off = bt.offsets[j], job_end = bt.offsets[j + 1];
+        const long long lo = off > base ? off : base, hi = job_end < base + n ? job_end : base + n;
+        const long long m = hi - lo < npix ? hi - lo : npix;
+        for (long long t = tid; t < m; t += nthr) {
+            const long long g = lo + t;
+            const bool first = J.frame.fresh && g - off < npix;
+            film_pixel(J.sum + 3 * ((g - off) % npix), J.sumsq + 3 * ((g - off) % npix), first, g - base, hi - base, npix,
+                       [&](long long k) { return rad[k * stride]; });
         }
-        su[0] = s0; su[1] = s1; su[2] = s2;
-        sq[0] = q0; sq[1] = q1; sq[2] = q2;
     }
+}
+__global__ void k_film_batch(PathPool pool, BatchTables bt) {
+    film_batch(bt, pool.rad.p, 2, pool.wave[0], pool.wave[1]);
+}
+
+__global__ void k_film_batch_walk(BatchTables bt, WalkArgs wa) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) *wa.ticket = 0u;
+    film_batch(bt, wa.film, 1, wa.base, wa.n);
 }
 
 // Raw nearest-hit queries (tests and tools): per ray (o.xyz, d.xyz) the region, the

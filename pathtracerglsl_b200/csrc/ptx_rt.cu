@@ -28,6 +28,7 @@
 #include "device/lbvh.cuh"
 #include "device/rails.cuh"
 #include "host/accel_build.h"
+#include "walk.h"
 
 using namespace ptx;
 
@@ -39,6 +40,9 @@ struct SpecKernels {
     const void* shadow = nullptr;
     const void* shade_adj = nullptr;    // the adjoint replay's shading and shadow kernels
     const void* shadow_adj = nullptr;   // (compiled at the first ptr_backward)
+    const void* walk = nullptr;         // scenes on the one-kernel walk: these two instead
+    const void* walk_adj = nullptr;
+    bool any() const { return shade || walk; }
 };
 
 struct ptr_ctx {
@@ -58,6 +62,8 @@ struct ptr_scene {
     DevScene dev{};
     std::vector<void*> allocs;
     int has_media = 0;
+    bool has_mesh = false;   // some region is a triangle mesh or instances one
+    bool walk = false;       // rendered by the one-kernel walk
     int max_stack_depth = 0;
     int n_lights = 0, n_delta_lights = 0, env_samplable = 0;
     std::vector<ptr_material> h_materials;   // host copies for ptr_update_params / ptr_backward
@@ -88,6 +94,14 @@ struct ptr_program {
     std::vector<void*> pool_allocs;
     PathPool pool{};
     FrameParams* fp_dev = nullptr;
+    unsigned char* ctl = nullptr;   // counters, statistics, wave cursor and tickets (kCtl*)
+    // the one-kernel walk's per-path output of a wave (radiance; first-hit samples)
+    float4* walk_film = nullptr;
+    float4* walk_aov = nullptr;
+    size_t walk_cap = 0, walk_aov_cap = 0;
+    // batched renders: the device copies of the job tables
+    unsigned char* tables = nullptr;
+    size_t tables_n = 0;
     // graph cache
     cudaGraphExec_t graph = nullptr;
     const ptr_scene* graph_scene = nullptr;
@@ -193,12 +207,54 @@ struct Launcher {
         cudaLaunchKernel(kern, dim3((unsigned)g), dim3((unsigned)block), argv, smem, st);
         if (count) ++*count;
     }
+    // at most `blocks` blocks of the resident grid (a kernel with less work than the grid)
+    template <class... A>
+    void raw_upto(int blocks, const void* kern, size_t smem, A... args) const {
+        const int g = std::max(1, std::min(blocks, resident_grid(kern, block, smem, n_sm)));
+        void* argv[] = {(void*)&args...};
+        cudaLaunchKernel(kern, dim3((unsigned)g), dim3((unsigned)block), argv, smem, st);
+        if (count) ++*count;
+    }
 };
 
+// The control block: queue counts, statistics, the wave cursor and the work tickets.
+constexpr size_t kCtlCnt = 0, kCtlStats = 64, kCtlWave = 128, kCtlFetch = 192, kCtlBytes = 256;
+void bind_ctl(ptr_program* p) {
+    p->pool.cnt = (unsigned*)(p->ctl + kCtlCnt);
+    p->pool.stats = (unsigned long long*)(p->ctl + kCtlStats);
+    p->pool.wave = (long long*)(p->ctl + kCtlWave);
+    p->pool.fetch = (unsigned*)(p->ctl + kCtlFetch);
+}
+int ensure_ctl(ptr_program* p) {
+    if (!p->ctl) {
+        if (cudaMalloc(&p->ctl, kCtlBytes) != cudaSuccess) { p->ctl = nullptr; return fail(p->ctx, PTR_E_NOMEM, "control block cudaMalloc"); }
+    }
+    bind_ctl(p);
+    return PTR_OK;
+}
+// The one-kernel walk's film record: 16 bytes per path of a wave (32 more with AOVs).
+int ensure_walk(ptr_program* p, size_t cap, bool aov) {
+    if (p->walk_cap < cap) {
+        cudaFree(p->walk_film);
+        p->walk_film = nullptr;
+        p->walk_cap = 0;
+        if (cudaMalloc(&p->walk_film, cap * sizeof(float4)) != cudaSuccess) return fail(p->ctx, PTR_E_NOMEM, "walk film cudaMalloc");
+        p->walk_cap = cap;
+    }
+    if (aov && p->walk_aov_cap < cap) {
+        cudaFree(p->walk_aov);
+        p->walk_aov = nullptr;
+        p->walk_aov_cap = 0;
+        if (cudaMalloc(&p->walk_aov, cap * 2 * sizeof(float4)) != cudaSuccess) return fail(p->ctx, PTR_E_NOMEM, "AOV pool allocation failed");
+        p->walk_aov_cap = cap;
+    }
+    return PTR_OK;
+}
 void free_pool(ptr_program* p) {
     for (void* a : p->pool_allocs) cudaFree(a);
     p->pool_allocs.clear();
     p->pool = PathPool{};
+    if (p->ctl) bind_ctl(p);
     p->capacity = 0;
     if (p->graph) { cudaGraphExecDestroy(p->graph); p->graph = nullptr; }
 }
@@ -206,6 +262,7 @@ void free_pool(ptr_program* p) {
 int alloc_pool(ptr_program* p, int capacity, bool slot2, bool adj = false, bool spectral = false) {
     free_pool(p);
     ptr_ctx* ctx = p->ctx;
+    if (int r = ensure_ctl(p)) return r;
     auto get = [&](size_t bytes, void** out) -> int {
         cudaError_t e = cudaMalloc(out, bytes);
         if (e != cudaSuccess) return fail(ctx, PTR_E_NOMEM, std::string("path pool cudaMalloc: ") + cudaGetErrorString(e));
@@ -228,19 +285,13 @@ int alloc_pool(ptr_program* p, int capacity, bool slot2, bool adj = false, bool 
         (rc = get(c * 8, (void**)&q.rng)) || (rc = pair(q.hit, q.hit_i)) ||
         (rc = pair(q.sh_o, q.sh_d)) || (rc = pair(q.sh_lp, q.sh_c)) || (rc = get(c * 4, (void**)&q.q[0])) ||
         (rc = get(c * 4, (void**)&q.q[1])) || (rc = get(c * 4, (void**)&q.shq)) ||
-        (rc = get(c * 4, (void**)&q.job)) ||
-        (rc = get(64, (void**)&q.cnt)) || (rc = get(64, (void**)&q.stats)) ||
-        (rc = get(64, (void**)&q.wave)) || (rc = get(c * 4, (void**)&q.q_sorted)) ||
+        (rc = get(c * 4, (void**)&q.q_sorted)) ||
         (rc = get(c, (void**)&q.sort_key)) || (rc = get((size_t)kMaxKeys * kSortChunks * sizeof(unsigned), (void**)&q.sort_hist)) ||
-        (rc = get(4 * sizeof(unsigned), (void**)&q.fetch)) || (rc = get(c, (void**)&q.rkey)) ||
+        (rc = get(c, (void**)&q.rkey)) ||
         (rc = get(c, (void**)&q.skey)) || (rc = get(c * 4, (void**)&q.q_ray)) ||
         (rc = get(c * 4, (void**)&q.shq_s))) {
         free_pool(p);
         return rc;
-    }
-    if (cudaMemset(q.fetch, 0, 4 * sizeof(unsigned)) != cudaSuccess) {
-        free_pool(p);
-        return fail(ctx, PTR_E_CUDA, "path pool: clearing the work tickets failed");
     }
     // the second shadow slot only for programs with the per-segment equiangular site
     if (slot2 && ((rc = pair(q.sh2_o, q.sh2_d)) || (rc = pair(q.sh2_lp, q.sh2_c)) ||
@@ -464,6 +515,42 @@ void launch_replay(ptr_program* p, const ptr_scene* s, cudaStream_t st, int iter
         }
     }
     k_advance<<<1, 32, 0, st>>>(pool);
+}
+
+// ---- the one-kernel walk (k_walk) ---------------------------------------------------------
+ProgParams prog_params(const ptr_program_desc& d) {
+    ProgParams P;
+    P.max_bounces = d.max_bounces;
+    P.direct = d.direct;
+    P.rr_start = d.rr_start;
+    P.max_null = d.max_null_crossings;
+    P.rr_max_survival = d.rr_max_survival;
+    P.scattering = d.scattering;
+    P.equiangular = d.equiangular;
+    P.light_tree = d.light_tree;
+    return P;
+}
+// Whether a frame whose waves hold `paths` paths takes the one-kernel walk.  Scenes with
+// triangle meshes keep the wavefront kernels, whose traversals refill idle lanes inside a
+// query.  Spectral programs do from 2^22 paths on: their shading is several times the code of
+// an RGB program, and large waves run it denser in the wavefront's compacted queues (media
+// and spectral workload, 1024 x 1024, per-scene kernels: 16 spp 21.2 ms against 35.6 ms, 4 spp
+// 9.8 against 10.4; 512 x 512 at 4 spp 5.1 against 3.7).
+bool walk_route(const ptr_program* p, const ptr_scene* s, long long paths) {
+    return s->walk && !(p->desc.color == PTR_COLOR_SPECTRAL && paths >= (1ll << 22));
+}
+// Lockstep keeps a block's warps in the same part of an iteration, so that one pass of a
+// part's instructions through the instruction cache serves them all (the walk's code is far
+// larger than that cache: without it the media workload took 128 ms against 41 ms at 16 spp,
+// the adjoint 15.4 against 9.3).  Tracking through heterogeneous media runs loops of very
+// uneven length, whose short ones would wait there for the longest: they go without (fog room,
+// 256 x 256 x 4 spp: 24.6 ms against 42.3).
+int walk_lockstep(bool heterogeneous) { return heterogeneous ? 0 : 1; }
+
+// Launches one wave's walk: n paths, one lane each at a time.
+void launch_walk(const Launcher& L, const void* kern, size_t smem, const DevScene& S, const ProgParams& P, const FrameParams& F,
+                 const BatchTables& bt, const WalkArgs& wa, const AdjParams& adj) {
+    L.raw_upto((int)((wa.n + (unsigned)L.block - 1u) / (unsigned)L.block), kern, smem, S, P, F, bt, wa, adj);
 }
 
 // One wave of a batched render: the same kernel sequence over the concatenated job space;
@@ -1305,28 +1392,12 @@ int upload_region_bvh(ptr_ctx* ctx, ptr_scene* s, const ptr_scene_desc* d) {
     return PTR_OK;
 }
 
-// The first-hit pictures' FP64 sums (programs with AOVs), sized and cleared with the film.
-int prepare_aov_film(ptr_program* p, const ptr_frame* f, size_t npix, cudaStream_t st) {
-    ptr_ctx* ctx = p->ctx;
-    if (p->desc.aovs) {
-        if (!p->aov_sum || p->aov_n != npix) {
-            if (p->aov_sum) cudaFree(p->aov_sum);
-            p->aov_sum = nullptr;
-            if (cudaMalloc(&p->aov_sum, npix * 6 * sizeof(double)) != cudaSuccess) return fail(ctx, PTR_E_NOMEM, "AOV film allocation failed");
-            p->aov_n = npix;
-            CK(ctx, cudaMemsetAsync(p->aov_sum, 0, npix * 6 * sizeof(double), st));
-        } else if (!f->accumulate) {
-            CK(ctx, cudaMemsetAsync(p->aov_sum, 0, npix * 6 * sizeof(double), st));
-        }
-        p->pool.aov_sum = p->aov_sum;
-    }
-    return PTR_OK;
-}
-
-// Size (and clear unless accumulating) a program's FP64 film for a frame.
-int prepare_film(ptr_program* p, const ptr_frame* f, cudaStream_t st) {
+// Size a program's FP64 film for a frame.  fresh: the film pass starts every pixel from zero
+// (a new film, or a frame that does not accumulate), so nothing is cleared here.
+int prepare_film(ptr_program* p, const ptr_frame* f, bool& fresh) {
     ptr_ctx* ctx = p->ctx;
     const size_t npix = (size_t)f->width * f->height;
+    fresh = !f->accumulate;
     if (p->fw != f->width || p->fh != f->height || !p->sum) {
         if (p->sum) cudaFree(p->sum);
         if (p->sumsq) cudaFree(p->sumsq);
@@ -1339,15 +1410,15 @@ int prepare_film(ptr_program* p, const ptr_frame* f, cudaStream_t st) {
             return fail(ctx, PTR_E_NOMEM, "film allocation failed");
         p->fw = f->width;
         p->fh = f->height;
-        p->nsamples = 0.0;
-        CK(ctx, cudaMemsetAsync(p->sum, 0, npix * 3 * sizeof(double), st));
-        CK(ctx, cudaMemsetAsync(p->sumsq, 0, npix * 3 * sizeof(double), st));
-    } else if (!f->accumulate) {
-        p->nsamples = 0.0;
-        CK(ctx, cudaMemsetAsync(p->sum, 0, npix * 3 * sizeof(double), st));
-        CK(ctx, cudaMemsetAsync(p->sumsq, 0, npix * 3 * sizeof(double), st));
+        fresh = true;
     }
-    if (int rc = prepare_aov_film(p, f, npix, st)) return rc;
+    if (fresh) p->nsamples = 0.0;
+    if (p->desc.aovs && (!p->aov_sum || p->aov_n != npix)) {   // the first-hit pictures' sums beside it
+        if (p->aov_sum) cudaFree(p->aov_sum);
+        p->aov_sum = nullptr;
+        if (cudaMalloc(&p->aov_sum, npix * 6 * sizeof(double)) != cudaSuccess) return fail(ctx, PTR_E_NOMEM, "AOV film allocation failed");
+        p->aov_n = npix;
+    }
     return PTR_OK;
 }
 
@@ -1383,6 +1454,129 @@ int check_color(ptr_ctx* ctx, const ptr_program* p, const ptr_scene* s) {
     return PTR_OK;
 }
 
+FrameParams frame_params(const ptr_frame* f, long long total, int cap, bool fresh) {
+    FrameParams F{};
+    F.width = f->width;
+    F.height = f->height;
+    F.spp = f->spp;
+    F.first_sample = f->first_sample;
+    F.salt = f->reset_salt;
+    F.px_off = f->pixel_offset[0];
+    F.py_off = f->pixel_offset[1];
+    F.img_w = f->image_size[0] > 0 ? f->image_size[0] : f->width;
+    F.img_h = f->image_size[1] > 0 ? f->image_size[1] : f->height;
+    F.total = total;
+    F.capacity = cap;
+    F.cam = f->camera;
+    F.fresh = fresh ? 1 : 0;
+    return F;
+}
+
+// Sums an instrumented render's event pairs per kernel class (the stream is idle).
+void fold_profile(ptr_program* p, std::vector<ProfRec>& prof) {
+    for (int k = 0; k < PTR_PROFILE_CLASSES; ++k) { p->prof_ms[k] = 0.f; p->prof_launches[k] = 0; }
+    for (ProfRec& r : prof) {
+        float ms = 0.f;
+        cudaEventElapsedTime(&ms, r.a, r.b);
+        p->prof_ms[r.cls] += ms;
+        p->prof_launches[r.cls] += r.n;
+        cudaEventDestroy(r.a);
+        cudaEventDestroy(r.b);
+    }
+}
+
+// A frame on the one-kernel walk: per wave one walk and one film pass, launched directly (two
+// launches leave nothing for a graph to save).  An instrumented render reports the walk under
+// class 2 (shade) and the film pass under class 4.
+int render_walk(ptr_program* p, ptr_scene* s, const ptr_frame* f, const FrameParams& F, float* samples_dev) {
+    ptr_ctx* ctx = p->ctx;
+    cudaStream_t st = ctx->stream;
+    const bool profiling = (p->profile_next & PTR_PROFILE_TIMING) != 0;
+    p->profile_next = 0;
+    p->work_valid = 0;
+    p->last_scene = s;
+    if (int rc = ensure_ctl(p)) return rc;
+    if (int rc = ensure_walk(p, (size_t)F.capacity, p->desc.aovs != 0)) return rc;
+    CK(ctx, cudaMemsetAsync(p->ctl, 0, kCtlBytes, st));
+    DevScene S = s->dev;
+    S.accel = p->desc.accel;
+    S.inst_accel = p->desc.instance_accel;
+    S.work = nullptr;
+    const ProgParams P = prog_params(p->desc);
+    const void* kern = p->spec.scene_id == s->id && p->spec.walk
+                           ? p->spec.walk
+                           : ptx_host::walk_kernel(P.direct, s->has_media != 0, p->desc.color == PTR_COLOR_SPECTRAL, false, false);
+    WalkArgs wa{};
+    wa.film = p->walk_film;
+    wa.aov = p->desc.aovs ? p->walk_aov : nullptr;
+    wa.ticket = p->pool.fetch;
+    wa.stats = p->pool.stats;
+    wa.iters = wave_iterations(p, s);
+    wa.lockstep = walk_lockstep(s->dev.has_het != 0);
+    const Launcher L{tuning_of(p).block, device_sms(ctx->device), st, false};
+    std::vector<ProfRec> prof;
+    auto event = [&](int cls, bool begin) {
+        if (!profiling) return;
+        if (begin) {
+            prof.push_back(ProfRec{cls, nullptr, nullptr, 0, 1});
+            cudaEventCreate(&prof.back().a);
+            cudaEventCreate(&prof.back().b);
+        }
+        cudaEventRecord(begin ? prof.back().a : prof.back().b, st);
+    };
+    for (wa.base = 0; wa.base < F.total; wa.base += F.capacity) {
+        wa.n = (unsigned)std::min<long long>(F.capacity, F.total - wa.base);
+        event(2, true);
+        launch_walk(L, kern, 0, S, P, F, BatchTables{}, wa, AdjParams{});
+        event(2, false);
+        event(4, true);
+        L(k_film_walk, 0, F, wa, p->desc.aovs ? p->aov_sum : (double*)nullptr, p->sum, p->sumsq, samples_dev);
+        event(4, false);
+    }
+    CK(ctx, cudaGetLastError());
+    if (profiling) {
+        CK(ctx, cudaStreamSynchronize(st));
+        fold_profile(p, prof);
+    }
+    p->nsamples += (double)f->spp;
+    return PTR_OK;
+}
+
+// The adjoint on the one-kernel walk: per wave the forward walk, which leaves every path's
+// radiance and logs its first log_iters iterations, then its replay.
+int backward_walk(ptr_program* p, ptr_scene* s, const FrameParams& F, const AdjParams& adj, int iters, int log_iters) {
+    ptr_ctx* ctx = p->ctx;
+    cudaStream_t st = ctx->stream;
+    DevScene S = s->dev;
+    S.accel = p->desc.accel;
+    S.inst_accel = p->desc.instance_accel;
+    S.work = nullptr;
+    const ProgParams P = prog_params(p->desc);
+    const SpecKernels* sk = p->spec.scene_id == s->id ? &p->spec : nullptr;
+    const bool media = s->has_media != 0;
+    const void* fwd = sk && sk->walk ? sk->walk : ptx_host::walk_kernel(P.direct, media, false, false, false);
+    const void* rep = sk && sk->walk_adj ? sk->walk_adj : ptx_host::walk_kernel(P.direct, media, false, false, true);
+    const size_t smem = sizeof(double) * PTR_GRAD_SLOTS * (size_t)S.n_materials;
+    WalkArgs wa{};
+    wa.film = p->walk_film;
+    wa.stats = p->pool.stats;
+    wa.iters = iters;
+    wa.lockstep = walk_lockstep(false);   // (heterogeneous media are not differentiated)
+    wa.hit_log = log_iters > 0 ? p->hit_log : nullptr;
+    wa.hit_log_stride = F.capacity;
+    wa.hit_log_iters = log_iters;
+    const Launcher L{tuning_of(p).block, device_sms(ctx->device), st, false};
+    for (wa.base = 0; wa.base < F.total; wa.base += F.capacity) {
+        wa.n = (unsigned)std::min<long long>(F.capacity, F.total - wa.base);
+        if (wa.base > 0) CK(ctx, cudaMemsetAsync(p->pool.fetch, 0, 2 * sizeof(unsigned), st));
+        wa.ticket = p->pool.fetch;
+        launch_walk(L, fwd, 0, S, P, F, BatchTables{}, wa, AdjParams{});
+        wa.ticket = p->pool.fetch + 1;
+        launch_walk(L, rep, smem, S, P, F, BatchTables{}, wa, adj);
+    }
+    return PTR_OK;
+}
+
 int render_impl(ptr_program* p, ptr_scene* s, const ptr_frame* f, float* samples_dev) {
     ptr_ctx* ctx = p->ctx;
     if (int rc = check_color(ctx, p, s)) return rc;
@@ -1392,27 +1586,8 @@ int render_impl(ptr_program* p, ptr_scene* s, const ptr_frame* f, float* samples
     CK(ctx, cudaSetDevice(ctx->device));
     cudaStream_t st = ctx->stream;
     const size_t npix = (size_t)f->width * f->height;
-    if (p->fw != f->width || p->fh != f->height || !p->sum) {
-        if (p->sum) cudaFree(p->sum);
-        if (p->sumsq) cudaFree(p->sumsq);
-        if (p->export_buf) cudaFree(p->export_buf);
-        p->sum = p->sumsq = nullptr;
-        p->export_buf = nullptr;
-        if (cudaMalloc(&p->sum, npix * 3 * sizeof(double)) != cudaSuccess ||
-            cudaMalloc(&p->sumsq, npix * 3 * sizeof(double)) != cudaSuccess ||
-            cudaMalloc(&p->export_buf, npix * 3 * sizeof(float)) != cudaSuccess)
-            return fail(ctx, PTR_E_NOMEM, "film allocation failed");
-        p->fw = f->width;
-        p->fh = f->height;
-        p->nsamples = 0.0;
-        CK(ctx, cudaMemsetAsync(p->sum, 0, npix * 3 * sizeof(double), st));
-        CK(ctx, cudaMemsetAsync(p->sumsq, 0, npix * 3 * sizeof(double), st));
-    } else if (!f->accumulate) {
-        p->nsamples = 0.0;
-        CK(ctx, cudaMemsetAsync(p->sum, 0, npix * 3 * sizeof(double), st));
-        CK(ctx, cudaMemsetAsync(p->sumsq, 0, npix * 3 * sizeof(double), st));
-    }
-    if (int rc = prepare_aov_film(p, f, npix, st)) return rc;
+    bool fresh = true;
+    if (int rc = prepare_film(p, f, fresh)) return rc;
     const long long total = (long long)npix * f->spp;
     // capacity: whole sample passes when a pass fits the pool, else a chunk of pixels
     long long cap_max = ctx->tune.capacity > 0 ? ctx->tune.capacity : (1ll << 24);
@@ -1422,6 +1597,13 @@ int render_impl(ptr_program* p, ptr_scene* s, const ptr_frame* f, float* samples
     if ((long long)npix <= cap_max) cap = (cap_max / (long long)npix) * (long long)npix;
     else cap = cap_max;
     if (cap > total) cap = total;
+    const bool profiling = (p->profile_next & PTR_PROFILE_TIMING) != 0;
+    const bool counting = (p->profile_next & PTR_PROFILE_WORK) != 0;
+    FrameParams F = frame_params(f, total, (int)cap, fresh);
+    F.wavelengths = p->desc.wavelengths;
+    F.lambda_min = p->desc.lambda_min;
+    F.lambda_max = p->desc.lambda_max;
+    if (walk_route(p, s, cap) && !counting) return render_walk(p, s, f, F, samples_dev);
     const bool slot2 = p->desc.equiangular != 0;
     const bool spectral = p->desc.color == PTR_COLOR_SPECTRAL;
     if (p->capacity < cap || (slot2 && !p->pool.sh2_o) || (spectral && !p->pool.wl)) {
@@ -1440,32 +1622,12 @@ int render_impl(ptr_program* p, ptr_scene* s, const ptr_frame* f, float* samples
     if (!p->fp_dev) CK(ctx, cudaMalloc(&p->fp_dev, sizeof(FrameParams)));
     // The frame's parameters travel as a kernel argument into a device block: no host
     // synchronisation, and the captured graph (which reads the block) stays valid.
-    FrameParams F;
-    F.width = f->width;
-    F.height = f->height;
-    F.spp = f->spp;
-    F.first_sample = f->first_sample;
-    F.salt = f->reset_salt;
-    F.px_off = f->pixel_offset[0];
-    F.py_off = f->pixel_offset[1];
-    F.img_w = f->image_size[0] > 0 ? f->image_size[0] : f->width;
-    F.img_h = f->image_size[1] > 0 ? f->image_size[1] : f->height;
-    F.total = total;
-    F.capacity = (int)cap;
-    F.cam = f->camera;
-    F.wavelengths = p->desc.wavelengths;
-    F.lambda_min = p->desc.lambda_min;
-    F.lambda_max = p->desc.lambda_max;
     k_set_frame<<<1, 1, 0, st>>>(p->fp_dev, F);
     CK(ctx, cudaGetLastError());
-    CK(ctx, cudaMemsetAsync(p->pool.wave, 0, 64, st));
-    CK(ctx, cudaMemsetAsync(p->pool.stats, 0, 64, st));
-    CK(ctx, cudaMemsetAsync(p->pool.cnt, 0, 64, st));
+    CK(ctx, cudaMemsetAsync(p->ctl, 0, kCtlBytes, st));
     const int iters = wave_iterations(p, s);
     const long long waves = (total + cap - 1) / cap;
     const int n_sm = device_sms(ctx->device);
-    const bool profiling = (p->profile_next & PTR_PROFILE_TIMING) != 0;
-    const bool counting = (p->profile_next & PTR_PROFILE_WORK) != 0;
     p->last_scene = s;
     if (counting) {
         if (!p->work_dev) CK(ctx, cudaMalloc(&p->work_dev, 64));
@@ -1506,15 +1668,7 @@ int render_impl(ptr_program* p, ptr_scene* s, const ptr_frame* f, float* samples
         for (long long w = 0; w < waves; ++w) launch_wave(p, s, st, iters, samples_dev, n_sm, &prof);
         CK(ctx, cudaGetLastError());
         CK(ctx, cudaStreamSynchronize(st));
-        for (int k = 0; k < PTR_PROFILE_CLASSES; ++k) { p->prof_ms[k] = 0.f; p->prof_launches[k] = 0; }
-        for (ProfRec& r : prof) {
-            float ms = 0.f;
-            cudaEventElapsedTime(&ms, r.a, r.b);
-            p->prof_ms[r.cls] += ms;
-            p->prof_launches[r.cls] += r.n;
-            cudaEventDestroy(r.a);
-            cudaEventDestroy(r.b);
-        }
+        fold_profile(p, prof);
         p->profile_next = 0;
     } else {
         for (long long w = 0; w < waves; ++w) launch_wave(p, s, st, iters, samples_dev, n_sm);
@@ -1571,7 +1725,13 @@ std::string lib_dir() {
     size_t k = f.find_last_of('/');
     return k == std::string::npos ? std::string(".") : f.substr(0, k);
 }
-struct SpecModule { cudaLibrary_t lib = nullptr; const void* closest = nullptr; const void* shade = nullptr; const void* shadow = nullptr; };
+struct SpecModule {
+    cudaLibrary_t lib = nullptr;
+    const void* closest = nullptr;
+    const void* shade = nullptr;
+    const void* shadow = nullptr;
+    const void* walk = nullptr;
+};
 // The occupant census a set of kernels is compiled for: material models, light kinds,
 // environment kinds and region shapes present (bit masks), the regions in order when
 // there are at most 16 (0 otherwise), the light tree, the direct-lighting mode, media,
@@ -1581,7 +1741,10 @@ struct Census {
     int nregions = 0;
     unsigned long long shape_code = 0;
     bool tree = false, media = false, spectral = false, batch = false;
+    bool mesh = false;                 // some region is a triangle mesh or instances one
+    bool het = false;                  // some medium has a coefficient field
     bool adj = false;                  // the replay's kernels (ADJ = true) instead of the forward's
+    bool walk = false;                 // the one-kernel walk instead of the wavefront's three kernels
     int direct = 0;
 };
 Census census_of(const ptr_program* p, const ptr_scene* sc) {
@@ -1596,6 +1759,9 @@ Census census_of(const ptr_program* p, const ptr_scene* sc) {
     c.media = sc->has_media != 0;
     c.spectral = p->desc.color == PTR_COLOR_SPECTRAL;
     c.direct = p->desc.direct;
+    c.walk = sc->walk;
+    c.mesh = sc->has_mesh;
+    c.het = sc->dev.has_het != 0;
     return c;
 }
 // The union census of a job mix (the batched kernels serve every job of it): masks OR-ed,
@@ -1603,8 +1769,12 @@ Census census_of(const ptr_program* p, const ptr_scene* sc) {
 Census census_of_batch(const ptr_batch_job* jobs, int n) {
     Census c;
     c.batch = true;
+    c.walk = true;
     for (int j = 0; j < n; ++j) {
         const Census k = census_of(jobs[j].prog, jobs[j].scene);
+        c.walk = c.walk && k.walk;
+        c.mesh = c.mesh || k.mesh;
+        c.het = c.het || k.het;
         c.mats |= k.mats;
         c.lights |= k.lights;
         c.envs |= k.envs;
@@ -1620,6 +1790,8 @@ std::vector<std::string> census_options(const Census& c) {
             "-DPTR_SPEC_LIGHTS=" + std::to_string(c.lights) + "u",
             "-DPTR_SPEC_ENVS=" + std::to_string(c.envs) + "u",
             "-DPTR_SPEC_SHAPES=" + std::to_string(c.shapes) + "u",
+            std::string("-DPTR_SPEC_MESH=") + (c.mesh ? "1" : "0"),
+            std::string("-DPTR_SPEC_HET=") + (c.het ? "1" : "0"),
             "-DPTR_SPEC_NREGIONS=" + std::to_string(c.nregions),
             "-DPTR_SPEC_SHAPE_CODE=" + std::to_string(c.shape_code) + "ull",
             std::string("-DPTR_SPEC_TREE=") + (c.tree ? "1" : "0")};
@@ -1628,9 +1800,10 @@ std::string census_key(const Census& c) {
     std::string k;
     for (const auto& o : census_options(c)) k += o + "\n";
     return k + std::to_string(c.direct) + (c.media ? "m" : "-") + (c.spectral ? "s" : "-") + (c.batch ? "b" : "-") +
-           (c.adj ? "a" : "-");
+           (c.adj ? "a" : "-") + (c.walk ? "w" : "-");
 }
-// Compile (or fetch) the closest-hit, shading and shadow kernels for a census.  Modules are
+// Compile (or fetch) the census's kernels: the one-kernel walk, or the wavefront's
+// closest-hit, shading and shadow kernels.  Modules are
 // cached by census for the process, so equal scenes (and equal mixes) share one module.
 int spec_compile(ptr_ctx* ctx, const Census& c, SpecModule& out, bool& compiled) {
     compiled = false;
@@ -1670,7 +1843,16 @@ int spec_compile(ptr_ctx* ctx, const Census& c, SpecModule& out, bool& compiled)
     }
     std::string key;
     for (const auto& o : opts) key += o + "\n";
-    key += n_closest + "\n" + n_shade + "\n" + n_shadow;
+    const std::string n_walk = std::string("ptx::k_walk<") + col + ", " + std::to_string(c.direct) + ", " + md + ", " + bt + ", " + adj + ">";
+    struct Want { std::string name; const void* SpecModule::*slot; };
+    std::vector<Want> wants;
+    if (c.walk) wants.push_back({n_walk, &SpecModule::walk});
+    if (!c.walk || c.spectral) {   // large spectral frames take the wavefront (walk_route)
+        wants.push_back({n_closest, &SpecModule::closest});
+        wants.push_back({n_shade, &SpecModule::shade});
+        wants.push_back({n_shadow, &SpecModule::shadow});
+    }
+    for (const Want& wnt : wants) key += wnt.name + "\n";
     std::lock_guard<std::mutex> lk(mu);
     auto it = cache.find(key);
     if (it != cache.end()) { out = it->second; return PTR_OK; }
@@ -1682,9 +1864,7 @@ int spec_compile(ptr_ctx* ctx, const Census& c, SpecModule& out, bool& compiled)
     Nvrtc::Prog prog = nullptr;
     if (nv.create(&prog, kSource, "ptr_specialize.cu", 0, nullptr, nullptr) != 0)
         return fail(ctx, PTR_E_CUDA, "ptr_specialize: nvrtcCreateProgram failed");
-    nv.add_name(prog, n_closest.c_str());
-    nv.add_name(prog, n_shade.c_str());
-    nv.add_name(prog, n_shadow.c_str());
+    for (const Want& wnt : wants) nv.add_name(prog, wnt.name.c_str());
     std::vector<const char*> argv;
     for (const auto& o : opts) argv.push_back(o.c_str());
     const int rc = nv.compile(prog, (int)argv.size(), argv.data());
@@ -1700,24 +1880,22 @@ int spec_compile(ptr_ctx* ctx, const Census& c, SpecModule& out, bool& compiled)
     nv.cubin_size(prog, &nbin);
     std::vector<char> bin(nbin);
     nv.cubin(prog, bin.data());
-    const char *l_closest = nullptr, *l_shade = nullptr, *l_shadow = nullptr;
-    nv.lowered(prog, n_closest.c_str(), &l_closest);
-    nv.lowered(prog, n_shade.c_str(), &l_shade);
-    nv.lowered(prog, n_shadow.c_str(), &l_shadow);
-    const std::string s_closest = l_closest ? l_closest : "", s_shade = l_shade ? l_shade : "",
-                      s_shadow = l_shadow ? l_shadow : "";
+    std::vector<std::string> lowered;
+    for (const Want& wnt : wants) {
+        const char* l = nullptr;
+        nv.lowered(prog, wnt.name.c_str(), &l);
+        lowered.push_back(l ? l : "");
+    }
     nv.destroy(&prog);
     SpecModule m;
     cudaError_t e = cudaLibraryLoadData(&m.lib, bin.data(), nullptr, nullptr, 0, nullptr, nullptr, 0);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "ptr_specialize: cudaLibraryLoadData");
-    cudaKernel_t kc = nullptr, ks = nullptr, kw = nullptr;
-    if ((e = cudaLibraryGetKernel(&kc, m.lib, s_closest.c_str())) != cudaSuccess ||
-        (e = cudaLibraryGetKernel(&ks, m.lib, s_shade.c_str())) != cudaSuccess ||
-        (e = cudaLibraryGetKernel(&kw, m.lib, s_shadow.c_str())) != cudaSuccess)
-        return cuda_fail(ctx, e, "ptr_specialize: cudaLibraryGetKernel");
-    m.closest = (const void*)kc;
-    m.shade = (const void*)ks;
-    m.shadow = (const void*)kw;
+    for (size_t k = 0; k < wants.size(); ++k) {
+        cudaKernel_t kern = nullptr;
+        if ((e = cudaLibraryGetKernel(&kern, m.lib, lowered[k].c_str())) != cudaSuccess)
+            return cuda_fail(ctx, e, "ptr_specialize: cudaLibraryGetKernel");
+        m.*(wants[k].slot) = (const void*)kern;
+    }
     cache[key] = m;
     out = m;
     compiled = true;
@@ -1983,6 +2161,21 @@ static int upload_scene(ptr_ctx* ctx, const ptr_scene_desc* d, const ptr_rails* 
     }
     rc = upload_accels(ctx, s, d, rails);
     if (!rc) rc = upload_region_bvh(ctx, s, d);
+    if (!rc && d->n_regions > 0) {   // the scans' per-region values
+        std::vector<float4> scan((size_t)d->n_regions, make_float4(0.f, 0.f, 0.f, 0.f));
+        for (int i = 0; i < d->n_regions; ++i) {
+            const float* q = d->regions[i].p;
+            if (d->regions[i].shape == PTR_SHAPE_SPHERE) {
+                scan[i] = make_float4(q[0], q[1], q[2], q[3] * q[3] * (1.0f + kScanPad));
+            } else if (d->regions[i].shape == PTR_SHAPE_QUAD) {
+                // binary32 products in dot()'s order, as the kernels would round them
+                auto dot3 = [](const float* a, const float* b) { return a[0] * b[0] + a[1] * b[1] + a[2] * b[2]; };
+                const float e11 = dot3(q + 3, q + 3), e22 = dot3(q + 6, q + 6), e12 = dot3(q + 3, q + 6);
+                scan[i] = make_float4(e11, e22, e12, e11 * e22 - e12 * e12);
+            }
+        }
+        rc = dev_copy(ctx, s->allocs, scan.data(), scan.size(), &S.region_scan);
+    }
     if (!rc && !S.region_bvh && d->n_regions > 0) {   // the scan's same-shape runs
         std::vector<int4> runs;
         for (int i = 0; i < d->n_regions; ++i) {
@@ -2003,6 +2196,15 @@ static int upload_scene(ptr_ctx* ctx, const ptr_scene_desc* d, const ptr_rails* 
                 flat = i;
         }
         s->dev.flat_region = (accel_regions == 1 && !s->dev.region_bvh) ? flat : -1;
+        // scenes whose queries are short run the one-kernel walk: analytic regions and
+        // instanced spheres; scenes with triangle meshes keep the wavefront kernels, whose
+        // traversals refill idle lanes inside a query
+        for (int i = 0; i < d->n_regions; ++i) {
+            const ptr_region& g = d->regions[i];
+            s->has_mesh |= g.shape == PTR_SHAPE_MESH ||
+                           (g.shape == PTR_SHAPE_INSTANCES && d->batches[g.ref].prototype_shape == PTR_SHAPE_MESH);
+        }
+        s->walk = !s->has_mesh;
         // occupant census for ptr_specialize
         static std::atomic<uint64_t> next_id{1};
         s->id = next_id++;
@@ -2078,6 +2280,10 @@ int ptr_free_program(ptr_program* p) {
     if (p->aov_sum) cudaFree(p->aov_sum);
     if (p->export_buf) cudaFree(p->export_buf);
     if (p->fp_dev) cudaFree(p->fp_dev);
+    cudaFree(p->ctl);
+    cudaFree(p->walk_film);
+    cudaFree(p->walk_aov);
+    cudaFree(p->tables);
     if (p->work_dev) cudaFree(p->work_dev);
     if (p->adj_dl) cudaFree(p->adj_dl);
     if (p->adj_grads) cudaFree(p->adj_grads);
@@ -2096,7 +2302,7 @@ int ptr_render_batch(ptr_ctx* ctx, const ptr_batch_job* jobs, int n_jobs) {
     CK(ctx, cudaSetDevice(ctx->device));
     cudaStream_t st = ctx->stream;
     const int direct = jobs[0].prog ? jobs[0].prog->desc.direct : -1;
-    bool media = false, equi = false;
+    bool media = false, equi = false, het = false, walk = true;
     for (int j = 0; j < n_jobs; ++j) {
         const ptr_batch_job& J = jobs[j];
         if (!J.prog || !J.scene || J.prog->ctx != ctx || J.scene->ctx != ctx)
@@ -2106,6 +2312,7 @@ int ptr_render_batch(ptr_ctx* ctx, const ptr_batch_job* jobs, int n_jobs) {
         if (J.frame.width <= 0 || J.frame.height <= 0 || J.frame.spp <= 0)
             return fail(ctx, PTR_E_INVALID, "ptr_render_batch: job " + std::to_string(j) + " has an empty frame");
         if (J.scene->has_media) media = true;
+        if (J.scene->dev.has_het) het = true;
         if (J.prog->desc.color != PTR_COLOR_RGB)
             return fail(ctx, PTR_E_UNSUPPORTED, "ptr_render_batch: spectral programs render one per launch (ptr_render)");
         if (int rc = check_equiangular(ctx, J.prog, J.scene)) return rc;
@@ -2129,36 +2336,18 @@ int ptr_render_batch(ptr_ctx* ctx, const ptr_batch_job* jobs, int n_jobs) {
     for (int j = 0; j < n_jobs; ++j) {
         const ptr_batch_job& J = jobs[j];
         ptr_program* p = J.prog;
-        int rc = prepare_film(p, &J.frame, st);
+        bool fresh = true;
+        int rc = prepare_film(p, &J.frame, fresh);
         if (rc) return rc;
+        walk = walk && J.scene->walk;
         scenes[j] = J.scene->dev;
         scenes[j].accel = p->desc.accel;
         scenes[j].inst_accel = p->desc.instance_accel;
         scenes[j].work = nullptr;
-        ProgParams& P = progs[j];
-        P.max_bounces = p->desc.max_bounces;
-        P.direct = p->desc.direct;
-        P.rr_start = p->desc.rr_start;
-        P.max_null = p->desc.max_null_crossings;
-        P.rr_max_survival = p->desc.rr_max_survival;
-        P.scattering = p->desc.scattering;
-        P.equiangular = p->desc.equiangular;
-        P.light_tree = p->desc.light_tree;
-        if (P.equiangular) equi = true;
+        progs[j] = prog_params(p->desc);
+        if (progs[j].equiangular) equi = true;
         const long long total_j = (long long)J.frame.width * J.frame.height * J.frame.spp;
-        FrameParams& F = bjobs[j].frame;
-        F.width = J.frame.width;
-        F.height = J.frame.height;
-        F.spp = J.frame.spp;
-        F.first_sample = J.frame.first_sample;
-        F.salt = J.frame.reset_salt;
-        F.px_off = J.frame.pixel_offset[0];
-        F.py_off = J.frame.pixel_offset[1];
-        F.img_w = J.frame.image_size[0] > 0 ? J.frame.image_size[0] : J.frame.width;
-        F.img_h = J.frame.image_size[1] > 0 ? J.frame.image_size[1] : J.frame.height;
-        F.total = total_j;
-        F.capacity = 0;
-        F.cam = J.frame.camera;
+        bjobs[j].frame = frame_params(&J.frame, total_j, 0, fresh);
         bjobs[j].sum = p->sum;
         bjobs[j].sumsq = p->sumsq;
         offsets[j + 1] = offsets[j] + total_j;
@@ -2174,23 +2363,34 @@ int ptr_render_batch(ptr_ctx* ctx, const ptr_batch_job* jobs, int n_jobs) {
     long long cap_max = ctx->tune.capacity > 0 ? ctx->tune.capacity : (1ll << 24);
     if (const char* env = std::getenv("PTR_CAPACITY")) cap_max = std::max(1024ll, (long long)std::atoll(env));
     long long cap = std::min(total, cap_max);
-    if (bp->capacity < cap || (equi && !bp->pool.sh2_o)) {
+    if (walk) {
+        if (int rc = ensure_ctl(bp)) return rc;
+        if (int rc = ensure_walk(bp, (size_t)cap, false)) return rc;
+    } else if (bp->capacity < cap || (equi && !bp->pool.sh2_o)) {
         int rc = alloc_pool(bp, (int)std::max<long long>(cap, bp->capacity), equi || bp->pool.sh2_o);
         if (rc) return rc;
     }
-    // device tables (a few KB; refreshed every call)
-    DevScene* d_scenes = nullptr;
-    ProgParams* d_progs = nullptr;
-    BatchJob* d_jobs = nullptr;
-    long long* d_off = nullptr;
-    if (cudaMalloc(&d_scenes, sizeof(DevScene) * n_jobs) != cudaSuccess || cudaMalloc(&d_progs, sizeof(ProgParams) * n_jobs) != cudaSuccess ||
-        cudaMalloc(&d_jobs, sizeof(BatchJob) * n_jobs) != cudaSuccess || cudaMalloc(&d_off, sizeof(long long) * (n_jobs + 1)) != cudaSuccess) {
-        cudaFree(d_scenes); cudaFree(d_progs); cudaFree(d_jobs); cudaFree(d_off);
-        return fail(ctx, PTR_E_NOMEM, "ptr_render_batch: tables");
+    // device tables (a few KB; refreshed every call from one host image, one copy)
+    const size_t o_progs = sizeof(DevScene) * n_jobs, o_jobs = o_progs + (sizeof(ProgParams) * n_jobs + 15) / 16 * 16,
+                 o_off = o_jobs + sizeof(BatchJob) * n_jobs, n_tables = o_off + sizeof(long long) * (n_jobs + 1);
+    static_assert(sizeof(DevScene) % 16 == 0 || alignof(DevScene) <= 8, "table sections");
+    if (bp->tables_n < n_tables) {
+        cudaFree(bp->tables);
+        bp->tables = nullptr;
+        bp->tables_n = 0;
+        if (cudaMalloc(&bp->tables, n_tables) != cudaSuccess) return fail(ctx, PTR_E_NOMEM, "ptr_render_batch: tables");
+        bp->tables_n = n_tables;
     }
+    std::vector<unsigned char> image(n_tables);
+    std::memcpy(image.data(), scenes.data(), o_progs);
+    std::memcpy(image.data() + o_progs, progs.data(), sizeof(ProgParams) * n_jobs);
+    std::memcpy(image.data() + o_jobs, bjobs.data(), sizeof(BatchJob) * n_jobs);
+    std::memcpy(image.data() + o_off, offsets.data(), sizeof(long long) * (n_jobs + 1));
+    const DevScene* d_scenes = (const DevScene*)bp->tables;
+    const ProgParams* d_progs = (const ProgParams*)(bp->tables + o_progs);
+    const BatchJob* d_jobs = (const BatchJob*)(bp->tables + o_jobs);
+    const long long* d_off = (const long long*)(bp->tables + o_off);
     int rc = PTR_OK;
-    cudaGraph_t g = nullptr;
-    cudaGraphExec_t ge = nullptr;
     BatchTables bt{};
     bt.scenes = d_scenes;
     bt.progs = d_progs;
@@ -2208,16 +2408,45 @@ int ptr_render_batch(ptr_ctx* ctx, const ptr_batch_job* jobs, int n_jobs) {
         for (long long k = j; k < n_jobs && offsets[k] < hi; ++k) wave_iters[(size_t)w] = std::max(wave_iters[(size_t)w], job_iters[(size_t)k]);
     }
     const int n_sm = device_sms(ctx->device);
-    cudaError_t e = cudaMemcpyAsync(d_scenes, scenes.data(), sizeof(DevScene) * n_jobs, cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(d_progs, progs.data(), sizeof(ProgParams) * n_jobs, cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(d_jobs, bjobs.data(), sizeof(BatchJob) * n_jobs, cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(d_off, offsets.data(), sizeof(long long) * (n_jobs + 1), cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(bp->pool.wave, 0, 64, st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(bp->pool.stats, 0, 64, st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(bp->pool.cnt, 0, 64, st);
+    cudaError_t e = cudaMemcpyAsync(bp->tables, image.data(), n_tables, cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess) e = cudaMemsetAsync(bp->ctl, 0, kCtlBytes, st);
     const bool profiling = (bp->profile_next & PTR_PROFILE_TIMING) != 0;
     bp->profile_next = 0;
-    if (profiling) {
+    if (walk) {
+        // per wave one walk over its jobs' paths and one film pass; an instrumented render
+        // reports them under classes 2 and 4
+        std::vector<ProfRec> prof;
+        auto event = [&](int cls, bool begin) {
+            if (!profiling) return;
+            if (begin) {
+                prof.push_back(ProfRec{cls, nullptr, nullptr, 0, 1});
+                cudaEventCreate(&prof.back().a);
+                cudaEventCreate(&prof.back().b);
+            }
+            cudaEventRecord(begin ? prof.back().a : prof.back().b, st);
+        };
+        const void* kern = sk && sk->walk ? sk->walk : ptx_host::walk_kernel(direct, media, false, true, false);
+        const Launcher L{ctx->tune.block, n_sm, st, false};
+        WalkArgs wa{};
+        wa.film = bp->walk_film;
+        wa.ticket = bp->pool.fetch;
+        wa.stats = bp->pool.stats;
+        wa.lockstep = walk_lockstep(het);
+        for (long long w = 0; e == cudaSuccess && w < waves; ++w) {
+            wa.base = w * cap;
+            wa.n = (unsigned)std::min(cap, total - wa.base);
+            wa.iters = wave_iters[(size_t)w];
+            event(2, true);
+            launch_walk(L, kern, 0, jobs[0].scene->dev, ProgParams{}, FrameParams{}, bt, wa, AdjParams{});
+            event(2, false);
+            event(4, true);
+            L(k_film_batch_walk, 0, bt, wa);
+            event(4, false);
+            e = cudaGetLastError();
+        }
+        if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+        if (profiling && e == cudaSuccess) fold_profile(bp, prof);
+    } else if (profiling) {
         // instrumented: plain launches with events around each (no graph)
         std::vector<ProfRec> prof;
         prof.reserve((size_t)waves * (iters * 5 + 2));
@@ -2226,15 +2455,7 @@ int ptr_render_batch(ptr_ctx* ctx, const ptr_batch_job* jobs, int n_jobs) {
             e = cudaGetLastError();
         }
         if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-        for (int k = 0; k < PTR_PROFILE_CLASSES; ++k) { bp->prof_ms[k] = 0.0f; bp->prof_launches[k] = 0; }
-        for (ProfRec& pr : prof) {
-            float ms = 0.0f;
-            if (e == cudaSuccess) cudaEventElapsedTime(&ms, pr.a, pr.b);
-            bp->prof_ms[pr.cls] += ms;
-            bp->prof_launches[pr.cls] += pr.n;
-            cudaEventDestroy(pr.a);
-            cudaEventDestroy(pr.b);
-        }
+        if (e == cudaSuccess) fold_profile(bp, prof);
     } else {
         // occupancy queries outside capture, then one captured wave per iteration count the
         // waves need
@@ -2264,9 +2485,6 @@ int ptr_render_batch(ptr_ctx* ctx, const ptr_batch_job* jobs, int n_jobs) {
         }
     }
     if (e != cudaSuccess) rc = cuda_fail(ctx, e, "ptr_render_batch");
-    if (ge) cudaGraphExecDestroy(ge);
-    if (g) cudaGraphDestroy(g);
-    cudaFree(d_scenes); cudaFree(d_progs); cudaFree(d_jobs); cudaFree(d_off);
     if (rc) return rc;
     for (int j = 0; j < n_jobs; ++j) jobs[j].prog->nsamples += (double)jobs[j].frame.spp;
     bp->last_scene = nullptr;
@@ -2377,11 +2595,16 @@ int ptr_backward(ptr_program* p, ptr_scene* s, const ptr_frame* f, const float* 
     if (const char* env = std::getenv("PTR_CAPACITY")) cap_max = std::max(1024ll, (long long)std::atoll(env));
     long long cap = (long long)npix <= cap_max ? (cap_max / (long long)npix) * (long long)npix : cap_max;
     if (cap > total) cap = total;
-    if (p->capacity < cap || !p->pool.l_rem) {
-        int rc = alloc_pool(p, (int)std::max<long long>(cap, p->capacity), p->pool.sh2_o.p != nullptr, true);
-        if (rc) return rc;
+    if (s->walk) {
+        if (int rc = ensure_ctl(p)) return rc;
+        if (int rc = ensure_walk(p, (size_t)cap, false)) return rc;
+    } else {
+        if (p->capacity < cap || !p->pool.l_rem) {
+            int rc = alloc_pool(p, (int)std::max<long long>(cap, p->capacity), p->pool.sh2_o.p != nullptr, true);
+            if (rc) return rc;
+        }
+        if (!p->fp_dev) CK(ctx, cudaMalloc(&p->fp_dev, sizeof(FrameParams)));
     }
-    if (!p->fp_dev) CK(ctx, cudaMalloc(&p->fp_dev, sizeof(FrameParams)));
     if (p->adj_dl_n < npix * 3) {
         if (p->adj_dl) cudaFree(p->adj_dl);
         p->adj_dl = nullptr;
@@ -2395,27 +2618,14 @@ int ptr_backward(ptr_program* p, ptr_scene* s, const ptr_frame* f, const float* 
         if (cudaMalloc(&p->adj_grads, ng * sizeof(double)) != cudaSuccess) return fail(ctx, PTR_E_NOMEM, "ptr_backward: gradients");
         p->adj_grads_n = ng;
     }
-    // the graph of a previous ptr_render reads the same pool; it is re-captured on demand
-    FrameParams F;
-    F.width = f->width;
-    F.height = f->height;
-    F.spp = f->spp;
-    F.first_sample = f->first_sample;
-    F.salt = f->reset_salt;
-    F.px_off = f->pixel_offset[0];
-    F.py_off = f->pixel_offset[1];
-    F.img_w = f->image_size[0] > 0 ? f->image_size[0] : f->width;
-    F.img_h = f->image_size[1] > 0 ? f->image_size[1] : f->height;
-    F.total = total;
-    F.capacity = (int)cap;
-    F.cam = f->camera;
-    k_set_frame<<<1, 1, 0, st>>>(p->fp_dev, F);
-    CK(ctx, cudaGetLastError());
+    const FrameParams F = frame_params(f, total, (int)cap, true);
+    if (!s->walk) {
+        k_set_frame<<<1, 1, 0, st>>>(p->fp_dev, F);
+        CK(ctx, cudaGetLastError());
+    }
     CK(ctx, cudaMemcpyAsync(p->adj_dl, dl_dimage, npix * 3 * sizeof(float), cudaMemcpyHostToDevice, st));
     CK(ctx, cudaMemsetAsync(p->adj_grads, 0, ng * sizeof(double), st));
-    CK(ctx, cudaMemsetAsync(p->pool.wave, 0, 64, st));
-    CK(ctx, cudaMemsetAsync(p->pool.stats, 0, 64, st));
-    CK(ctx, cudaMemsetAsync(p->pool.cnt, 0, 64, st));
+    CK(ctx, cudaMemsetAsync(p->ctl, 0, kCtlBytes, st));
     AdjParams adj;
     adj.dl_image = p->adj_dl;
     adj.inv_spp = 1.0f / (float)f->spp;
@@ -2424,7 +2634,7 @@ int ptr_backward(ptr_program* p, ptr_scene* s, const ptr_frame* f, const float* 
     const long long waves = (total + cap - 1) / cap;
     const int n_sm = device_sms(ctx->device);
     // a specialised program: the replay's kernels for the same census (NVRTC, once)
-    if (p->spec.scene_id == s->id && p->spec.shade && !p->spec.shade_adj) {
+    if (p->spec.scene_id == s->id && p->spec.any() && !p->spec.shade_adj && !p->spec.walk_adj) {
         Census c = census_of(p, s);
         c.adj = true;
         SpecModule m;
@@ -2432,11 +2642,13 @@ int ptr_backward(ptr_program* p, ptr_scene* s, const ptr_frame* f, const float* 
         if (int rc = spec_compile(ctx, c, m, compiled)) return rc;
         p->spec.shade_adj = m.shade;
         p->spec.shadow_adj = m.shadow;
+        p->spec.walk_adj = m.walk;
     }
     // the forward walk logs its closest hits and slot-0 shadow queries for the replay, as many
     // walk iterations as 4 GiB holds (64 bytes per path slot and iteration; PTR_HIT_LOG_BYTES
     // overrides the bound); later iterations are walked again
-    const long long per_iter = 64ll * p->capacity;
+    const long long log_stride = s->walk ? cap : p->capacity;
+    const long long per_iter = 64ll * log_stride;
     long long log_budget = 4ll << 30;
     if (const char* env = std::getenv("PTR_HIT_LOG_BYTES")) log_budget = std::max(0ll, (long long)std::atoll(env));
     int log_iters = (int)std::min<long long>(iters, log_budget / std::max<long long>(per_iter, 1));
@@ -2447,6 +2659,9 @@ int ptr_backward(ptr_program* p, ptr_scene* s, const ptr_frame* f, const float* 
         if (cudaMalloc(&p->hit_log, (size_t)(per_iter * log_iters)) == cudaSuccess) p->hit_log_bytes = (size_t)(per_iter * log_iters);
         else { cudaGetLastError(); log_iters = 0; }   // no log: the replay walks every query
     }
+    if (s->walk) {
+        if (int rc = backward_walk(p, s, F, adj, iters, log_iters)) return rc;
+    } else {
     const int saved_profile = p->profile_next;
     p->profile_next = 0;
     p->pool.hit_log = log_iters > 0 ? p->hit_log : nullptr;
@@ -2462,6 +2677,7 @@ int ptr_backward(ptr_program* p, ptr_scene* s, const ptr_frame* f, const float* 
     p->pool.hit_log_iters = 0;
     p->pool.hit_log_mode = 0;
     p->profile_next = saved_profile;
+    }
     CK(ctx, cudaGetLastError());
     CK(ctx, cudaMemcpyAsync(grads, p->adj_grads, ng * sizeof(double), cudaMemcpyDeviceToHost, st));
     CK(ctx, cudaStreamSynchronize(st));
@@ -2520,6 +2736,7 @@ int ptr_specialize(ptr_program* p, ptr_scene* s, double* seconds_out) {
     p->spec.closest = m.closest;
     p->spec.shade = m.shade;
     p->spec.shadow = m.shadow;
+    p->spec.walk = m.walk;
     if (seconds_out && compiled) *seconds_out = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
     return PTR_OK;
 }
@@ -2544,6 +2761,7 @@ int ptr_specialize_batch(ptr_ctx* ctx, const ptr_batch_job* jobs, int n_jobs, do
     k.closest = m.closest;
     k.shade = m.shade;
     k.shadow = m.shadow;
+    k.walk = m.walk;
     ctx->batch_spec[census_key(c)] = k;
     if (seconds_out && compiled) *seconds_out = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
     return PTR_OK;
@@ -2816,10 +3034,6 @@ extern "C" int ptr_render_noalloc(const ptr_scene_desc* d, const ptr_program_des
     // the previous call's counters, statistics and wave cursor must not leak in
     if (cudaMemsetAsync(base, 0, kNaFrame, st) != cudaSuccess) return PTR_E_CUDA;
     const size_t npix = (size_t)f->width * f->height;
-    if (!f->accumulate) {
-        if (cudaMemsetAsync(sum_dev, 0, npix * 3 * sizeof(double), st) != cudaSuccess) return PTR_E_CUDA;
-        if (cudaMemsetAsync(sumsq_dev, 0, npix * 3 * sizeof(double), st) != cudaSuccess) return PTR_E_CUDA;
-    }
     DevScene S{};
     S.regions = (const ptr_region*)(base + kNaRegions);
     S.materials = (const ptr_material*)(base + kNaMaterials);
@@ -2845,19 +3059,7 @@ extern "C" int ptr_render_noalloc(const ptr_scene_desc* d, const ptr_program_des
     long long cap = (long long)npix <= kNoAllocMaxPaths ? (kNoAllocMaxPaths / (long long)npix) * (long long)npix
                                                         : (long long)kNoAllocMaxPaths;
     if (cap > total) cap = total;
-    FrameParams F;
-    F.width = f->width;
-    F.height = f->height;
-    F.spp = f->spp;
-    F.first_sample = f->first_sample;
-    F.salt = f->reset_salt;
-    F.px_off = f->pixel_offset[0];
-    F.py_off = f->pixel_offset[1];
-    F.img_w = f->image_size[0] > 0 ? f->image_size[0] : f->width;
-    F.img_h = f->image_size[1] > 0 ? f->image_size[1] : f->height;
-    F.total = total;
-    F.capacity = (int)cap;
-    F.cam = f->camera;
+    const FrameParams F = frame_params(f, total, (int)cap, !f->accumulate);
     FrameParams* fp = (FrameParams*)(base + kNaFrame);
     k_set_frame<<<1, 1, 0, st>>>(fp, F);
 
