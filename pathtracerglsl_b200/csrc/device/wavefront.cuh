@@ -111,7 +111,8 @@ struct PathPool {
     // 2 replay) are set per launch.
     float4* hit_log;
     long long hit_log_stride;
-    int hit_log_iters, hit_log_mode, iter, pad_log;
+    int hit_log_iters, hit_log_mode, iter;
+    int lockstep;      // k_shade: a block's warps run each part of an iteration together
 };
 
 constexpr int kRayBuckets = 64;   // ray_key values
@@ -145,6 +146,26 @@ struct QueueCursor {
         k += stride;
         out = k;
         return k < ((n + 31u) & ~31u);
+    }
+};
+
+// The same cursor with the option of a block's warps starting every round together (lockstep:
+// uniform over the grid; needs the ticket counter).
+struct ShadeCursor {
+    QueueCursor warp;
+    bool lockstep;
+    __device__ __forceinline__ ShadeCursor(unsigned n, unsigned* t, bool lock) : warp(n, t), lockstep(lock && t) {}
+    __device__ __forceinline__ bool next(unsigned& out) {
+        if (!lockstep) return warp.next(out);
+        __shared__ unsigned base;
+        __syncthreads();
+        if (threadIdx.x == 0) base = atomicAdd(warp.ticket, blockDim.x);
+        __syncthreads();
+        out = base + threadIdx.x;
+        return base < warp.n;
+    }
+    __device__ __forceinline__ void phase() const {
+        if (lockstep) __syncthreads();
     }
 };
 
@@ -1416,14 +1437,15 @@ __global__ void __launch_bounds__(256, PTR_SHADE_MIN_BLOCKS) k_shade(DevScene S0
     int* qout = pool.q[in ^ 1];
     if (blockIdx.x == 0 && threadIdx.x == 0 && pool.fetch) pool.fetch[0] = 0u;   // the next k_closest's ticket
     const WaveJobs wj = BATCH ? WaveJobs(pool, bt) : WaveJobs{};
-    QueueCursor cur(n, pool.fetch ? pool.fetch + 3 : nullptr);
+    ShadeCursor cur(n, pool.fetch ? pool.fetch + 3 : nullptr, pool.lockstep != 0);
     unsigned k;
     while (cur.next(k)) {
         bool alive = false, shadow = false, shadow2 = false;
         int i = -1;
         unsigned rk = 0u, sk = 0u;   // ray-coherence keys of the spawned ray / shadow query
-        if (k < n) {
-            i = q[k];
+        const bool live = k < n;
+        if (live || cur.lockstep) {   // a lane past the end reads the last path and stores nothing
+            i = q[live ? k : n - 1u];
             const int job = BATCH ? wj.of(bt, i) : 0;
             const DevScene& S = BATCH ? bt.scenes[job] : S0;
             const ProgParams& P = BATCH ? bt.progs[job] : P0;
@@ -1461,7 +1483,7 @@ __global__ void __launch_bounds__(256, PTR_SHADE_MIN_BLOCKS) k_shade(DevScene S0
             hr.t = hf.x; hr.u = hf.y; hr.v = hf.z;
             hr.region = hi.x; hr.element = hi.y; hr.prim = hi.z;
             PoolSink<Col> sink(pool, i);
-            alive = walk_iteration<Col, DIRECT, MEDIA, ADJ>(S, P, ws, hr, sink, ga, sh_mat, sg, true, [] {});
+            alive = walk_iteration<Col, DIRECT, MEDIA, ADJ>(S, P, ws, hr, sink, ga, sh_mat, sg, live, [&] { cur.phase(); });
             shadow = sink.shadow;
             shadow2 = sink.shadow2;
             if (pool.ray_sort) {
@@ -1471,10 +1493,12 @@ __global__ void __launch_bounds__(256, PTR_SHADE_MIN_BLOCKS) k_shade(DevScene S0
                     sk = ray_key(S, xyz(so), xyz(sd));
                 }
             }
-            pool.rad[i] = col_st(ws.rad, 0.0f);
-            pool.thr[i] = col_st(ws.thr, 0.0f);   // with rad: the whole record, for a dying path too
+            if (live) {
+                pool.rad[i] = col_st(ws.rad, 0.0f);
+                pool.thr[i] = col_st(ws.thr, 0.0f);   // with rad: the whole record, for a dying path too
+            }
             if constexpr (ADJ) {
-                pool.l_rem[i] = f4(ws.lrem, 0.0f);
+                if (live) pool.l_rem[i] = f4(ws.lrem, 0.0f);
                 if (shadow) {
                     pool.sh_g[i] = f4(sg.dnee, sg.dw);
                     pool.sh_gm[i] = sh_mat | (sg.kind << 16);

@@ -350,6 +350,25 @@ void launch_ray_sort(const Launcher& L, const PathPool& pool, int in, bool shado
 }
 const ptr_tuning& tuning_of(const ptr_program* p) { return p->ctx ? p->ctx->tune : kDefaultTuning; }
 
+ProgParams prog_params(const ptr_program_desc& d) {
+    ProgParams P;
+    P.max_bounces = d.max_bounces;
+    P.direct = d.direct;
+    P.rr_start = d.rr_start;
+    P.max_null = d.max_null_crossings;
+    P.rr_max_survival = d.rr_max_survival;
+    P.scattering = d.scattering;
+    P.equiangular = d.equiangular;
+    P.light_tree = d.light_tree;
+    return P;
+}
+// Whether k_shade runs in lockstep (PathPool::lockstep).  The media arms make its code several
+// times the instruction cache: the media and spectral workload at 1024 x 1024 x 16 took 25.6 ms
+// without and 22.1 with, fog lit by 256 lamps at 512 x 384 x 8 30.9 and 23.3.  Without media
+// the barriers cost what they save (mesh workload 82.9 to 87.7 ms over two runs), and tracking
+// loops through heterogeneous media are too uneven to wait for one another.
+int shade_lockstep(bool media, bool heterogeneous) { return media && !heterogeneous ? 1 : 0; }
+
 // Event pairs around each launch of an instrumented render (kernel class, start, end).
 struct ProfRec { int cls; cudaEvent_t a, b; int n0, n; };   // n: kernels launched in the region
 
@@ -377,20 +396,13 @@ void launch_wave_t(ptr_program* p, const ptr_scene* s, cudaStream_t st, int iter
         r->n = n_launched - r->n0;
     };
     const DevScene& S = Sp;
-    ProgParams P;
-    P.max_bounces = p->desc.max_bounces;
-    P.direct = p->desc.direct;
-    P.rr_start = p->desc.rr_start;
-    P.max_null = p->desc.max_null_crossings;
-    P.rr_max_survival = p->desc.rr_max_survival;
-    P.scattering = p->desc.scattering;
-    P.equiangular = p->desc.equiangular;
-    P.light_tree = p->desc.light_tree;
+    const ProgParams P = prog_params(p->desc);
     const int block = tuning_of(p).block;
     const Launcher L{block, n_sm, st, dry, &n_launched};
     PathPool pool = p->pool;
     pool.sort_buckets = tuning_of(p).sort_buckets;
     pool.ray_sort = tuning_of(p).ray_sort;
+    pool.lockstep = shade_lockstep(s->has_media != 0, S.has_het != 0);
     ProfRec* r = mark(0);
     const BatchTables nob{};
     // this scene's compiled kernels (ptr_specialize); the counting pass keeps the generic ones
@@ -472,16 +484,10 @@ void launch_replay(ptr_program* p, const ptr_scene* s, cudaStream_t st, int iter
     S.accel = p->desc.accel;
     S.inst_accel = p->desc.instance_accel;
     S.work = nullptr;
-    const PathPool& pool = p->pool;
-    ProgParams P;
-    P.max_bounces = p->desc.max_bounces;
-    P.direct = p->desc.direct;
-    P.rr_start = p->desc.rr_start;
-    P.max_null = p->desc.max_null_crossings;
-    P.rr_max_survival = p->desc.rr_max_survival;
-    P.scattering = p->desc.scattering;
+    PathPool pool = p->pool;
+    pool.lockstep = shade_lockstep(s->has_media != 0, S.has_het != 0);
+    ProgParams P = prog_params(p->desc);
     P.equiangular = 0;
-    P.light_tree = p->desc.light_tree;
     const int block = tuning_of(p).block;
     const Launcher L{block, n_sm, st, false};
     const size_t smem = sizeof(double) * PTR_GRAD_SLOTS * (size_t)S.n_materials;
@@ -518,18 +524,6 @@ void launch_replay(ptr_program* p, const ptr_scene* s, cudaStream_t st, int iter
 }
 
 // ---- the one-kernel walk (k_walk) ---------------------------------------------------------
-ProgParams prog_params(const ptr_program_desc& d) {
-    ProgParams P;
-    P.max_bounces = d.max_bounces;
-    P.direct = d.direct;
-    P.rr_start = d.rr_start;
-    P.max_null = d.max_null_crossings;
-    P.rr_max_survival = d.rr_max_survival;
-    P.scattering = d.scattering;
-    P.equiangular = d.equiangular;
-    P.light_tree = d.light_tree;
-    return P;
-}
 // Whether a frame whose waves hold `paths` paths takes the one-kernel walk.  Scenes with
 // triangle meshes keep the wavefront kernels, whose traversals refill idle lanes inside a
 // query.  Spectral programs do from 2^22 paths on: their shading is several times the code of
@@ -557,7 +551,7 @@ void launch_walk(const Launcher& L, const void* kern, size_t smem, const DevScen
 // scene, program knobs and frame come from the per-job tables.
 // sk: the mix's compiled batched kernels (ptr_specialize_batch), or null for the generic ones.
 void launch_batch_wave(const DevScene& S0, const PathPool& pool_in, const BatchTables& bt, int direct, bool media,
-                       bool equiangular, cudaStream_t st, int iters, int n_sm, const ptr_tuning& tune,
+                       bool het, bool equiangular, cudaStream_t st, int iters, int n_sm, const ptr_tuning& tune,
                        const SpecKernels* sk, std::vector<ProfRec>* prof = nullptr, bool dry = false) {
     const int block = tune.block;
     int n_launched = 0;
@@ -565,6 +559,7 @@ void launch_batch_wave(const DevScene& S0, const PathPool& pool_in, const BatchT
     PathPool pool = pool_in;
     pool.sort_buckets = tune.sort_buckets;
     pool.ray_sort = tune.ray_sort;
+    pool.lockstep = shade_lockstep(media, het);
     ProgParams P0{};
     auto mark = [&](int cls) -> ProfRec* {
         if (!prof) return nullptr;
@@ -2451,7 +2446,7 @@ int ptr_render_batch(ptr_ctx* ctx, const ptr_batch_job* jobs, int n_jobs) {
         std::vector<ProfRec> prof;
         prof.reserve((size_t)waves * (iters * 5 + 2));
         for (long long w = 0; e == cudaSuccess && w < waves; ++w) {
-            launch_batch_wave(jobs[0].scene->dev, bp->pool, bt, direct, media, equi, st, wave_iters[(size_t)w], n_sm, ctx->tune, sk, &prof);
+            launch_batch_wave(jobs[0].scene->dev, bp->pool, bt, direct, media, het, equi, st, wave_iters[(size_t)w], n_sm, ctx->tune, sk, &prof);
             e = cudaGetLastError();
         }
         if (e == cudaSuccess) e = cudaStreamSynchronize(st);
@@ -2459,7 +2454,7 @@ int ptr_render_batch(ptr_ctx* ctx, const ptr_batch_job* jobs, int n_jobs) {
     } else {
         // occupancy queries outside capture, then one captured wave per iteration count the
         // waves need
-        launch_batch_wave(jobs[0].scene->dev, bp->pool, bt, direct, media, equi, st, iters, n_sm, ctx->tune, sk, nullptr, true);
+        launch_batch_wave(jobs[0].scene->dev, bp->pool, bt, direct, media, het, equi, st, iters, n_sm, ctx->tune, sk, nullptr, true);
         std::map<int, std::pair<cudaGraph_t, cudaGraphExec_t>> graphs;
         for (long long w = 0; e == cudaSuccess && w < waves; ++w) {
             const int it = wave_iters[(size_t)w];
@@ -2469,7 +2464,7 @@ int ptr_render_batch(ptr_ctx* ctx, const ptr_batch_job* jobs, int n_jobs) {
                 cudaGraphExec_t gew = nullptr;
                 e = cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal);
                 if (e == cudaSuccess) {
-                    launch_batch_wave(jobs[0].scene->dev, bp->pool, bt, direct, media, equi, st, it, n_sm, ctx->tune, sk);
+                    launch_batch_wave(jobs[0].scene->dev, bp->pool, bt, direct, media, het, equi, st, it, n_sm, ctx->tune, sk);
                     e = cudaStreamEndCapture(st, &gw);
                 }
                 if (e == cudaSuccess) e = cudaGraphInstantiate(&gew, gw, 0);
