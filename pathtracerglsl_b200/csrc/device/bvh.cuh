@@ -16,9 +16,6 @@
 
 namespace ptx {
 
-#ifndef PTR_CW_NEARFAR
-#define PTR_CW_NEARFAR 0
-#endif
 constexpr float kBvhTfarPad = 1.00000024f;   // BVH_TFAR_PAD (Ize 2013 far-plane pad)
 constexpr int kBvhStack = 64;                // BVH_STACK_DEPTH
 constexpr int kCwStack = 24;                 // CWBVH_STACK_DEPTH
@@ -120,12 +117,6 @@ __device__ __forceinline__ bool walk_binary(const DevScene& S, const float4* nod
 
 // ---- compressed wide BVH walk ---------------------------------------------------------------
 __device__ __forceinline__ int find_msb24(unsigned v) { return 31 - __clz(v); }
-// Byte k of word as a float, exactly: the byte is permuted into the mantissa of 2^23
-// (bits 0x4B0000bb) and 2^23 is subtracted.  One PRMT + one FADD on the integer / FMA pipes
-// instead of an I2F conversion (the conversion unit was the walk's busiest pipe).
-__device__ __forceinline__ float byte_as_float(unsigned word, unsigned k) {
-    return __fadd_rn(__uint_as_float(__byte_perm(word, 0x4B000000u, 0x7540u | k)), -8388608.0f);
-}
 __device__ __forceinline__ float clamp_dir(float d) { return fabsf(d) < 1e-20f ? (d < 0.0f ? -1e-20f : 1e-20f) : d; }
 
 // Per-ray set-up of a wide walk: the direction with zero components clamped (slab
@@ -141,54 +132,61 @@ __device__ __forceinline__ CwRay cw_ray(f3 rd) {
 // One CWBVH node against the ray: the hit internal children as an octant-ordered bit mask
 // (hits, with the node's child base and internal-child mask for the group) and the hit
 // leaf triangles as bits above the node's triangle base (leaf_bits, leaf_base).
+//
+// The walk is bound by instruction issue, so a child costs as few instructions as the test
+// allows, and no branch: the ray's octant picks the near and the far plane of each axis once
+// per node; a quantized byte b becomes the float 1 + b 2^-15 by one byte permute and its
+// plane's distance by one FMA with the offset folded in (the folded offset rounds to 2^-9 of
+// a quantization cell, kCwPad widens every box by four times that, so no child the exact
+// slab meets is lost); internal and leaf children are told apart on the 8-bit hit mask.
 struct CwNodeHits { unsigned hits, leaf_bits, child_base, imask, leaf_base; };
+constexpr float kCwPad = 0.0078125f;   // 2^-7 of a cell
+__device__ __forceinline__ float cw_plane(unsigned word, unsigned k, float scale, float offset) {
+    return __fmaf_rn(__uint_as_float(__byte_perm(word, 0x3F800000u, 0x7604u | (k << 4))), scale, offset);
+}
 __device__ __forceinline__ CwNodeHits cw_node(const uint4* nd, f3 ro, const CwRay& cr, float tmax) {
-    uint4 n0 = __ldg(nd), n1 = __ldg(nd + 1), n2 = __ldg(nd + 2), n3 = __ldg(nd + 3), n4 = __ldg(nd + 4);
-    f3 p(__uint_as_float(n0.x), __uint_as_float(n0.y), __uint_as_float(n0.z));
-    f3 dq = f3(__uint_as_float((n0.w & 0xFFu) << 23), __uint_as_float(((n0.w >> 8) & 0xFFu) << 23),
-               __uint_as_float(((n0.w >> 16) & 0xFFu) << 23)) * cr.inv;
-    f3 oq = (p - ro) * cr.inv;
-#if PTR_CW_NEARFAR
-    // the ray's octant picks which quantized bound of each axis is the near plane (the slab
-    // values are the same as min / max of the two, without computing both orders)
-    const bool nx = (cr.octinv & 1u) == 0u, ny = (cr.octinv & 2u) == 0u, nz = (cr.octinv & 4u) == 0u;
-#endif
+    const uint4 n0 = __ldg(nd), n1 = __ldg(nd + 1), n2 = __ldg(nd + 2), n3 = __ldg(nd + 3), n4 = __ldg(nd + 4);
+    const f3 p(__uint_as_float(n0.x), __uint_as_float(n0.y), __uint_as_float(n0.z));
+    const f3 dq = f3(__uint_as_float((n0.w & 0xFFu) << 23), __uint_as_float(((n0.w >> 8) & 0xFFu) << 23),
+                     __uint_as_float(((n0.w >> 16) & 0xFFu) << 23)) * cr.inv;
+    const f3 sc = dq * 32768.0f;
+    const f3 c = (p - ro) * cr.inv - sc;
+    const f3 pad(fabsf(dq.x) * kCwPad, fabsf(dq.y) * kCwPad, fabsf(dq.z) * kCwPad);
+    const f3 cn = c - pad, cf = c + pad;
+    const bool px = (cr.octinv & 1u) != 0u, py = (cr.octinv & 2u) != 0u, pz = (cr.octinv & 4u) != 0u;   // direction >= 0
+    unsigned hm = 0u;
+#pragma unroll
+    for (unsigned half = 0u; half < 2u; ++half) {
+        const unsigned lx = half ? n2.y : n2.x, ly = half ? n2.w : n2.z, lz = half ? n3.y : n3.x;
+        const unsigned hx = half ? n3.w : n3.z, hy = half ? n4.y : n4.x, hz = half ? n4.w : n4.z;
+        const unsigned nx = px ? lx : hx, ny = py ? ly : hy, nz = pz ? lz : hz;
+        const unsigned fx = px ? hx : lx, fy = py ? hy : ly, fz = pz ? hz : lz;
+#pragma unroll
+        for (unsigned k = 0u; k < 4u; ++k) {
+            const float tn = fmaxf(fmaxf(cw_plane(nx, k, sc.x, cn.x), cw_plane(ny, k, sc.y, cn.y)),
+                                   fmaxf(cw_plane(nz, k, sc.z, cn.z), 0.0f));
+            const float tf = fminf(fminf(cw_plane(fx, k, sc.x, cf.x), cw_plane(fy, k, sc.y, cf.y)),
+                                   fminf(cw_plane(fz, k, sc.z, cf.z), tmax)) * kBvhTfarPad;
+            if (!(tf < tn)) hm |= 1u << (4u * half + k);
+        }
+    }
     CwNodeHits o;
-    o.hits = 0u;
-    o.leaf_bits = 0u;
     o.child_base = n1.x;
     o.leaf_base = n1.y;
     o.imask = (n0.w >> 24) & 0xFFu;
-#pragma unroll
-    for (unsigned sl = 0u; sl < 8u; sl++) {
-        const unsigned sh = 8u * (sl & 3u);
-        unsigned m = ((sl < 4u ? n1.z : n1.w) >> sh) & 0xFFu;
-        if (m == 0u) continue;
-        const unsigned kb = sl & 3u;
-        const unsigned wlx = sl < 4u ? n2.x : n2.y, wly = sl < 4u ? n2.z : n2.w, wlz = sl < 4u ? n3.x : n3.y;
-        const unsigned whx = sl < 4u ? n3.z : n3.w, why = sl < 4u ? n4.x : n4.y, whz = sl < 4u ? n4.z : n4.w;
-#if PTR_CW_NEARFAR
-        float nearx = __fmaf_rn(byte_as_float(nx ? whx : wlx, kb), dq.x, oq.x);
-        float fary = __fmaf_rn(byte_as_float(ny ? wly : why, kb), dq.y, oq.y);
-        float neary = __fmaf_rn(byte_as_float(ny ? why : wly, kb), dq.y, oq.y);
-        float farx = __fmaf_rn(byte_as_float(nx ? wlx : whx, kb), dq.x, oq.x);
-        float nearz = __fmaf_rn(byte_as_float(nz ? whz : wlz, kb), dq.z, oq.z);
-        float farz = __fmaf_rn(byte_as_float(nz ? wlz : whz, kb), dq.z, oq.z);
-        float tn = gmax(gmax(nearx, neary), gmax(nearz, 0.0f));
-        float tf = gmin(gmin(farx, fary), gmin(farz, tmax)) * kBvhTfarPad;
-#else
-        float qlx = byte_as_float(wlx, kb), qly = byte_as_float(wly, kb), qlz = byte_as_float(wlz, kb);
-        float qhx = byte_as_float(whx, kb), qhy = byte_as_float(why, kb), qhz = byte_as_float(whz, kb);
-        float lox = __fmaf_rn(qlx, dq.x, oq.x), hix = __fmaf_rn(qhx, dq.x, oq.x);
-        float loy = __fmaf_rn(qly, dq.y, oq.y), hiy = __fmaf_rn(qhy, dq.y, oq.y);
-        float loz = __fmaf_rn(qlz, dq.z, oq.z), hiz = __fmaf_rn(qhz, dq.z, oq.z);
-        float tn = gmax(gmax(gmin(lox, hix), gmin(loy, hiy)), gmax(gmin(loz, hiz), 0.0f));
-        float tf = gmin(gmin(gmax(lox, hix), gmax(loy, hiy)), gmin(gmax(loz, hiz), tmax)) * kBvhTfarPad;
-#endif
-        if (tf < tn) continue;
-        if ((m & 0xE0u) == 0x20u && (m & 0x1Fu) >= 24u) o.hits |= 1u << ((((m & 0x1Fu) - 24u) ^ cr.octinv) & 7u);
-        else o.leaf_bits |= (m >> 5) << (m & 0x1Fu);
+    o.leaf_bits = 0u;
+    // hit leaf children: their items' bits (an empty slot has none)
+    for (unsigned lm = hm & ~o.imask; lm != 0u; lm &= lm - 1u) {
+        const unsigned sl = (unsigned)__ffs((int)lm) - 1u;
+        const unsigned m = ((sl < 4u ? n1.z : n1.w) >> (8u * (sl & 3u))) & 0xFFu;
+        o.leaf_bits |= (m >> 5) << (m & 0x1Fu);
     }
+    // hit internal children, slot s at bit s ^ octinv
+    unsigned h = hm & o.imask;
+    if (cr.octinv & 1u) h = ((h & 0x55u) << 1) | ((h >> 1) & 0x55u);
+    if (cr.octinv & 2u) h = ((h & 0x33u) << 2) | ((h >> 2) & 0x33u);
+    if (cr.octinv & 4u) h = ((h & 0x0Fu) << 4) | (h >> 4);
+    o.hits = h;
     return o;
 }
 // The next child of a node group: pops the highest hit bit and maps it to the child index.
@@ -238,6 +236,11 @@ __device__ __forceinline__ bool walk_wide(const DevScene& S, const uint4* nodes,
     return false;
 }
 
+// Whether the program walks this mesh's compressed wide BVH (else its binary one).
+__device__ __forceinline__ bool walks_cwbvh(const DevScene& S, const DevMesh& m) {
+    return (PTR_SPEC_ACCEL < 0 ? S.accel : PTR_SPEC_ACCEL) == PTR_ACCEL_CWBVH && m.cwbvh;
+}
+
 // ---- one mesh BLAS in a given frame (ro/rd already in the mesh's local frame) --------------
 // tie_in(): whether this walk wins a tie with the incoming tmax (a lower instance index
 // than the hit that set it); ties inside the walk go to the lower triangle index.
@@ -245,11 +248,11 @@ template <class Tie = NoTie>
 __device__ __forceinline__ bool mesh_nearest(const DevScene& S, const DevMesh& m, f3 ro, f3 rd, float& tmax, int& prim,
                                              Work* w = nullptr, Tie tie_in = Tie{}) {
     bool found = false;
-    const float4* tri = (S.accel == PTR_ACCEL_CWBVH && m.cwbvh) ? m.tri_w : m.tri;
+    const float4* tri = walks_cwbvh(S, m) ? m.tri_w : m.tri;
     auto take = [&](int i, float t) {
         return t > 0.0f && (t < tmax || (t == tmax && (found ? tri_orig(tri, i) < tri_orig(tri, prim) : tie_in())));
     };
-    if (S.accel == PTR_ACCEL_CWBVH && m.cwbvh) {
+    if (walks_cwbvh(S, m)) {
         walk_wide(S, m.cwbvh, ro, rd, tmax, [&](int i) {
             f3 a, e1, e2;
             if (w) w->tris++;
@@ -273,7 +276,7 @@ __device__ __forceinline__ bool mesh_nearest(const DevScene& S, const DevMesh& m
     return found;
 }
 __device__ __forceinline__ bool mesh_any(const DevScene& S, const DevMesh& m, f3 ro, f3 rd, float max_dist, Work* w = nullptr) {
-    if (S.accel == PTR_ACCEL_CWBVH && m.cwbvh) {
+    if (walks_cwbvh(S, m)) {
         const float4* tri = m.tri_w;
         return walk_wide(S, m.cwbvh, ro, rd, max_dist, [&](int i) {
             f3 a, e1, e2;
@@ -296,159 +299,227 @@ __device__ __forceinline__ bool mesh_any(const DevScene& S, const DevMesh& m, f3
     }, w ? &w->nodes : nullptr);
 }
 
-// ---- instanced meshes: binary TLAS over CWBVH BLAS as one flat loop -------------------------
+// ---- instanced meshes: TLAS over BLAS as one flat loop --------------------------------------
 // The nested form (accel_closest / accel_any) runs each instance's BLAS walk to the end
 // inside the TLAS leaf that reached it, so in a warp every lane whose TLAS step did not
 // enter an instance waits for the other lanes' whole BLAS walks.  Here one loop advances
-// each lane by one step — a TLAS node, the next instance of the current TLAS leaf, or a
-// BLAS node with its leaf triangles — so lanes at different levels proceed together.  Per
-// lane the sequence of node visits, leaf tests and tmax updates is that of the nested
-// walks, so hits (and the work tallies) are identical.  ANY: stop at the first triangle hit.
-// The walk as a resumable state: init() for one ray, then step() until it reports the end.
-// A step runs the bookkeeping transitions in line instead of spending a loop iteration on
-// each: a TLAS leaf enters its first instance and that instance's BLAS root in the same
-// step, a group pop goes straight on to the popped node, and a finished BLAS walk hands
-// over to the next instance or TLAS node at the start of the next step.
-struct InstFlat {
-    f3 winv;                               // TLAS: world-ray reciprocal, node stack, leaf range
-    int tstack[kBvhStack];
-    int tptr, li, lend;
-    f3 ro, rd;                             // BLAS: the entered instance's frame and group stack
-    CwRay cr;
-    uint2 stack[kCwStack];
-    int ptr;
-    unsigned g_base, g_hits, g_imask;
-    float t, t_near;                       // t: BLAS tmax; t_near: TLAS culling distance
-    int prim, inst, phase;                 // phase: 0 TLAS node, 1 next instance, 2 BLAS step
-    bool found;
-    __device__ __forceinline__ void init(const Ray& r, float t0) {
-        winv = f3(1.0f / r.d.x, 1.0f / r.d.y, 1.0f / r.d.z);
-        tptr = 0;
-        tstack[0] = 0;
-        li = lend = 0;
-        ptr = -1;
-        g_hits = 0u;
-        t_near = t0;
-        phase = 0;
-        found = false;
+// each lane by one node, whichever tree the node belongs to: TLAS and BLAS are walked in the
+// same node format by the same code (wide: compressed nodes of the wide TLAS and the CWBVH;
+// binary: the two-float4 nodes of the binary TLAS and BVH), so lanes at either level do the
+// same work and differ only in the ray's frame and the node array.  Entering an instance and
+// leaving its BLAS are done on the way to the next node.  Hits and ties are those of the
+// nested walks.  ANY: stop at the first triangle hit.
+//
+// The walk is resumable: init() for one ray, then step() until it reports the end.
+// h takes every nearer hit at once; h.element is the placement's index in the order hit
+// queries report (the binary TLAS leaf order unless the program walks the wide TLAS).
+struct FlatScene {                         // what a walk reads of its batch and prototype
+    const void* tlas;
+    const void* blas;
+    const float4* place;
+    const float4* tri;
+    const int* id;                         // caller's index of each placement of this walk's order
+    const int* element;                    // reported index of each placement (NULL: its own)
+    const int* element_id;                 // caller's index of a reported element
+};
+template <bool WIDE>
+__device__ __forceinline__ FlatScene flat_scene(const DevScene& S, const DevBatch& b) {
+    const DevMesh& m = S.meshes[b.proto_mesh];
+    if (!WIDE) return FlatScene{b.tlas, m.bvh, b.place, m.tri, b.inst_id, nullptr, b.inst_id};
+    const bool wide_ids = S.inst_accel == PTR_ACCEL_CWBVH;
+    return FlatScene{b.tlas_w, m.cwbvh, b.place_w, m.tri_w, b.inst_id_w, wide_ids ? nullptr : b.slot_of_w,
+                     wide_ids ? b.inst_id_w : b.inst_id};
+}
+template <bool WIDE> struct FlatStack { using Entry = uint2; static constexpr int kSize = 2 * kCwStack; };
+template <> struct FlatStack<false> { using Entry = int; static constexpr int kSize = 2 * kBvhStack; };
+template <bool WIDE>
+struct FlatWalk {
+    using Entry = typename FlatStack<WIDE>::Entry;
+    Entry stack[FlatStack<WIDE>::kSize];   // both levels share it
+    f3 ro, rd;                             // the ray in the frame of the level walked last
+    CwRay cr;                              // its reciprocal (wide: and octant)
+    int ptr, bottom;                       // stack top; the top when the current instance was entered
+    unsigned g_base, g_hits, g_imask;      // wide: the node group under way
+    float A, B;                            // binary: words of the node to expand, g_base, when g_hits != 0
+    unsigned leaf_base, leaf_left;         // the TLAS leaf's placements still to enter (wide: bits, binary: count)
+    int inst;
+    bool blas, world, found;               // level; the frame is the world's; this instance holds the hit
+    __device__ __forceinline__ void frame(const f3 o, const f3 d) {
+        ro = o;
+        rd = d;
+        if (WIDE) cr = cw_ray(d);
+        else cr.inv = f3(1.0f / d.x, 1.0f / d.y, 1.0f / d.z);
     }
-    // One step; false once the query is over.  Closest (ANY = false): h takes every nearer
-    // instance hit.  Any-hit: returns false with `found` set at the first hit.
-    template <bool ANY>
-    __device__ __forceinline__ bool step(const DevScene& S, const DevBatch& b, const DevMesh& m, int region, const Ray& r,
-                                         HitRec& h, float max_dist, Work* w) {
-        if (phase == 2 && g_hits == 0u && ptr < 0) {   // the BLAS walk is done
-            if (!ANY && found) {
-                t_near = t;
-                h.t = t;
-                h.region = region;
-                h.element = inst;
-                h.prim = prim;
-            }
-            phase = li < lend ? 1 : 0;
-        }
-        if (phase == 0) {
-            if (tptr < 0) return false;
-            const int ni = tstack[tptr--];
-            if (w) w->tlas++;
-            const float4 n0 = __ldg(b.tlas + 2 * ni), n1 = __ldg(b.tlas + 2 * ni + 1);
-            if (!aabb_hit(n0, n1, r.o, winv, t_near)) return true;
-            if (n0.w >= 0.0f) {
-                li = (int)n1.w;
-                lend = li + (int)n0.w;
-                phase = 1;                 // enter its first instance in this step
-            } else {
-                const int axis = (int)(-n0.w - 1.0f);
-                const int L = ni + 1, R = (int)n1.w;
-                const bool nf = (axis == 0 ? r.d.x : (axis == 1 ? r.d.y : r.d.z)) >= 0.0f;
-                if (tptr + 2 < kBvhStack) {
-                    tstack[++tptr] = nf ? R : L;
-                    tstack[++tptr] = nf ? L : R;
-                } else {
-                    flag_error(S, kErrBvhStack);
-                }
-                return true;
-            }
-        }
-        if (phase == 1) {
-            if (li >= lend) { phase = 0; return true; }
-            inst = li++;
-            const float4 q = __ldg(b.place + 2 * inst), ts = __ldg(b.place + 2 * inst + 1);
-            const float s = ts.w;
-            if (w) w->inst++;
-            ro = placement_rigid(q, ts, r.o) / s;
-            rd = qrot(q, r.d) / s;
-            cr = cw_ray(rd);
-            ptr = -1;
+    __device__ __forceinline__ void root(const FlatScene& fs, float tmax, Work* w) {
+        if constexpr (WIDE) {
             g_base = 0u;
             g_hits = 1u << (cr.octinv & 7u);
             g_imask = 1u;
-            t = t_near;
-            prim = -1;
-            found = false;
-            phase = 2;                     // and walk its BLAS root in this step
+        } else {
+            load(fs, 0, tmax, w);
         }
-        if (g_hits == 0u) {                // pop a group (the stack is not empty here)
-            const uint2 top = stack[ptr];
-            g_base = top.x;
-            g_hits = top.y & 0xFFu;
-            g_imask = top.y >> 8;
-            ptr--;
+    }
+    __device__ __forceinline__ void push(const DevScene& S, Entry e) {
+        if (ptr + 1 < FlatStack<WIDE>::kSize) stack[++ptr] = e;
+        else flag_error(S, WIDE ? kErrCwStack : kErrBvhStack);
+    }
+    __device__ __forceinline__ void push_group(const DevScene& S) {
+        if constexpr (WIDE) push(S, make_uint2(g_base, g_hits | (g_imask << 8)));
+    }
+    // Binary: node ni becomes the one to expand if the ray meets its box.
+    __device__ __forceinline__ void load(const FlatScene& fs, int ni, float tmax, Work* w) {
+        const float4* nodes = (const float4*)(blas ? fs.blas : fs.tlas);
+        const float4 n0 = __ldg(nodes + 2 * (size_t)ni), n1 = __ldg(nodes + 2 * (size_t)ni + 1);
+        if (w) { if (blas) w->nodes++; else w->tlas++; }
+        g_hits = aabb_hit(n0, n1, ro, cr.inv, tmax) ? 1u : 0u;
+        g_base = (unsigned)ni;
+        A = n0.w;
+        B = n1.w;
+    }
+    // Binary: both children of an inner node are met here, the nearer along the split axis
+    // goes on and the other waits, so a node the ray misses costs no step of its own.
+    __device__ __forceinline__ void expand(const DevScene& S, const FlatScene& fs, float tmax, Work* w) {
+        const int axis = (int)(-A - 1.0f);
+        const bool nf = (axis == 0 ? rd.x : (axis == 1 ? rd.y : rd.z)) >= 0.0f;
+        const int L = (int)g_base + 1, R = (int)B, near = nf ? L : R, far = nf ? R : L;
+        const float4* nodes = (const float4*)(blas ? fs.blas : fs.tlas);
+        const float4 a0 = __ldg(nodes + 2 * (size_t)near), a1 = __ldg(nodes + 2 * (size_t)near + 1);
+        const float4 b0 = __ldg(nodes + 2 * (size_t)far), b1 = __ldg(nodes + 2 * (size_t)far + 1);
+        if (w) { if (blas) w->nodes += 2; else w->tlas += 2; }
+        const bool ha = aabb_hit(a0, a1, ro, cr.inv, tmax), hb = aabb_hit(b0, b1, ro, cr.inv, tmax);
+        g_hits = ha || hb ? 1u : 0u;
+        g_base = (unsigned)(ha ? near : far);
+        A = ha ? a0.w : b0.w;
+        B = ha ? a1.w : b1.w;
+        if constexpr (!WIDE) {
+            if (ha && hb) push(S, far);
         }
-        const unsigned child = cw_next_child(g_hits, g_base, g_imask, cr.octinv);
-        if (g_hits != 0u) {
-            if (ptr + 1 < kCwStack) { ptr++; stack[ptr] = make_uint2(g_base, g_hits | (g_imask << 8)); }
-            else flag_error(S, kErrCwStack);
-        }
-        if (w) w->nodes++;
-        const CwNodeHits nh = cw_node(m.cwbvh + 5 * (size_t)child, ro, cr, ANY ? max_dist : t);
-        unsigned leaf_bits = nh.leaf_bits;
-        while (leaf_bits != 0u) {
-            const int lb = find_msb24(leaf_bits);
-            leaf_bits &= ~(1u << (unsigned)lb);
-            const int i = (int)nh.leaf_base + lb;
-            f3 a, e1, e2;
-            if (w) w->tris++;
-            load_tri(m.tri_w, i, a, e1, e2);
-            float tt;
-            if (ANY) {
-                if (tri_test(ro, rd, a, e1, e2, tt) && tt > 0.0f && tt < max_dist) {
-                    found = true;
-                    return false;
+    }
+    __device__ __forceinline__ void init(const FlatScene& fs, const Ray& r, float tmax, Work* w) {
+        frame(r.o, r.d);
+        ptr = bottom = -1;
+        leaf_left = 0u;
+        blas = found = false;
+        world = true;
+        root(fs, tmax, w);
+    }
+    // One node; false once the query is over (any-hit: with found set at the first hit).
+    template <bool ANY>
+    __device__ __forceinline__ bool step(const DevScene& S, const FlatScene& fs, int region, const Ray& r, HitRec& h, float max_dist, Work* w) {
+        if (g_hits == 0u && blas && ptr == bottom) blas = false;   // the instance is done
+        if (!blas && leaf_left != 0u) {                            // enter the TLAS leaf's next placement
+            if (WIDE) {
+                if (g_hits != 0u) push_group(S);
+                const int lb = find_msb24(leaf_left);
+                leaf_left &= ~(1u << (unsigned)lb);
+                inst = (int)leaf_base + lb;
+            } else {
+                inst = (int)leaf_base++;
+                leaf_left--;
+            }
+            const float4 q = __ldg(fs.place + 2 * (size_t)inst), ts = __ldg(fs.place + 2 * (size_t)inst + 1);
+            if (w) w->inst++;
+            frame(placement_rigid(q, ts, r.o) / ts.w, qrot(q, r.d) / ts.w);
+            blas = true;
+            world = found = false;
+            bottom = ptr;
+            root(fs, ANY ? max_dist : h.t, w);
+        } else {
+            if (g_hits == 0u && ptr < 0) return false;
+            if (!blas && !world) {
+                frame(r.o, r.d);
+                world = true;
+            }
+            if (g_hits == 0u) {
+                const Entry top = stack[ptr--];
+                if constexpr (WIDE) {
+                    g_base = top.x;
+                    g_hits = top.y & 0xFFu;
+                    g_imask = top.y >> 8;
+                } else {
+                    load(fs, top, ANY ? max_dist : h.t, w);   // against the hit found since it was pushed
                 }
-            } else if (tri_test(ro, rd, a, e1, e2, tt) && tt > 0.0f &&
-                       (tt < t || (tt == t && (found ? tri_orig(m.tri_w, i) < tri_orig(m.tri_w, prim)
-                                                     : (h.region == region && __ldg(b.inst_id + inst) < __ldg(b.inst_id + h.element)))))) {
-                t = tt;
-                prim = i;
-                found = true;
             }
         }
-        if (nh.hits != 0u) { g_base = nh.child_base; g_hits = nh.hits; g_imask = nh.imask; }
-        else g_hits = 0u;
+        if constexpr (!WIDE) {
+            if (g_hits == 0u) return true;
+            if (A < 0.0f) {
+                expand(S, fs, ANY ? max_dist : h.t, w);
+                if (g_hits == 0u || A < 0.0f) return true;
+            }
+            g_hits = 0u;                                       // a leaf of A items from B
+            if (!blas) {
+                leaf_base = (unsigned)B;
+                leaf_left = (unsigned)A;
+                return true;
+            }
+            for (int i = (int)B; i < (int)B + (int)A; ++i)
+                if (triangle<ANY>(fs, i, region, h, max_dist, w)) return false;
+        } else {
+            const unsigned child = cw_next_child(g_hits, g_base, g_imask, cr.octinv);
+            if (g_hits != 0u) push_group(S);
+            if (w) { if (blas) w->nodes++; else w->tlas++; }
+            const CwNodeHits nh = cw_node((const uint4*)(blas ? fs.blas : fs.tlas) + 5 * (size_t)child, ro, cr, ANY ? max_dist : h.t);
+            g_base = nh.child_base;
+            g_hits = nh.hits;
+            g_imask = nh.imask;
+            if (!blas) {
+                leaf_base = nh.leaf_base;
+                leaf_left = nh.leaf_bits;
+                return true;
+            }
+            for (unsigned bits = nh.leaf_bits; bits != 0u;) {
+                const int lb = find_msb24(bits);
+                bits &= ~(1u << (unsigned)lb);
+                if (triangle<ANY>(fs, (int)nh.leaf_base + lb, region, h, max_dist, w)) return false;
+            }
+        }
         return true;
+    }
+    // Leaf triangle i; true ends an any-hit query.
+    template <bool ANY>
+    __device__ __forceinline__ bool triangle(const FlatScene& fs, int i, int region, HitRec& h, float max_dist, Work* w) {
+        f3 a, e1, e2;
+        if (w) w->tris++;
+        load_tri(fs.tri, i, a, e1, e2);
+        float t;
+        if (!tri_test(ro, rd, a, e1, e2, t) || !(t > 0.0f)) return false;
+        if (ANY) {
+            found = t < max_dist;
+            return found;
+        }
+        if (t < h.t || (t == h.t && (found ? tri_orig(fs.tri, i) < tri_orig(fs.tri, h.prim)
+                                           : (h.region == region && __ldg(fs.id + inst) < __ldg(fs.element_id + h.element))))) {
+            h.t = t;
+            h.region = region;
+            h.element = fs.element ? __ldg(fs.element + inst) : inst;
+            h.prim = i;
+            found = true;
+        }
+        return false;
     }
 };
 constexpr int kFlatGuard = 1 << 22;        // steps of one query before the walk gives up
-template <bool ANY>
-__device__ __forceinline__ bool inst_mesh_flat(const DevScene& S, const DevBatch& b, int region, const Ray& r, HitRec& h,
-                                               float max_dist, Work* w) {
-    const DevMesh& m = S.meshes[b.proto_mesh];
-    InstFlat f;
-    f.init(r, ANY ? max_dist : h.t);
+template <bool WIDE, bool ANY>
+__device__ __forceinline__ bool flat_walk(const DevScene& S, const DevBatch& b, int region, const Ray& r, HitRec& h, float max_dist, Work* w) {
+    const FlatScene fs = flat_scene<WIDE>(S, b);
+    FlatWalk<WIDE> f;
+    f.init(fs, r, ANY ? max_dist : h.t, w);
     for (int guard = 0; guard < kFlatGuard; ++guard)
-        if (!f.step<ANY>(S, b, m, region, r, h, max_dist, w)) return ANY && f.found;
+        if (!f.template step<ANY>(S, fs, region, r, h, max_dist, w)) return ANY && f.found;
     flag_error(S, kErrCwGuard);
     return false;
 }
-// The flat loop applies to mesh prototypes walked as CWBVH under the binary TLAS
-// (PTR_FLAT_INST=0 builds keep the nested walks everywhere).
-#ifndef PTR_FLAT_INST
-#define PTR_FLAT_INST 1
-#endif
-__device__ __forceinline__ bool inst_mesh_flat_ok(const DevScene& S, const DevBatch& b) {
-    return kHasMesh && PTR_FLAT_INST && b.proto_shape == PTR_SHAPE_MESH && S.accel == PTR_ACCEL_CWBVH &&
-           !(S.inst_accel == PTR_ACCEL_CWBVH && b.tlas_w) && S.meshes[b.proto_mesh].cwbvh != nullptr;
+// The flat loops a batch takes: wide for mesh prototypes walked as CWBVH (with the wide TLAS,
+// whichever TLAS the program names: hits do not depend on it), binary for prototypes walked
+// as binary BVH under the binary TLAS.  The rest keep the nested walks.
+__device__ __forceinline__ bool flat_wide_ok(const DevScene& S, const DevBatch& b) {
+    return kHasMesh && PTR_SPEC_ACCEL != PTR_ACCEL_BVH && b.proto_shape == PTR_SHAPE_MESH && b.tlas_w &&
+           walks_cwbvh(S, S.meshes[b.proto_mesh]);
+}
+__device__ __forceinline__ bool flat_binary_ok(const DevScene& S, const DevBatch& b) {
+    return kHasMesh && PTR_SPEC_ACCEL != PTR_ACCEL_CWBVH && b.proto_shape == PTR_SHAPE_MESH &&
+           !walks_cwbvh(S, S.meshes[b.proto_mesh]) && !(S.inst_accel == PTR_ACCEL_CWBVH && b.tlas_w);
 }
 
 // ---- region arms ------------------------------------------------------------------------
@@ -467,10 +538,8 @@ __device__ __forceinline__ void accel_closest(const DevScene& S, const ptr_regio
         return;
     }
     const DevBatch& b = S.batches[g.ref];
-    if (inst_mesh_flat_ok(S, b)) {
-        inst_mesh_flat<false>(S, b, region, r, h, 0.0f, w);
-        return;
-    }
+    if (flat_wide_ok(S, b)) { flat_walk<true, false>(S, b, region, r, h, 0.0f, w); return; }
+    if (flat_binary_ok(S, b)) { flat_walk<false, false>(S, b, region, r, h, 0.0f, w); return; }
     float t_near = h.t;
     const bool wide = S.inst_accel == PTR_ACCEL_CWBVH && b.tlas_w;
     const float4* place = wide ? b.place_w : b.place;
@@ -513,10 +582,9 @@ __device__ __forceinline__ bool accel_any(const DevScene& S, const ptr_region& g
                                           Work* w = nullptr) {
     if (kHasMesh && g.shape == PTR_SHAPE_MESH) return mesh_any(S, S.meshes[g.ref], r.o, r.d, max_dist, w);
     const DevBatch& b = S.batches[g.ref];
-    if (inst_mesh_flat_ok(S, b)) {
-        HitRec unused;
-        return inst_mesh_flat<true>(S, b, 0, r, unused, max_dist, w);
-    }
+    HitRec unused;
+    if (flat_wide_ok(S, b)) return flat_walk<true, true>(S, b, 0, r, unused, max_dist, w);
+    if (flat_binary_ok(S, b)) return flat_walk<false, true>(S, b, 0, r, unused, max_dist, w);
     const bool wide = S.inst_accel == PTR_ACCEL_CWBVH && b.tlas_w;
     const float4* place = wide ? b.place_w : b.place;
     auto instance = [&](int i) -> bool {
@@ -588,7 +656,7 @@ __device__ __forceinline__ f3 accel_hit_normal(const DevScene& S, const ptr_regi
         }
         const DevMesh& m = S.meshes[b.proto_mesh];
         float4 q = __ldg(place + 2 * hr.element);
-        const float4* tri = (S.accel == PTR_ACCEL_CWBVH && m.cwbvh) ? m.tri_w : m.tri;
+        const float4* tri = walks_cwbvh(S, m) ? m.tri_w : m.tri;
         f3 a, e1, e2;
         load_tri(tri, hr.prim, a, e1, e2);
         f3 gl = cross(e1, e2);
@@ -598,7 +666,7 @@ __device__ __forceinline__ f3 accel_hit_normal(const DevScene& S, const ptr_regi
         return normalize(placement_normal(q, gl));
     }
     const DevMesh& m = S.meshes[g.ref];
-    const float4* tri = (S.accel == PTR_ACCEL_CWBVH && m.cwbvh) ? m.tri_w : m.tri;
+    const float4* tri = walks_cwbvh(S, m) ? m.tri_w : m.tri;
     f3 a, e1, e2;
     load_tri(tri, hr.prim, a, e1, e2);
     f3 gl = cross(e1, e2);

@@ -52,6 +52,9 @@ PTR_M1(m_tanh, tanh) PTR_M1(m_atanh, atanh) PTR_M1(m_cosh, cosh) PTR_M2(m_atan2,
 #ifndef PTR_SPEC_TREE
 #define PTR_SPEC_TREE 1         // 0: the build never selects lights with the light tree
 #endif
+#ifndef PTR_SPEC_ACCEL
+#define PTR_SPEC_ACCEL (-1)     // PTR_ACCEL_* the program walks meshes with (-1: read at run time)
+#endif
 #ifndef PTR_SPEC_HET
 #define PTR_SPEC_HET 1          // 0: no medium of the build has a coefficient field
 #endif

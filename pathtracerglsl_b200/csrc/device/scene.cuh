@@ -43,6 +43,7 @@ struct DevBatch {
     // rule between instances, and the element a hit query reports)
     const int* inst_id;
     const int* inst_id_w;
+    const int* slot_of_w;     // the binary leaf slot of each wide one (NULL without a wide TLAS)
 };
 
 struct DevScene {

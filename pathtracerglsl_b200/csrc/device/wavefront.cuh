@@ -770,15 +770,17 @@ __device__ __forceinline__ unsigned shade_key(const DevScene& S, int region, int
 #ifndef PTR_REFILL
 #define PTR_REFILL 1
 #endif
-constexpr int kRefillMin = 8;
-template <bool COUNT>
+#ifndef PTR_REFILL_MIN
+#define PTR_REFILL_MIN 8
+#endif
+constexpr int kRefillMin = PTR_REFILL_MIN;
+template <bool COUNT, bool WIDE>
 __device__ __forceinline__ void closest_refill(const DevScene& S, const PathPool& pool, const int* q, unsigned n, int buckets,
                                                unsigned* ticket, Work* w) {
     const int fr = S.flat_region;
-    const DevBatch& b = S.batches[S.regions[fr].ref];
-    const DevMesh& m = S.meshes[b.proto_mesh];
+    const FlatScene fs = flat_scene<WIDE>(S, S.batches[S.regions[fr].ref]);
     const unsigned lane = threadIdx.x & 31u;
-    InstFlat f;
+    FlatWalk<WIDE> f;
     Ray r;
     HitRec h;
     int i = -1, steps = 0;
@@ -807,7 +809,7 @@ __device__ __forceinline__ void closest_refill(const DevScene& S, const PathPool
                             float t;
                             if (analytic_root(S.regions[g], r, t) && t < h.t) { h.t = t; h.region = g; h.element = 0; h.prim = -1; }
                         }
-                        f.init(r, h.t);
+                        f.init(fs, r, h.t, COUNT ? w : nullptr);
                         steps = 0;
                         active = true;
                     }
@@ -816,7 +818,7 @@ __device__ __forceinline__ void closest_refill(const DevScene& S, const PathPool
         }
         if (!__any_sync(0xffffffffu, active)) break;
         if (!active) continue;
-        bool more = f.step<false>(S, b, m, fr, r, h, 0.0f, COUNT ? w : nullptr);
+        bool more = f.template step<false>(S, fs, fr, r, h, 0.0f, COUNT ? w : nullptr);
         if (more && ++steps >= kFlatGuard) {
             flag_error(S, kErrCwGuard);
             more = false;
@@ -847,10 +849,15 @@ __global__ void __launch_bounds__(256, PTR_TRACE_MIN_BLOCKS) k_closest(DevScene 
     }
     const int* q = closest_queue(pool, in);
     Work w{0u, 0u, 0u, 0u};
-    if (PTR_REFILL && !BATCH && pool.fetch && S0.flat_region >= 0 && inst_mesh_flat_ok(S0, S0.batches[S0.regions[S0.flat_region].ref])) {
-        closest_refill<COUNT>(S0, pool, q, n, buckets, pool.fetch + 0, &w);
-        if (COUNT) flush_work(S0, w);
-        return;
+    if (PTR_REFILL && kHasMesh && !BATCH && pool.fetch && S0.flat_region >= 0) {
+        const DevBatch& b = S0.batches[S0.regions[S0.flat_region].ref];
+        const bool wide = flat_wide_ok(S0, b), binary = flat_binary_ok(S0, b);
+        if (wide) closest_refill<COUNT, true>(S0, pool, q, n, buckets, pool.fetch + 0, &w);
+        else if (binary) closest_refill<COUNT, false>(S0, pool, q, n, buckets, pool.fetch + 0, &w);
+        if (wide || binary) {
+            if (COUNT) flush_work(S0, w);
+            return;
+        }
     }
     const WaveJobs wj = BATCH ? WaveJobs(pool, bt) : WaveJobs{};
     // the adjoint's hit log: this launch's slice, when its iteration is logged
@@ -1642,16 +1649,15 @@ __device__ __forceinline__ void shadow_grads(const DevScene& S, const ProgParams
 // Opaque shadow queries over the same scene form, with the same per-lane refill: the
 // regions before the instanced one, the flat any-hit walk, then the regions after it (the
 // order of scene_any); an unoccluded query adds its stored contribution as k_shadow does.
-template <class Col, bool COUNT>
+template <class Col, bool COUNT, bool WIDE>
 __device__ __forceinline__ void shadow_refill(const DevScene& S, const PathPool& pool, const int* shq, unsigned n, int slot,
                                               const Pair<float4> a_o, const Pair<float4> a_d, const Pair<float4> a_lp,
                                               const Pair<float4> a_c, unsigned* ticket, Work* w) {
     constexpr bool SPECTRAL = sizeof(Col) == sizeof(s4);
     const int fr = S.flat_region;
-    const DevBatch& b = S.batches[S.regions[fr].ref];
-    const DevMesh& m = S.meshes[b.proto_mesh];
+    const FlatScene fs = flat_scene<WIDE>(S, S.batches[S.regions[fr].ref]);
     const unsigned lane = threadIdx.x & 31u;
-    InstFlat f;
+    FlatWalk<WIDE> f;
     Ray r;
     HitRec unused;
     float max_dist = 0.0f;
@@ -1680,7 +1686,7 @@ __device__ __forceinline__ void shadow_refill(const DevScene& S, const PathPool&
                             blocked = analytic_root(S.regions[g], r, t) && t < max_dist;
                         }
                         if (!blocked) {            // an occluded query is finished: nothing to add
-                            f.init(r, max_dist);
+                            f.init(fs, r, max_dist, COUNT ? w : nullptr);
                             steps = 0;
                             active = true;
                         }
@@ -1690,7 +1696,7 @@ __device__ __forceinline__ void shadow_refill(const DevScene& S, const PathPool&
         }
         if (!__any_sync(0xffffffffu, active)) break;
         if (!active) continue;
-        bool more = f.step<true>(S, b, m, fr, r, unused, max_dist, COUNT ? w : nullptr);
+        bool more = f.template step<true>(S, fs, fr, r, unused, max_dist, COUNT ? w : nullptr);
         if (more && ++steps >= kFlatGuard) {
             flag_error(S, kErrCwGuard);
             more = false;
@@ -1739,11 +1745,16 @@ __global__ void __launch_bounds__(256, PTR_TRACE_MIN_BLOCKS) k_shadow(DevScene S
             slog = pool.hit_log + 4 * (size_t)pool.iter * (size_t)pool.hit_log_stride + 2;
     const bool rec = !ADJ && slog && pool.hit_log_mode == 1;
     const bool rep = ADJ && slog && pool.hit_log_mode == 2;
-    if (PTR_REFILL && !MEDIA && !BATCH && !ADJ && !rec && pool.fetch && S0.flat_region >= 0 &&
-        inst_mesh_flat_ok(S0, S0.batches[S0.regions[S0.flat_region].ref])) {
-        shadow_refill<Col, COUNT>(S0, pool, shq, n, slot, a_o, a_d, a_lp, a_c, pool.fetch + 1 + slot, &wk);
-        if (COUNT) flush_work(S0, wk);
-        return;
+    if (PTR_REFILL && kHasMesh && !MEDIA && !BATCH && !ADJ && !rec && pool.fetch && S0.flat_region >= 0) {
+        const DevBatch& b = S0.batches[S0.regions[S0.flat_region].ref];
+        const bool wide = flat_wide_ok(S0, b), binary = flat_binary_ok(S0, b);
+        unsigned* ticket = pool.fetch + 1 + slot;
+        if (wide) shadow_refill<Col, COUNT, true>(S0, pool, shq, n, slot, a_o, a_d, a_lp, a_c, ticket, &wk);
+        else if (binary) shadow_refill<Col, COUNT, false>(S0, pool, shq, n, slot, a_o, a_d, a_lp, a_c, ticket, &wk);
+        if (wide || binary) {
+            if (COUNT) flush_work(S0, wk);
+            return;
+        }
     }
     const WaveJobs wj = BATCH ? WaveJobs(pool, bt) : WaveJobs{};
     QueueCursor cur(n, pool.fetch ? pool.fetch + 1 + slot : nullptr);
@@ -2146,7 +2157,7 @@ __global__ void k_trace_rays(DevScene S, const float* rays, int n, int* region, 
         if (h.region >= 0 && h.prim >= 0) {
             const ptr_region& g = S.regions[h.region];
             const DevMesh& m = S.meshes[g.shape == PTR_SHAPE_MESH ? g.ref : S.batches[g.ref].proto_mesh];
-            const float4* tri = (S.accel == PTR_ACCEL_CWBVH && m.cwbvh) ? m.tri_w : m.tri;
+            const float4* tri = walks_cwbvh(S, m) ? m.tri_w : m.tri;
             orig = __float_as_int(tri[3 * h.prim].w);
         }
         int el = h.element;

@@ -1008,6 +1008,7 @@ int rail_batch(ptr_ctx* ctx, ptr_scene* s, const ptr_rails& R, const RailDev& D,
     b.tlas_w = nullptr;
     b.place_w = nullptr;
     b.inst_id_w = nullptr;
+    b.slot_of_w = nullptr;
     ptx_host::WideBvh wt = ptx_host::build_cwbvh(boxes.data(), N, ptx_host::kCwbvhCPrim);
     if (!wt.error && wt.node_count > 0) {
         std::vector<float4> rec_w(2 * (size_t)N);
@@ -1025,6 +1026,9 @@ int rail_batch(ptr_ctx* ctx, ptr_scene* s, const ptr_rails& R, const RailDev& D,
         b.place_w = p4;
         if ((rc = dev_copy(ctx, s->allocs, ids_w.data(), ids_w.size(), &pi))) return rc;
         b.inst_id_w = pi;
+        std::vector<int> slots(wt.order.begin(), wt.order.begin() + N);
+        if ((rc = dev_copy(ctx, s->allocs, slots.data(), slots.size(), &pi))) return rc;
+        b.slot_of_w = pi;
         if (bd.light_base >= 0) {
             if ((rc = dev_copy(ctx, s->allocs, lo_w.data(), lo_w.size(), &pi))) return rc;
             b.light_of_w = pi;
@@ -1251,6 +1255,7 @@ int upload_accels(ptr_ctx* ctx, ptr_scene* s, const ptr_scene_desc* d, const ptr
             b.inst_id = pi;
         }
         b.inst_id_w = nullptr;
+        b.slot_of_w = nullptr;
         if ((rc = dev_copy(ctx, s->allocs, (const float4*)tl.nodes.data(), 2 * (size_t)tl.node_count, &p4))) return rc;
         b.tlas = p4;
         // the compressed wide twin of the TLAS (instanceAccel 'cwbvh', cwbvh.ts:80-372 over
@@ -1271,6 +1276,11 @@ int upload_accels(ptr_ctx* ctx, ptr_scene* s, const ptr_scene_desc* d, const ptr
             const int* pid = nullptr;
             if ((rc = dev_copy(ctx, s->allocs, ids.data(), ids.size(), &pid))) return rc;
             b.inst_id_w = pid;
+            std::vector<int> slot_of(N), slots(N);
+            for (int i = 0; i < N; ++i) slot_of[tl.order[i]] = i;
+            for (int i = 0; i < N; ++i) slots[i] = slot_of[wt.order[i]];
+            if ((rc = dev_copy(ctx, s->allocs, slots.data(), slots.size(), &pid))) return rc;
+            b.slot_of_w = pid;
             if (bd.light_base >= 0) {
                 std::vector<int> lo(N);
                 for (int i = 0; i < N; ++i) lo[i] = bd.light_base + (int)wt.order[i];
@@ -1738,6 +1748,7 @@ struct Census {
     bool tree = false, media = false, spectral = false, batch = false;
     bool mesh = false;                 // some region is a triangle mesh or instances one
     bool het = false;                  // some medium has a coefficient field
+    int accel = -1;                    // PTR_ACCEL_* of the mesh walks (-1: no meshes, or a mix)
     bool adj = false;                  // the replay's kernels (ADJ = true) instead of the forward's
     bool walk = false;                 // the one-kernel walk instead of the wavefront's three kernels
     int direct = 0;
@@ -1757,6 +1768,7 @@ Census census_of(const ptr_program* p, const ptr_scene* sc) {
     c.walk = sc->walk;
     c.mesh = sc->has_mesh;
     c.het = sc->dev.has_het != 0;
+    c.accel = sc->has_mesh ? p->desc.accel : -1;
     return c;
 }
 // The union census of a job mix (the batched kernels serve every job of it): masks OR-ed,
@@ -1787,6 +1799,7 @@ std::vector<std::string> census_options(const Census& c) {
             "-DPTR_SPEC_SHAPES=" + std::to_string(c.shapes) + "u",
             std::string("-DPTR_SPEC_MESH=") + (c.mesh ? "1" : "0"),
             std::string("-DPTR_SPEC_HET=") + (c.het ? "1" : "0"),
+            "-DPTR_SPEC_ACCEL=(" + std::to_string(c.accel) + ")",
             "-DPTR_SPEC_NREGIONS=" + std::to_string(c.nregions),
             "-DPTR_SPEC_SHAPE_CODE=" + std::to_string(c.shape_code) + "ull",
             std::string("-DPTR_SPEC_TREE=") + (c.tree ? "1" : "0")};
