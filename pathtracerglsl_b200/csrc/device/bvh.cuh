@@ -523,8 +523,15 @@ __device__ __forceinline__ bool flat_binary_ok(const DevScene& S, const DevBatch
 }
 
 // ---- region arms ------------------------------------------------------------------------
-__device__ __forceinline__ void accel_closest(const DevScene& S, const ptr_region& g, int region, const Ray& r, HitRec& h,
-                                              Work* w = nullptr) {
+// The per-scene kernels inline these arms; the library's generic kernels call them (ptx_rt.cu
+// defines PTR_ACCEL_CALL): inlined next to every other arm, the tree walks' registers spilled
+// across the region scans (fog with 256 lamps and a mesh, 512 x 384 x 8: 25.3 ms inlined, 20.7
+// called).
+#ifndef PTR_ACCEL_CALL
+#define PTR_ACCEL_CALL __forceinline__
+#endif
+__device__ PTR_ACCEL_CALL HitRec accel_closest(const DevScene& S, const ptr_region& g, int region, Ray r, HitRec h,
+                                               Work* w = nullptr) {
     if (kHasMesh && g.shape == PTR_SHAPE_MESH) {
         const DevMesh& m = S.meshes[g.ref];
         int prim = -1;
@@ -535,11 +542,11 @@ __device__ __forceinline__ void accel_closest(const DevScene& S, const ptr_regio
             h.element = 0;
             h.prim = prim;
         }
-        return;
+        return h;
     }
     const DevBatch& b = S.batches[g.ref];
-    if (flat_wide_ok(S, b)) { flat_walk<true, false>(S, b, region, r, h, 0.0f, w); return; }
-    if (flat_binary_ok(S, b)) { flat_walk<false, false>(S, b, region, r, h, 0.0f, w); return; }
+    if (flat_wide_ok(S, b)) { flat_walk<true, false>(S, b, region, r, h, 0.0f, w); return h; }
+    if (flat_binary_ok(S, b)) { flat_walk<false, false>(S, b, region, r, h, 0.0f, w); return h; }
     float t_near = h.t;
     const bool wide = S.inst_accel == PTR_ACCEL_CWBVH && b.tlas_w;
     const float4* place = wide ? b.place_w : b.place;
@@ -570,15 +577,16 @@ __device__ __forceinline__ void accel_closest(const DevScene& S, const ptr_regio
     };
     if (wide) {   // the reference's CWBVH instance accel (intersection/index.ts:99-158)
         walk_wide(S, b.tlas_w, r.o, r.d, t_near, [&](int i) { instance(i); return false; }, w ? &w->tlas : nullptr);
-        return;
+        return h;
     }
     walk_binary(S, b.tlas, r.o, r.d, t_near, [&](int off, int cnt) {
         for (int i = off; i < off + cnt; ++i) instance(i);
         return false;
     }, w ? &w->tlas : nullptr);
+    return h;
 }
 
-__device__ __forceinline__ bool accel_any(const DevScene& S, const ptr_region& g, const Ray& r, float max_dist,
+__device__ PTR_ACCEL_CALL bool accel_any(const DevScene& S, const ptr_region& g, Ray r, float max_dist,
                                           Work* w = nullptr) {
     if (kHasMesh && g.shape == PTR_SHAPE_MESH) return mesh_any(S, S.meshes[g.ref], r.o, r.d, max_dist, w);
     const DevBatch& b = S.batches[g.ref];
@@ -611,7 +619,7 @@ __device__ __forceinline__ bool accel_any(const DevScene& S, const ptr_region& g
 // Containment of an instanced SPHERE batch (the TLAS point descent of scene_region_at):
 // the least-negative signed distance among the instances that contain p, else 1e20.
 // Mesh batches are thin (no containment).
-__device__ __forceinline__ float accel_region_sdf(const DevScene& S, const ptr_region& g, f3 p) {
+__device__ PTR_ACCEL_CALL float accel_region_sdf(const DevScene& S, const ptr_region& g, f3 p) {
     const DevBatch& b = S.batches[g.ref];
     if (b.proto_shape != PTR_SHAPE_SPHERE) return 1.0e20f;
     float best = -1.0e20f;

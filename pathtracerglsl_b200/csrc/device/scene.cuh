@@ -75,7 +75,7 @@ struct DevScene {
     int flat_region = -1;     // the one acceleration region when every other region is analytic
                               // and there is no region BVH (refilling closest-hit loop), else -1
     int has_het;              // some medium has a coefficient field (heterogeneous media)
-    int pad_i2;
+    int has_null;             // some region is a null interface (a shadow query may pass through it)
     float sort_c[4];          // centre of the bounded geometry (ray-coherence keys)
     // environment
     int env_kind, env_samplable, env_select_live, env_w;

@@ -347,7 +347,7 @@ __device__ __forceinline__ HitRec scene_closest(const DevScene& S, const Ray& r,
     };
     auto arm = [&](int i, const ptr_region& g, int shape) {
         if (has_accel() && shape >= PTR_SHAPE_MESH) {
-            accel_closest(S, g, i, r, h, w);
+            h = accel_closest(S, g, i, r, h, w);
             return;
         }
         float t;
@@ -837,7 +837,7 @@ __device__ __forceinline__ void closest_refill(const DevScene& S, const PathPool
 }
 
 template <bool COUNT, bool BATCH>
-__global__ void __launch_bounds__(256, PTR_TRACE_MIN_BLOCKS) k_closest(DevScene S0, PathPool pool, int in, BatchTables bt) {
+__global__ void __launch_bounds__(256, PTR_TRACE_MIN_BLOCKS) k_closest(const __grid_constant__ DevScene S0, PathPool pool, int in, BatchTables bt) {
     const int buckets = pool.sort_buckets;
     unsigned n = pool.cnt[in];
     if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -1431,7 +1431,7 @@ struct PoolSink {
 // memory: PTR_GRAD_SLOTS doubles per material).
 // Col: f3 (RGB) or s4 (spectral, four wavelength lanes; the adjoint is RGB only).
 template <class Col, int DIRECT, bool MEDIA, bool BATCH, bool ADJ = false>
-__global__ void __launch_bounds__(256, PTR_SHADE_MIN_BLOCKS) k_shade(DevScene S0, PathPool pool, ProgParams P0, int in, BatchTables bt,
+__global__ void __launch_bounds__(256, PTR_SHADE_MIN_BLOCKS) k_shade(const __grid_constant__ DevScene S0, PathPool pool, ProgParams P0, int in, BatchTables bt,
                                                                      AdjParams adj = AdjParams{}) {
     constexpr bool SPECTRAL = sizeof(Col) == sizeof(s4);
     static_assert(!(ADJ && SPECTRAL), "the adjoint replay is RGB only");
@@ -1565,39 +1565,51 @@ __device__ __forceinline__ Col shadow_visibility(const DevScene& S, const ProgPa
     Col T(1.0f);
     Rng srng;
     bool srng_live = false;
-    int medium = scene_region_at(S, sr.o);
+    // the medium of a segment attenuates only a query that gets past it: a query that an
+    // optical surface blocks is done without its point classification and transmittance
+    auto attenuate = [&](const Ray& seg, int medium, float seg_len) {
+        const int med_mat = material_of(S, medium);
+        if (!mat_has_medium(S, med_mat)) return;
+        bool het = false;
+        if constexpr (!SPECTRAL) {
+            const ptr_material& smm = S.materials[med_mat];
+            if (PTR_SPEC_HET && S.has_het && mat_is_het(smm)) {   // ratio tracking on the query's own stream
+                het = true;
+                if (!srng_live) { srng = seed_of(); srng_live = true; }
+                T = T * medium_ratio_track(S, smm, seg, seg_len, srng, scatter_live(S, P, med_mat));
+            }
+        }
+        if (!het) T = T * medium_transmittance<Col>(S, P, med_mat, seg_len, wl);
+        if (collect) {
+            int e = 0;
+            while (e < mm.n && mm.id[e] != med_mat) e++;
+            if (e < mm.n) mm.len[e] += seg_len;
+            else if (mm.n < kAdjMaxMedia) { mm.id[mm.n] = med_mat; mm.len[mm.n] = seg_len; mm.n++; }
+            else if (flag_more) flag_error(S, kErrAdjMedia);
+        }
+    };
+    if (!S.has_null) {   // every surface is optical: any hit before the light blocks the query
+        const float remaining = length(light_p - sr.o) - kShadowBackoff;
+        if (remaining <= 0.0f) return T;
+        if (scene_any(S, sr, gmin(remaining, kMaxDist), work)) return Col(0.0f);
+        attenuate(sr, scene_region_at(S, sr.o), remaining);
+        return T;
+    }
+    int medium = 0;
     Ray seg = sr;
     for (int crossed = 0; crossed <= crossings_left; crossed++) {
         float remaining = length(light_p - seg.o) - kShadowBackoff;
         if (remaining <= 0.0f) return T;
         HitRec hr = scene_closest(S, seg, work);
         bool hit_boundary = hr.region >= 0 && hr.t < remaining;
-        float seg_len = hit_boundary ? hr.t : remaining;
-        int med_mat = material_of(S, medium);
-        if (mat_has_medium(S, med_mat)) {
-            bool het = false;
-            if constexpr (!SPECTRAL) {
-                const ptr_material& smm = S.materials[med_mat];
-                if ((PTR_SPEC_HET && S.has_het) && mat_is_het(smm)) {   // ratio tracking on the query's own stream
-                    het = true;
-                    if (!srng_live) { srng = seed_of(); srng_live = true; }
-                    T = T * medium_ratio_track(S, smm, seg, seg_len, srng, scatter_live(S, P, med_mat));
-                }
-            }
-            if (!het) T = T * medium_transmittance<Col>(S, P, med_mat, seg_len, wl);
-            if (collect) {
-                int e = 0;
-                while (e < mm.n && mm.id[e] != med_mat) e++;
-                if (e < mm.n) mm.len[e] += seg_len;
-                else if (mm.n < kAdjMaxMedia) { mm.id[mm.n] = med_mat; mm.len[mm.n] = seg_len; mm.n++; }
-                else if (flag_more) flag_error(S, kErrAdjMedia);
-            }
+        // an optical surface blocks the query: decided from the hit region alone
+        if (hit_boundary) {
+            const int om = material_of(S, hr.region);
+            if (!(om >= 0 && S.materials[om].model == PTR_MAT_NONE)) return Col(0.0f);
         }
+        if (crossed == 0) medium = scene_region_at(S, sr.o);
+        attenuate(seg, medium, hit_boundary ? hr.t : remaining);
         if (!hit_boundary) return T;
-        // an optical surface blocks the query: decided from the hit region alone,
-        // before the hit's frame and its region classification
-        const int om = material_of(S, hr.region);
-        if (!(om >= 0 && S.materials[om].model == PTR_MAT_NONE)) return Col(0.0f);
         Hit h;
         fill_hit(S, seg, hr, h, false, true);
         medium = h.region_to;
@@ -1722,7 +1734,7 @@ __device__ __forceinline__ void shadow_refill(const DevScene& S, const PathPool&
 }
 
 template <class Col, bool MEDIA, bool COUNT, bool BATCH, bool ADJ = false>
-__global__ void __launch_bounds__(256, PTR_TRACE_MIN_BLOCKS) k_shadow(DevScene S0, PathPool pool, ProgParams P0, BatchTables bt,
+__global__ void __launch_bounds__(256, PTR_TRACE_MIN_BLOCKS) k_shadow(const __grid_constant__ DevScene S0, PathPool pool, ProgParams P0, BatchTables bt,
                                                                       int slot, AdjParams adj = AdjParams{}) {
     constexpr bool SPECTRAL = sizeof(Col) == sizeof(s4);
     static_assert(!(ADJ && SPECTRAL), "the adjoint replay is RGB only");
@@ -1868,7 +1880,7 @@ struct WalkSink {
 #define PTR_WALK_REFILL 1
 #endif
 template <class Col, int DIRECT, bool MEDIA, bool BATCH, bool ADJ = false>
-__global__ void __launch_bounds__(256, PTR_WALK_MIN_BLOCKS) k_walk(DevScene S0, ProgParams P0, FrameParams F0, BatchTables bt,
+__global__ void __launch_bounds__(256, PTR_WALK_MIN_BLOCKS) k_walk(const __grid_constant__ DevScene S0, ProgParams P0, FrameParams F0, BatchTables bt,
                                                                    WalkArgs wa, AdjParams adj = AdjParams{}) {
     constexpr bool SPECTRAL = sizeof(Col) == sizeof(s4);
     static_assert(!(ADJ && SPECTRAL), "the adjoint replay is RGB only");

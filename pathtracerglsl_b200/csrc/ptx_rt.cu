@@ -24,6 +24,7 @@
 #include <string>
 #include <dlfcn.h>
 
+#define PTR_ACCEL_CALL __noinline__   // the generic kernels call the acceleration arms (bvh.cuh)
 #include "device/wavefront.cuh"
 #include "device/lbvh.cuh"
 #include "device/rails.cuh"
@@ -2060,6 +2061,12 @@ int check_scene_desc(const ptr_scene_desc* d, std::string& why) {
 }
 }  // namespace
 
+static int scene_has_null(const ptr_scene_desc* d) {
+    for (int i = 0; i < d->n_regions; ++i)
+        if (d->materials[d->regions[i].material].model == PTR_MAT_NONE) return 1;
+    return 0;
+}
+
 static int upload_scene(ptr_ctx* ctx, const ptr_scene_desc* d, const ptr_rails* rails, ptr_scene** out);
 
 int ptr_upload_scene(ptr_ctx* ctx, const ptr_scene_desc* d, ptr_scene** out) { return upload_scene(ctx, d, nullptr, out); }
@@ -2120,6 +2127,7 @@ static int upload_scene(ptr_ctx* ctx, const ptr_scene_desc* d, const ptr_rails* 
     for (int i = 0; i < d->n_materials; ++i)
         if (d->materials[i].flags & PTR_MATF_MEDIUM) media = true;
     S.has_media = media ? 1 : 0;
+    S.has_null = scene_has_null(d);
     s->has_media = S.has_media;
     s->n_lights = d->n_lights;
     s->h_materials.assign(d->materials, d->materials + d->n_materials);
@@ -3055,6 +3063,7 @@ extern "C" int ptr_render_noalloc(const ptr_scene_desc* d, const ptr_program_des
     for (int i = 0; i < d->n_materials; ++i)
         if (d->materials[i].flags & PTR_MATF_MEDIUM) media = true;
     S.has_media = media ? 1 : 0;
+    S.has_null = scene_has_null(d);
     S.env_kind = d->env.kind;
     S.env_samplable = d->env.kind != PTR_ENV_NONE && d->env.sample_as_light;
     S.env_select_live = S.env_samplable && d->n_lights > 0;
