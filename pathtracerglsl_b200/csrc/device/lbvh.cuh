@@ -270,9 +270,12 @@ __device__ __forceinline__ float half_area(float4 a, float4 b) {
 }
 // counters: [0] wide nodes allocated, [1] leaf items placed, [2] next level's tasks,
 // [3] error flag (quantization range)
+// counters: [0] nodes, [1] items, [3] error flags, [4 + l] the tasks of level l.
+constexpr int kCollapseCounters = 32;
 __global__ void k_collapse(int n, const int* child, const int2* range, const float4* nlo, const float4* nhi,
-                           const unsigned long long* keys, const int2* tasks, int n_tasks, int2* next,
-                           unsigned* counters, uint32_t* nodes, uint32_t* order) {
+                           const unsigned long long* keys, const int2* tasks, int2* next,
+                           unsigned* counters, int level, uint32_t* nodes, uint32_t* order) {
+    const int n_tasks = (int)counters[4 + level];
     for (int ti = blockIdx.x * blockDim.x + threadIdx.x; ti < n_tasks; ti += gridDim.x * blockDim.x) {
         const int b = tasks[ti].x, w = tasks[ti].y;
         int mem[8];
@@ -329,7 +332,7 @@ __global__ void k_collapse(int n, const int* child, const int2* range, const flo
         if (ebx > 254 || eby > 254 || ebz > 254) { atomicOr(&counters[3], 1u); continue; }
         const int child_base = n_int ? (int)atomicAdd(&counters[0], (unsigned)n_int) : 0;
         const int prim_base = n_items ? (int)atomicAdd(&counters[1], (unsigned)n_items) : 0;
-        const int task_base = n_int ? (int)atomicAdd(&counters[2], (unsigned)n_int) : 0;
+        const int task_base = n_int ? (int)atomicAdd(&counters[4 + level + 1], (unsigned)n_int) : 0;
         const float sx = pow2_of(ebx), sy = pow2_of(eby), sz = pow2_of(ebz);
         uint32_t qlo[24], qhi[24], meta[8];
         for (int s = 0; s < 8; ++s) {

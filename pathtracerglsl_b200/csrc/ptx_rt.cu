@@ -12,6 +12,7 @@
 #include <cmath>
 #include <map>
 #include <mutex>
+#include <set>
 #include <tuple>
 #include <type_traits>
 #include <cstdio>
@@ -56,12 +57,18 @@ struct ptr_ctx {
     // by census key
     std::map<std::string, SpecKernels> batch_spec;
     int accel_build = PTR_BUILD_HOST;   // where ptr_upload_scene builds mesh BVHs (ptr_set_accel_build)
+    cudaMemPool_t pool = nullptr;       // the device's pool (acquire_pool)
+    std::set<void*> big;                // allocations outside it (kPoolMax)
 };
 
 struct ptr_scene {
     ptr_ctx* ctx = nullptr;
     DevScene dev{};
     std::vector<void*> allocs;
+    // the small tables' staged block (dev_copy): host image, its place on the device
+    std::vector<unsigned char> stage;
+    unsigned char* stage_dev = nullptr;
+    size_t stage_used = 0, stage_left = 0;
     int has_media = 0;
     bool has_mesh = false;   // some region is a triangle mesh or instances one
     bool walk = false;       // rendered by the one-kernel walk
@@ -147,15 +154,106 @@ int cuda_fail(ptr_ctx* ctx, cudaError_t e, const char* what) {
         if (e_ != cudaSuccess) return cuda_fail((ctx), e_, #call); \
     } while (0)
 
+// Device memory of the contexts' objects.  A scene, program or build takes a few dozen blocks,
+// and cudaMalloc / cudaFree cost 0.1 to several ms each (38 of each made 18 of the 25 ms of
+// uploading a 327,680-triangle scene).  So the contexts on one device share a stream-ordered
+// pool: allocating and freeing is then a few microseconds while it holds enough.  It keeps at
+// most kPoolKeep bytes that no object uses and goes with the device's last context.  Blocks
+// above kPoolMax come from cudaMalloc: the pool maps memory in small pieces, and the 8.7 GB
+// path pool of a 2^25-path wave took 80 ms from it against 5.
+constexpr unsigned long long kPoolKeep = 512ull << 20;
+constexpr size_t kPoolMax = 256ull << 20;
+constexpr int kPoolDevices = 64;
+struct DevicePool { cudaMemPool_t pool = nullptr; int users = 0; };
+std::mutex g_pool_mutex;
+DevicePool g_pools[kPoolDevices];
+cudaMemPool_t acquire_pool(int device) {
+    if (device >= kPoolDevices) return nullptr;
+    std::lock_guard<std::mutex> lock(g_pool_mutex);
+    DevicePool& d = g_pools[device];
+    if (!d.pool) {
+        cudaMemPoolProps props{};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = device;
+        unsigned long long keep = kPoolKeep;
+        if (cudaMemPoolCreate(&d.pool, &props) != cudaSuccess) { d.pool = nullptr; return nullptr; }
+        if (cudaMemPoolSetAttribute(d.pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
+            cudaMemPoolDestroy(d.pool);
+            d.pool = nullptr;
+            return nullptr;
+        }
+    }
+    ++d.users;
+    return d.pool;
+}
+void release_pool(int device) {
+    std::lock_guard<std::mutex> lock(g_pool_mutex);
+    DevicePool& d = g_pools[device];
+    if (--d.users > 0) return;
+    cudaMemPoolDestroy(d.pool);
+    d.pool = nullptr;
+}
+
+// Memory of a context's object, ordered on its stream (every use is).
 template <typename T>
-int dev_copy(ptr_ctx* ctx, std::vector<void*>& allocs, const T* host, size_t n, const T** out) {
+cudaError_t dev_alloc(ptr_ctx* ctx, T** out, size_t bytes) {
+    void* p = nullptr;
+    const bool big = bytes > kPoolMax;
+    const cudaError_t e = big ? cudaMalloc(&p, bytes) : cudaMallocFromPoolAsync(&p, bytes, ctx->pool, ctx->stream);
+    if (e != cudaSuccess) { p = nullptr; cudaGetLastError(); }
+    else if (big) ctx->big.insert(p);
+    *out = (T*)p;
+    return e;
+}
+void dev_free(ptr_ctx* ctx, void* p) {
+    if (!p) return;
+    if (ctx->big.erase(p)) cudaFree(p);
+    else cudaFreeAsync(p, ctx->stream);
+}
+
+// A device copy of a host array that lives with the scene.  Tables up to kStageMax bytes are
+// laid into one staged block (one allocation and one copy for a scene's dozens of small
+// tables); they are on the device after flush_stage.  Larger arrays are copied on the spot.  The
+// caller synchronises the stream before the host array may go.
+constexpr size_t kStageMax = 32u << 10, kStageBlock = 256u << 10;
+int flush_stage(ptr_scene* s) {
+    if (s->stage_used == 0) return PTR_OK;
+    CK(s->ctx, cudaMemcpyAsync(s->stage_dev, s->stage.data(), s->stage_used, cudaMemcpyHostToDevice, s->ctx->stream));
+    // a pageable source is staged by the copy itself, so the block's host image may be reused
+    s->stage_dev += s->stage_used;
+    s->stage_left -= s->stage_used;
+    s->stage_used = 0;
+    return PTR_OK;
+}
+template <typename T>
+int dev_copy(ptr_scene* s, const T* host, size_t n, const T** out) {
+    ptr_ctx* ctx = s->ctx;
     *out = nullptr;
     if (n == 0) return PTR_OK;
-    void* p = nullptr;
-    cudaError_t e = cudaMalloc(&p, n * sizeof(T));
-    if (e != cudaSuccess) return fail(ctx, PTR_E_NOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
-    allocs.push_back(p);
-    CK(ctx, cudaMemcpy(p, host, n * sizeof(T), cudaMemcpyHostToDevice));
+    const size_t bytes = n * sizeof(T), room = (bytes + 255) / 256 * 256;
+    const bool staged = bytes <= kStageMax;
+    if (staged && s->stage_left >= s->stage_used + room) {
+        std::memcpy(s->stage.data() + s->stage_used, host, bytes);
+        *out = (const T*)(s->stage_dev + s->stage_used);
+        s->stage_used += room;
+        return PTR_OK;
+    }
+    if (staged) {
+        if (int rc = flush_stage(s)) return rc;
+    }
+    unsigned char* p = nullptr;
+    cudaError_t e = dev_alloc(ctx, &p, staged ? kStageBlock : bytes);
+    if (e != cudaSuccess) return fail(ctx, PTR_E_NOMEM, std::string("device allocation: ") + cudaGetErrorString(e));
+    s->allocs.push_back(p);
+    if (staged) {
+        s->stage.resize(kStageBlock);
+        s->stage_dev = p;
+        s->stage_left = kStageBlock;
+        s->stage_used = 0;
+        return dev_copy(s, host, n, out);
+    }
+    CK(ctx, cudaMemcpyAsync(p, host, bytes, cudaMemcpyHostToDevice, ctx->stream));
     *out = (const T*)p;
     return PTR_OK;
 }
@@ -228,7 +326,7 @@ void bind_ctl(ptr_program* p) {
 }
 int ensure_ctl(ptr_program* p) {
     if (!p->ctl) {
-        if (cudaMalloc(&p->ctl, kCtlBytes) != cudaSuccess) { p->ctl = nullptr; return fail(p->ctx, PTR_E_NOMEM, "control block cudaMalloc"); }
+        if (dev_alloc(p->ctx, &p->ctl, kCtlBytes) != cudaSuccess) return fail(p->ctx, PTR_E_NOMEM, "control block allocation failed");
     }
     bind_ctl(p);
     return PTR_OK;
@@ -236,23 +334,21 @@ int ensure_ctl(ptr_program* p) {
 // The one-kernel walk's film record: 16 bytes per path of a wave (32 more with AOVs).
 int ensure_walk(ptr_program* p, size_t cap, bool aov) {
     if (p->walk_cap < cap) {
-        cudaFree(p->walk_film);
-        p->walk_film = nullptr;
+        dev_free(p->ctx, p->walk_film);
         p->walk_cap = 0;
-        if (cudaMalloc(&p->walk_film, cap * sizeof(float4)) != cudaSuccess) return fail(p->ctx, PTR_E_NOMEM, "walk film cudaMalloc");
+        if (dev_alloc(p->ctx, &p->walk_film, cap * sizeof(float4)) != cudaSuccess) return fail(p->ctx, PTR_E_NOMEM, "walk film allocation failed");
         p->walk_cap = cap;
     }
     if (aov && p->walk_aov_cap < cap) {
-        cudaFree(p->walk_aov);
-        p->walk_aov = nullptr;
+        dev_free(p->ctx, p->walk_aov);
         p->walk_aov_cap = 0;
-        if (cudaMalloc(&p->walk_aov, cap * 2 * sizeof(float4)) != cudaSuccess) return fail(p->ctx, PTR_E_NOMEM, "AOV pool allocation failed");
+        if (dev_alloc(p->ctx, &p->walk_aov, cap * 2 * sizeof(float4)) != cudaSuccess) return fail(p->ctx, PTR_E_NOMEM, "AOV pool allocation failed");
         p->walk_aov_cap = cap;
     }
     return PTR_OK;
 }
 void free_pool(ptr_program* p) {
-    for (void* a : p->pool_allocs) cudaFree(a);
+    for (void* a : p->pool_allocs) dev_free(p->ctx, a);
     p->pool_allocs.clear();
     p->pool = PathPool{};
     if (p->ctl) bind_ctl(p);
@@ -264,54 +360,68 @@ int alloc_pool(ptr_program* p, int capacity, bool slot2, bool adj = false, bool 
     free_pool(p);
     ptr_ctx* ctx = p->ctx;
     if (int r = ensure_ctl(p)) return r;
-    auto get = [&](size_t bytes, void** out) -> int {
-        cudaError_t e = cudaMalloc(out, bytes);
-        if (e != cudaSuccess) return fail(ctx, PTR_E_NOMEM, std::string("path pool cudaMalloc: ") + cudaGetErrorString(e));
-        p->pool_allocs.push_back(*out);
-        return PTR_OK;
-    };
-    size_t c = (size_t)capacity;
+    // one block, carved twice: for its size, then for the arrays
+    const size_t c = (size_t)capacity;
     PathPool& q = p->pool;
-    int rc = PTR_OK;
-    // a two-field record: 32 bytes per path, the first field at +0, the second at +16
-    auto pair = [&](auto& a, auto& b) -> int {
-        void* base = nullptr;
-        if (int r = get(c * 32, &base)) return r;
-        a.p = (std::remove_reference_t<decltype(*a.p)>*)base;
-        b.p = (std::remove_reference_t<decltype(*b.p)>*)((char*)base + 16);
-        return PTR_OK;
+    auto carve = [&](unsigned char* base) -> size_t {
+        size_t at = 0;
+        auto get = [&](size_t bytes, auto& out) {
+            out = base ? (std::remove_reference_t<decltype(out)>)(base + at) : nullptr;
+            at += (bytes + 255) / 256 * 256;
+        };
+        // a two-field record: 32 bytes per path, the first field at +0, the second at +16
+        auto pair = [&](auto& f, auto& g) {
+            unsigned char* rec = nullptr;
+            get(c * 32, rec);
+            f.p = (std::remove_reference_t<decltype(*f.p)>*)rec;
+            g.p = rec ? (std::remove_reference_t<decltype(*g.p)>*)(rec + 16) : nullptr;
+        };
+        pair(q.ray_o, q.ray_d);
+        pair(q.thr, q.rad);
+        pair(q.prev_q, q.st);
+        pair(q.hit, q.hit_i);
+        pair(q.sh_o, q.sh_d);
+        pair(q.sh_lp, q.sh_c);
+        get(c * 16, q.prev_n);
+        get(c * 8, q.rng);
+        get(c * 4, q.sh_seed);
+        get(c * 4, q.q[0]);
+        get(c * 4, q.q[1]);
+        get(c * 4, q.shq);
+        get(c * 4, q.q_sorted);
+        get(c * 4, q.q_ray);
+        get(c * 4, q.shq_s);
+        get(c, q.sort_key);
+        get(c, q.rkey);
+        get(c, q.skey);
+        get((size_t)kMaxKeys * kSortChunks * sizeof(unsigned), q.sort_hist);
+        if (slot2) {      // the second shadow slot: programs with the per-segment equiangular site
+            pair(q.sh2_o, q.sh2_d);
+            pair(q.sh2_lp, q.sh2_c);
+            get(c * 4, q.shq2);
+        }
+        if (adj) {        // the adjoint replay's per-path records
+            get(c * 16, q.l_rem);
+            get(c * 16, q.dl);
+            get(c * 16, q.sh_g);
+            get(c * 4, q.sh_gm);
+        }
+        if (spectral) {   // the spectral colour model's wavelengths and shadow pdfs
+            get(c * 16, q.wl);
+            get(c * 16, q.wl_pdf);
+            get(c * 4, q.sh_pdf);
+            get(c * 4, q.sh2_pdf);
+        }
+        return at;
     };
-    if ((rc = pair(q.ray_o, q.ray_d)) || (rc = pair(q.thr, q.rad)) ||
-        (rc = pair(q.prev_q, q.st)) || (rc = get(c * 16, (void**)&q.prev_n)) || (rc = get(c * 4, (void**)&q.sh_seed)) ||
-        (rc = get(c * 8, (void**)&q.rng)) || (rc = pair(q.hit, q.hit_i)) ||
-        (rc = pair(q.sh_o, q.sh_d)) || (rc = pair(q.sh_lp, q.sh_c)) || (rc = get(c * 4, (void**)&q.q[0])) ||
-        (rc = get(c * 4, (void**)&q.q[1])) || (rc = get(c * 4, (void**)&q.shq)) ||
-        (rc = get(c * 4, (void**)&q.q_sorted)) ||
-        (rc = get(c, (void**)&q.sort_key)) || (rc = get((size_t)kMaxKeys * kSortChunks * sizeof(unsigned), (void**)&q.sort_hist)) ||
-        (rc = get(c, (void**)&q.rkey)) ||
-        (rc = get(c, (void**)&q.skey)) || (rc = get(c * 4, (void**)&q.q_ray)) ||
-        (rc = get(c * 4, (void**)&q.shq_s))) {
+    unsigned char* block = nullptr;
+    const cudaError_t e = dev_alloc(ctx, &block, carve(nullptr));
+    if (e != cudaSuccess) {
         free_pool(p);
-        return rc;
+        return fail(ctx, PTR_E_NOMEM, std::string("path pool allocation: ") + cudaGetErrorString(e));
     }
-    // the second shadow slot only for programs with the per-segment equiangular site
-    if (slot2 && ((rc = pair(q.sh2_o, q.sh2_d)) || (rc = pair(q.sh2_lp, q.sh2_c)) ||
-                  (rc = get(c * 4, (void**)&q.shq2)))) {
-        free_pool(p);
-        return rc;
-    }
-    // the adjoint replay's per-path records
-    if (adj && ((rc = get(c * 16, (void**)&q.l_rem)) || (rc = get(c * 16, (void**)&q.dl)) ||
-                (rc = get(c * 16, (void**)&q.sh_g)) || (rc = get(c * 4, (void**)&q.sh_gm)))) {
-        free_pool(p);
-        return rc;
-    }
-    // the spectral colour model's wavelengths and shadow pdfs
-    if (spectral && ((rc = get(c * 16, (void**)&q.wl)) || (rc = get(c * 16, (void**)&q.wl_pdf)) ||
-                     (rc = get(c * 4, (void**)&q.sh_pdf)) || (rc = get(c * 4, (void**)&q.sh2_pdf)))) {
-        free_pool(p);
-        return rc;
-    }
+    p->pool_allocs.push_back(block);
+    carve(block);
     p->capacity = capacity;
     return PTR_OK;
 }
@@ -647,47 +757,59 @@ int build_mesh_device_core(ptr_ctx* ctx, ptr_scene* s, const float* d_pos, const
     const int grid = n_sm * 8, block = 256;
     int n_pad = kBitonicTile;
     while (n_pad < n) n_pad <<= 1;
-    std::vector<void*> tmp;
-    auto alloc = [&](size_t bytes, bool keep) -> void* {
-        void* p = nullptr;
-        if (cudaMalloc(&p, bytes) != cudaSuccess) return nullptr;
-        (keep ? s->allocs : tmp).push_back(p);
-        return p;
-    };
-    auto release = [&]() { for (void* p : tmp) cudaFree(p); tmp.clear(); };
+    static_assert(kCollapseCounters > 4 + ptx_host::kCwbvhStackDepth, "a task counter per level and one past the last");
     const int total = 2 * n - 1;
     const int n_int = std::max(n - 1, 1);
-    float4* lo = (float4*)alloc(sizeof(float4) * (size_t)n, false);
-    float4* hi = (float4*)alloc(sizeof(float4) * (size_t)n, false);
-    int* cb = (int*)alloc(sizeof(int) * 8, false);
-    unsigned long long* keys = (unsigned long long*)alloc(sizeof(unsigned long long) * (size_t)n_pad, false);
-    int* child = (int*)alloc(sizeof(int) * 2 * (size_t)n_int, false);
-    int* parent = (int*)alloc(sizeof(int) * (size_t)total, false);
-    int2* range = (int2*)alloc(sizeof(int2) * (size_t)total, false);
-    unsigned* arrivals = (unsigned*)alloc(sizeof(unsigned) * (size_t)n_int, false);
-    float4* nlo = (float4*)alloc(sizeof(float4) * (size_t)total, false);
-    float4* nhi = (float4*)alloc(sizeof(float4) * (size_t)total, false);
-    int2* ta = (int2*)alloc(sizeof(int2) * (size_t)n, false);
-    int2* tb = (int2*)alloc(sizeof(int2) * (size_t)n, false);
-    unsigned* counters = (unsigned*)alloc(sizeof(unsigned) * 8, false);
-    uint32_t* wide_big = (uint32_t*)alloc(sizeof(uint32_t) * 20 * (size_t)n, false);
-    uint32_t* order = (uint32_t*)alloc(sizeof(uint32_t) * (size_t)n, false);
-    float4* bvh = binary ? (float4*)alloc(sizeof(float4) * 2 * (size_t)total, true) : nullptr;
-    float4* tri = binary ? (float4*)alloc(sizeof(float4) * 3 * (size_t)n, true) : nullptr;
-    float4* tri_w = (float4*)alloc(sizeof(float4) * 3 * (size_t)n, true);
-    if (!lo || !hi || !cb || !keys || !child || !parent || !range ||
-        !arrivals || !nlo || !nhi || !ta || !tb || !counters || !wide_big || !order || (binary && (!bvh || !tri)) || !tri_w) {
-        release();
-        return fail(ctx, PTR_E_NOMEM, "scene: device BVH build: cudaMalloc");
-    }
+    float4 *lo, *hi, *nlo, *nhi;
+    int *cb, *child, *parent;
+    int2 *range, *ta, *tb;
+    unsigned long long* keys;
+    unsigned *arrivals, *counters;
+    uint32_t *wide_big, *order;
+    // the build's temporaries in one block, carved twice: for its size, then for the arrays
+    auto carve = [&](unsigned char* base) -> size_t {
+        size_t at = 0;
+        auto get = [&](size_t count, auto& out) {
+            out = (std::remove_reference_t<decltype(out)>)(base + at);
+            at += (count * sizeof(*out) + 255) / 256 * 256;
+        };
+        get((size_t)n, lo);
+        get((size_t)n, hi);
+        get((size_t)total, nlo);
+        get((size_t)total, nhi);
+        get((size_t)n_pad, keys);
+        get((size_t)total, range);
+        get((size_t)n, ta);
+        get((size_t)n, tb);
+        get(2 * (size_t)n_int, child);
+        get((size_t)total, parent);
+        get((size_t)n_int, arrivals);
+        get((size_t)8, cb);
+        get((size_t)kCollapseCounters, counters);
+        get(20 * (size_t)n, wide_big);
+        get((size_t)n, order);
+        return at;
+    };
+    unsigned char* tmp = nullptr;
+    auto release = [&]() { dev_free(ctx, tmp); tmp = nullptr; };
+    auto keep = [&](size_t bytes) -> void* {
+        void* p = nullptr;
+        if (dev_alloc(ctx, &p, bytes) == cudaSuccess) s->allocs.push_back(p);
+        return p;
+    };
+    float4* bvh = binary ? (float4*)keep(sizeof(float4) * 2 * (size_t)total) : nullptr;
+    float4* tri = binary ? (float4*)keep(sizeof(float4) * 3 * (size_t)n) : nullptr;
+    float4* tri_w = (float4*)keep(sizeof(float4) * 3 * (size_t)n);
+    if ((binary && (!bvh || !tri)) || !tri_w || dev_alloc(ctx, &tmp, carve(nullptr)) != cudaSuccess)
+        return fail(ctx, PTR_E_NOMEM, "scene: device BVH build: allocation failed");
+    carve(tmp);
     const int cb_init[8] = {0x7FFFFFFF, 0x7FFFFFFF, 0x7FFFFFFF, (int)0x80000000, (int)0x80000000, (int)0x80000000, 0, 0};
-    const unsigned cnt_init[8] = {1u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
+    unsigned cnt[kCollapseCounters] = {1u, 0u, 0u, 0u, 1u};   // one node (the root), one task on level 0
     const int2 root_task = make_int2(0, 0);   // binary node 0 (internal root, or the one leaf) -> wide node 0
     cudaError_t e = cudaMemcpyAsync(cb, cb_init, sizeof(cb_init), cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(counters, cnt_init, sizeof(cnt_init), cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(counters, cnt, sizeof(cnt), cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(ta, &root_task, sizeof(int2), cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = cudaMemsetAsync(arrivals, 0, sizeof(unsigned) * (size_t)n_int, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);   // the small host tables are copied before the launches
     if (e != cudaSuccess) { release(); return cuda_fail(ctx, e, "scene: device BVH build"); }
     k_boxes<<<grid, block, 0, st>>>(d_pos, d_idx, n, lo, hi, cb);
     k_keys<<<grid, block, 0, st>>>(lo, hi, n, n_pad, cb, keys);
@@ -700,34 +822,31 @@ int build_mesh_device_core(ptr_ctx* ctx, ptr_scene* s, const float* d_pos, const
     k_refit<<<grid, block, 0, st>>>(keys, lo, hi, n, child, parent, arrivals, nlo, nhi);
     int* depth_dev = cb + 6;   // the binary layout's deepest level (initialised to 0)
     if (binary) k_binary_layout<<<grid, block, 0, st>>>(n, child, parent, range, nlo, nhi, bvh, depth_dev);
-    // the wide nodes, one level of tasks per launch
-    int n_tasks = 1, levels = 0;
+    // the wide nodes, one level of tasks per launch: every level the walk's stack admits is
+    // launched, each reads its task count on the device (a level without tasks returns at
+    // once), so the host waits once instead of once per level
     int2 *tin = ta, *tout = tb;
-    unsigned cnt[4] = {0u, 0u, 0u, 0u};
-    e = cudaGetLastError();
-    while (n_tasks > 0 && e == cudaSuccess) {
-        if (++levels > 64) { cnt[3] |= 2u; break; }
-        e = cudaMemsetAsync(counters + 2, 0, sizeof(unsigned), st);
-        if (e != cudaSuccess) break;
-        k_collapse<<<std::min(grid, (n_tasks + block - 1) / block), block, 0, st>>>(n, child, range, nlo, nhi, keys, tin, n_tasks,
-                                                                                   tout, counters, wide_big, order);
-        e = cudaMemcpyAsync(cnt, counters, sizeof(cnt), cudaMemcpyDeviceToHost, st);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-        n_tasks = (int)cnt[2];
+    for (int l = 0; l < ptx_host::kCwbvhStackDepth; ++l) {
+        k_collapse<<<grid, block, 0, st>>>(n, child, range, nlo, nhi, keys, tin, tout, counters, l, wide_big, order);
         std::swap(tin, tout);
     }
+    e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaMemcpyAsync(cnt, counters, sizeof(cnt), cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    int levels = 0;
+    while (levels < ptx_host::kCwbvhStackDepth && cnt[4 + levels] > 0u) ++levels;
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) { release(); return cuda_fail(ctx, e, "scene: device BVH build"); }
-    if (cnt[3] != 0u || cnt[1] != (unsigned)n || cnt[0] == 0u || cnt[0] > (unsigned)std::max(n, 1)) {
-        release();
-        return fail(ctx, PTR_E_INVALID, "scene: device CWBVH build failed (exponent range, depth or item count)");
-    }
     if (levels >= ptx_host::kCwbvhStackDepth) {
         release();
         return fail(ctx, PTR_E_INVALID, "scene: device CWBVH depth " + std::to_string(levels) + " reaches the walk's stack depth");
     }
-    uint32_t* wide = (uint32_t*)alloc(sizeof(uint32_t) * 20 * (size_t)cnt[0], true);
-    if (!wide) { release(); return fail(ctx, PTR_E_NOMEM, "scene: device BVH build: cudaMalloc"); }
+    if (cnt[3] != 0u || cnt[1] != (unsigned)n || cnt[0] == 0u || cnt[0] > (unsigned)std::max(n, 1)) {
+        release();
+        return fail(ctx, PTR_E_INVALID, "scene: device CWBVH build failed (exponent range, depth or item count)");
+    }
+    uint32_t* wide = (uint32_t*)keep(sizeof(uint32_t) * 20 * (size_t)cnt[0]);
+    if (!wide) { release(); return fail(ctx, PTR_E_NOMEM, "scene: device BVH build: allocation failed"); }
     e = cudaMemcpyAsync(wide, wide_big, sizeof(uint32_t) * 20 * (size_t)cnt[0], cudaMemcpyDeviceToDevice, st);
     if (binary) k_emit_tris<<<grid, block, 0, st>>>(d_pos, d_idx, d_alpha, nullptr, keys, n, tri);
     k_emit_tris<<<grid, block, 0, st>>>(d_pos, d_idx, d_alpha, order, keys, n, tri_w);
@@ -762,10 +881,10 @@ int build_mesh_device(ptr_ctx* ctx, ptr_scene* s, const ptr_mesh_desc& md, DevMe
     float* d_pos = nullptr;
     unsigned* d_idx = nullptr;
     float* d_alpha = nullptr;
-    auto release = [&]() { cudaFree(d_pos); cudaFree(d_idx); cudaFree(d_alpha); };
-    if (cudaMalloc(&d_pos, sizeof(float) * 3 * (size_t)md.n_vertices) != cudaSuccess ||
-        cudaMalloc(&d_idx, sizeof(unsigned) * 3 * (size_t)n) != cudaSuccess ||
-        (md.tri_alpha && cudaMalloc(&d_alpha, sizeof(float) * (size_t)n) != cudaSuccess)) {
+    auto release = [&]() { dev_free(ctx, d_pos); dev_free(ctx, d_idx); dev_free(ctx, d_alpha); };
+    if (dev_alloc(ctx, &d_pos, sizeof(float) * 3 * (size_t)md.n_vertices) != cudaSuccess ||
+        dev_alloc(ctx, &d_idx, sizeof(unsigned) * 3 * (size_t)n) != cudaSuccess ||
+        (md.tri_alpha && dev_alloc(ctx, &d_alpha, sizeof(float) * (size_t)n) != cudaSuccess)) {
         release();
         return fail(ctx, PTR_E_NOMEM, "scene: device BVH build: cudaMalloc");
     }
@@ -873,14 +992,14 @@ int rail_mesh(ptr_ctx* ctx, ptr_scene* s, const ptr_rails& R, const RailDev& D, 
     unsigned* d_idx = nullptr;
     uint32_t* d_order = nullptr;
     float* d_alpha = nullptr;
-    auto release = [&]() { cudaFree(d_pos); cudaFree(d_idx); cudaFree(d_order); cudaFree(d_alpha); };
+    auto release = [&]() { dev_free(ctx, d_pos); dev_free(ctx, d_idx); dev_free(ctx, d_order); dev_free(ctx, d_alpha); };
     float4* tri = nullptr;
-    if (cudaMalloc(&d_pos, sizeof(float) * 3 * (size_t)V) != cudaSuccess ||
-        cudaMalloc(&d_idx, sizeof(unsigned) * 3 * (size_t)T) != cudaSuccess ||
-        (rm.tri_order && cudaMalloc(&d_order, sizeof(uint32_t) * (size_t)T) != cudaSuccess) ||
-        (rm.tri_alpha && cudaMalloc(&d_alpha, sizeof(float) * (size_t)T) != cudaSuccess) ||
-        cudaMalloc(&tri, sizeof(float4) * 3 * (size_t)T) != cudaSuccess) {
-        if (tri) cudaFree(tri);
+    if (dev_alloc(ctx, &d_pos, sizeof(float) * 3 * (size_t)V) != cudaSuccess ||
+        dev_alloc(ctx, &d_idx, sizeof(unsigned) * 3 * (size_t)T) != cudaSuccess ||
+        (rm.tri_order && dev_alloc(ctx, &d_order, sizeof(uint32_t) * (size_t)T) != cudaSuccess) ||
+        (rm.tri_alpha && dev_alloc(ctx, &d_alpha, sizeof(float) * (size_t)T) != cudaSuccess) ||
+        dev_alloc(ctx, &tri, sizeof(float4) * 3 * (size_t)T) != cudaSuccess) {
+        dev_free(ctx, tri);
         release();
         return fail(ctx, PTR_E_NOMEM, who + ": cudaMalloc");
     }
@@ -914,9 +1033,9 @@ int rail_mesh(ptr_ctx* ctx, ptr_scene* s, const ptr_rails& R, const RailDev& D, 
     if (ml) {
         float4* lt = nullptr;
         float* cdf = nullptr;
-        if (cudaMalloc(&lt, sizeof(float4) * 3 * (size_t)T) != cudaSuccess) return fail(ctx, PTR_E_NOMEM, who + ": cudaMalloc");
+        if (dev_alloc(ctx, &lt, sizeof(float4) * 3 * (size_t)T) != cudaSuccess) return fail(ctx, PTR_E_NOMEM, who + ": cudaMalloc");
         s->allocs.push_back(lt);
-        if (cudaMalloc(&cdf, sizeof(float) * (size_t)T) != cudaSuccess) return fail(ctx, PTR_E_NOMEM, who + ": cudaMalloc");
+        if (dev_alloc(ctx, &cdf, sizeof(float) * (size_t)T) != cudaSuccess) return fail(ctx, PTR_E_NOMEM, who + ": cudaMalloc");
         s->allocs.push_back(cdf);
         rails::k_light_tris<<<n_sm * 4, 256, 0, st>>>(D.v, ml->wpos_base, D.idx, rm.tbase, T, lt);
         rails::k_scalars<<<n_sm * 4, 256, 0, st>>>(D.rec, ml->cdf_base, T, cdf);
@@ -987,7 +1106,7 @@ int rail_batch(ptr_ctx* ctx, ptr_scene* s, const ptr_rails& R, const RailDev& D,
         b.place = D.rec + rb.placements_base;
     } else {
         float4* place = nullptr;
-        if (cudaMalloc(&place, sizeof(float4) * 2 * (size_t)N) != cudaSuccess) return fail(ctx, PTR_E_NOMEM, who + ": cudaMalloc");
+        if (dev_alloc(ctx, &place, sizeof(float4) * 2 * (size_t)N) != cudaSuccess) return fail(ctx, PTR_E_NOMEM, who + ": cudaMalloc");
         s->allocs.push_back(place);
         rails::k_restride<<<n_sm * 4, 256, 0, ctx->stream>>>(D.rec, rb.placements_base, N, place);
         if (cudaError_t e = cudaGetLastError()) return cuda_fail(ctx, e, who.c_str());
@@ -995,14 +1114,14 @@ int rail_batch(ptr_ctx* ctx, ptr_scene* s, const ptr_rails& R, const RailDev& D,
     }
     b.tlas = D.nodes + rb.tlas_base;
     const int* pi = nullptr;
-    if ((rc = dev_copy(ctx, s->allocs, ids.data(), ids.size(), &pi))) return rc;
+    if ((rc = dev_copy(s, ids.data(), ids.size(), &pi))) return rc;
     b.inst_id = pi;
     b.light_of = nullptr;
     b.light_of_w = nullptr;
     if (bd.light_base >= 0) {
         std::vector<int> lo((size_t)N);
         for (int i = 0; i < N; ++i) lo[(size_t)i] = bd.light_base + ids[(size_t)i];
-        if ((rc = dev_copy(ctx, s->allocs, lo.data(), lo.size(), &pi))) return rc;
+        if ((rc = dev_copy(s, lo.data(), lo.size(), &pi))) return rc;
         b.light_of = pi;
     }
     // the wide twin over the leaf slots' boxes; its leaves index leaf slots
@@ -1023,18 +1142,18 @@ int rail_batch(ptr_ctx* ctx, ptr_scene* s, const ptr_rails& R, const RailDev& D,
         }
         const float4* p4 = nullptr;
         const uint4* u4 = nullptr;
-        if ((rc = dev_copy(ctx, s->allocs, rec_w.data(), rec_w.size(), &p4))) return rc;
+        if ((rc = dev_copy(s, rec_w.data(), rec_w.size(), &p4))) return rc;
         b.place_w = p4;
-        if ((rc = dev_copy(ctx, s->allocs, ids_w.data(), ids_w.size(), &pi))) return rc;
+        if ((rc = dev_copy(s, ids_w.data(), ids_w.size(), &pi))) return rc;
         b.inst_id_w = pi;
         std::vector<int> slots(wt.order.begin(), wt.order.begin() + N);
-        if ((rc = dev_copy(ctx, s->allocs, slots.data(), slots.size(), &pi))) return rc;
+        if ((rc = dev_copy(s, slots.data(), slots.size(), &pi))) return rc;
         b.slot_of_w = pi;
         if (bd.light_base >= 0) {
-            if ((rc = dev_copy(ctx, s->allocs, lo_w.data(), lo_w.size(), &pi))) return rc;
+            if ((rc = dev_copy(s, lo_w.data(), lo_w.size(), &pi))) return rc;
             b.light_of_w = pi;
         }
-        if ((rc = dev_copy(ctx, s->allocs, (const uint4*)wt.nodes.data(), 5 * (size_t)wt.node_count, &u4))) return rc;
+        if ((rc = dev_copy(s, (const uint4*)wt.nodes.data(), 5 * (size_t)wt.node_count, &u4))) return rc;
         b.tlas_w = u4;
     }
     b.n_inst = N;
@@ -1054,11 +1173,12 @@ int upload_accels(ptr_ctx* ctx, ptr_scene* s, const ptr_scene_desc* d, const ptr
     RailDev rd;
     if (rails) {   // each channel to the device once, as the App packed it
         int rc0;
-        if ((rails->vertices_texels > 0 && (rc0 = dev_copy(ctx, s->allocs, (const float4*)rails->vertices, (size_t)rails->vertices_texels, &rd.v))) ||
-            (rails->indices_texels > 0 && (rc0 = dev_copy(ctx, s->allocs, (const float4*)rails->indices, (size_t)rails->indices_texels, &rd.idx))) ||
-            (rails->nodes_texels > 0 && (rc0 = dev_copy(ctx, s->allocs, (const float4*)rails->nodes, (size_t)rails->nodes_texels, &rd.nodes))) ||
-            (rails->records_texels > 0 && (rc0 = dev_copy(ctx, s->allocs, (const float4*)rails->records, (size_t)rails->records_texels, &rd.rec))))
+        if ((rails->vertices_texels > 0 && (rc0 = dev_copy(s, (const float4*)rails->vertices, (size_t)rails->vertices_texels, &rd.v))) ||
+            (rails->indices_texels > 0 && (rc0 = dev_copy(s, (const float4*)rails->indices, (size_t)rails->indices_texels, &rd.idx))) ||
+            (rails->nodes_texels > 0 && (rc0 = dev_copy(s, (const float4*)rails->nodes, (size_t)rails->nodes_texels, &rd.nodes))) ||
+            (rails->records_texels > 0 && (rc0 = dev_copy(s, (const float4*)rails->records, (size_t)rails->records_texels, &rd.rec))))
             return rc0;
+        if (int rc1 = flush_stage(s)) return rc1;   // device gathers read the channels
     }
     // the bounded geometry's box: its centre splits ray origins into octants for the
     // ray-coherence queue keys
@@ -1125,13 +1245,13 @@ int upload_accels(ptr_ctx* ctx, ptr_scene* s, const ptr_scene_desc* d, const ptr
             if (wide.error) return fail(ctx, PTR_E_INVALID, "scene: CWBVH build failed (exponent range or DP invariant)");
             std::vector<float4> tri_b = tri_array(bin.order), tri_w = tri_array(wide.order);
             const uint4* u4 = nullptr;
-            if ((rc = dev_copy(ctx, s->allocs, tri_b.data(), tri_b.size(), &p4))) return rc;
+            if ((rc = dev_copy(s, tri_b.data(), tri_b.size(), &p4))) return rc;
             m.tri = p4;
-            if ((rc = dev_copy(ctx, s->allocs, tri_w.data(), tri_w.size(), &p4))) return rc;
+            if ((rc = dev_copy(s, tri_w.data(), tri_w.size(), &p4))) return rc;
             m.tri_w = p4;
-            if ((rc = dev_copy(ctx, s->allocs, (const float4*)bin.nodes.data(), 2 * (size_t)bin.node_count, &p4))) return rc;
+            if ((rc = dev_copy(s, (const float4*)bin.nodes.data(), 2 * (size_t)bin.node_count, &p4))) return rc;
             m.bvh = p4;
-            if ((rc = dev_copy(ctx, s->allocs, (const uint4*)wide.nodes.data(), 5 * (size_t)wide.node_count, &u4))) return rc;
+            if ((rc = dev_copy(s, (const uint4*)wide.nodes.data(), 5 * (size_t)wide.node_count, &u4))) return rc;
             m.cwbvh = u4;
             n_nodes = bin.node_count;
             n_cw_nodes = wide.node_count;
@@ -1167,9 +1287,9 @@ int upload_accels(ptr_ctx* ctx, ptr_scene* s, const ptr_scene_desc* d, const ptr
             }
             cdf[T - 1] = 1.0f;
             const float* pf = nullptr;
-            if ((rc = dev_copy(ctx, s->allocs, cdf.data(), cdf.size(), &pf))) return rc;
+            if ((rc = dev_copy(s, cdf.data(), cdf.size(), &pf))) return rc;
             m.light_cdf = pf;
-            if ((rc = dev_copy(ctx, s->allocs, lt.data(), lt.size(), &p4))) return rc;
+            if ((rc = dev_copy(s, lt.data(), lt.size(), &p4))) return rc;
             m.light_tri = p4;
         }
         m.n_tris = T;
@@ -1244,20 +1364,20 @@ int upload_accels(ptr_ctx* ctx, ptr_scene* s, const ptr_scene_desc* d, const ptr
             std::vector<int> lo(N);
             for (int i = 0; i < N; ++i) lo[i] = bd.light_base + (int)tl.order[i];
             const int* pi = nullptr;
-            if ((rc = dev_copy(ctx, s->allocs, lo.data(), lo.size(), &pi))) return rc;
+            if ((rc = dev_copy(s, lo.data(), lo.size(), &pi))) return rc;
             b.light_of = pi;
         }
-        if ((rc = dev_copy(ctx, s->allocs, rec_leaf.data(), rec_leaf.size(), &p4))) return rc;
+        if ((rc = dev_copy(s, rec_leaf.data(), rec_leaf.size(), &p4))) return rc;
         b.place = p4;
         {
             std::vector<int> ids(tl.order.begin(), tl.order.begin() + N);
             const int* pi = nullptr;
-            if ((rc = dev_copy(ctx, s->allocs, ids.data(), ids.size(), &pi))) return rc;
+            if ((rc = dev_copy(s, ids.data(), ids.size(), &pi))) return rc;
             b.inst_id = pi;
         }
         b.inst_id_w = nullptr;
         b.slot_of_w = nullptr;
-        if ((rc = dev_copy(ctx, s->allocs, (const float4*)tl.nodes.data(), 2 * (size_t)tl.node_count, &p4))) return rc;
+        if ((rc = dev_copy(s, (const float4*)tl.nodes.data(), 2 * (size_t)tl.node_count, &p4))) return rc;
         b.tlas = p4;
         // the compressed wide twin of the TLAS (instanceAccel 'cwbvh', cwbvh.ts:80-372 over
         // the same instance boxes) with the placements in its leaf order
@@ -1271,25 +1391,25 @@ int upload_accels(ptr_ctx* ctx, ptr_scene* s, const ptr_scene_desc* d, const ptr
                 rec_w[2 * (size_t)i + 1] = rec[2 * (size_t)wt.order[i] + 1];
             }
             const uint4* u4 = nullptr;
-            if ((rc = dev_copy(ctx, s->allocs, rec_w.data(), rec_w.size(), &p4))) return rc;
+            if ((rc = dev_copy(s, rec_w.data(), rec_w.size(), &p4))) return rc;
             b.place_w = p4;
             std::vector<int> ids(wt.order.begin(), wt.order.begin() + N);
             const int* pid = nullptr;
-            if ((rc = dev_copy(ctx, s->allocs, ids.data(), ids.size(), &pid))) return rc;
+            if ((rc = dev_copy(s, ids.data(), ids.size(), &pid))) return rc;
             b.inst_id_w = pid;
             std::vector<int> slot_of(N), slots(N);
             for (int i = 0; i < N; ++i) slot_of[tl.order[i]] = i;
             for (int i = 0; i < N; ++i) slots[i] = slot_of[wt.order[i]];
-            if ((rc = dev_copy(ctx, s->allocs, slots.data(), slots.size(), &pid))) return rc;
+            if ((rc = dev_copy(s, slots.data(), slots.size(), &pid))) return rc;
             b.slot_of_w = pid;
             if (bd.light_base >= 0) {
                 std::vector<int> lo(N);
                 for (int i = 0; i < N; ++i) lo[i] = bd.light_base + (int)wt.order[i];
                 const int* pi = nullptr;
-                if ((rc = dev_copy(ctx, s->allocs, lo.data(), lo.size(), &pi))) return rc;
+                if ((rc = dev_copy(s, lo.data(), lo.size(), &pi))) return rc;
                 b.light_of_w = pi;
             }
-            if ((rc = dev_copy(ctx, s->allocs, (const uint4*)wt.nodes.data(), 5 * (size_t)wt.node_count, &u4))) return rc;
+            if ((rc = dev_copy(s, (const uint4*)wt.nodes.data(), 5 * (size_t)wt.node_count, &u4))) return rc;
             b.tlas_w = u4;
         }
         b.n_inst = N;
@@ -1300,15 +1420,15 @@ int upload_accels(ptr_ctx* ctx, ptr_scene* s, const ptr_scene_desc* d, const ptr
     int rc;
     const DevMesh* dm = nullptr;
     const DevBatch* db = nullptr;
-    if ((rc = dev_copy(ctx, s->allocs, meshes.data(), meshes.size(), &dm))) return rc;
-    if ((rc = dev_copy(ctx, s->allocs, batches.data(), batches.size(), &db))) return rc;
+    if ((rc = dev_copy(s, meshes.data(), meshes.size(), &dm))) return rc;
+    if ((rc = dev_copy(s, batches.data(), batches.size(), &db))) return rc;
     S.meshes = dm;
     S.batches = db;
     S.n_meshes = (int)meshes.size();
     S.n_batches = (int)batches.size();
     unsigned zero = 0;
     const unsigned* ef = nullptr;
-    if ((rc = dev_copy(ctx, s->allocs, &zero, 1, &ef))) return rc;
+    if ((rc = dev_copy(s, &zero, 1, &ef))) return rc;
     S.err_flags = (unsigned*)ef;
     for (int i = 0; i < d->n_regions; ++i) {
         const ptr_region& g = d->regions[i];
@@ -1387,9 +1507,9 @@ int upload_region_bvh(ptr_ctx* ctx, ptr_scene* s, const ptr_scene_desc* d) {
     const float4* nodes = nullptr;
     const int* it = nullptr;
     const int* lin = nullptr;
-    if ((rc = dev_copy(ctx, s->allocs, (const float4*)bvh.nodes.data(), 2 * (size_t)bvh.node_count, &nodes))) return rc;
-    if ((rc = dev_copy(ctx, s->allocs, items.data(), items.size(), &it))) return rc;
-    if (!linear.empty() && (rc = dev_copy(ctx, s->allocs, linear.data(), linear.size(), &lin))) return rc;
+    if ((rc = dev_copy(s, (const float4*)bvh.nodes.data(), 2 * (size_t)bvh.node_count, &nodes))) return rc;
+    if ((rc = dev_copy(s, items.data(), items.size(), &it))) return rc;
+    if (!linear.empty() && (rc = dev_copy(s, linear.data(), linear.size(), &lin))) return rc;
     S.region_bvh = nodes;
     S.region_items = it;
     S.linear_regions = lin;
@@ -1405,24 +1525,27 @@ int prepare_film(ptr_program* p, const ptr_frame* f, bool& fresh) {
     const size_t npix = (size_t)f->width * f->height;
     fresh = !f->accumulate;
     if (p->fw != f->width || p->fh != f->height || !p->sum) {
-        if (p->sum) cudaFree(p->sum);
-        if (p->sumsq) cudaFree(p->sumsq);
-        if (p->export_buf) cudaFree(p->export_buf);
+        dev_free(ctx, p->sum);
+        dev_free(ctx, p->sumsq);
+        dev_free(ctx, p->export_buf);
         p->sum = p->sumsq = nullptr;
         p->export_buf = nullptr;
-        if (cudaMalloc(&p->sum, npix * 3 * sizeof(double)) != cudaSuccess ||
-            cudaMalloc(&p->sumsq, npix * 3 * sizeof(double)) != cudaSuccess ||
-            cudaMalloc(&p->export_buf, npix * 3 * sizeof(float)) != cudaSuccess)
+        if (dev_alloc(ctx, &p->sum, npix * 3 * sizeof(double)) != cudaSuccess ||
+            dev_alloc(ctx, &p->sumsq, npix * 3 * sizeof(double)) != cudaSuccess ||
+            dev_alloc(ctx, &p->export_buf, npix * 3 * sizeof(float)) != cudaSuccess)
             return fail(ctx, PTR_E_NOMEM, "film allocation failed");
         p->fw = f->width;
         p->fh = f->height;
         fresh = true;
+        // a captured graph holds the old film's address
+        if (p->graph) { cudaGraphExecDestroy(p->graph); p->graph = nullptr; }
     }
     if (fresh) p->nsamples = 0.0;
     if (p->desc.aovs && (!p->aov_sum || p->aov_n != npix)) {   // the first-hit pictures' sums beside it
-        if (p->aov_sum) cudaFree(p->aov_sum);
+        dev_free(ctx, p->aov_sum);
         p->aov_sum = nullptr;
-        if (cudaMalloc(&p->aov_sum, npix * 6 * sizeof(double)) != cudaSuccess) return fail(ctx, PTR_E_NOMEM, "AOV film allocation failed");
+        if (p->graph) { cudaGraphExecDestroy(p->graph); p->graph = nullptr; }
+        if (dev_alloc(ctx, &p->aov_sum, npix * 6 * sizeof(double)) != cudaSuccess) return fail(ctx, PTR_E_NOMEM, "AOV film allocation failed");
         p->aov_n = npix;
     }
     return PTR_OK;
@@ -1619,13 +1742,13 @@ int render_impl(ptr_program* p, ptr_scene* s, const ptr_frame* f, float* samples
     }
     if (p->desc.aovs && !p->pool.aov) {   // two float4 per path slot; a captured graph predates them
         void* a = nullptr;
-        if (cudaMalloc(&a, (size_t)p->capacity * 32) != cudaSuccess) return fail(ctx, PTR_E_NOMEM, "AOV pool allocation failed");
+        if (dev_alloc(ctx, &a, (size_t)p->capacity * 32) != cudaSuccess) return fail(ctx, PTR_E_NOMEM, "AOV pool allocation failed");
         p->pool_allocs.push_back(a);
         p->pool.aov = (float4*)a;
         if (p->graph) { cudaGraphExecDestroy(p->graph); p->graph = nullptr; }
     }
     p->pool.aov_sum = p->desc.aovs ? p->aov_sum : nullptr;
-    if (!p->fp_dev) CK(ctx, cudaMalloc(&p->fp_dev, sizeof(FrameParams)));
+    if (!p->fp_dev) CK(ctx, dev_alloc(ctx, &p->fp_dev, sizeof(FrameParams)));
     // The frame's parameters travel as a kernel argument into a device block: no host
     // synchronisation, and the captured graph (which reads the block) stays valid.
     k_set_frame<<<1, 1, 0, st>>>(p->fp_dev, F);
@@ -1636,7 +1759,7 @@ int render_impl(ptr_program* p, ptr_scene* s, const ptr_frame* f, float* samples
     const int n_sm = device_sms(ctx->device);
     p->last_scene = s;
     if (counting) {
-        if (!p->work_dev) CK(ctx, cudaMalloc(&p->work_dev, 64));
+        if (!p->work_dev) CK(ctx, dev_alloc(ctx, &p->work_dev, 64));
         CK(ctx, cudaMemsetAsync(p->work_dev, 0, 64, st));
         p->work_valid = 1;
     } else {
@@ -1929,8 +2052,15 @@ int ptr_create(int device_ordinal, ptr_ctx** out) {
         delete c;
         return PTR_E_CUDA;
     }
+    c->pool = acquire_pool(device_ordinal);
+    if (!c->pool) {
+        cudaStreamDestroy(c->stream);
+        delete c;
+        return PTR_E_CUDA;
+    }
     // the counting sort's scan stages its whole table in shared memory (above the 48 KB default)
     if (cudaFuncSetAttribute((const void*)k_sort_scan, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSortScanSmem) != cudaSuccess) {
+        release_pool(device_ordinal);
         cudaStreamDestroy(c->stream);
         delete c;
         return PTR_E_CUDA;
@@ -1944,6 +2074,8 @@ int ptr_destroy(ptr_ctx* ctx) {
     cudaSetDevice(ctx->device);
     cudaStreamSynchronize(ctx->stream);
     if (ctx->batch) ptr_free_program(ctx->batch);
+    cudaStreamSynchronize(ctx->stream);   // the frees above
+    release_pool(ctx->device);
     cudaStreamDestroy(ctx->stream);
     delete ctx;
     return PTR_OK;
@@ -2096,10 +2228,10 @@ static int upload_scene(ptr_ctx* ctx, const ptr_scene_desc* d, const ptr_rails* 
     std::vector<int> lor(d->n_regions > 0 ? d->n_regions : 1, -1);
     for (int i = 0; i < d->n_lights; ++i)
         if (d->lights[i].region >= 0) lor[d->lights[i].region] = i;
-    if ((rc = dev_copy(ctx, s->allocs, d->regions, (size_t)d->n_regions, &S.regions)) ||
-        (rc = dev_copy(ctx, s->allocs, d->materials, (size_t)d->n_materials, &S.materials)) ||
-        (rc = dev_copy(ctx, s->allocs, d->lights, (size_t)d->n_lights, &S.lights)) ||
-        (rc = dev_copy(ctx, s->allocs, lor.data(), lor.size(), &S.light_of_region))) {
+    if ((rc = dev_copy(s, d->regions, (size_t)d->n_regions, &S.regions)) ||
+        (rc = dev_copy(s, d->materials, (size_t)d->n_materials, &S.materials)) ||
+        (rc = dev_copy(s, d->lights, (size_t)d->n_lights, &S.lights)) ||
+        (rc = dev_copy(s, lor.data(), lor.size(), &S.light_of_region))) {
         ptr_free_scene(s);
         return rc;
     }
@@ -2109,13 +2241,13 @@ static int upload_scene(ptr_ctx* ctx, const ptr_scene_desc* d, const ptr_rails* 
     bool has_het = false;
     for (int i = 0; i < d->n_materials; ++i) has_het |= d->materials[i].field_a || d->materials[i].field_s;
     S.has_het = has_het ? 1 : 0;
-    if (has_het && (rc = dev_copy(ctx, s->allocs, d->field_code, (size_t)d->n_field_code, &S.field_code))) {
+    if (has_het && (rc = dev_copy(s, d->field_code, (size_t)d->n_field_code, &S.field_code))) {
         ptr_free_scene(s);
         return rc;
     }
     if (d->n_tree_nodes > 0 &&
-        ((rc = dev_copy(ctx, s->allocs, (const float4*)d->light_tree, 2 * (size_t)d->n_tree_nodes, &S.light_tree)) ||
-         (rc = dev_copy(ctx, s->allocs, (const uint2*)d->light_trails, (size_t)d->n_lights, &S.light_trails)))) {
+        ((rc = dev_copy(s, (const float4*)d->light_tree, 2 * (size_t)d->n_tree_nodes, &S.light_tree)) ||
+         (rc = dev_copy(s, (const uint2*)d->light_trails, (size_t)d->n_lights, &S.light_trails)))) {
         ptr_free_scene(s);
         return rc;
     }
@@ -2144,9 +2276,9 @@ static int upload_scene(ptr_ctx* ctx, const ptr_scene_desc* d, const ptr_rails* 
             return fail(ctx, PTR_E_INVALID, "scene: incomplete spectral tables");
         }
         const float4* curves = nullptr;
-        if ((rc = dev_copy(ctx, s->allocs, sp->materials, (size_t)d->n_materials, &S.spec_mats)) ||
-            (rc = dev_copy(ctx, s->allocs, sp->lights, (size_t)d->n_lights, &S.spec_lights)) ||
-            (rc = dev_copy(ctx, s->allocs, (const float4*)sp->curves, (size_t)95, &curves))) {
+        if ((rc = dev_copy(s, sp->materials, (size_t)d->n_materials, &S.spec_mats)) ||
+            (rc = dev_copy(s, sp->lights, (size_t)d->n_lights, &S.spec_lights)) ||
+            (rc = dev_copy(s, (const float4*)sp->curves, (size_t)95, &curves))) {
             ptr_free_scene(s);
             return rc;
         }
@@ -2167,9 +2299,9 @@ static int upload_scene(ptr_ctx* ctx, const ptr_scene_desc* d, const ptr_rails* 
         S.env_w = d->env.width;
         S.env_h = d->env.height;
         const float* m = nullptr;
-        if ((rc = dev_copy(ctx, s->allocs, (const float4*)d->env.radiance, (size_t)S.env_w * S.env_h, &S.env_map)) ||
-            (rc = dev_copy(ctx, s->allocs, d->env.marginal, (size_t)S.env_h, &S.env_marg)) ||
-            (rc = dev_copy(ctx, s->allocs, d->env.conditional, (size_t)S.env_h * S.env_w, &m))) {
+        if ((rc = dev_copy(s, (const float4*)d->env.radiance, (size_t)S.env_w * S.env_h, &S.env_map)) ||
+            (rc = dev_copy(s, d->env.marginal, (size_t)S.env_h, &S.env_marg)) ||
+            (rc = dev_copy(s, d->env.conditional, (size_t)S.env_h * S.env_w, &m))) {
             ptr_free_scene(s);
             return rc;
         }
@@ -2190,7 +2322,7 @@ static int upload_scene(ptr_ctx* ctx, const ptr_scene_desc* d, const ptr_rails* 
                 scan[i] = make_float4(e11, e22, e12, e11 * e22 - e12 * e12);
             }
         }
-        rc = dev_copy(ctx, s->allocs, scan.data(), scan.size(), &S.region_scan);
+        rc = dev_copy(s, scan.data(), scan.size(), &S.region_scan);
     }
     if (!rc && !S.region_bvh && d->n_regions > 0) {   // the scan's same-shape runs
         std::vector<int4> runs;
@@ -2199,7 +2331,7 @@ static int upload_scene(ptr_ctx* ctx, const ptr_scene_desc* d, const ptr_rails* 
             if (!runs.empty() && runs.back().x == sh) runs.back().z++;
             else runs.push_back(make_int4(sh, i, 1, 0));
         }
-        if ((rc = dev_copy(ctx, s->allocs, runs.data(), runs.size(), &S.region_runs)) == PTR_OK) S.n_runs = (int)runs.size();
+        if ((rc = dev_copy(s, runs.data(), runs.size(), &S.region_runs)) == PTR_OK) S.n_runs = (int)runs.size();
     }
     if (!rc) {
         // the refilling closest-hit loop's scene form: analytic regions and exactly one
@@ -2236,6 +2368,15 @@ static int upload_scene(ptr_ctx* ctx, const ptr_scene_desc* d, const ptr_rails* 
                 s->spec_shape_code |= (unsigned long long)(d->regions[i].shape & 15) << (4 * i);
         }
     }
+    // the caller's arrays (pinned ones are read while the copies run) and the staged tables
+    // may go once the call returns
+    if (!rc) rc = flush_stage(s);
+    if (!rc) {
+        s->stage = std::vector<unsigned char>();
+        s->stage_left = 0;
+        const cudaError_t e = cudaStreamSynchronize(ctx->stream);
+        if (e != cudaSuccess) rc = cuda_fail(ctx, e, "scene upload");
+    }
     if (rc) {
         ptr_free_scene(s);
         return rc;
@@ -2250,7 +2391,7 @@ int ptr_free_scene(ptr_scene* s) {
         cudaSetDevice(s->ctx->device);
         cudaStreamSynchronize(s->ctx->stream);
     }
-    for (void* a : s->allocs) cudaFree(a);
+    for (void* a : s->allocs) dev_free(s->ctx, a);
     delete s;
     return PTR_OK;
 }
@@ -2291,19 +2432,10 @@ int ptr_free_program(ptr_program* p) {
     cudaSetDevice(p->ctx->device);
     cudaStreamSynchronize(p->ctx->stream);
     free_pool(p);
-    if (p->sum) cudaFree(p->sum);
-    if (p->sumsq) cudaFree(p->sumsq);
-    if (p->aov_sum) cudaFree(p->aov_sum);
-    if (p->export_buf) cudaFree(p->export_buf);
-    if (p->fp_dev) cudaFree(p->fp_dev);
-    cudaFree(p->ctl);
-    cudaFree(p->walk_film);
-    cudaFree(p->walk_aov);
-    cudaFree(p->tables);
-    if (p->work_dev) cudaFree(p->work_dev);
-    if (p->adj_dl) cudaFree(p->adj_dl);
-    if (p->adj_grads) cudaFree(p->adj_grads);
-    if (p->hit_log) cudaFree(p->hit_log);
+    for (void* a : {(void*)p->sum, (void*)p->sumsq, (void*)p->aov_sum, (void*)p->export_buf, (void*)p->fp_dev, (void*)p->ctl,
+                    (void*)p->walk_film, (void*)p->walk_aov, (void*)p->tables, (void*)p->work_dev, (void*)p->adj_dl,
+                    (void*)p->adj_grads, (void*)p->hit_log})
+        dev_free(p->ctx, a);
     delete p;
     return PTR_OK;
 }
@@ -2391,10 +2523,9 @@ int ptr_render_batch(ptr_ctx* ctx, const ptr_batch_job* jobs, int n_jobs) {
                  o_off = o_jobs + sizeof(BatchJob) * n_jobs, n_tables = o_off + sizeof(long long) * (n_jobs + 1);
     static_assert(sizeof(DevScene) % 16 == 0 || alignof(DevScene) <= 8, "table sections");
     if (bp->tables_n < n_tables) {
-        cudaFree(bp->tables);
-        bp->tables = nullptr;
+        dev_free(ctx, bp->tables);
         bp->tables_n = 0;
-        if (cudaMalloc(&bp->tables, n_tables) != cudaSuccess) return fail(ctx, PTR_E_NOMEM, "ptr_render_batch: tables");
+        if (dev_alloc(ctx, &bp->tables, n_tables) != cudaSuccess) return fail(ctx, PTR_E_NOMEM, "ptr_render_batch: tables");
         bp->tables_n = n_tables;
     }
     std::vector<unsigned char> image(n_tables);
@@ -2536,7 +2667,7 @@ int ptr_render_samples(ptr_program* p, ptr_scene* s, const ptr_frame* f, float* 
     if (n < need) return fail(ctx, PTR_E_INVALID, "ptr_render_samples: destination too small");
     float* dev = nullptr;
     CK(ctx, cudaSetDevice(ctx->device));
-    if (cudaMalloc(&dev, need * sizeof(float)) != cudaSuccess) return fail(ctx, PTR_E_NOMEM, "samples buffer");
+    if (dev_alloc(ctx, &dev, need * sizeof(float)) != cudaSuccess) return fail(ctx, PTR_E_NOMEM, "samples buffer");
     int rc = render_impl(p, s, f, dev);
     if (rc == PTR_OK) {
         cudaError_t e = cudaMemcpyAsync(host_out, dev, need * sizeof(float), cudaMemcpyDeviceToHost, ctx->stream);
@@ -2544,7 +2675,7 @@ int ptr_render_samples(ptr_program* p, ptr_scene* s, const ptr_frame* f, float* 
         if (e != cudaSuccess) rc = cuda_fail(ctx, e, "samples readback");
     }
     if (p->graph) { cudaGraphExecDestroy(p->graph); p->graph = nullptr; }
-    cudaFree(dev);
+    dev_free(ctx, dev);
     return rc;
 }
 
@@ -2553,20 +2684,19 @@ int ptr_trace_closest(ptr_ctx* ctx, ptr_scene* s, int accel, const float* rays, 
     if (!ctx || !s || !rays || n < 0 || !region || !element || !prim || !t) return fail(ctx, PTR_E_INVALID, "ptr_trace_closest: null argument");
     if (n == 0) return PTR_OK;
     CK(ctx, cudaSetDevice(ctx->device));
+    // the rays and the four answer arrays in one block
+    const size_t nn = (size_t)n;
     float* d_rays = nullptr;
-    int *d_reg = nullptr, *d_el = nullptr, *d_prim = nullptr;
-    float* d_t = nullptr;
-    size_t nn = (size_t)n;
-    if (cudaMalloc(&d_rays, nn * 6 * sizeof(float)) != cudaSuccess || cudaMalloc(&d_reg, nn * 4) != cudaSuccess ||
-        cudaMalloc(&d_el, nn * 4) != cudaSuccess || cudaMalloc(&d_prim, nn * 4) != cudaSuccess || cudaMalloc(&d_t, nn * 4) != cudaSuccess) {
-        cudaFree(d_rays); cudaFree(d_reg); cudaFree(d_el); cudaFree(d_prim); cudaFree(d_t);
-        return fail(ctx, PTR_E_NOMEM, "ptr_trace_closest: buffers");
-    }
+    if (dev_alloc(ctx, &d_rays, nn * 10 * sizeof(float)) != cudaSuccess) return fail(ctx, PTR_E_NOMEM, "ptr_trace_closest: buffers");
+    int *d_reg = (int*)(d_rays + 6 * nn), *d_el = d_reg + nn, *d_prim = d_el + nn;
+    float* d_t = (float*)(d_prim + nn);
     DevScene S = s->dev;
     S.accel = accel;
     cudaError_t e = cudaMemcpyAsync(d_rays, rays, nn * 6 * sizeof(float), cudaMemcpyHostToDevice, ctx->stream);
     if (e == cudaSuccess) {
-        k_trace_rays<<<256, 128, 0, ctx->stream>>>(S, d_rays, n, d_reg, d_el, d_prim, d_t);
+        // as many threads as stay resident: a query is a chain of dependent loads
+        const int grid = std::min((n + 127) / 128, resident_grid((const void*)k_trace_rays, 128, 0, device_sms(ctx->device)));
+        k_trace_rays<<<grid, 128, 0, ctx->stream>>>(S, d_rays, n, d_reg, d_el, d_prim, d_t);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaMemcpyAsync(region, d_reg, nn * 4, cudaMemcpyDeviceToHost, ctx->stream);
@@ -2574,7 +2704,7 @@ int ptr_trace_closest(ptr_ctx* ctx, ptr_scene* s, int accel, const float* rays, 
     if (e == cudaSuccess) e = cudaMemcpyAsync(prim, d_prim, nn * 4, cudaMemcpyDeviceToHost, ctx->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(t, d_t, nn * 4, cudaMemcpyDeviceToHost, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-    cudaFree(d_rays); cudaFree(d_reg); cudaFree(d_el); cudaFree(d_prim); cudaFree(d_t);
+    dev_free(ctx, d_rays);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "ptr_trace_closest");
     return PTR_OK;
 }
@@ -2619,19 +2749,19 @@ int ptr_backward(ptr_program* p, ptr_scene* s, const ptr_frame* f, const float* 
             int rc = alloc_pool(p, (int)std::max<long long>(cap, p->capacity), p->pool.sh2_o.p != nullptr, true);
             if (rc) return rc;
         }
-        if (!p->fp_dev) CK(ctx, cudaMalloc(&p->fp_dev, sizeof(FrameParams)));
+        if (!p->fp_dev) CK(ctx, dev_alloc(ctx, &p->fp_dev, sizeof(FrameParams)));
     }
     if (p->adj_dl_n < npix * 3) {
-        if (p->adj_dl) cudaFree(p->adj_dl);
+        dev_free(ctx, p->adj_dl);
         p->adj_dl = nullptr;
-        if (cudaMalloc(&p->adj_dl, npix * 3 * sizeof(float)) != cudaSuccess) return fail(ctx, PTR_E_NOMEM, "ptr_backward: adjoint image");
+        if (dev_alloc(ctx, &p->adj_dl, npix * 3 * sizeof(float)) != cudaSuccess) return fail(ctx, PTR_E_NOMEM, "ptr_backward: adjoint image");
         p->adj_dl_n = npix * 3;
     }
     const size_t ng = (size_t)PTR_GRAD_SLOTS * n_mat;
     if (p->adj_grads_n < ng) {
-        if (p->adj_grads) cudaFree(p->adj_grads);
+        dev_free(ctx, p->adj_grads);
         p->adj_grads = nullptr;
-        if (cudaMalloc(&p->adj_grads, ng * sizeof(double)) != cudaSuccess) return fail(ctx, PTR_E_NOMEM, "ptr_backward: gradients");
+        if (dev_alloc(ctx, &p->adj_grads, ng * sizeof(double)) != cudaSuccess) return fail(ctx, PTR_E_NOMEM, "ptr_backward: gradients");
         p->adj_grads_n = ng;
     }
     const FrameParams F = frame_params(f, total, (int)cap, true);
@@ -2669,10 +2799,10 @@ int ptr_backward(ptr_program* p, ptr_scene* s, const ptr_frame* f, const float* 
     if (const char* env = std::getenv("PTR_HIT_LOG_BYTES")) log_budget = std::max(0ll, (long long)std::atoll(env));
     int log_iters = (int)std::min<long long>(iters, log_budget / std::max<long long>(per_iter, 1));
     if (log_iters > 0 && p->hit_log_bytes < (size_t)(per_iter * log_iters)) {
-        if (p->hit_log) cudaFree(p->hit_log);
+        dev_free(ctx, p->hit_log);
         p->hit_log = nullptr;
         p->hit_log_bytes = 0;
-        if (cudaMalloc(&p->hit_log, (size_t)(per_iter * log_iters)) == cudaSuccess) p->hit_log_bytes = (size_t)(per_iter * log_iters);
+        if (dev_alloc(ctx, &p->hit_log, (size_t)(per_iter * log_iters)) == cudaSuccess) p->hit_log_bytes = (size_t)(per_iter * log_iters);
         else { cudaGetLastError(); log_iters = 0; }   // no log: the replay walks every query
     }
     if (s->walk) {

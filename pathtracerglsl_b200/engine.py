@@ -12,6 +12,7 @@ Mirrors the reference's Engine surface (``src/engine/Engine.ts:83-438``):
 Errors from the library raise ``EngineError`` carrying ``ptr_last_error``.
 """
 import ctypes as C
+import functools
 
 import numpy as np
 
@@ -51,8 +52,10 @@ def plan_tiles(width, height, tile_size):
     return {"cols": cols, "rows": rows, "size": size, "tiles": tiles}
 
 
+@functools.lru_cache(maxsize=1)
 def _source_revision():
-    """The source revision of this package (git HEAD), or 'unknown' outside a checkout."""
+    """The source revision of this package (git HEAD), or 'unknown' outside a checkout;
+    asked for once per process (a fork of a process that holds a GPU takes milliseconds)."""
     import os
     import subprocess
     try:
