@@ -9,6 +9,7 @@
 #include "scene.cuh"
 #include "sample.cuh"
 #include "lights/registry.cuh"
+#include "field_ops.h"
 
 namespace ptx {
 
@@ -416,112 +417,136 @@ __device__ __forceinline__ int emitter_light(const DevScene& S, const Hit& hit) 
 template <class Col> struct MediumSample { bool scattered; Col weight; f3 exit_p, exit_dir; };
 
 // ---- heterogeneous media (transport/volume/delta_tracking/delta_tracking.glsl) ----------
-// A coefficient field: the stack program of a GLSL expression of p (validated at upload:
-// known opcodes, stack depth within PTR_FIELD_MAX_STACK, END inside the table).
 __device__ __forceinline__ float fract_(float x) { return x - floorf(x); }
-// One copy of the interpreter serves every tracking loop (inlined, its copies crowd the
-// instruction cache: the walk's kernels stall on instruction fetch first).
+// A coefficient field at p: its typed program (field_ops.h), the stack's top in registers, the
+// rest in local memory (a scalar's y and z are not kept).  A tracking walk through the escaping
+// part of a fog takes thousands of evaluations in a row, so an evaluation's instructions are
+// what bounds it: typed, a scalar expression computes one value instead of three per
+// operation and takes its constants in place.  One copy of the interpreter serves every
+// tracking loop (inlined, its copies crowd the instruction cache).
 __device__ __noinline__ f3 field_eval(const uint32_t* code, f3 p) {
-    f3 st[PTR_FIELD_MAX_STACK];
+    float sx[PTR_FIELD_MAX_STACK], sy[PTR_FIELD_MAX_STACK], sz[PTR_FIELD_MAX_STACK];
     int sp = 0;
-    for (int pc = 0;;) {
-        const uint32_t op = __ldg(code + pc++);
-        if (op == PTR_FOP_END) break;
-        if (op == PTR_FOP_CONST) {
-            st[sp++] = f3(__uint_as_float(__ldg(code + pc)), __uint_as_float(__ldg(code + pc + 1)),
-                          __uint_as_float(__ldg(code + pc + 2)));
-            pc += 3;
+    f3 top(0.0f);
+    for (;;) {
+        const unsigned w = __ldg(code++);
+        const unsigned op = w & 0xFFu;
+        const bool vec = (w & kFieldVec) != 0u;
+        if (op == kFieldEnd) return vec ? top : f3(top.x);
+        if (op <= kFieldPushCV) {
+            if (!(w & kFieldFirst)) {
+                sx[sp] = top.x;
+                if (w & kFieldA) { sy[sp] = top.y; sz[sp] = top.z; }
+                ++sp;
+            }
+            if (op == kFieldPushP) {
+                const unsigned c = w >> 16;
+                top.x = c == 0u ? p.x : c == 1u ? p.y : p.z;
+            } else if (op == kFieldPushC) {
+                top.x = __uint_as_float(__ldg(code++));
+            } else if (op == kFieldPushPV) {
+                top = p;
+            } else {
+                top = f3(__uint_as_float(__ldg(code)), __uint_as_float(__ldg(code + 1)), __uint_as_float(__ldg(code + 2)));
+                code += 3;
+            }
             continue;
         }
-        if (op == PTR_FOP_P) { st[sp++] = p; continue; }
-        if (op == PTR_FOP_SWZ) {
-            const uint32_t c = __ldg(code + pc++);
-            f3 v = st[sp - 1];
-            float x = c == 0 ? v.x : c == 1 ? v.y : v.z;
-            st[sp - 1] = f3(x, x, x);
+        if (op <= kFieldAddC) {   // the component of a vector, or an immediate constant
+            if (op == kFieldSwz) {
+                const unsigned c = w >> 16;
+                top.x = c == 0u ? top.x : c == 1u ? top.y : top.z;
+                continue;
+            }
+            const float k = __uint_as_float(__ldg(code++));
+            if (op == kFieldMulC) {
+                top.x = top.x * k;
+                if (vec) { top.y = top.y * k; top.z = top.z * k; }
+            } else {
+                top.x = top.x + k;
+                if (vec) { top.y = top.y + k; top.z = top.z + k; }
+            }
             continue;
         }
-        if (op >= PTR_FOP_ADD && op <= PTR_FOP_DIV) {
-            f3 b = st[--sp], a = st[sp - 1];
-            st[sp - 1] = op == PTR_FOP_ADD ? a + b : op == PTR_FOP_SUB ? a - b
-                       : op == PTR_FOP_MUL ? a * b : f3(a.x / b.x, a.y / b.y, a.z / b.z);
-            continue;
-        }
-        if (op >= PTR_FOP_NEG && op <= PTR_FOP_FRACT) {
-            f3 a = st[sp - 1];
+        if (op <= kFieldLength) {
+            if (op == kFieldLength) {
+                const f3 v = (w & kFieldA) ? top : f3(top.x);
+                top.x = sqrtf(dot(v, v));
+                continue;
+            }
 #pragma unroll 1
-            for (int k = 0; k < 3; ++k) {   // lane by lane, rotating: one copy of each function
-                float x = a.x;
+            for (int k = vec ? 3 : 1; k > 0; --k) {   // component by component, rotating: one copy of each function
+                float x = top.x;
                 switch (op) {
-                    case PTR_FOP_NEG: x = -x; break;
-                    case PTR_FOP_EXP: x = m_exp(x); break;
-                    case PTR_FOP_LOG: x = m_log(x); break;
-                    case PTR_FOP_SIN: x = m_sin(x); break;
-                    case PTR_FOP_COS: x = m_cos(x); break;
-                    case PTR_FOP_SQRT: x = sqrtf(x); break;
-                    case PTR_FOP_ABS: x = fabsf(x); break;
-                    case PTR_FOP_FLOOR: x = floorf(x); break;
+                    case kFieldNeg: x = -x; break;
+                    case kFieldExp: x = m_exp(x); break;
+                    case kFieldLog: x = m_log(x); break;
+                    case kFieldSin: x = m_sin(x); break;
+                    case kFieldCos: x = m_cos(x); break;
+                    case kFieldSqrt: x = sqrtf(x); break;
+                    case kFieldAbs: x = fabsf(x); break;
+                    case kFieldFloor: x = floorf(x); break;
                     default: x = fract_(x); break;
                 }
-                a = f3(a.y, a.z, x);
+                if (vec) top = f3(top.y, top.z, x);
+                else top.x = x;
             }
-            st[sp - 1] = a;
             continue;
         }
-        if (op >= PTR_FOP_POW && op <= PTR_FOP_STEP) {
-            f3 b = st[--sp], a = st[sp - 1];
+        if (op <= kFieldDot) {
+            --sp;
+            const bool swap = (w & kFieldSwap) != 0u, va = (w & kFieldA) != 0u, vb = (w & kFieldB) != 0u;
+            f3 under(sx[sp]);
+            if (swap ? vb : va) { under.y = sy[sp]; under.z = sz[sp]; }
+            f3 a = swap ? top : under, b = swap ? under : top;
+            if (!va) a = f3(a.x);
+            if (!vb) b = f3(b.x);
+            if (op == kFieldDot) { top.x = dot(a, b); continue; }
 #pragma unroll 1
-            for (int k = 0; k < 3; ++k) {
+            for (int k = vec ? 3 : 1; k > 0; --k) {
                 float x = a.x, y = b.x;
                 switch (op) {
-                    case PTR_FOP_POW: x = m_pow(x, y); break;
-                    case PTR_FOP_MIN: x = y < x ? y : x; break;
-                    case PTR_FOP_MAX: x = x < y ? y : x; break;
-                    case PTR_FOP_MOD: x = x - y * floorf(x / y); break;
+                    case kFieldAdd: x = x + y; break;
+                    case kFieldSub: x = x - y; break;
+                    case kFieldMul: x = x * y; break;
+                    case kFieldDiv: x = x / y; break;
+                    case kFieldPow: x = m_pow(x, y); break;
+                    case kFieldMin: x = y < x ? y : x; break;
+                    case kFieldMax: x = x < y ? y : x; break;
+                    case kFieldMod: x = x - y * floorf(x / y); break;
                     default: x = y < x ? 0.0f : 1.0f; break;   // step(edge = a, x = b)
                 }
-                a = f3(a.y, a.z, x);
-                b = f3(b.y, b.z, b.x);
+                if (vec) { a = f3(a.y, a.z, x); b = f3(b.y, b.z, b.x); }
+                else a.x = x;
             }
-            st[sp - 1] = a;
+            top = a;
             continue;
         }
-        if (op >= PTR_FOP_CLAMP && op <= PTR_FOP_SMOOTHSTEP) {
-            f3 c = st[--sp], b = st[--sp], a = st[sp - 1];
-            float ra[3] = {a.x, a.y, a.z}, rb[3] = {b.x, b.y, b.z}, rc[3] = {c.x, c.y, c.z};
-            for (int k = 0; k < 3; ++k) {
-                float x;
-                if (op == PTR_FOP_CLAMP) {
-                    x = ra[k] < rb[k] ? rb[k] : ra[k];
-                    x = rc[k] < x ? rc[k] : x;
-                } else if (op == PTR_FOP_MIX) {
-                    x = ra[k] * (1.0f - rc[k]) + rb[k] * rc[k];
-                } else {   // smoothstep(e0 = a, e1 = b, x = c)
-                    float t = (rc[k] - ra[k]) / (rb[k] - ra[k]);
-                    t = t < 0.0f ? 0.0f : (t > 1.0f ? 1.0f : t);
-                    x = t * t * (3.0f - 2.0f * t);
-                }
-                ra[k] = x;
+        // three operands: the top two of the stack and the top
+        sp -= 2;
+        f3 a(sx[sp]), b(sx[sp + 1]), c = (w & kFieldC) ? top : f3(top.x);
+        if (w & kFieldA) { a.y = sy[sp]; a.z = sz[sp]; }
+        if (w & kFieldB) { b.y = sy[sp + 1]; b.z = sz[sp + 1]; }
+        if (op == kFieldVec3) { top = f3(a.x, b.x, c.x); continue; }   // three scalars
+#pragma unroll 1
+        for (int k = 0; k < 3; ++k) {
+            float x;
+            if (op == kFieldClamp) {
+                x = a.x < b.x ? b.x : a.x;
+                x = c.x < x ? c.x : x;
+            } else if (op == kFieldMix) {
+                x = a.x * (1.0f - c.x) + b.x * c.x;
+            } else {   // smoothstep(e0 = a, e1 = b, x = c)
+                float t = (c.x - a.x) / (b.x - a.x);
+                t = t < 0.0f ? 0.0f : (t > 1.0f ? 1.0f : t);
+                x = t * t * (3.0f - 2.0f * t);
             }
-            st[sp - 1] = f3(ra[0], ra[1], ra[2]);
-            continue;
+            a = f3(a.y, a.z, x);
+            b = f3(b.y, b.z, b.x);
+            c = f3(c.y, c.z, c.x);
         }
-        if (op == PTR_FOP_DOT) {
-            f3 b = st[--sp], a = st[sp - 1];
-            float d = dot(a, b);
-            st[sp - 1] = f3(d, d, d);
-            continue;
-        }
-        if (op == PTR_FOP_LENGTH) {
-            float l = sqrtf(dot(st[sp - 1], st[sp - 1]));
-            st[sp - 1] = f3(l, l, l);
-            continue;
-        }
-        // PTR_FOP_VEC3: three broadcast scalars into one vector
-        f3 z = st[--sp], y = st[--sp], x = st[sp - 1];
-        st[sp - 1] = f3(x.x, y.x, z.x);
+        top = a;
     }
-    return st[0];
 }
 __device__ __forceinline__ bool mat_is_het(const ptr_material& m) { return PTR_SPEC_HET && (m.field_a | m.field_s) != 0; }
 // The rendered medium at p: the fields (or constants), scaled down proportionally where the
@@ -529,8 +554,9 @@ __device__ __forceinline__ bool mat_is_het(const ptr_material& m) { return PTR_S
 struct HetProps { f3 sa, ss; };
 __device__ __forceinline__ HetProps het_props(const DevScene& S, const ptr_material& m, f3 p) {
     HetProps h;
-    h.sa = m.field_a ? field_eval(S.field_code + (m.field_a - 1), p) : ld3(m.sigma_a);
-    h.ss = m.field_s ? field_eval(S.field_code + (m.field_s - 1), p) : ld3(m.sigma_s);
+    // the word at a program's offset is the place of its typed form in the table
+    h.sa = m.field_a ? field_eval(S.field_code + __ldg(S.field_code + (m.field_a - 1)), p) : ld3(m.sigma_a);
+    h.ss = m.field_s ? field_eval(S.field_code + __ldg(S.field_code + (m.field_s - 1)), p) : ld3(m.sigma_s);
     f3 st = h.sa + h.ss;
     float smax = gmax(st.x, gmax(st.y, st.z));
     float scale = smax > m.majorant ? m.majorant / smax : 1.0f;

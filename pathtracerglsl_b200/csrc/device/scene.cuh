@@ -97,7 +97,8 @@ struct DevScene {
     // max.xyz, link), and the two trail words of every light
     const float4* light_tree;
     const uint2* light_trails;
-    // heterogeneous media: the coefficient fields' stack programs (NULL: none)
+    // heterogeneous media: the coefficient fields' programs, typed (field_ops.h); the word at a
+    // program's uploaded offset holds its place in this table (NULL: none)
     const uint32_t* field_code;
 };
 

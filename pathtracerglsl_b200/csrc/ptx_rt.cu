@@ -30,6 +30,7 @@
 #include "device/lbvh.cuh"
 #include "device/rails.cuh"
 #include "host/accel_build.h"
+#include "host/field_compile.h"
 #include "walk.h"
 
 using namespace ptx;
@@ -2241,9 +2242,19 @@ static int upload_scene(ptr_ctx* ctx, const ptr_scene_desc* d, const ptr_rails* 
     bool has_het = false;
     for (int i = 0; i < d->n_materials; ++i) has_het |= d->materials[i].field_a || d->materials[i].field_s;
     S.has_het = has_het ? 1 : 0;
-    if (has_het && (rc = dev_copy(s, d->field_code, (size_t)d->n_field_code, &S.field_code))) {
-        ptr_free_scene(s);
-        return rc;
+    if (has_het) {
+        std::vector<uint32_t> code(d->field_code, d->field_code + d->n_field_code);
+        for (int i = 0; i < d->n_materials; ++i)
+            for (int f : {d->materials[i].field_a, d->materials[i].field_s}) {
+                if (!f) continue;
+                const std::vector<uint32_t> typed = ptx_host::compile_field(d->field_code, f - 1);
+                code[(size_t)f - 1] = (uint32_t)code.size();
+                code.insert(code.end(), typed.begin(), typed.end());
+            }
+        if ((rc = dev_copy(s, code.data(), code.size(), &S.field_code))) {
+            ptr_free_scene(s);
+            return rc;
+        }
     }
     if (d->n_tree_nodes > 0 &&
         ((rc = dev_copy(s, (const float4*)d->light_tree, 2 * (size_t)d->n_tree_nodes, &S.light_tree)) ||
