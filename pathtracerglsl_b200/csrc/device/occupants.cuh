@@ -571,43 +571,53 @@ __device__ __forceinline__ int tracking_cap(float lambda) {
 }
 // Delta tracking of a scattering segment (Kutz et al. 2017, Algorithm 4, with the
 // history-aware average-based probabilities): xi are the site's two numbers, later
-// collisions draw from the path's stream.  Absorption terminates (weight 0).
-__device__ MediumSample<f3> medium_sample_delta(const DevScene& S, const ptr_material& m, const Ray& r, float t_max,
-                                                float x0, float x1, Rng& rng) {
+// collisions draw from the path's stream.  Absorption terminates (weight 0).  Resumable:
+// advance() runs at most `steps` tentative collisions and returns true when ms is decided.
+struct DeltaTrack {
     MediumSample<f3> ms;
-    ms.scattered = false;
-    ms.weight = f3(1.0f);
-    const float sbar = m.majorant;
-    f3 w(1.0f);
-    float t = 0.0f, xd = x0, xe = x1;
-    const int cap = tracking_cap(sbar * t_max);
-    for (int i = 0; i < cap; ++i) {
-        t += -m_log(1.0f - xd) / sbar;
-        if (t >= t_max) { ms.weight = w; return ms; }
-        f3 p = r.o + r.d * t;
-        HetProps h = het_props(S, m, p);
-        f3 sn = vmax(f3(sbar) - (h.sa + h.ss), f3(0.0f));
-        float pa = spectrum_average(h.sa * w);
-        float ps = spectrum_average(h.ss * w);
-        float pn = spectrum_average(sn * w);
-        float c = pa + ps + pn;
-        if (c <= 0.0f) { ms.weight = f3(0.0f); return ms; }
-        pa /= c; ps /= c; pn /= c;
-        if (xe < pa) { ms.weight = f3(0.0f); return ms; }
-        if (xe < pa + ps) {
-            ms.scattered = true;
-            ms.exit_p = p;
-            ms.exit_dir = r.d;
-            ms.weight = w * h.ss / (sbar * gmax(ps, 1e-20f));
-            return ms;
-        }
-        w = w * sn / (sbar * gmax(pn, 1e-20f));
-        xd = rng.next();
-        xe = rng.next();
+    f3 w;
+    float t, xd, xe;
+    int left;              // tentative collisions before the walk gives up
+    __device__ __forceinline__ void begin(const ptr_material& m, float t_max, float x0, float x1) {
+        ms.scattered = false;
+        ms.weight = f3(1.0f);
+        w = f3(1.0f);
+        t = 0.0f;
+        xd = x0;
+        xe = x1;
+        left = tracking_cap(m.majorant * t_max);
     }
-    ms.weight = w;
-    return ms;
-}
+    __device__ __forceinline__ bool advance(const DevScene& S, const ptr_material& m, const Ray& r, float t_max, Rng& rng, int steps) {
+        const float sbar = m.majorant;
+        for (; left > 0; --left) {
+            if (steps-- <= 0) return false;
+            t += -m_log(1.0f - xd) / sbar;
+            if (t >= t_max) { ms.weight = w; return true; }
+            f3 p = r.o + r.d * t;
+            HetProps h = het_props(S, m, p);
+            f3 sn = vmax(f3(sbar) - (h.sa + h.ss), f3(0.0f));
+            float pa = spectrum_average(h.sa * w);
+            float ps = spectrum_average(h.ss * w);
+            float pn = spectrum_average(sn * w);
+            float c = pa + ps + pn;
+            if (c <= 0.0f) { ms.weight = f3(0.0f); return true; }
+            pa /= c; ps /= c; pn /= c;
+            if (xe < pa) { ms.weight = f3(0.0f); return true; }
+            if (xe < pa + ps) {
+                ms.scattered = true;
+                ms.exit_p = p;
+                ms.exit_dir = r.d;
+                ms.weight = w * h.ss / (sbar * gmax(ps, 1e-20f));
+                return true;
+            }
+            w = w * sn / (sbar * gmax(pn, 1e-20f));
+            xd = rng.next();
+            xe = rng.next();
+        }
+        ms.weight = w;
+        return true;
+    }
+};
 // Ratio tracking of exp(-int sigma) along a segment (Novak et al. 2014): sigma_a alone
 // for the absorbing-only pass-through of the walk, sigma_t with pbrt's roulette (below
 // 0.05, survive 1/4 with weight 4) for shadow segments.

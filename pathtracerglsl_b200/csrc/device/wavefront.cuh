@@ -1113,9 +1113,12 @@ struct WalkState {
 // ADJ: also scatters the gradient terms through ga and leaves the slot-0 query's vertex
 // material and lobe derivative in sh_mat / sg.
 // live: this lane has a path; phase() is called by every lane between the parts of the iteration.
-template <class Col, int DIRECT, bool MEDIA, bool ADJ, class Sink, class Phase>
+// tracked: the outcome of the segment's delta tracking where the caller ran it (TRACKED; the
+// site's two numbers are drawn then).
+template <class Col, int DIRECT, bool MEDIA, bool ADJ, bool TRACKED = false, class Sink, class Phase>
 __device__ __forceinline__ bool walk_iteration(const DevScene& S, const ProgParams& P, WalkState<Col>& ws, const HitRec& hr,
-                                               Sink& sink, const GradAcc& ga, int& sh_mat, NeeGrad& sg, bool live, Phase phase) {
+                                               Sink& sink, const GradAcc& ga, int& sh_mat, NeeGrad& sg, bool live, Phase phase,
+                                               const MediumSample<f3>* tracked = nullptr) {
     constexpr bool SPECTRAL = sizeof(Col) == sizeof(s4);
     using CM = Colors<Col>;
     const bool nee = DIRECT != PTR_DIRECT_NONE;
@@ -1152,11 +1155,14 @@ __device__ __forceinline__ bool walk_iteration(const DevScene& S, const ProgPara
                 if (equiangular_site<Col>(S, med_mat, r, boundary ? hr.t : kMaxDist, rng, thr, wl, eq))
                     sink.segment_query(eq.p_evt, eq.wi, P.max_null - nulls, eq.light_pos, eq.contrib, eq.denom);
             }
-            float x0 = rng.next();
-            float x1 = rng.next();
-            float t_max = boundary ? hr.t : kMaxDist;
             // heterogeneous media take the tracking arms (delta_tracking.glsl)
             het = !SPECTRAL && PTR_SPEC_HET && S.has_het && mat_is_het(mm);
+            float x0 = 0.0f, x1 = 0.0f;
+            if (!(TRACKED && het && scatter_live(S, P, med_mat))) {
+                x0 = rng.next();
+                x1 = rng.next();
+            }
+            float t_max = boundary ? hr.t : kMaxDist;
             if (!scatter_live(S, P, med_mat) && !het) {
                 thr = thr * vexp(-CM::sigma_a(S, med_mat, wl) * t_max);
                 if constexpr (ADJ) {   // w = exp(-(1-a) st t)
@@ -1166,18 +1172,25 @@ __device__ __forceinline__ bool walk_iteration(const DevScene& S, const ProgPara
                 }
             } else {
                 MediumSample<Col> ms;
-                bool tracked = false;
+                bool done = false;
                 if constexpr (!SPECTRAL && PTR_SPEC_HET) {
                     if (het && scatter_live(S, P, med_mat)) {
-                        ms = medium_sample_delta(S, mm, r, t_max, x0, x1, rng);
-                        tracked = true;
+                        if constexpr (TRACKED) {
+                            ms = *tracked;
+                        } else {
+                            DeltaTrack track;
+                            track.begin(mm, t_max, x0, x1);
+                            track.advance(S, mm, r, t_max, rng, track.left);
+                            ms = track.ms;
+                        }
+                        done = true;
                     } else if (het) {   // absorbing only: the ratio-tracked pass-through
                         ms.scattered = false;
                         ms.weight = medium_ratio_track(S, mm, r, t_max, rng, false);
-                        tracked = true;
+                        done = true;
                     }
                 }
-                if (!tracked)
+                if (!done)
                     ms = medium_sample_analytic<Col>(CM::sigma_a(S, med_mat, wl), CM::sigma_s(S, med_mat, wl), r, t_max, x0, x1);
                 thr = thr * ms.weight;
                 if constexpr (ADJ) {   // scattered at t: w = a st exp(-st t)/pdf; passed: exp(-st t_max)/P
@@ -1824,11 +1837,19 @@ __global__ void __launch_bounds__(256, PTR_TRACE_MIN_BLOCKS) k_shadow(const __gr
 // ---- the whole walk in one kernel ------------------------------------------------------
 // k_walk runs every iteration of a path in one thread, its state in registers: no path
 // record, queue or shadow query travels through memory, only 16 bytes of radiance per path
-// go to the film pass.  A lane whose path has ended takes the next one (warp-aggregated
+// go to the film pass.  A lane whose path has ended takes the next one at once (warp-aggregated
 // tickets), so lanes stay busy whatever the paths' lengths, and a wave is one launch instead
 // of three per iteration.  The arithmetic and the order of the random numbers and radiance
 // sums are walk_iteration's and shadow_visibility's, so samples are bit-identical to the
 // wavefront kernels'.
+// What bounds it is instruction issue (65 % of the slots, 17 of 32 lanes on the Cornell box)
+// and, first of all, the instruction cache: the code of a walk is 70 to 500 KB.  A block's
+// warps therefore run each part of an iteration together, so that one pass of the part's code
+// through the cache serves them all (media and spectral workload, 16.8 M paths: 128 ms with
+// free-running warps, 41 ms in step; adjoint 15.4 and 9.3; fog room in tiles 50.0 and 48.4).
+// 80 registers (3 blocks of 256 per SM) measured faster than 128 (2): Cornell 1.73 ms against
+// 2.03 for 4.2 M paths, the 64-job mix 343 against 363; refilling at the first idle lane
+// faster than at the eighth (363 against 372).
 struct WalkArgs {
     float4* film;                 // radiance of path base + i at [i]
     float4* aov;                  // first-hit samples, two per path (null: none)
@@ -1837,7 +1858,6 @@ struct WalkArgs {
     long long base;               // the wave's paths: [base, base + n) of the frame or job space
     unsigned n;
     int iters;                    // walk iterations at most
-    int lockstep;                 // the block's warps run each part of an iteration together
     float4* hit_log;              // PathPool::hit_log of the adjoint (null: none)
     long long hit_log_stride;
     int hit_log_iters;
@@ -1879,6 +1899,10 @@ struct WalkSink {
 #ifndef PTR_WALK_REFILL
 #define PTR_WALK_REFILL 1
 #endif
+#ifndef PTR_TRACK_STEPS
+#define PTR_TRACK_STEPS 32
+#endif
+constexpr int kTrackSteps = PTR_TRACK_STEPS;
 template <class Col, int DIRECT, bool MEDIA, bool BATCH, bool ADJ = false>
 __global__ void __launch_bounds__(256, PTR_WALK_MIN_BLOCKS) k_walk(const __grid_constant__ DevScene S0, ProgParams P0, FrameParams F0, BatchTables bt,
                                                                    WalkArgs wa, AdjParams adj = AdjParams{}) {
@@ -1895,7 +1919,15 @@ __global__ void __launch_bounds__(256, PTR_WALK_MIN_BLOCKS) k_walk(const __grid_
     ga.s = s_grad;
     int i = -1, job = 0, it = 0;
     bool active = false, exhausted = false;
-    auto phase = [&] { if (wa.lockstep) __syncthreads(); else __syncwarp(); };
+    // Delta tracking runs kTrackSteps collisions at a time between the other lanes' iterations:
+    // a ray that escapes through an ambient fog takes thousands, one that scatters a few, and
+    // a warp that finished each segment in turn would wait for its longest.
+    constexpr bool TRACK = MEDIA && !SPECTRAL && !ADJ && PTR_SPEC_HET;
+    DeltaTrack track;
+    bool tracking = false;
+    HitRec hr;
+    // the block's warps run each part of an iteration together
+    auto phase = [] { __syncthreads(); };
     for (;;) {
         const unsigned idle = __ballot_sync(0xffffffffu, !active);
         if (!exhausted && __popc(idle) >= PTR_WALK_REFILL) {
@@ -1938,14 +1970,13 @@ __global__ void __launch_bounds__(256, PTR_WALK_MIN_BLOCKS) k_walk(const __grid_
                 }
             }
         }
-        if (wa.lockstep ? !__syncthreads_or(active) : !__any_sync(0xffffffffu, active)) break;
+        if (!__syncthreads_or(active)) break;
         const DevScene& S = BATCH ? bt.scenes[job] : S0;
         const ProgParams& P = BATCH ? bt.progs[job] : P0;
         // this iteration's record of the adjoint's walk log: the closest hit, then the query
         float4* rec = (!BATCH && !SPECTRAL && active && wa.hit_log && it < wa.hit_log_iters)
                           ? wa.hit_log + 4 * ((size_t)it * (size_t)wa.hit_log_stride + (size_t)i) : nullptr;
-        HitRec hr;
-        if (active) {
+        if (active && !tracking) {
             if (ADJ && rec) {
                 const float4 hf = rec[0];
                 const int4 hi = float4_as_int4(rec[1]);
@@ -1961,11 +1992,27 @@ __global__ void __launch_bounds__(256, PTR_WALK_MIN_BLOCKS) k_walk(const __grid_
             n_closest++;
         }
         phase();
+        if constexpr (TRACK) {
+            if (active && S.has_het) {
+                const int med_mat = material_of(S, ws.cur_med);
+                if (mat_has_medium(S, med_mat) && mat_is_het(S.materials[med_mat]) && scatter_live(S, P, med_mat)) {
+                    const ptr_material& mm = S.materials[med_mat];
+                    const float t_max = hr.region >= 0 ? hr.t : kMaxDist;
+                    if (!tracking) {
+                        const float x0 = ws.rng.next(), x1 = ws.rng.next();
+                        track.begin(mm, t_max, x0, x1);
+                    }
+                    tracking = !track.advance(S, mm, ws.r, t_max, ws.rng, kTrackSteps);
+                }
+            }
+            phase();
+        }
+        const bool live = active && !tracking;
         bool alive = false;
         int sh_mat = 0;
         NeeGrad sg{kGradKindNone, f3(0.0f), 0.0f};
         sink.seg.live = sink.vtx.live = false;
-        alive = walk_iteration<Col, DIRECT, MEDIA, ADJ>(S, P, ws, hr, sink, ga, sh_mat, sg, active, phase);
+        alive = walk_iteration<Col, DIRECT, MEDIA, ADJ, TRACK>(S, P, ws, hr, sink, ga, sh_mat, sg, live, phase, &track.ms);
         phase();
         if constexpr (MEDIA && DIRECT == PTR_DIRECT_NEE && !ADJ) {   // the equiangular segment query comes first
             if (sink.seg.live) {
@@ -2004,7 +2051,7 @@ __global__ void __launch_bounds__(256, PTR_WALK_MIN_BLOCKS) k_walk(const __grid_
             }
             phase();
         }
-        if (active && (!alive || ++it >= wa.iters)) {
+        if (live && (!alive || ++it >= wa.iters)) {
             active = false;
             if constexpr (SPECTRAL) {
                 const f3 px = color_to_pixel(S, col_st(ws.rad, 0.0f), ws.wl.lambda, wavelength_pdfs(BATCH ? bt.jobs[job].frame : F0, ws.wl.lambda));

@@ -259,9 +259,6 @@ int dev_copy(ptr_scene* s, const T* host, size_t n, const T** out) {
     return PTR_OK;
 }
 
-// Grid of the grid-stride wavefront kernels: 2048 resident threads per SM.
-int launch_grid(int n_sm, int block = 256) { return n_sm * (2048 / block); }
-
 // One wave of resident blocks per SM for a kernel (the occupancy calculator's figure for its
 // registers / shared memory at this block size, cached per kernel): a grid-stride kernel
 // sized for more blocks than fit runs them in a second wave whose tail leaves SMs idle.
@@ -645,14 +642,6 @@ void launch_replay(ptr_program* p, const ptr_scene* s, cudaStream_t st, int iter
 bool walk_route(const ptr_program* p, const ptr_scene* s, long long paths) {
     return s->walk && !(p->desc.color == PTR_COLOR_SPECTRAL && paths >= (1ll << 22));
 }
-// Lockstep keeps a block's warps in the same part of an iteration, so that one pass of a
-// part's instructions through the instruction cache serves them all (the walk's code is far
-// larger than that cache: without it the media workload took 128 ms against 41 ms at 16 spp,
-// the adjoint 15.4 against 9.3).  Tracking through heterogeneous media runs loops of very
-// uneven length, whose short ones would wait there for the longest: they go without (fog room,
-// 256 x 256 x 4 spp: 24.6 ms against 42.3).
-int walk_lockstep(bool heterogeneous) { return heterogeneous ? 0 : 1; }
-
 // Launches one wave's walk: n paths, one lane each at a time.
 void launch_walk(const Launcher& L, const void* kern, size_t smem, const DevScene& S, const ProgParams& P, const FrameParams& F,
                  const BatchTables& bt, const WalkArgs& wa, const AdjParams& adj) {
@@ -1642,7 +1631,6 @@ int render_walk(ptr_program* p, ptr_scene* s, const ptr_frame* f, const FramePar
     wa.ticket = p->pool.fetch;
     wa.stats = p->pool.stats;
     wa.iters = wave_iterations(p, s);
-    wa.lockstep = walk_lockstep(s->dev.has_het != 0);
     const Launcher L{tuning_of(p).block, device_sms(ctx->device), st, false};
     std::vector<ProfRec> prof;
     auto event = [&](int cls, bool begin) {
@@ -1691,7 +1679,6 @@ int backward_walk(ptr_program* p, ptr_scene* s, const FrameParams& F, const AdjP
     wa.film = p->walk_film;
     wa.stats = p->pool.stats;
     wa.iters = iters;
-    wa.lockstep = walk_lockstep(false);   // (heterogeneous media are not differentiated)
     wa.hit_log = log_iters > 0 ? p->hit_log : nullptr;
     wa.hit_log_stride = F.capacity;
     wa.hit_log_iters = log_iters;
@@ -2589,7 +2576,6 @@ int ptr_render_batch(ptr_ctx* ctx, const ptr_batch_job* jobs, int n_jobs) {
         wa.film = bp->walk_film;
         wa.ticket = bp->pool.fetch;
         wa.stats = bp->pool.stats;
-        wa.lockstep = walk_lockstep(het);
         for (long long w = 0; e == cudaSuccess && w < waves; ++w) {
             wa.base = w * cap;
             wa.n = (unsigned)std::min(cap, total - wa.base);
