@@ -1847,9 +1847,10 @@ __global__ void __launch_bounds__(256, PTR_TRACE_MIN_BLOCKS) k_shadow(const __gr
 // warps therefore run each part of an iteration together, so that one pass of the part's code
 // through the cache serves them all (media and spectral workload, 16.8 M paths: 128 ms with
 // free-running warps, 41 ms in step; adjoint 15.4 and 9.3; fog room in tiles 50.0 and 48.4).
-// 80 registers (3 blocks of 256 per SM) measured faster than 128 (2): Cornell 1.73 ms against
-// 2.03 for 4.2 M paths, the 64-job mix 343 against 363; refilling at the first idle lane
-// faster than at the eighth (363 against 372).
+// 64 registers (1024 threads per SM) measured faster than 80 or 128, and two blocks of 512
+// faster than four of 256 (fewer passes through the cache; the 64-job mix 279 ms at 80
+// registers, 276 with four blocks, 267 with two; the adjoint 7.4, 7.1 and 6.5); refilling at
+// the first idle lane faster than at the eighth (363 against 372).
 struct WalkArgs {
     float4* film;                 // radiance of path base + i at [i]
     float4* aov;                  // first-hit samples, two per path (null: none)
@@ -1893,18 +1894,10 @@ struct WalkSink {
     __device__ __forceinline__ float4* aov() const { return aov_p; }
 };
 
-#ifndef PTR_WALK_MIN_BLOCKS
-#define PTR_WALK_MIN_BLOCKS 3
-#endif
-#ifndef PTR_WALK_REFILL
-#define PTR_WALK_REFILL 1
-#endif
-#ifndef PTR_TRACK_STEPS
-#define PTR_TRACK_STEPS 32
-#endif
-constexpr int kTrackSteps = PTR_TRACK_STEPS;
+constexpr int kWalkBlock = 512;   // threads per block at most (2 blocks per SM)
+constexpr int kTrackSteps = 32;   // 16, 32 and 128: 50.4, 50.0 and 67.7 ms for the fog room in tiles
 template <class Col, int DIRECT, bool MEDIA, bool BATCH, bool ADJ = false>
-__global__ void __launch_bounds__(256, PTR_WALK_MIN_BLOCKS) k_walk(const __grid_constant__ DevScene S0, ProgParams P0, FrameParams F0, BatchTables bt,
+__global__ void __launch_bounds__(kWalkBlock, 2) k_walk(const __grid_constant__ DevScene S0, ProgParams P0, FrameParams F0, BatchTables bt,
                                                                    WalkArgs wa, AdjParams adj = AdjParams{}) {
     constexpr bool SPECTRAL = sizeof(Col) == sizeof(s4);
     static_assert(!(ADJ && SPECTRAL), "the adjoint replay is RGB only");
@@ -1930,7 +1923,7 @@ __global__ void __launch_bounds__(256, PTR_WALK_MIN_BLOCKS) k_walk(const __grid_
     auto phase = [] { __syncthreads(); };
     for (;;) {
         const unsigned idle = __ballot_sync(0xffffffffu, !active);
-        if (!exhausted && __popc(idle) >= PTR_WALK_REFILL) {
+        if (!exhausted && idle != 0u) {
             unsigned first = 0u;
             if ((threadIdx.x & 31u) == 0u) first = atomicAdd(wa.ticket, (unsigned)__popc(idle));
             first = __shfl_sync(0xffffffffu, first, 0);

@@ -645,7 +645,11 @@ bool walk_route(const ptr_program* p, const ptr_scene* s, long long paths) {
 // Launches one wave's walk: n paths, one lane each at a time.
 void launch_walk(const Launcher& L, const void* kern, size_t smem, const DevScene& S, const ProgParams& P, const FrameParams& F,
                  const BatchTables& bt, const WalkArgs& wa, const AdjParams& adj) {
-    L.raw_upto((int)((wa.n + (unsigned)L.block - 1u) / (unsigned)L.block), kern, smem, S, P, F, bt, wa, adj);
+    // the largest block that still puts one on every SM: a small wave spreads over the chip
+    Launcher W = L;
+    W.block = kWalkBlock;
+    while (W.block > 64 && wa.n < (unsigned)W.block * (unsigned)L.n_sm) W.block /= 2;
+    W.raw_upto((int)((wa.n + (unsigned)W.block - 1u) / (unsigned)W.block), kern, smem, S, P, F, bt, wa, adj);
 }
 
 // One wave of a batched render: the same kernel sequence over the concatenated job space;
