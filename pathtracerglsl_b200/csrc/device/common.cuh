@@ -52,6 +52,12 @@ PTR_M1(m_tanh, tanh) PTR_M1(m_atanh, atanh) PTR_M1(m_cosh, cosh) PTR_M2(m_atan2,
 #ifndef PTR_SPEC_TREE
 #define PTR_SPEC_TREE 1         // 0: the build never selects lights with the light tree
 #endif
+#ifndef PTR_SPEC_BVH
+#define PTR_SPEC_BVH 1          // 0: no scene of the build has a region BVH
+#endif
+#ifndef PTR_SPEC_NULL
+#define PTR_SPEC_NULL (-1)      // whether some region is a null interface (-1: read at run time)
+#endif
 #ifndef PTR_SPEC_ACCEL
 #define PTR_SPEC_ACCEL (-1)     // PTR_ACCEL_* the program walks meshes with (-1: read at run time)
 #endif

@@ -366,7 +366,7 @@ __device__ __forceinline__ HitRec scene_closest(const DevScene& S, const Ray& r,
         if (hit) take(k, t);
     }
 #else
-    const bool tabled = S.region_bvh != nullptr;
+    const bool tabled = PTR_SPEC_BVH && S.region_bvh != nullptr;
     if (!tabled && S.region_runs) {
         for_region_runs(S, [&](auto sc, int a, int b) {
             constexpr int SH = decltype(sc)::value;
@@ -434,7 +434,7 @@ __device__ __forceinline__ bool scene_any(const DevScene& S, const Ray& r, float
         }
     }
 #else
-    const bool tabled = S.region_bvh != nullptr;
+    const bool tabled = PTR_SPEC_BVH && S.region_bvh != nullptr;
     if (!tabled && S.region_runs) {
         bool hit = false;
         for (int q = 0; q < S.n_runs && !hit; ++q) {
@@ -484,7 +484,7 @@ __device__ __forceinline__ int scene_region_at(const DevScene& S, f3 p) {
 #pragma unroll
     for (int k = 0; k < PTR_SPEC_NREGIONS; ++k) arm(k, S.regions[k], spec_shape(k));
 #else
-    const bool tabled = S.region_bvh != nullptr;
+    const bool tabled = PTR_SPEC_BVH && S.region_bvh != nullptr;
     if (!tabled && S.region_runs) {
         for_region_runs(S, [&](auto sc, int a, int b) {
             constexpr int SH = decltype(sc)::value;
@@ -682,8 +682,7 @@ __device__ __forceinline__ void camera_path(const FrameParams& F, int pix, int s
     r.o = ld3(F.cam.position);
 }
 // path_state_init of path slot i.
-__device__ __forceinline__ void init_slot(const DevScene& S, const PathPool& pool, long long i, const Rng& rng, const Ray& r) {
-    int medium = S.has_media ? scene_region_at(S, r.o) : -1;
+__device__ __forceinline__ void init_slot(const PathPool& pool, long long i, const Rng& rng, const Ray& r, int medium) {
     pool.ray_o[i] = f4(r.o, 0.0f);
     pool.ray_d[i] = f4(r.d, 1.0f);
     pool.thr[i] = make_float4(1.f, 1.f, 1.f, 1.f);   // the spectral model's fourth lane included
@@ -708,6 +707,8 @@ __global__ void k_generate(DevScene S, PathPool pool, const FrameParams* fp, Adj
         if (pool.fetch) pool.fetch[0] = 0u;
     }
     const unsigned npix = (unsigned)F.width * (unsigned)F.height;
+    // every path starts at the pinhole: its region is found once per thread
+    const int medium = S.has_media ? scene_region_at(S, ld3(F.cam.position)) : -1;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         int pix, sample;
         split_path(base + i, npix, pix, sample);
@@ -724,7 +725,7 @@ __global__ void k_generate(DevScene S, PathPool pool, const FrameParams* fp, Adj
             const float* g = adj.dl_image + 3 * (size_t)pix;
             pool.dl[i] = make_float4(g[0] * adj.inv_spp, g[1] * adj.inv_spp, g[2] * adj.inv_spp, 0.f);
         }
-        init_slot(S, pool, i, rng, r);
+        init_slot(pool, i, rng, r, medium);
         if (pool.aov) { pool.aov[2 * i] = make_float4(0.f, 0.f, 0.f, 0.f); pool.aov[2 * i + 1] = make_float4(0.f, 0.f, 0.f, 0.f); }
     }
 }
@@ -1601,13 +1602,14 @@ __device__ __forceinline__ Col shadow_visibility(const DevScene& S, const ProgPa
             else if (flag_more) flag_error(S, kErrAdjMedia);
         }
     };
-    if (!S.has_null) {   // every surface is optical: any hit before the light blocks the query
+    if (PTR_SPEC_NULL < 0 ? !S.has_null : !PTR_SPEC_NULL) {   // every surface is optical: any hit before the light blocks the query
         const float remaining = length(light_p - sr.o) - kShadowBackoff;
         if (remaining <= 0.0f) return T;
         if (scene_any(S, sr, gmin(remaining, kMaxDist), work)) return Col(0.0f);
         attenuate(sr, scene_region_at(S, sr.o), remaining);
         return T;
     }
+    if (PTR_SPEC_NULL == 0) return T;
     int medium = 0;
     Ray seg = sr;
     for (int crossed = 0; crossed <= crossings_left; crossed++) {
@@ -1905,6 +1907,8 @@ __global__ void __launch_bounds__(kWalkBlock, 2) k_walk(const __grid_constant__ 
     if constexpr (ADJ) grad_block_init(s_grad, PTR_GRAD_SLOTS * S0.n_materials);
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&wa.stats[2], (unsigned long long)wa.n);
     const WaveJobs wj = BATCH ? WaveJobs(wa.base, (long long)wa.n, bt) : WaveJobs{};
+    // the region every path starts in (a pinhole's rays share their origin): once per thread
+    int cam_med = !BATCH && MEDIA ? scene_region_at(S0, ld3(F0.cam.position)) : -1;
     unsigned n_closest = 0u, n_shadow = 0u;
     WalkState<Col> ws;
     WalkSink<Col> sink;
@@ -1947,7 +1951,8 @@ __global__ void __launch_bounds__(kWalkBlock, 2) k_walk(const __grid_constant__ 
                 ws.rad = Col(0.0f);
                 ws.prev_qp = ws.r.o;
                 ws.bounce = 0;
-                ws.cur_med = S.has_media ? scene_region_at(S, ws.r.o) : -1;
+                if (BATCH) cam_med = S.has_media ? scene_region_at(S, ws.r.o) : -1;
+                ws.cur_med = cam_med;
                 ws.nulls = 0;
                 ws.prev_delta = true;
                 if constexpr (ADJ) {   // the forward walk left this path's total radiance
@@ -2161,7 +2166,8 @@ __global__ void k_generate_batch(PathPool pool, BatchTables bt) {
         Ray r;
         float4 unused;
         camera_path<false>(F, pix, sample, rng, r, unused);
-        init_slot(bt.scenes[j], pool, i, rng, r);
+        const DevScene& S = bt.scenes[j];
+        init_slot(pool, i, rng, r, S.has_media ? scene_region_at(S, r.o) : -1);
     }
 }
 

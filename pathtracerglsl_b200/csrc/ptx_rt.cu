@@ -1865,6 +1865,8 @@ struct Census {
     bool mesh = false;                 // some region is a triangle mesh or instances one
     bool het = false;                  // some medium has a coefficient field
     int accel = -1;                    // PTR_ACCEL_* of the mesh walks (-1: no meshes, or a mix)
+    bool bvh = false;                  // some scene has a region BVH
+    int null = -1;                     // null interfaces: 0 none, 1 every scene has some, -1 a mix
     bool adj = false;                  // the replay's kernels (ADJ = true) instead of the forward's
     bool walk = false;                 // the one-kernel walk instead of the wavefront's three kernels
     int direct = 0;
@@ -1885,6 +1887,8 @@ Census census_of(const ptr_program* p, const ptr_scene* sc) {
     c.mesh = sc->has_mesh;
     c.het = sc->dev.has_het != 0;
     c.accel = sc->has_mesh ? p->desc.accel : -1;
+    c.bvh = sc->dev.region_bvh != nullptr;
+    c.null = sc->dev.has_null;
     return c;
 }
 // The union census of a job mix (the batched kernels serve every job of it): masks OR-ed,
@@ -1898,6 +1902,8 @@ Census census_of_batch(const ptr_batch_job* jobs, int n) {
         c.walk = c.walk && k.walk;
         c.mesh = c.mesh || k.mesh;
         c.het = c.het || k.het;
+        c.bvh = c.bvh || k.bvh;
+        c.null = j == 0 || c.null == k.null ? k.null : -1;
         c.mats |= k.mats;
         c.lights |= k.lights;
         c.envs |= k.envs;
@@ -1916,6 +1922,8 @@ std::vector<std::string> census_options(const Census& c) {
             std::string("-DPTR_SPEC_MESH=") + (c.mesh ? "1" : "0"),
             std::string("-DPTR_SPEC_HET=") + (c.het ? "1" : "0"),
             "-DPTR_SPEC_ACCEL=(" + std::to_string(c.accel) + ")",
+            std::string("-DPTR_SPEC_BVH=") + (c.bvh ? "1" : "0"),
+            "-DPTR_SPEC_NULL=(" + std::to_string(c.null) + ")",
             "-DPTR_SPEC_NREGIONS=" + std::to_string(c.nregions),
             "-DPTR_SPEC_SHAPE_CODE=" + std::to_string(c.shape_code) + "ull",
             std::string("-DPTR_SPEC_TREE=") + (c.tree ? "1" : "0")};
