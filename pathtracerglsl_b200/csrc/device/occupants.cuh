@@ -680,8 +680,8 @@ __device__ __forceinline__ MediumSample<Col> medium_sample_analytic(Col sigma_a,
 // is uniform in the angle subtended at the light point.  Returns true when a shadow query
 // is due: from p_evt towards light_pos, adding contrib * visibility / denom.
 template <class Col> struct EquiangularQuery { f3 p_evt, wi, light_pos; Col contrib; float denom; };
-template <class Col>
-__device__ __forceinline__ bool equiangular_site(const DevScene& S, int med_mat, const Ray& r, float t_max,
+template <class Col, class SigA, class SigS>
+__device__ __forceinline__ bool equiangular_site(const DevScene& S, int med_mat, SigA sigma_a_of, SigS sigma_s_of, const Ray& r, float t_max,
                                                  Rng& rng, Col thr, const Wl& wl, EquiangularQuery<Col>& q) {
     const ptr_material& mm = S.materials[med_mat];
     float uc = rng.next();
@@ -713,9 +713,9 @@ __device__ __forceinline__ bool equiangular_site(const DevScene& S, int med_mat,
     float t = t_c + h * m_tan(theta);
     float pdf_t = h / ((theta_b - theta_a) * (h2 + (t - t_c) * (t - t_c)));
     q.p_evt = r.o + r.d * t;
-    Col sigma_s = Colors<Col>::sigma_s(S, med_mat, wl);
+    Col sigma_s = sigma_s_of(med_mat);
     if (spectrum_is_black(sigma_s)) return false;
-    Col T_seg = vexp(-(Colors<Col>::sigma_a(S, med_mat, wl) + sigma_s) * t);
+    Col T_seg = vexp(-(sigma_a_of(med_mat) + sigma_s) * t);
     f3 to_light = pos - q.p_evt;
     float d2 = gmax(dot(to_light, to_light), 1e-8f);
     float dist = sqrtf(d2);
