@@ -2,11 +2,12 @@
 //
 // One context = one CUDA device + one stream.  A program owns its film (FP64 per-pixel
 // sum and sum of squares) and its path pool; ptr_render renders frame.spp samples per
-// pixel as waves of at most `capacity` paths, each wave a CUDA graph of
+// pixel as waves of at most `capacity` paths.  Without triangle meshes a wave is two plain
+// launches, k_walk and k_film_walk (walk_route says when); else it is a CUDA graph of
 //   k_generate, (k_closest, k_shade, k_shadow) x iterations, k_film, k_advance
 // captured once per (program, scene, image size) and replayed for every wave and frame.
 // Frame-varying values (sample index, salt, camera) live in a device-side FrameParams
-// block refreshed by one cudaMemcpyAsync before the replays, so the graph stays valid.
+// block written by one tiny kernel before the replays, so the graph stays valid.
 #include <cuda_runtime.h>
 #include <chrono>
 #include <cmath>
@@ -635,12 +636,12 @@ void launch_replay(ptr_program* p, const ptr_scene* s, cudaStream_t st, int iter
 // ---- the one-kernel walk (k_walk) ---------------------------------------------------------
 // Whether a frame whose waves hold `paths` paths takes the one-kernel walk.  Scenes with
 // triangle meshes keep the wavefront kernels, whose traversals refill idle lanes inside a
-// query.  Spectral programs do from 2^22 paths on: their shading is several times the code of
+// query.  Spectral programs do above 2^22 paths: their shading is several times the code of
 // an RGB program, and large waves run it denser in the wavefront's compacted queues (media
-// and spectral workload, 1024 x 1024, per-scene kernels: 16 spp 21.2 ms against 35.6 ms, 4 spp
-// 9.8 against 10.4; 512 x 512 at 4 spp 5.1 against 3.7).
+// and spectral workload, 1024 x 1024, per-scene kernels, wavefront against walk: 16 spp 20.5 and
+// 25.4 ms, 8 spp 12.2 and 13.5, 5 spp 9.22 and 9.35, 4 spp 8.26 and 7.69).
 bool walk_route(const ptr_program* p, const ptr_scene* s, long long paths) {
-    return s->walk && !(p->desc.color == PTR_COLOR_SPECTRAL && paths >= (1ll << 22));
+    return s->walk && !(p->desc.color == PTR_COLOR_SPECTRAL && paths > (1ll << 22));
 }
 // Launches one wave's walk: n paths, one lane each at a time.
 void launch_walk(const Launcher& L, const void* kern, size_t smem, const DevScene& S, const ProgParams& P, const FrameParams& F,
