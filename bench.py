@@ -280,14 +280,44 @@ def run_reference_batch(args):
     print(json.dumps(line), flush=True)
 
 
-# DRAM bytes of the roofline kernel per closest-hit query (a shaded path, for k_shade), from
+# DRAM bytes of the roofline kernel per closest-hit query, from
 # one ncu capture of one whole wave of the workload at 1 spp with the autotuner's pick
 # (dram__bytes_read.sum + dram__bytes_write.sum over the wave's launches / the wave's
 # queries).  Scaled to a launch of the timed configuration by its queries per launch; the
 # line labels it "ncu capture, scaled" (it is not measured in the timed run).
-NCU_TRAFFIC_PER_QUERY = {("mesh", "closest"): 216.18, ("cornell", "shade"): 311.37}
-# the kernel each workload's roofline is reported for (its dominant traversal / shading kernel)
-ROOFLINE_KERNEL = {"mesh": "closest", "mesh-bvh": "closest", "cornell": "shade", "media": "shade"}
+NCU_TRAFFIC_PER_QUERY = {("mesh", "closest"): 208.89}
+# the kernel each workload's roofline is reported for (its dominant traversal / shading kernel);
+# on the one-kernel walk it is that kernel
+ROOFLINE_KERNEL = {"mesh": "closest", "mesh-bvh": "closest", "media": "shade"}
+
+
+def on_walk(prof):
+    """Whether the instrumented render took the one-kernel walk (k_walk), which the profile
+    reports in the shading class, with no closest-hit launches."""
+    return prof["closest"][1] == 0 and prof["shade"][1] > 0
+
+
+def roofline_of(prof, counters, name=None, cw=True, note=""):
+    """The roofline record of an instrumented render's dominant kernel class."""
+    walk = on_walk(prof)
+    kernel = "walk" if walk else ROOFLINE_KERNEL.get(name) or max(prof.items(), key=lambda kv: kv[1][0])[0]
+    kms, launches = prof["shade" if walk else kernel]
+    peak, peak_kind = measured_peaks()
+    launch_ms = kms / max(launches, 1)
+    bytes_per_launch = algorithmic_bytes(kernel, counters, cw) / max(launches, 1)
+    achieved = bytes_per_launch / (launch_ms / 1000.0) / 1e9
+    total_ms = sum(v[0] for v in prof.values())
+    traffic = NCU_TRAFFIC_PER_QUERY.get((name, kernel))
+    rec = {"bound": "hbm", "kernel": "k_" + kernel + note, "achieved": achieved, "peak": peak, "unit": "GB/s",
+           "frac": achieved / peak, "peak_source": peak_kind,
+           "traffic": None if traffic is None else traffic * counters["closest_queries"] / max(launches, 1),
+           "traffic_source": None if traffic is None else "ncu capture of one wave at 1 spp, scaled by queries per launch",
+           "bytes_per_launch": bytes_per_launch, "launch_ms": launch_ms,
+           "share": {("walk" if walk and k == "shade" else k): v[0] / total_ms for k, v in prof.items()}}
+    if walk:
+        rec["reading"] = ("the walk keeps its paths in registers and writes one 16-byte film record per path: "
+                          "instruction issue bounds it, not memory")
+    return rec
 
 
 def algorithmic_bytes(kernel, c, cw=True):
@@ -311,7 +341,7 @@ def algorithmic_bytes(kernel, c, cw=True):
         return shadow * (4 + 64 + 32) + trav("shadow_")
     if kernel == "generate":
         return paths * (104 + 4 + 16)
-    if kernel == "film":
+    if kernel in ("film", "walk"):   # the walk's paths stay in registers: its film record
         return paths * 16
     return 0
 
@@ -513,22 +543,8 @@ def measure_ours(args, name, rank, local, world, dist, tuning=None, cpu_leg=True
     eng.reset()
     eng.profile_render(w, h, spp, _abi.PROFILE_WORK)
     cnt = eng.counters()
-    kernel = ROOFLINE_KERNEL.get(name) or max(prof.items(), key=lambda kv: kv[1][0])[0]
-    kms, klaunch = prof[kernel]
-    peak, peak_kind = measured_peaks()
-    launch_ms = kms / max(klaunch, 1)
-    bytes_per_launch = algorithmic_bytes(kernel, cnt, cfg.get("mesh_accel", "cwbvh") == "cwbvh") / max(klaunch, 1)
-    achieved = bytes_per_launch / (launch_ms / 1000.0) / 1e9
-    total_prof_ms = sum(v[0] for v in prof.values())
-    roofline = {"bound": "hbm", "kernel": "k_" + kernel, "achieved": achieved, "peak": peak, "unit": "GB/s",
-                "frac": achieved / peak, "peak_source": peak_kind,
-                "traffic": (NCU_TRAFFIC_PER_QUERY[(name, kernel)] * cnt["closest_queries"] / max(klaunch, 1)
-                            if (name, kernel) in NCU_TRAFFIC_PER_QUERY else None),
-                "traffic_source": ("ncu capture of one wave at 1 spp, scaled by queries per launch"
-                                   if (name, kernel) in NCU_TRAFFIC_PER_QUERY else None),
-                "bytes_per_launch": bytes_per_launch, "launch_ms": launch_ms,
-                "share": {k: v[0] / total_prof_ms for k, v in prof.items()}}
-    launches = sum(v[1] for v in prof.values()) + 1   # + the frame-parameter kernel
+    roofline = roofline_of(prof, cnt, name, cfg.get("mesh_accel", "cwbvh") == "cwbvh")
+    launches = sum(v[1] for v in prof.values()) + (not on_walk(prof))   # + the wavefront's frame-parameter kernel
 
     if rank == 0:
         line = {"metric": METRIC, "value": value, "unit": "samples/s", "n_gpus": world, "steps": args.steps,
@@ -685,16 +701,7 @@ def measure_batch(args, rank, local, world, dist, cpu_leg=True):
 
     prof = b.profile(frames)
     cnt = b.counters()
-    kernel, (kms, klaunch) = max(prof.items(), key=lambda kv: kv[1][0])
-    peak, peak_kind = measured_peaks()
-    launch_ms = kms / max(klaunch, 1)
-    bytes_per_launch = algorithmic_bytes(kernel, cnt) / max(klaunch, 1)
-    achieved = bytes_per_launch / (launch_ms / 1000.0) / 1e9
-    total_prof_ms = sum(v[0] for v in prof.values())
-    roofline = {"bound": "hbm", "kernel": "k_" + kernel, "achieved": achieved, "peak": peak, "unit": "GB/s",
-                "frac": achieved / peak, "peak_source": peak_kind, "traffic": None,
-                "bytes_per_launch": bytes_per_launch, "launch_ms": launch_ms,
-                "share": {k: v[0] / total_prof_ms for k, v in prof.items()}}
+    roofline = roofline_of(prof, cnt)
     launches = sum(v[1] for v in prof.values())
     line = None
     if rank == 0:
@@ -874,12 +881,6 @@ def measure_adjoint(args, rank, local, world, dist, cpu_leg=True):
     eng.profile_render(w, h, spp_a, _abi.PROFILE_WORK)
     cnt = eng.counters()
     if rank == 0:
-        kernel, (kms, klaunch) = max(prof.items(), key=lambda kv: kv[1][0])
-        peak, peak_kind = measured_peaks()
-        launch_ms = kms / max(klaunch, 1)
-        bytes_per_launch = algorithmic_bytes(kernel, cnt) / max(klaunch, 1)
-        achieved = bytes_per_launch / (launch_ms / 1000.0) / 1e9
-        total_prof_ms = sum(v[0] for v in prof.values())
         line = {"metric": METRIC, "value": value, "unit": "samples/s", "n_gpus": world, "steps": args.steps,
                 "warmup": args.warmup, "ms_per_step": adj_ms / args.steps, "higher_is_better": True,
                 "scaling": "weak", "vs_baseline": None, "dtype": "f32", "data": "synthetic",
@@ -894,11 +895,9 @@ def measure_adjoint(args, rank, local, world, dist, cpu_leg=True):
                             "adjoint_over_forward_cost": adj_ms / fwd_ms},
                 "loss": loss, "gradient_l2": float(np.linalg.norm(g[mask])),
                 "e2e": e2e, "clocks": clk,
-                "roofline": {"bound": "hbm", "kernel": "k_" + kernel + " (forward pass of the step)", "achieved": achieved,
-                             "peak": peak, "unit": "GB/s", "frac": achieved / peak, "peak_source": peak_kind,
-                             "traffic": None, "bytes_per_launch": bytes_per_launch, "launch_ms": launch_ms,
-                             "share": {k: v[0] / total_prof_ms for k, v in prof.items()}},
-                "gpu_launches": args.steps * 2 * sum(v[1] for v in prof.values())}
+                "roofline": roofline_of(prof, cnt, note=" (forward pass of the step)"),
+                # forward walk and replay: one k_walk each per wave, or the wavefront's launches twice
+                "gpu_launches": args.steps * 2 * (prof["shade"][1] if on_walk(prof) else sum(v[1] for v in prof.values()))}
         if cpu_leg and not args.no_cpu_baseline:
             line["cpu_baseline"] = cpu_baseline(sc, st, w, h, spp_a)
             line["cpu_baseline"]["sample"] = "forward only (the oracle has no adjoint): " + line["cpu_baseline"]["sample"]

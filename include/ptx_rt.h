@@ -382,10 +382,12 @@ int ptr_free_program(ptr_program* prog);
 int ptr_render(ptr_program* prog, ptr_scene* scene, const ptr_frame* frame);
 
 /* Batched rendering: many scenes x programs x frames of uneven size in ONE wavefront —
- * the jobs' paths share one path pool and every wave is one CUDA graph of the
- * generate / closest / shade / shadow / film kernels over the concatenated job space,
- * with per-job scene, program and frame tables (paths of shallow jobs retire early;
- * compaction keeps the queues dense).  Each job accumulates into its own program's film
+ * the jobs' paths share the waves over the concatenated job space, with per-job scene,
+ * program and frame tables.  A mix without triangle meshes runs each wave as one kernel that
+ * walks whole paths (a lane whose path ends takes the next one) and one film kernel; else
+ * every wave is one CUDA graph of the generate / closest / shade / shadow / film kernels over
+ * one path pool (paths of shallow jobs retire early; compaction keeps the queues dense).
+ * Each job accumulates into its own program's film
  * (read it with ptr_read_export).  All jobs must share directLighting.  Synchronises.
  * No counterpart in the reference (one fragment draw per renderer and frame). */
 typedef struct ptr_batch_job {
@@ -397,7 +399,7 @@ int ptr_render_batch(ptr_ctx* ctx, const ptr_batch_job* jobs, int n_jobs);
 /* Counters of the last batched render (paths, closest and shadow queries). */
 int ptr_get_batch_counters(ptr_ctx* ctx, ptr_counters* out);
 /* Instrument the next ptr_render_batch (PTR_PROFILE_TIMING: CUDA events around every
- * launch, no graph) and read the per-kernel-class times like ptr_get_profile. */
+ * kernel class's launches, no graph) and read the per-kernel-class times like ptr_get_profile. */
 int ptr_profile_batch_next(ptr_ctx* ctx, int mode);
 int ptr_get_batch_profile(ptr_ctx* ctx, float* ms_out, int* launches_out, int n);
 
@@ -504,14 +506,15 @@ int ptr_update_params(ptr_scene* scene, const ptr_material* materials, int n_mat
 /* ---- per-scene kernels (replaces the reference's per scene x strategy code generation:
  * Generate emits GLSL for each scene x strategy, src/compiler/generate/Generator.ts:10-91,
  * compiled by the WebGL driver in RenderExecutor.ts:86-107).
- * Compiles the program's closest-hit, shading and shadow kernels for this scene with NVRTC
- * (sm_100a): material models, light kinds, environment kind and region shapes the scene
+ * Compiles the kernels the program renders this scene with (the one-kernel walk of scenes
+ * without triangle meshes; closest-hit, shading and shadow otherwise; all four for spectral
+ * programs) with NVRTC (sm_100a): material models, light kinds, environment kind and region shapes the scene
  * lacks fold away, and with at most 16 regions the region loops unroll into one arm per
  * region with its intersection routine fixed, like the reference's generated arms (in
  * place of the region BVH, which returns the same hits).  Later ptr_render calls of the
  * program with this scene use them (samples are bit-identical to the generic kernels), and
- * so does ptr_backward's forward walk; its replay kernels (shading and shadow with the
- * adjoint terms) are compiled for the same census at the first ptr_backward that follows.
+ * so does ptr_backward's forward walk; its replay kernels (those with the adjoint terms) are
+ * compiled for the same census at the first ptr_backward that follows.
  * The counting passes keep the generic kernels (a batch takes ptr_specialize_batch).
  * Modules are cached per occupant census for the process.
  * seconds_out (may be NULL): compile time (0 for a cached module).  scene = NULL returns
@@ -545,7 +548,9 @@ int ptr_set_accel_build(ptr_ctx* ctx, int where);
  * sort_buckets: the occupant-sorted shading queue — 1 = off, 8 = live paths grouped by the
  * material model they shade, 16 = by model and whether the segment starts in a medium;
  * ray_sort: the ray-coherence order of the traversal queues.  Every knob changes the order
- * of work only: each path's samples are bit-identical under any tuning.
+ * of work only: each path's samples are bit-identical under any tuning.  The one-kernel walk
+ * of scenes without triangle meshes has no queues and chooses its own block size; of these
+ * knobs it uses the capacity.
  * Applies to every later ptr_render / ptr_render_batch / ptr_backward on the context.
  * pathtracerglsl_b200.autotune picks and records these per workload. */
 typedef struct ptr_tuning {
@@ -578,7 +583,8 @@ int ptr_get_counters(ptr_program* prog, ptr_counters* out);
  * walk iteration on the context's stream — ptr_get_profile then returns, per kernel
  * class k (0 generate, 1 closest-hit, 2 shade, 3 shadow, 4 film, 5 queue sorts), the
  * summed device time ms_out[k] and the number of kernel launches launches_out[k]
- * (n <= PTR_PROFILE_CLASSES entries); PTR_PROFILE_WORK runs the traversal kernels'
+ * (n <= PTR_PROFILE_CLASSES entries; the one-kernel walk counts as class 2 and leaves
+ * classes 0, 1, 3 and 5 at zero); PTR_PROFILE_WORK runs the traversal kernels'
  * counting variants, which tally nodes, triangles, TLAS nodes and instances into
  * ptr_counters. */
 #define PTR_PROFILE_TIMING 1

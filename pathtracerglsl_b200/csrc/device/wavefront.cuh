@@ -1,8 +1,11 @@
-// wavefront.cuh — the transport loop as a wavefront of kernels over a path pool.
+// wavefront.cuh — the transport loop, as a wavefront of kernels over a path pool and as one
+// kernel per wave.
 //
 // The reference runs the whole walk (transport/integrators/pt/pt.ts:299-464) as one
-// fragment per pixel.  Here each path lives in struct-of-arrays state in HBM and the walk
-// is split at its two traversals:
+// fragment per pixel.  Scenes without triangle meshes do so here too: k_walk runs a path in
+// one thread, its state in registers, and k_film_walk / k_film_batch_walk fold the wave into
+// the film.  With meshes (and for large spectral frames) each path lives in struct-of-arrays
+// state in HBM and the walk is split at its two traversals:
 //
 //   k_generate  camera rays + path_state_init for one wave of (pixel, sample) paths
 //   k_closest   nearest hit of every live path (the scene_intersect traversal)
@@ -13,6 +16,7 @@
 //               the owning path's radiance
 //   k_film      per-pixel FP64 sum and sum of squares over the wave's samples
 //
+// Both forms share one iteration (walk_iteration) and one shadow query (shadow_visibility).
 // Every path draws its random numbers in exactly the order of the reference's walk
 // (the sampler is counter-based, so a path's stream does not depend on scheduling), and
 // its radiance is accumulated in the same order: emission, then the vertex's NEE term,
@@ -1855,8 +1859,8 @@ __global__ void __launch_bounds__(256, PTR_TRACE_MIN_BLOCKS) k_shadow(const __gr
 // of three per iteration.  The arithmetic and the order of the random numbers and radiance
 // sums are walk_iteration's and shadow_visibility's, so samples are bit-identical to the
 // wavefront kernels'.
-// What bounds it is instruction issue (65 % of the slots, 17 of 32 lanes on the Cornell box)
-// and, first of all, the instruction cache: the code of a walk is 70 to 500 KB.  A block's
+// What bounds it is instruction issue (70 % of the slots, 17.5 of 32 lanes on the Cornell box)
+// and, were its warps to run free, the instruction cache: a walk is 70 to 500 KB of code.  A block's
 // warps therefore run each part of an iteration together, so that one pass of the part's code
 // through the cache serves them all (media and spectral workload, 16.8 M paths: 128 ms with
 // free-running warps, 41 ms in step; adjoint 15.4 and 9.3; fog room in tiles 50.0 and 48.4).
