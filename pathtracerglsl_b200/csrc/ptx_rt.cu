@@ -68,7 +68,7 @@ struct ptr_scene {
     DevScene dev{};
     std::vector<void*> allocs;
     // the small tables' staged block (dev_copy): host image, its place on the device
-    std::vector<unsigned char> stage;
+    std::vector<std::vector<unsigned char>> stage;   // host images of the staged blocks, the last one in use
     unsigned char* stage_dev = nullptr;
     size_t stage_used = 0, stage_left = 0;
     int has_media = 0;
@@ -216,13 +216,15 @@ void dev_free(ptr_ctx* ctx, void* p) {
 
 // A device copy of a host array that lives with the scene.  Tables up to kStageMax bytes are
 // laid into one staged block (one allocation and one copy for a scene's dozens of small
-// tables); they are on the device after flush_stage.  Larger arrays are copied on the spot.  The
-// caller synchronises the stream before the host array may go.
+// tables); they are on the device after flush_stage, and their host image lives until upload_scene
+// has waited for the stream.  Larger arrays are on the device when this returns: many are a
+// builder's own, gone soon after.
 constexpr size_t kStageMax = 32u << 10, kStageBlock = 256u << 10;
 int flush_stage(ptr_scene* s) {
     if (s->stage_used == 0) return PTR_OK;
-    CK(s->ctx, cudaMemcpyAsync(s->stage_dev, s->stage.data(), s->stage_used, cudaMemcpyHostToDevice, s->ctx->stream));
-    // a pageable source is staged by the copy itself, so the block's host image may be reused
+    // the image mirrors the block and is written once: the copy may read it until the stream is waited for
+    const unsigned char* image = s->stage.back().data() + (kStageBlock - s->stage_left);
+    CK(s->ctx, cudaMemcpyAsync(s->stage_dev, image, s->stage_used, cudaMemcpyHostToDevice, s->ctx->stream));
     s->stage_dev += s->stage_used;
     s->stage_left -= s->stage_used;
     s->stage_used = 0;
@@ -236,7 +238,7 @@ int dev_copy(ptr_scene* s, const T* host, size_t n, const T** out) {
     const size_t bytes = n * sizeof(T), room = (bytes + 255) / 256 * 256;
     const bool staged = bytes <= kStageMax;
     if (staged && s->stage_left >= s->stage_used + room) {
-        std::memcpy(s->stage.data() + s->stage_used, host, bytes);
+        std::memcpy(s->stage.back().data() + (kStageBlock - s->stage_left) + s->stage_used, host, bytes);
         *out = (const T*)(s->stage_dev + s->stage_used);
         s->stage_used += room;
         return PTR_OK;
@@ -249,13 +251,14 @@ int dev_copy(ptr_scene* s, const T* host, size_t n, const T** out) {
     if (e != cudaSuccess) return fail(ctx, PTR_E_NOMEM, std::string("device allocation: ") + cudaGetErrorString(e));
     s->allocs.push_back(p);
     if (staged) {
-        s->stage.resize(kStageBlock);
+        s->stage.emplace_back(kStageBlock);
         s->stage_dev = p;
         s->stage_left = kStageBlock;
         s->stage_used = 0;
         return dev_copy(s, host, n, out);
     }
     CK(ctx, cudaMemcpyAsync(p, host, bytes, cudaMemcpyHostToDevice, ctx->stream));
+    CK(ctx, cudaStreamSynchronize(ctx->stream));
     *out = (const T*)p;
     return PTR_OK;
 }
@@ -2379,13 +2382,13 @@ static int upload_scene(ptr_ctx* ctx, const ptr_scene_desc* d, const ptr_rails* 
                 s->spec_shape_code |= (unsigned long long)(d->regions[i].shape & 15) << (4 * i);
         }
     }
-    // the caller's arrays (pinned ones are read while the copies run) and the staged tables
-    // may go once the call returns
+    // the staged tables' host image may go once the copies have run, and the caller's arrays
+    // once the call returns
     if (!rc) rc = flush_stage(s);
     if (!rc) {
-        s->stage = std::vector<unsigned char>();
-        s->stage_left = 0;
         const cudaError_t e = cudaStreamSynchronize(ctx->stream);
+        s->stage.clear();
+        s->stage_left = 0;
         if (e != cudaSuccess) rc = cuda_fail(ctx, e, "scene upload");
     }
     if (rc) {
