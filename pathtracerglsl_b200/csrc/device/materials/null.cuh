@@ -9,6 +9,7 @@ namespace ptx {
 
 struct Null : MaterialModel {
     static constexpr int kId = PTR_MAT_NONE;
+    static constexpr bool kUsesIor = true;   // without media (with them the walk never samples it)
     template <class Col>
     __device__ static ISample<Col> sample(const MatSite<Col>& s, f3 wo, float uc, float, float) {
         return dielectric_sample(wo, s.hit, Colors<Col>::tint(s.S, s.mat, s.wl), s.n_from, s.n_to, uc);
