@@ -96,8 +96,8 @@ struct ptr_program {
     double* sum = nullptr;
     double* sumsq = nullptr;
     double* aov_sum = nullptr;   // first-hit pictures: 6 doubles per pixel (programs with aovs)
-    size_t aov_n = 0;
     double nsamples = 0.0;
+    bool film_fresh = true;      // the sums hold nothing: the next frame's film pass starts them from zero
     float* export_buf = nullptr;
     // path pool
     int capacity = 0;
@@ -1516,37 +1516,42 @@ int upload_region_bvh(ptr_ctx* ctx, ptr_scene* s, const ptr_scene_desc* d) {
     return PTR_OK;
 }
 
-// Size a program's FP64 film for a frame.  fresh: the film pass starts every pixel from zero
-// (a new film, or a frame that does not accumulate), so nothing is cleared here.
-int prepare_film(ptr_program* p, const ptr_frame* f, bool& fresh) {
+void free_film(ptr_program* p) {
+    if (p->graph) { cudaGraphExecDestroy(p->graph); p->graph = nullptr; }   // it holds the film's addresses
+    for (void* a : {(void*)p->sum, (void*)p->sumsq, (void*)p->aov_sum, (void*)p->export_buf}) dev_free(p->ctx, a);
+    p->sum = p->sumsq = p->aov_sum = nullptr;
+    p->export_buf = nullptr;
+    p->fw = p->fh = 0;
+    p->nsamples = 0.0;
+    p->film_fresh = true;
+}
+// Size a program's FP64 film (and its first-hit sums) for a frame.  Nothing is cleared here: a
+// new film, or a frame that does not accumulate, makes the film fresh, and the film pass
+// starts every pixel of a fresh film from zero.  It stays fresh until a frame has been
+// launched whole, so a frame after one that failed starts from zero too.
+int prepare_film(ptr_program* p, const ptr_frame* f) {
     ptr_ctx* ctx = p->ctx;
     const size_t npix = (size_t)f->width * f->height;
-    fresh = !f->accumulate;
-    if (p->fw != f->width || p->fh != f->height || !p->sum) {
-        dev_free(ctx, p->sum);
-        dev_free(ctx, p->sumsq);
-        dev_free(ctx, p->export_buf);
-        p->sum = p->sumsq = nullptr;
-        p->export_buf = nullptr;
+    if (p->fw != f->width || p->fh != f->height) {
+        free_film(p);
         if (dev_alloc(ctx, &p->sum, npix * 3 * sizeof(double)) != cudaSuccess ||
             dev_alloc(ctx, &p->sumsq, npix * 3 * sizeof(double)) != cudaSuccess ||
-            dev_alloc(ctx, &p->export_buf, npix * 3 * sizeof(float)) != cudaSuccess)
+            dev_alloc(ctx, &p->export_buf, npix * 3 * sizeof(float)) != cudaSuccess ||
+            (p->desc.aovs && dev_alloc(ctx, &p->aov_sum, npix * 6 * sizeof(double)) != cudaSuccess)) {
+            free_film(p);
             return fail(ctx, PTR_E_NOMEM, "film allocation failed");
+        }
         p->fw = f->width;
         p->fh = f->height;
-        fresh = true;
-        // a captured graph holds the old film's address
-        if (p->graph) { cudaGraphExecDestroy(p->graph); p->graph = nullptr; }
     }
-    if (fresh) p->nsamples = 0.0;
-    if (p->desc.aovs && (!p->aov_sum || p->aov_n != npix)) {   // the first-hit pictures' sums beside it
-        dev_free(ctx, p->aov_sum);
-        p->aov_sum = nullptr;
-        if (p->graph) { cudaGraphExecDestroy(p->graph); p->graph = nullptr; }
-        if (dev_alloc(ctx, &p->aov_sum, npix * 6 * sizeof(double)) != cudaSuccess) return fail(ctx, PTR_E_NOMEM, "AOV film allocation failed");
-        p->aov_n = npix;
-    }
+    if (!f->accumulate) p->film_fresh = true;
+    if (p->film_fresh) p->nsamples = 0.0;
     return PTR_OK;
+}
+// A frame's passes are all launched: the film holds its samples.
+void film_done(ptr_program* p, const ptr_frame* f) {
+    p->film_fresh = false;
+    p->nsamples += (double)f->spp;
 }
 
 // The scene-dependent pins of the equiangular site: the reference admits delta lights only
@@ -1664,7 +1669,7 @@ int render_walk(ptr_program* p, ptr_scene* s, const ptr_frame* f, const FramePar
         CK(ctx, cudaStreamSynchronize(st));
         fold_profile(p, prof);
     }
-    p->nsamples += (double)f->spp;
+    film_done(p, f);
     return PTR_OK;
 }
 
@@ -1711,8 +1716,7 @@ int render_impl(ptr_program* p, ptr_scene* s, const ptr_frame* f, float* samples
     CK(ctx, cudaSetDevice(ctx->device));
     cudaStream_t st = ctx->stream;
     const size_t npix = (size_t)f->width * f->height;
-    bool fresh = true;
-    if (int rc = prepare_film(p, f, fresh)) return rc;
+    if (int rc = prepare_film(p, f)) return rc;
     const long long total = (long long)npix * f->spp;
     // capacity: whole sample passes when a pass fits the pool, else a chunk of pixels
     long long cap_max = ctx->tune.capacity > 0 ? ctx->tune.capacity : (1ll << 24);
@@ -1724,7 +1728,7 @@ int render_impl(ptr_program* p, ptr_scene* s, const ptr_frame* f, float* samples
     if (cap > total) cap = total;
     const bool profiling = (p->profile_next & PTR_PROFILE_TIMING) != 0;
     const bool counting = (p->profile_next & PTR_PROFILE_WORK) != 0;
-    FrameParams F = frame_params(f, total, (int)cap, fresh);
+    FrameParams F = frame_params(f, total, (int)cap, p->film_fresh);
     F.wavelengths = p->desc.wavelengths;
     F.lambda_min = p->desc.lambda_min;
     F.lambda_max = p->desc.lambda_max;
@@ -1800,7 +1804,7 @@ int render_impl(ptr_program* p, ptr_scene* s, const ptr_frame* f, float* samples
         CK(ctx, cudaGetLastError());
         p->profile_next = 0;
     }
-    p->nsamples += (double)f->spp;
+    film_done(p, f);
     return PTR_OK;
 }
 
@@ -2446,7 +2450,8 @@ int ptr_free_program(ptr_program* p) {
     cudaSetDevice(p->ctx->device);
     cudaStreamSynchronize(p->ctx->stream);
     free_pool(p);
-    for (void* a : {(void*)p->sum, (void*)p->sumsq, (void*)p->aov_sum, (void*)p->export_buf, (void*)p->fp_dev, (void*)p->ctl,
+    free_film(p);
+    for (void* a : {(void*)p->fp_dev, (void*)p->ctl,
                     (void*)p->walk_film, (void*)p->walk_aov, (void*)p->tables, (void*)p->work_dev, (void*)p->adj_dl,
                     (void*)p->adj_grads, (void*)p->hit_log})
         dev_free(p->ctx, a);
@@ -2498,9 +2503,7 @@ int ptr_render_batch(ptr_ctx* ctx, const ptr_batch_job* jobs, int n_jobs) {
     for (int j = 0; j < n_jobs; ++j) {
         const ptr_batch_job& J = jobs[j];
         ptr_program* p = J.prog;
-        bool fresh = true;
-        int rc = prepare_film(p, &J.frame, fresh);
-        if (rc) return rc;
+        if (int rc = prepare_film(p, &J.frame)) return rc;
         walk = walk && J.scene->walk;
         scenes[j] = J.scene->dev;
         scenes[j].accel = p->desc.accel;
@@ -2509,7 +2512,7 @@ int ptr_render_batch(ptr_ctx* ctx, const ptr_batch_job* jobs, int n_jobs) {
         progs[j] = prog_params(p->desc);
         if (progs[j].equiangular) equi = true;
         const long long total_j = (long long)J.frame.width * J.frame.height * J.frame.spp;
-        bjobs[j].frame = frame_params(&J.frame, total_j, 0, fresh);
+        bjobs[j].frame = frame_params(&J.frame, total_j, 0, p->film_fresh);
         bjobs[j].sum = p->sum;
         bjobs[j].sumsq = p->sumsq;
         offsets[j + 1] = offsets[j] + total_j;
@@ -2646,7 +2649,7 @@ int ptr_render_batch(ptr_ctx* ctx, const ptr_batch_job* jobs, int n_jobs) {
     }
     if (e != cudaSuccess) rc = cuda_fail(ctx, e, "ptr_render_batch");
     if (rc) return rc;
-    for (int j = 0; j < n_jobs; ++j) jobs[j].prog->nsamples += (double)jobs[j].frame.spp;
+    for (int j = 0; j < n_jobs; ++j) film_done(jobs[j].prog, &jobs[j].frame);
     bp->last_scene = nullptr;
     return PTR_OK;
 }
@@ -2987,6 +2990,12 @@ static int export_impl(ptr_program* p, const char* name, float* dst, size_t n, b
     else if (std::strcmp(name, "normal") == 0 && (p->desc.aovs & PTR_AOV_NORMAL) && p->aov_sum) what = 3;
     else return fail(ctx, PTR_E_INVALID, std::string("export: unknown export '") + name + "'");
     if (n < npix * 3) return fail(ctx, PTR_E_INVALID, "export: destination too small");
+    if (p->film_fresh) {   // the only frame of this film failed: no samples, so its sums are zero
+        CK(ctx, cudaMemsetAsync(p->sum, 0, npix * 3 * sizeof(double), ctx->stream));
+        CK(ctx, cudaMemsetAsync(p->sumsq, 0, npix * 3 * sizeof(double), ctx->stream));
+        if (p->aov_sum) CK(ctx, cudaMemsetAsync(p->aov_sum, 0, npix * 6 * sizeof(double), ctx->stream));
+        p->film_fresh = false;
+    }
     float* target = device_dst ? dst : p->export_buf;
     const double* src = what == 2 ? p->aov_sum : what == 3 ? p->aov_sum + 3 * npix : p->sum;   // a picture's mean
     k_export<<<256, 256, 0, ctx->stream>>>(src, p->sumsq, p->nsamples > 0 ? p->nsamples : 1.0, (int)npix, what >= 2 ? 0 : what, target);
