@@ -32,6 +32,7 @@
 #include "device/rails.cuh"
 #include "host/accel_build.h"
 #include "host/field_compile.h"
+#include "host/stream_guard.h"
 #include "walk.h"
 
 using namespace ptx;
@@ -804,6 +805,9 @@ int build_mesh_device_core(ptr_ctx* ctx, ptr_scene* s, const float* d_pos, const
     const int cb_init[8] = {0x7FFFFFFF, 0x7FFFFFFF, 0x7FFFFFFF, (int)0x80000000, (int)0x80000000, (int)0x80000000, 0, 0};
     unsigned cnt[kCollapseCounters] = {1u, 0u, 0u, 0u, 1u};   // one node (the root), one task on level 0
     const int2 root_task = make_int2(0, 0);   // binary node 0 (internal root, or the one leaf) -> wide node 0
+    float4 rb[2];
+    int depth = 0;
+    ptx_host::StreamGuard guard(st);          // over the values above
     cudaError_t e = cudaMemcpyAsync(cb, cb_init, sizeof(cb_init), cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(counters, cnt, sizeof(cnt), cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(ta, &root_task, sizeof(int2), cudaMemcpyHostToDevice, st);
@@ -848,11 +852,12 @@ int build_mesh_device_core(ptr_ctx* ctx, ptr_scene* s, const float* d_pos, const
     e = cudaMemcpyAsync(wide, wide_big, sizeof(uint32_t) * 20 * (size_t)cnt[0], cudaMemcpyDeviceToDevice, st);
     if (binary) k_emit_tris<<<grid, block, 0, st>>>(d_pos, d_idx, d_alpha, nullptr, keys, n, tri);
     k_emit_tris<<<grid, block, 0, st>>>(d_pos, d_idx, d_alpha, order, keys, n, tri_w);
-    float4 rb[2];
-    int depth = 0;
     if (e == cudaSuccess && binary) e = cudaMemcpyAsync(rb, bvh, sizeof(rb), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(&depth, depth_dev, sizeof(int), cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    if (e == cudaSuccess) {
+        e = cudaStreamSynchronize(st);
+        guard.waited();
+    }
     if (e == cudaSuccess) e = cudaGetLastError();
     release();
     if (e != cudaSuccess) return cuda_fail(ctx, e, "scene: device BVH build");
@@ -891,7 +896,7 @@ int build_mesh_device(ptr_ctx* ctx, ptr_scene* s, const ptr_mesh_desc& md, DevMe
     if (e == cudaSuccess && d_alpha) e = cudaMemcpyAsync(d_alpha, md.tri_alpha, sizeof(float) * (size_t)n, cudaMemcpyHostToDevice, st);
     if (e != cudaSuccess) { release(); return cuda_fail(ctx, e, "scene: device BVH build"); }
     const int rc = build_mesh_device_core(ctx, s, d_pos, d_idx, d_alpha, n, m, root, n_nodes, n_cw_nodes, bin_depth);
-    release();   // the core synchronised the stream before it returned
+    release();   // the core waited for the stream before it returned
     return rc;
 }
 
@@ -2546,6 +2551,7 @@ int ptr_render_batch(ptr_ctx* ctx, const ptr_batch_job* jobs, int n_jobs) {
         bp->tables_n = n_tables;
     }
     std::vector<unsigned char> image(n_tables);
+    ptx_host::StreamGuard guard(st);
     std::memcpy(image.data(), scenes.data(), o_progs);
     std::memcpy(image.data() + o_progs, progs.data(), sizeof(ProgParams) * n_jobs);
     std::memcpy(image.data() + o_jobs, bjobs.data(), sizeof(BatchJob) * n_jobs);
@@ -2554,7 +2560,6 @@ int ptr_render_batch(ptr_ctx* ctx, const ptr_batch_job* jobs, int n_jobs) {
     const ProgParams* d_progs = (const ProgParams*)(bp->tables + o_progs);
     const BatchJob* d_jobs = (const BatchJob*)(bp->tables + o_jobs);
     const long long* d_off = (const long long*)(bp->tables + o_off);
-    int rc = PTR_OK;
     BatchTables bt{};
     bt.scenes = d_scenes;
     bt.progs = d_progs;
@@ -2647,8 +2652,8 @@ int ptr_render_batch(ptr_ctx* ctx, const ptr_batch_job* jobs, int n_jobs) {
             if (kv.second.first) cudaGraphDestroy(kv.second.first);
         }
     }
-    if (e != cudaSuccess) rc = cuda_fail(ctx, e, "ptr_render_batch");
-    if (rc) return rc;
+    if (e != cudaSuccess) return cuda_fail(ctx, e, "ptr_render_batch");
+    guard.waited();
     for (int j = 0; j < n_jobs; ++j) film_done(jobs[j].prog, &jobs[j].frame);
     bp->last_scene = nullptr;
     return PTR_OK;
@@ -2708,6 +2713,7 @@ int ptr_trace_closest(ptr_ctx* ctx, ptr_scene* s, int accel, const float* rays, 
     float* d_t = (float*)(d_prim + nn);
     DevScene S = s->dev;
     S.accel = accel;
+    ptx_host::StreamGuard guard(ctx->stream);   // over the caller's arrays
     cudaError_t e = cudaMemcpyAsync(d_rays, rays, nn * 6 * sizeof(float), cudaMemcpyHostToDevice, ctx->stream);
     if (e == cudaSuccess) {
         // as many threads as stay resident: a query is a chain of dependent loads
@@ -2719,7 +2725,10 @@ int ptr_trace_closest(ptr_ctx* ctx, ptr_scene* s, int accel, const float* rays, 
     if (e == cudaSuccess) e = cudaMemcpyAsync(element, d_el, nn * 4, cudaMemcpyDeviceToHost, ctx->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(prim, d_prim, nn * 4, cudaMemcpyDeviceToHost, ctx->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(t, d_t, nn * 4, cudaMemcpyDeviceToHost, ctx->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+    if (e == cudaSuccess) {
+        e = cudaStreamSynchronize(ctx->stream);
+        guard.waited();
+    }
     dev_free(ctx, d_rays);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "ptr_trace_closest");
     return PTR_OK;
