@@ -32,6 +32,7 @@
 #include "device/rails.cuh"
 #include "host/accel_build.h"
 #include "host/field_compile.h"
+#include "host/profile_events.h"
 #include "host/stream_guard.h"
 #include "walk.h"
 
@@ -483,32 +484,17 @@ ProgParams prog_params(const ptr_program_desc& d) {
 // loops through heterogeneous media are too uneven to wait for one another.
 int shade_lockstep(bool media, bool heterogeneous) { return media && !heterogeneous ? 1 : 0; }
 
-// Event pairs around each launch of an instrumented render (kernel class, start, end).
-struct ProfRec { int cls; cudaEvent_t a, b; int n0, n; };   // n: kernels launched in the region
-
 template <class Col>
 void launch_wave_t(ptr_program* p, const ptr_scene* s, cudaStream_t st, int iters, float* samples, int n_sm,
-                   std::vector<ProfRec>* prof, bool film, bool dry) {
+                   ptx_host::ProfList* prof, bool film, bool dry) {
     constexpr bool SPECTRAL = sizeof(Col) == sizeof(s4);
     DevScene Sp = s->dev;
     Sp.accel = p->desc.accel;
     Sp.inst_accel = p->desc.instance_accel;
     Sp.work = (p->profile_next & PTR_PROFILE_WORK) ? p->work_dev : nullptr;
     int n_launched = 0;
-    auto mark = [&](int cls) -> ProfRec* {
-        if (!prof) return nullptr;
-        ProfRec r{cls, nullptr, nullptr, n_launched, 0};
-        cudaEventCreate(&r.a);
-        cudaEventCreate(&r.b);
-        cudaEventRecord(r.a, st);
-        prof->push_back(r);
-        return &prof->back();
-    };
-    auto done = [&](ProfRec* r) {
-        if (!r) return;
-        cudaEventRecord(r->b, st);
-        r->n = n_launched - r->n0;
-    };
+    auto mark = [&](int cls) { if (prof) prof->begin(cls, n_launched, st); };
+    auto done = [&] { if (prof) prof->end(n_launched, st); };
     const DevScene& S = Sp;
     const ProgParams P = prog_params(p->desc);
     const int block = tuning_of(p).block;
@@ -517,29 +503,29 @@ void launch_wave_t(ptr_program* p, const ptr_scene* s, cudaStream_t st, int iter
     pool.sort_buckets = tuning_of(p).sort_buckets;
     pool.ray_sort = tuning_of(p).ray_sort;
     pool.lockstep = shade_lockstep(s->has_media != 0, S.has_het != 0);
-    ProfRec* r = mark(0);
+    mark(0);
     const BatchTables nob{};
     // this scene's compiled kernels (ptr_specialize); the counting pass keeps the generic ones
     const SpecKernels* sk = (p->spec.scene_id == s->id && p->spec.shade) ? &p->spec : nullptr;
     L(k_generate<false, SPECTRAL>, 0, S, pool, p->fp_dev, AdjParams{});
-    done(r);
+    done();
     for (int it = 0; it < iters; ++it) {
         int in = it & 1;
         PathPool pi = pool;   // camera rays keep their generation order; later queues are key-sorted
         pi.ray_in = pool.ray_sort && it > 0;
         pi.iter = it;
-        r = mark(1);
+        mark(1);
         if (S.work) L(k_closest<true, false>, 0, S, pi, in, nob);
         else if (sk) L.raw(sk->closest, 0, S, pi, in, nob);
         else L(k_closest<false, false>, 0, S, pi, in, nob);
-        done(r);
+        done();
         if (pool.sort_buckets > 1) {   // occupant-sorted shading queue
-            r = mark(5);
+            mark(5);
             launch_shade_sort(L, pi, in);
-            done(r);
+            done();
         }
         const bool media = s->has_media != 0;
-        r = mark(2);
+        mark(2);
         if (sk) L.raw(sk->shade, 0, S, pi, P, in, nob, AdjParams{});
         else switch (P.direct * 2 + (media ? 1 : 0)) {
             case 0: L(k_shade<Col, PTR_DIRECT_NONE, false, false>, 0, S, pi, P, in, nob, AdjParams{}); break;
@@ -549,14 +535,14 @@ void launch_wave_t(ptr_program* p, const ptr_scene* s, cudaStream_t st, int iter
             case 4: L(k_shade<Col, PTR_DIRECT_MIS, false, false>, 0, S, pi, P, in, nob, AdjParams{}); break;
             default: L(k_shade<Col, PTR_DIRECT_MIS, true, false>, 0, S, pi, P, in, nob, AdjParams{}); break;
         }
-        done(r);
+        done();
         if (pool.ray_sort) {
-            r = mark(5);
+            mark(5);
             launch_ray_sort(L, pool, in, P.direct != PTR_DIRECT_NONE);
-            done(r);
+            done();
         }
         if (P.direct != PTR_DIRECT_NONE) {
-            r = mark(3);
+            mark(3);
             PathPool ps = pool;
             ps.iter = it;
             // slot 1 (equiangular segment queries) before slot 0 (surface / vertex NEE)
@@ -573,19 +559,19 @@ void launch_wave_t(ptr_program* p, const ptr_scene* s, cudaStream_t st, int iter
                     else L(k_shadow<Col, false, false, false>, 0, S, ps, P, nob, slot, AdjParams{});
                 }
             }
-            done(r);
+            done();
         }
     }
     if (!film) return;
-    r = mark(4);
+    mark(4);
     L(k_film<SPECTRAL>, 0, pool, p->fp_dev, p->sum, p->sumsq, samples, S);
     if (!dry) k_advance<<<1, 32, 0, st>>>(pool);
     L.count_raw(1);
-    done(r);
+    done();
 }
 
 void launch_wave(ptr_program* p, const ptr_scene* s, cudaStream_t st, int iters, float* samples, int n_sm,
-                 std::vector<ProfRec>* prof = nullptr, bool film = true, bool dry = false) {
+                 ptx_host::ProfList* prof = nullptr, bool film = true, bool dry = false) {
     if (p->desc.color == PTR_COLOR_SPECTRAL) launch_wave_t<s4>(p, s, st, iters, samples, n_sm, prof, film, dry);
     else launch_wave_t<f3>(p, s, st, iters, samples, n_sm, prof, film, dry);
 }
@@ -662,7 +648,7 @@ void launch_walk(const Launcher& L, const void* kern, size_t smem, const DevScen
 // sk: the mix's compiled batched kernels (ptr_specialize_batch), or null for the generic ones.
 void launch_batch_wave(const DevScene& S0, const PathPool& pool_in, const BatchTables& bt, int direct, bool media,
                        bool het, bool equiangular, cudaStream_t st, int iters, int n_sm, const ptr_tuning& tune,
-                       const SpecKernels* sk, std::vector<ProfRec>* prof = nullptr, bool dry = false) {
+                       const SpecKernels* sk, ptx_host::ProfList* prof = nullptr, bool dry = false) {
     const int block = tune.block;
     int n_launched = 0;
     const Launcher L{block, n_sm, st, dry, &n_launched};
@@ -671,37 +657,25 @@ void launch_batch_wave(const DevScene& S0, const PathPool& pool_in, const BatchT
     pool.ray_sort = tune.ray_sort;
     pool.lockstep = shade_lockstep(media, het);
     ProgParams P0{};
-    auto mark = [&](int cls) -> ProfRec* {
-        if (!prof) return nullptr;
-        ProfRec r{cls, nullptr, nullptr, n_launched, 0};
-        cudaEventCreate(&r.a);
-        cudaEventCreate(&r.b);
-        cudaEventRecord(r.a, st);
-        prof->push_back(r);
-        return &prof->back();
-    };
-    auto done = [&](ProfRec* r) {
-        if (!r) return;
-        cudaEventRecord(r->b, st);
-        r->n = n_launched - r->n0;
-    };
-    ProfRec* r = mark(0);
+    auto mark = [&](int cls) { if (prof) prof->begin(cls, n_launched, st); };
+    auto done = [&] { if (prof) prof->end(n_launched, st); };
+    mark(0);
     L(k_generate_batch, 0, pool, bt);
-    done(r);
+    done();
     for (int it = 0; it < iters; ++it) {
         int in = it & 1;
         PathPool pi = pool;
         pi.ray_in = pool.ray_sort && it > 0;
-        r = mark(1);
+        mark(1);
         if (sk) L.raw(sk->closest, 0, S0, pi, in, bt);
         else L(k_closest<false, true>, 0, S0, pi, in, bt);
-        done(r);
+        done();
         if (pool.sort_buckets > 1) {
-            r = mark(5);
+            mark(5);
             launch_shade_sort(L, pi, in);
-            done(r);
+            done();
         }
-        r = mark(2);
+        mark(2);
         if (sk) L.raw(sk->shade, 0, S0, pi, P0, in, bt, AdjParams{});
         else switch (direct * 2 + (media ? 1 : 0)) {
             case 0: L(k_shade<f3, PTR_DIRECT_NONE, false, true>, 0, S0, pi, P0, in, bt, AdjParams{}); break;
@@ -711,27 +685,27 @@ void launch_batch_wave(const DevScene& S0, const PathPool& pool_in, const BatchT
             case 4: L(k_shade<f3, PTR_DIRECT_MIS, false, true>, 0, S0, pi, P0, in, bt, AdjParams{}); break;
             default: L(k_shade<f3, PTR_DIRECT_MIS, true, true>, 0, S0, pi, P0, in, bt, AdjParams{}); break;
         }
-        done(r);
+        done();
         if (pool.ray_sort) {
-            r = mark(5);
+            mark(5);
             launch_ray_sort(L, pool, in, direct != PTR_DIRECT_NONE);
-            done(r);
+            done();
         }
         if (direct != PTR_DIRECT_NONE) {
-            r = mark(3);
+            mark(3);
             for (int slot = equiangular ? 1 : 0; slot >= 0; --slot) {
                 if (sk) L.raw(sk->shadow, 0, S0, pool, P0, bt, slot, AdjParams{});
                 else if (media) L(k_shadow<f3, true, false, true>, 0, S0, pool, P0, bt, slot, AdjParams{});
                 else L(k_shadow<f3, false, false, true>, 0, S0, pool, P0, bt, slot, AdjParams{});
             }
-            done(r);
+            done();
         }
     }
-    r = mark(4);
+    mark(4);
     L(k_film_batch, 0, pool, bt);
     if (!dry) k_advance<<<1, 32, 0, st>>>(pool);
     L.count_raw(1);
-    done(r);
+    done();
 }
 
 int device_sms(int dev) {
@@ -1609,17 +1583,11 @@ FrameParams frame_params(const ptr_frame* f, long long total, int cap, bool fres
     return F;
 }
 
-// Sums an instrumented render's event pairs per kernel class (the stream is idle).
-void fold_profile(ptr_program* p, std::vector<ProfRec>& prof) {
+// An instrumented render's times and launches per kernel class (the stream is idle); without a
+// list, zeros.
+void fold_profile(ptr_program* p, const ptx_host::ProfList* prof) {
     for (int k = 0; k < PTR_PROFILE_CLASSES; ++k) { p->prof_ms[k] = 0.f; p->prof_launches[k] = 0; }
-    for (ProfRec& r : prof) {
-        float ms = 0.f;
-        cudaEventElapsedTime(&ms, r.a, r.b);
-        p->prof_ms[r.cls] += ms;
-        p->prof_launches[r.cls] += r.n;
-        cudaEventDestroy(r.a);
-        cudaEventDestroy(r.b);
-    }
+    if (prof) prof->fold(p->prof_ms, p->prof_launches);
 }
 
 // A frame on the one-kernel walk: per wave one walk and one film pass, launched directly (two
@@ -1650,29 +1618,22 @@ int render_walk(ptr_program* p, ptr_scene* s, const ptr_frame* f, const FramePar
     wa.stats = p->pool.stats;
     wa.iters = wave_iterations(p, s);
     const Launcher L{tuning_of(p).block, device_sms(ctx->device), st, false};
-    std::vector<ProfRec> prof;
-    auto event = [&](int cls, bool begin) {
-        if (!profiling) return;
-        if (begin) {
-            prof.push_back(ProfRec{cls, nullptr, nullptr, 0, 1});
-            cudaEventCreate(&prof.back().a);
-            cudaEventCreate(&prof.back().b);
-        }
-        cudaEventRecord(begin ? prof.back().a : prof.back().b, st);
-    };
+    ptx_host::ProfList prof;
+    auto mark = [&](int cls) { if (profiling) prof.begin(cls, 0, st); };
+    auto done = [&] { if (profiling) prof.end(1, st); };
     for (wa.base = 0; wa.base < F.total; wa.base += F.capacity) {
         wa.n = (unsigned)std::min<long long>(F.capacity, F.total - wa.base);
-        event(2, true);
+        mark(2);
         launch_walk(L, kern, 0, S, P, F, BatchTables{}, wa, AdjParams{});
-        event(2, false);
-        event(4, true);
+        done();
+        mark(4);
         L(k_film_walk, 0, F, wa, p->desc.aovs ? p->aov_sum : (double*)nullptr, p->sum, p->sumsq, samples_dev);
-        event(4, false);
+        done();
     }
     CK(ctx, cudaGetLastError());
     if (profiling) {
         CK(ctx, cudaStreamSynchronize(st));
-        fold_profile(p, prof);
+        fold_profile(p, &prof);
     }
     film_done(p, f);
     return PTR_OK;
@@ -1797,12 +1758,11 @@ int render_impl(ptr_program* p, ptr_scene* s, const ptr_frame* f, float* samples
         }
         for (long long w = 0; w < waves; ++w) CK(ctx, cudaGraphLaunch(p->graph, st));
     } else if (profiling) {
-        std::vector<ProfRec> prof;
-        prof.reserve((size_t)waves * (iters * 5 + 2));
+        ptx_host::ProfList prof;
         for (long long w = 0; w < waves; ++w) launch_wave(p, s, st, iters, samples_dev, n_sm, &prof);
         CK(ctx, cudaGetLastError());
         CK(ctx, cudaStreamSynchronize(st));
-        fold_profile(p, prof);
+        fold_profile(p, &prof);
         p->profile_next = 0;
     } else {
         for (long long w = 0; w < waves; ++w) launch_wave(p, s, st, iters, samples_dev, n_sm);
@@ -2584,16 +2544,9 @@ int ptr_render_batch(ptr_ctx* ctx, const ptr_batch_job* jobs, int n_jobs) {
     if (walk) {
         // per wave one walk over its jobs' paths and one film pass; an instrumented render
         // reports them under classes 2 and 4
-        std::vector<ProfRec> prof;
-        auto event = [&](int cls, bool begin) {
-            if (!profiling) return;
-            if (begin) {
-                prof.push_back(ProfRec{cls, nullptr, nullptr, 0, 1});
-                cudaEventCreate(&prof.back().a);
-                cudaEventCreate(&prof.back().b);
-            }
-            cudaEventRecord(begin ? prof.back().a : prof.back().b, st);
-        };
+        ptx_host::ProfList prof;
+        auto mark = [&](int cls) { if (profiling) prof.begin(cls, 0, st); };
+        auto done = [&] { if (profiling) prof.end(1, st); };
         const void* kern = sk && sk->walk ? sk->walk : ptx_host::walk_kernel(direct, media, false, true, false);
         const Launcher L{ctx->tune.block, n_sm, st, false};
         WalkArgs wa{};
@@ -2604,26 +2557,25 @@ int ptr_render_batch(ptr_ctx* ctx, const ptr_batch_job* jobs, int n_jobs) {
             wa.base = w * cap;
             wa.n = (unsigned)std::min(cap, total - wa.base);
             wa.iters = wave_iters[(size_t)w];
-            event(2, true);
+            mark(2);
             launch_walk(L, kern, 0, jobs[0].scene->dev, ProgParams{}, FrameParams{}, bt, wa, AdjParams{});
-            event(2, false);
-            event(4, true);
+            done();
+            mark(4);
             L(k_film_batch_walk, 0, bt, wa);
-            event(4, false);
+            done();
             e = cudaGetLastError();
         }
         if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-        if (profiling && e == cudaSuccess) fold_profile(bp, prof);
+        if (profiling) fold_profile(bp, e == cudaSuccess ? &prof : nullptr);
     } else if (profiling) {
         // instrumented: plain launches with events around each (no graph)
-        std::vector<ProfRec> prof;
-        prof.reserve((size_t)waves * (iters * 5 + 2));
+        ptx_host::ProfList prof;
         for (long long w = 0; e == cudaSuccess && w < waves; ++w) {
             launch_batch_wave(jobs[0].scene->dev, bp->pool, bt, direct, media, het, equi, st, wave_iters[(size_t)w], n_sm, ctx->tune, sk, &prof);
             e = cudaGetLastError();
         }
         if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-        if (e == cudaSuccess) fold_profile(bp, prof);
+        fold_profile(bp, e == cudaSuccess ? &prof : nullptr);
     } else {
         // occupancy queries outside capture, then one captured wave per iteration count the
         // waves need
