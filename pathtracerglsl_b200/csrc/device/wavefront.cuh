@@ -125,6 +125,10 @@ __device__ __forceinline__ unsigned ray_key(const DevScene& S, f3 o, f3 d) {
     k = (k << 3) | (o.x > S.sort_c[0] ? 1u : 0u) | (o.y > S.sort_c[1] ? 2u : 0u) | (o.z > S.sort_c[2] ? 4u : 0u);
     return k;
 }
+// The adjoint's hit log of this launch's iteration (null where it is not logged).
+__device__ __forceinline__ float4* hit_log_slice(const PathPool& pool) {
+    return pool.hit_log && pool.iter < pool.hit_log_iters ? pool.hit_log + 4 * (size_t)pool.iter * (size_t)pool.hit_log_stride : nullptr;
+}
 // The queue a k_closest of iteration `in` reads.
 __device__ __forceinline__ const int* closest_queue(const PathPool& pool, int in);
 
@@ -833,8 +837,14 @@ __device__ __forceinline__ void closest_refill(const DevScene& S, const PathPool
                 float t;
                 if (analytic_root(S.regions[g], r, t) && t < h.t) { h.t = t; h.region = g; h.element = 0; h.prim = -1; }
             }
-            pool.hit[i] = make_float4(h.t, h.u, h.v, 0.f);
-            pool.hit_i[i] = make_int4(h.region, h.element, h.prim, 0);
+            const float4 hf = make_float4(h.t, h.u, h.v, 0.f);
+            const int4 hi = make_int4(h.region, h.element, h.prim, 0);
+            pool.hit[i] = hf;
+            pool.hit_i[i] = hi;
+            if (float4* log = pool.hit_log_mode == 1 ? hit_log_slice(pool) : nullptr) {
+                log[4 * (size_t)i] = hf;
+                log[4 * (size_t)i + 1] = int4_as_float4(hi);
+            }
             if (buckets > 1) pool.sort_key[i] = (unsigned char)shade_key(S, h.region, pool.st[i].y, buckets);
             active = false;
         }
@@ -854,7 +864,9 @@ __global__ void __launch_bounds__(256, PTR_TRACE_MIN_BLOCKS) k_closest(const __g
     }
     const int* q = closest_queue(pool, in);
     Work w{0u, 0u, 0u, 0u};
-    if (PTR_REFILL && kHasMesh && !BATCH && pool.fetch && S0.flat_region >= 0) {
+    float4* log = BATCH ? nullptr : hit_log_slice(pool);
+    // (a logged iteration of the replay walks nothing: it reads the log in the loop below)
+    if (PTR_REFILL && kHasMesh && !BATCH && pool.fetch && S0.flat_region >= 0 && !(log && pool.hit_log_mode == 2)) {
         const DevBatch& b = S0.batches[S0.regions[S0.flat_region].ref];
         const bool wide = flat_wide_ok(S0, b), binary = flat_binary_ok(S0, b);
         if (wide) closest_refill<COUNT, true>(S0, pool, q, n, buckets, pool.fetch + 0, &w);
@@ -865,9 +877,6 @@ __global__ void __launch_bounds__(256, PTR_TRACE_MIN_BLOCKS) k_closest(const __g
         }
     }
     const WaveJobs wj = BATCH ? WaveJobs(pool, bt) : WaveJobs{};
-    // the adjoint's hit log: this launch's slice, when its iteration is logged
-    float4* log = (!BATCH && pool.hit_log && pool.iter < pool.hit_log_iters)
-                      ? pool.hit_log + 4 * (size_t)pool.iter * (size_t)pool.hit_log_stride : nullptr;
     QueueCursor cur(n, pool.fetch ? pool.fetch + 0 : nullptr);
     unsigned k;
     while (cur.next(k)) {
@@ -1783,8 +1792,7 @@ __global__ void __launch_bounds__(256, PTR_TRACE_MIN_BLOCKS) k_shadow(const __gr
     // pairs; a count of -1 marks a query the replay walks again)
     float4* slog = nullptr;
     if constexpr (!BATCH && !SPECTRAL)
-        if (slot == 0 && pool.hit_log && pool.iter < pool.hit_log_iters)
-            slog = pool.hit_log + 4 * (size_t)pool.iter * (size_t)pool.hit_log_stride + 2;
+        if (slot == 0 && hit_log_slice(pool)) slog = hit_log_slice(pool) + 2;
     const bool rec = !ADJ && slog && pool.hit_log_mode == 1;
     const bool rep = ADJ && slog && pool.hit_log_mode == 2;
     if (PTR_REFILL && kHasMesh && !MEDIA && !BATCH && !ADJ && !rec && pool.fetch && S0.flat_region >= 0) {
