@@ -13,7 +13,6 @@
 #include <cmath>
 #include <map>
 #include <mutex>
-#include <set>
 #include <tuple>
 #include <type_traits>
 #include <cstdio>
@@ -31,6 +30,7 @@
 #include "device/lbvh.cuh"
 #include "device/rails.cuh"
 #include "host/accel_build.h"
+#include "host/device_memory.h"
 #include "host/field_compile.h"
 #include "host/profile_events.h"
 #include "host/stream_guard.h"
@@ -61,8 +61,7 @@ struct ptr_ctx {
     // by census key
     std::map<std::string, SpecKernels> batch_spec;
     int accel_build = PTR_BUILD_HOST;   // where ptr_upload_scene builds mesh BVHs (ptr_set_accel_build)
-    cudaMemPool_t pool = nullptr;       // the device's pool (acquire_pool)
-    std::set<void*> big;                // allocations outside it (kPoolMax)
+    ptx_host::DeviceMemory memory;
 };
 
 struct ptr_scene {
@@ -158,63 +157,14 @@ int cuda_fail(ptr_ctx* ctx, cudaError_t e, const char* what) {
         if (e_ != cudaSuccess) return cuda_fail((ctx), e_, #call); \
     } while (0)
 
-// Device memory of the contexts' objects.  A scene, program or build takes a few dozen blocks,
-// and cudaMalloc / cudaFree cost 0.1 to several ms each (38 of each made 18 of the 25 ms of
-// uploading a 327,680-triangle scene).  So the contexts on one device share a stream-ordered
-// pool: allocating and freeing is then a few microseconds while it holds enough.  It keeps at
-// most kPoolKeep bytes that no object uses and goes with the device's last context.  Blocks
-// above kPoolMax come from cudaMalloc: the pool maps memory in small pieces, and the 8.7 GB
-// path pool of a 2^25-path wave took 80 ms from it against 5.
-constexpr unsigned long long kPoolKeep = 512ull << 20;
-constexpr size_t kPoolMax = 256ull << 20;
-constexpr int kPoolDevices = 64;
-struct DevicePool { cudaMemPool_t pool = nullptr; int users = 0; };
-std::mutex g_pool_mutex;
-DevicePool g_pools[kPoolDevices];
-cudaMemPool_t acquire_pool(int device) {
-    if (device >= kPoolDevices) return nullptr;
-    std::lock_guard<std::mutex> lock(g_pool_mutex);
-    DevicePool& d = g_pools[device];
-    if (!d.pool) {
-        cudaMemPoolProps props{};
-        props.allocType = cudaMemAllocationTypePinned;
-        props.location.type = cudaMemLocationTypeDevice;
-        props.location.id = device;
-        unsigned long long keep = kPoolKeep;
-        if (cudaMemPoolCreate(&d.pool, &props) != cudaSuccess) { d.pool = nullptr; return nullptr; }
-        if (cudaMemPoolSetAttribute(d.pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
-            cudaMemPoolDestroy(d.pool);
-            d.pool = nullptr;
-            return nullptr;
-        }
-    }
-    ++d.users;
-    return d.pool;
-}
-void release_pool(int device) {
-    std::lock_guard<std::mutex> lock(g_pool_mutex);
-    DevicePool& d = g_pools[device];
-    if (--d.users > 0) return;
-    cudaMemPoolDestroy(d.pool);
-    d.pool = nullptr;
-}
-
-// Memory of a context's object, ordered on its stream (every use is).
 template <typename T>
 cudaError_t dev_alloc(ptr_ctx* ctx, T** out, size_t bytes) {
     void* p = nullptr;
-    const bool big = bytes > kPoolMax;
-    const cudaError_t e = big ? cudaMalloc(&p, bytes) : cudaMallocFromPoolAsync(&p, bytes, ctx->pool, ctx->stream);
-    if (e != cudaSuccess) { p = nullptr; cudaGetLastError(); }
-    else if (big) ctx->big.insert(p);
+    const cudaError_t e = ctx->memory.alloc(&p, bytes);
     *out = (T*)p;
     return e;
 }
-void dev_free(ptr_ctx* ctx, void* p) {
-    if (!p) return;
-    if (ctx->big.erase(p)) cudaFree(p);
-    else cudaFreeAsync(p, ctx->stream);
-}
+void dev_free(ptr_ctx* ctx, void* p) { ctx->memory.free(p); }
 
 // A device copy of a host array that lives with the scene.  Tables up to kStageMax bytes are
 // laid into one staged block (one allocation and one copy for a scene's dozens of small
@@ -2025,15 +1975,10 @@ int ptr_create(int device_ordinal, ptr_ctx** out) {
         delete c;
         return PTR_E_CUDA;
     }
-    c->pool = acquire_pool(device_ordinal);
-    if (!c->pool) {
-        cudaStreamDestroy(c->stream);
-        delete c;
-        return PTR_E_CUDA;
-    }
+    c->memory.open(device_ordinal, c->stream);
     // the counting sort's scan stages its whole table in shared memory (above the 48 KB default)
     if (cudaFuncSetAttribute((const void*)k_sort_scan, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSortScanSmem) != cudaSuccess) {
-        release_pool(device_ordinal);
+        c->memory.close();
         cudaStreamDestroy(c->stream);
         delete c;
         return PTR_E_CUDA;
@@ -2048,7 +1993,7 @@ int ptr_destroy(ptr_ctx* ctx) {
     cudaStreamSynchronize(ctx->stream);
     if (ctx->batch) ptr_free_program(ctx->batch);
     cudaStreamSynchronize(ctx->stream);   // the frees above
-    release_pool(ctx->device);
+    ctx->memory.close();
     cudaStreamDestroy(ctx->stream);
     delete ctx;
     return PTR_OK;
