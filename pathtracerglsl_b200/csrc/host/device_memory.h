@@ -77,16 +77,14 @@ public:
     }
     void close() { DevicePools::all().release(device_); }
     cudaError_t alloc(void** out, size_t bytes) {
-        void* p = nullptr;
         const bool pooled = pool_ && bytes <= kPoolMax;
-        const cudaError_t e = pooled ? cudaMallocFromPoolAsync(&p, bytes, pool_, stream_) : cudaMalloc(&p, bytes);
-        if (e != cudaSuccess) {
-            p = nullptr;
-            cudaGetLastError();
-        } else if (!pooled) {
-            direct_.insert(p);
+        cudaError_t e = take(out, bytes, pooled);
+        if (e == cudaErrorMemoryAllocation && pool_) {   // what the pool keeps idle may be what is missing
+            cudaStreamSynchronize(stream_);
+            cudaMemPoolTrimTo(pool_, 0);
+            e = take(out, bytes, pooled);
         }
-        *out = p;
+        if (e == cudaSuccess && !pooled) direct_.insert(*out);
         return e;
     }
     void free(void* p) {
@@ -96,6 +94,13 @@ public:
     }
 
 private:
+    cudaError_t take(void** out, size_t bytes, bool pooled) {
+        void* p = nullptr;
+        const cudaError_t e = pooled ? cudaMallocFromPoolAsync(&p, bytes, pool_, stream_) : cudaMalloc(&p, bytes);
+        if (e != cudaSuccess) cudaGetLastError();
+        *out = e == cudaSuccess ? p : nullptr;
+        return e;
+    }
     int device_ = 0;
     cudaStream_t stream_ = nullptr;
     cudaMemPool_t pool_ = nullptr;

@@ -102,3 +102,19 @@ def test_a_block_that_does_not_fit_is_null(tmp_path):
     m.close();
     """)
     assert "2 null" in " ".join(out) and out[-4:] == ["pooled", "0", "async1", "~pool0"]
+
+
+def test_idle_pool_memory_does_not_refuse_a_block(tmp_path):
+    """A block fits as long as it fits beside the blocks in use: what the pool keeps idle is given
+    back first, and a block that does not fit then is refused."""
+    out = _run(tmp_path, """
+    DeviceMemory m; m.open(0, nullptr);
+    left = 300u << 20; idle = 400u << 20;
+    std::printf("%d ", (int)m.alloc(&a, 600u << 20));
+    std::printf("%d ", (int)m.alloc(&b, 200u << 20));
+    idle = 150u << 20;
+    std::printf("%d ", (int)m.alloc(&b, 200u << 20));
+    m.free(a); m.free(b); m.close();
+    """)
+    assert out == ("pool0 keep512 malloc! wait trim0 malloc 0 pooled! wait trim0 pooled! 2 "
+                   "pooled! wait trim0 pooled 0 free1 async2 ~pool0").split()
