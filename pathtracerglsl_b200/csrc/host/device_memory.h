@@ -13,7 +13,8 @@ namespace ptx_host {
 // microseconds while it holds enough.  It keeps at most kPoolKeep bytes that no object uses and
 // goes with the device's last context.  Blocks above kPoolMax come from cudaMalloc: the pool maps
 // memory in small pieces, and the 8.7 GB path pool of a 2^25-path wave took 80 ms from it against
-// 5.  So does every block of a device that makes no pool.
+// 5.  So does every block of a device that makes no pool.  A block freed on one stream goes to
+// another only once it is idle: streams of the pool never wait for one another.
 constexpr unsigned long long kPoolKeep = 512ull << 20;
 constexpr size_t kPoolMax = 256ull << 20;
 
@@ -51,12 +52,14 @@ private:
         props.location.type = cudaMemLocationTypeDevice;
         props.location.id = device;
         unsigned long long keep = kPoolKeep;
+        int wait = 0;
         cudaMemPool_t pool = nullptr;
         if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) {
             cudaGetLastError();
             return nullptr;
         }
-        if (cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
+        if (cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess ||
+            cudaMemPoolSetAttribute(pool, cudaMemPoolReuseAllowInternalDependencies, &wait) != cudaSuccess) {
             cudaGetLastError();
             cudaMemPoolDestroy(pool);
             return nullptr;
@@ -67,7 +70,7 @@ private:
     std::map<int, Pool> pools_;
 };
 
-// One context's allocations, ordered on its stream (every use is).
+// Allocations of one of a context's streams, ordered on it: every use is, or follows a wait for it.
 class DeviceMemory {
 public:
     void open(int device, cudaStream_t stream) {
@@ -80,7 +83,7 @@ public:
         const bool pooled = pool_ && bytes <= kPoolMax;
         cudaError_t e = take(out, bytes, pooled);
         if (e == cudaErrorMemoryAllocation && pool_) {   // what the pool keeps idle may be what is missing
-            cudaStreamSynchronize(stream_);
+            cudaDeviceSynchronize();   // frees on every stream
             cudaMemPoolTrimTo(pool_, 0);
             e = take(out, bytes, pooled);
         }

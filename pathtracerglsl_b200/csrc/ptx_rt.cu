@@ -61,7 +61,11 @@ struct ptr_ctx {
     // by census key
     std::map<std::string, SpecKernels> batch_spec;
     int accel_build = PTR_BUILD_HOST;   // where ptr_upload_scene builds mesh BVHs (ptr_set_accel_build)
-    ptx_host::DeviceMemory memory;
+    // Scenes are uploaded (and their trees built) on a stream of their own, waited for before the
+    // upload returns, so an upload does not wait for frames in flight.
+    cudaStream_t upload = nullptr;
+    ptx_host::DeviceMemory memory;       // programs' and calls' blocks, ordered on stream
+    ptx_host::DeviceMemory scene_memory; // scenes' and builds' blocks, ordered on upload
 };
 
 struct ptr_scene {
@@ -158,13 +162,18 @@ int cuda_fail(ptr_ctx* ctx, cudaError_t e, const char* what) {
     } while (0)
 
 template <typename T>
-cudaError_t dev_alloc(ptr_ctx* ctx, T** out, size_t bytes) {
+cudaError_t dev_alloc(ptx_host::DeviceMemory& memory, T** out, size_t bytes) {
     void* p = nullptr;
-    const cudaError_t e = ctx->memory.alloc(&p, bytes);
+    const cudaError_t e = memory.alloc(&p, bytes);
     *out = (T*)p;
     return e;
 }
+template <typename T>
+cudaError_t dev_alloc(ptr_ctx* ctx, T** out, size_t bytes) { return dev_alloc(ctx->memory, out, bytes); }
 void dev_free(ptr_ctx* ctx, void* p) { ctx->memory.free(p); }
+template <typename T>
+cudaError_t scene_alloc(ptr_ctx* ctx, T** out, size_t bytes) { return dev_alloc(ctx->scene_memory, out, bytes); }
+void scene_free(ptr_ctx* ctx, void* p) { ctx->scene_memory.free(p); }
 
 // A device copy of a host array that lives with the scene.  Tables up to kStageMax bytes are
 // laid into one staged block (one allocation and one copy for a scene's dozens of small
@@ -176,7 +185,7 @@ int flush_stage(ptr_scene* s) {
     if (s->stage_used == 0) return PTR_OK;
     // the image mirrors the block and is written once: the copy may read it until the stream is waited for
     const unsigned char* image = s->stage.back().data() + (kStageBlock - s->stage_left);
-    CK(s->ctx, cudaMemcpyAsync(s->stage_dev, image, s->stage_used, cudaMemcpyHostToDevice, s->ctx->stream));
+    CK(s->ctx, cudaMemcpyAsync(s->stage_dev, image, s->stage_used, cudaMemcpyHostToDevice, s->ctx->upload));
     s->stage_dev += s->stage_used;
     s->stage_left -= s->stage_used;
     s->stage_used = 0;
@@ -199,7 +208,7 @@ int dev_copy(ptr_scene* s, const T* host, size_t n, const T** out) {
         if (int rc = flush_stage(s)) return rc;
     }
     unsigned char* p = nullptr;
-    cudaError_t e = dev_alloc(ctx, &p, staged ? kStageBlock : bytes);
+    cudaError_t e = scene_alloc(ctx, &p, staged ? kStageBlock : bytes);
     if (e != cudaSuccess) return fail(ctx, PTR_E_NOMEM, std::string("device allocation: ") + cudaGetErrorString(e));
     s->allocs.push_back(p);
     if (staged) {
@@ -209,8 +218,8 @@ int dev_copy(ptr_scene* s, const T* host, size_t n, const T** out) {
         s->stage_used = 0;
         return dev_copy(s, host, n, out);
     }
-    CK(ctx, cudaMemcpyAsync(p, host, bytes, cudaMemcpyHostToDevice, ctx->stream));
-    CK(ctx, cudaStreamSynchronize(ctx->stream));
+    CK(ctx, cudaMemcpyAsync(p, host, bytes, cudaMemcpyHostToDevice, ctx->upload));
+    CK(ctx, cudaStreamSynchronize(ctx->upload));
     *out = (const T*)p;
     return PTR_OK;
 }
@@ -675,7 +684,7 @@ int build_mesh_device_core(ptr_ctx* ctx, ptr_scene* s, const float* d_pos, const
                            int n, DevMesh& m, std::vector<double>& root, int& n_nodes, int& n_cw_nodes, int& bin_depth,
                            bool binary = true) {
     using namespace lbvh;
-    cudaStream_t st = ctx->stream;
+    cudaStream_t st = ctx->upload;
     const int n_sm = device_sms(ctx->device);
     const int grid = n_sm * 8, block = 256;
     int n_pad = kBitonicTile;
@@ -714,16 +723,16 @@ int build_mesh_device_core(ptr_ctx* ctx, ptr_scene* s, const float* d_pos, const
         return at;
     };
     unsigned char* tmp = nullptr;
-    auto release = [&]() { dev_free(ctx, tmp); tmp = nullptr; };
+    auto release = [&]() { scene_free(ctx, tmp); tmp = nullptr; };
     auto keep = [&](size_t bytes) -> void* {
         void* p = nullptr;
-        if (dev_alloc(ctx, &p, bytes) == cudaSuccess) s->allocs.push_back(p);
+        if (scene_alloc(ctx, &p, bytes) == cudaSuccess) s->allocs.push_back(p);
         return p;
     };
     float4* bvh = binary ? (float4*)keep(sizeof(float4) * 2 * (size_t)total) : nullptr;
     float4* tri = binary ? (float4*)keep(sizeof(float4) * 3 * (size_t)n) : nullptr;
     float4* tri_w = (float4*)keep(sizeof(float4) * 3 * (size_t)n);
-    if ((binary && (!bvh || !tri)) || !tri_w || dev_alloc(ctx, &tmp, carve(nullptr)) != cudaSuccess)
+    if ((binary && (!bvh || !tri)) || !tri_w || scene_alloc(ctx, &tmp, carve(nullptr)) != cudaSuccess)
         return fail(ctx, PTR_E_NOMEM, "scene: device BVH build: allocation failed");
     carve(tmp);
     const int cb_init[8] = {0x7FFFFFFF, 0x7FFFFFFF, 0x7FFFFFFF, (int)0x80000000, (int)0x80000000, (int)0x80000000, 0, 0};
@@ -804,14 +813,14 @@ int build_mesh_device_core(ptr_ctx* ctx, ptr_scene* s, const float* d_pos, const
 int build_mesh_device(ptr_ctx* ctx, ptr_scene* s, const ptr_mesh_desc& md, DevMesh& m, std::vector<double>& root,
                       int& n_nodes, int& n_cw_nodes, int& bin_depth) {
     const int n = md.n_triangles;
-    cudaStream_t st = ctx->stream;
+    cudaStream_t st = ctx->upload;
     float* d_pos = nullptr;
     unsigned* d_idx = nullptr;
     float* d_alpha = nullptr;
-    auto release = [&]() { dev_free(ctx, d_pos); dev_free(ctx, d_idx); dev_free(ctx, d_alpha); };
-    if (dev_alloc(ctx, &d_pos, sizeof(float) * 3 * (size_t)md.n_vertices) != cudaSuccess ||
-        dev_alloc(ctx, &d_idx, sizeof(unsigned) * 3 * (size_t)n) != cudaSuccess ||
-        (md.tri_alpha && dev_alloc(ctx, &d_alpha, sizeof(float) * (size_t)n) != cudaSuccess)) {
+    auto release = [&]() { scene_free(ctx, d_pos); scene_free(ctx, d_idx); scene_free(ctx, d_alpha); };
+    if (scene_alloc(ctx, &d_pos, sizeof(float) * 3 * (size_t)md.n_vertices) != cudaSuccess ||
+        scene_alloc(ctx, &d_idx, sizeof(unsigned) * 3 * (size_t)n) != cudaSuccess ||
+        (md.tri_alpha && scene_alloc(ctx, &d_alpha, sizeof(float) * (size_t)n) != cudaSuccess)) {
         release();
         return fail(ctx, PTR_E_NOMEM, "scene: device BVH build: cudaMalloc");
     }
@@ -914,19 +923,19 @@ int rail_mesh(ptr_ctx* ctx, ptr_scene* s, const ptr_rails& R, const RailDev& D, 
         for (int i = 0; i < T; ++i)
             if (!std::isfinite(R.records[4 * (ml->cdf_base + i)])) return fail(ctx, PTR_E_INVALID, who + ": non-finite light CDF");
     }
-    cudaStream_t st = ctx->stream;
+    cudaStream_t st = ctx->upload;
     float* d_pos = nullptr;
     unsigned* d_idx = nullptr;
     uint32_t* d_order = nullptr;
     float* d_alpha = nullptr;
-    auto release = [&]() { dev_free(ctx, d_pos); dev_free(ctx, d_idx); dev_free(ctx, d_order); dev_free(ctx, d_alpha); };
+    auto release = [&]() { scene_free(ctx, d_pos); scene_free(ctx, d_idx); scene_free(ctx, d_order); scene_free(ctx, d_alpha); };
     float4* tri = nullptr;
-    if (dev_alloc(ctx, &d_pos, sizeof(float) * 3 * (size_t)V) != cudaSuccess ||
-        dev_alloc(ctx, &d_idx, sizeof(unsigned) * 3 * (size_t)T) != cudaSuccess ||
-        (rm.tri_order && dev_alloc(ctx, &d_order, sizeof(uint32_t) * (size_t)T) != cudaSuccess) ||
-        (rm.tri_alpha && dev_alloc(ctx, &d_alpha, sizeof(float) * (size_t)T) != cudaSuccess) ||
-        dev_alloc(ctx, &tri, sizeof(float4) * 3 * (size_t)T) != cudaSuccess) {
-        dev_free(ctx, tri);
+    if (scene_alloc(ctx, &d_pos, sizeof(float) * 3 * (size_t)V) != cudaSuccess ||
+        scene_alloc(ctx, &d_idx, sizeof(unsigned) * 3 * (size_t)T) != cudaSuccess ||
+        (rm.tri_order && scene_alloc(ctx, &d_order, sizeof(uint32_t) * (size_t)T) != cudaSuccess) ||
+        (rm.tri_alpha && scene_alloc(ctx, &d_alpha, sizeof(float) * (size_t)T) != cudaSuccess) ||
+        scene_alloc(ctx, &tri, sizeof(float4) * 3 * (size_t)T) != cudaSuccess) {
+        scene_free(ctx, tri);
         release();
         return fail(ctx, PTR_E_NOMEM, who + ": cudaMalloc");
     }
@@ -960,9 +969,9 @@ int rail_mesh(ptr_ctx* ctx, ptr_scene* s, const ptr_rails& R, const RailDev& D, 
     if (ml) {
         float4* lt = nullptr;
         float* cdf = nullptr;
-        if (dev_alloc(ctx, &lt, sizeof(float4) * 3 * (size_t)T) != cudaSuccess) return fail(ctx, PTR_E_NOMEM, who + ": cudaMalloc");
+        if (scene_alloc(ctx, &lt, sizeof(float4) * 3 * (size_t)T) != cudaSuccess) return fail(ctx, PTR_E_NOMEM, who + ": cudaMalloc");
         s->allocs.push_back(lt);
-        if (dev_alloc(ctx, &cdf, sizeof(float) * (size_t)T) != cudaSuccess) return fail(ctx, PTR_E_NOMEM, who + ": cudaMalloc");
+        if (scene_alloc(ctx, &cdf, sizeof(float) * (size_t)T) != cudaSuccess) return fail(ctx, PTR_E_NOMEM, who + ": cudaMalloc");
         s->allocs.push_back(cdf);
         rails::k_light_tris<<<n_sm * 4, 256, 0, st>>>(D.v, ml->wpos_base, D.idx, rm.tbase, T, lt);
         rails::k_scalars<<<n_sm * 4, 256, 0, st>>>(D.rec, ml->cdf_base, T, cdf);
@@ -1033,9 +1042,9 @@ int rail_batch(ptr_ctx* ctx, ptr_scene* s, const ptr_rails& R, const RailDev& D,
         b.place = D.rec + rb.placements_base;
     } else {
         float4* place = nullptr;
-        if (dev_alloc(ctx, &place, sizeof(float4) * 2 * (size_t)N) != cudaSuccess) return fail(ctx, PTR_E_NOMEM, who + ": cudaMalloc");
+        if (scene_alloc(ctx, &place, sizeof(float4) * 2 * (size_t)N) != cudaSuccess) return fail(ctx, PTR_E_NOMEM, who + ": cudaMalloc");
         s->allocs.push_back(place);
-        rails::k_restride<<<n_sm * 4, 256, 0, ctx->stream>>>(D.rec, rb.placements_base, N, place);
+        rails::k_restride<<<n_sm * 4, 256, 0, ctx->upload>>>(D.rec, rb.placements_base, N, place);
         if (cudaError_t e = cudaGetLastError()) return cuda_fail(ctx, e, who.c_str());
         b.place = place;
     }
@@ -1975,10 +1984,18 @@ int ptr_create(int device_ordinal, ptr_ctx** out) {
         delete c;
         return PTR_E_CUDA;
     }
+    if (cudaStreamCreateWithFlags(&c->upload, cudaStreamNonBlocking) != cudaSuccess) {
+        cudaStreamDestroy(c->stream);
+        delete c;
+        return PTR_E_CUDA;
+    }
     c->memory.open(device_ordinal, c->stream);
+    c->scene_memory.open(device_ordinal, c->upload);
     // the counting sort's scan stages its whole table in shared memory (above the 48 KB default)
     if (cudaFuncSetAttribute((const void*)k_sort_scan, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSortScanSmem) != cudaSuccess) {
+        c->scene_memory.close();
         c->memory.close();
+        cudaStreamDestroy(c->upload);
         cudaStreamDestroy(c->stream);
         delete c;
         return PTR_E_CUDA;
@@ -1993,7 +2010,10 @@ int ptr_destroy(ptr_ctx* ctx) {
     cudaStreamSynchronize(ctx->stream);
     if (ctx->batch) ptr_free_program(ctx->batch);
     cudaStreamSynchronize(ctx->stream);   // the frees above
+    cudaStreamSynchronize(ctx->upload);
+    ctx->scene_memory.close();
     ctx->memory.close();
+    cudaStreamDestroy(ctx->upload);
     cudaStreamDestroy(ctx->stream);
     delete ctx;
     return PTR_OK;
@@ -2300,7 +2320,7 @@ static int upload_scene(ptr_ctx* ctx, const ptr_scene_desc* d, const ptr_rails* 
     // once the call returns
     if (!rc) rc = flush_stage(s);
     if (!rc) {
-        const cudaError_t e = cudaStreamSynchronize(ctx->stream);
+        const cudaError_t e = cudaStreamSynchronize(ctx->upload);
         s->stage.clear();
         s->stage_left = 0;
         if (e != cudaSuccess) rc = cuda_fail(ctx, e, "scene upload");
@@ -2317,9 +2337,10 @@ int ptr_free_scene(ptr_scene* s) {
     if (!s) return PTR_E_INVALID;
     if (s->ctx) {
         cudaSetDevice(s->ctx->device);
-        cudaStreamSynchronize(s->ctx->stream);
+        cudaStreamSynchronize(s->ctx->upload);   // a failed upload's copies
+        cudaStreamSynchronize(s->ctx->stream);   // frames of the scene
     }
-    for (void* a : s->allocs) dev_free(s->ctx, a);
+    for (void* a : s->allocs) scene_free(s->ctx, a);
     delete s;
     return PTR_OK;
 }

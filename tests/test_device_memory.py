@@ -12,7 +12,8 @@ STUB = """
 typedef int* cudaStream_t;
 typedef int* cudaMemPool_t;
 enum cudaError_t { cudaSuccess = 0, cudaErrorMemoryAllocation = 2, cudaErrorNotSupported = 801 };
-enum { cudaDevAttrMemoryPoolsSupported, cudaMemAllocationTypePinned, cudaMemLocationTypeDevice, cudaMemPoolAttrReleaseThreshold };
+enum { cudaDevAttrMemoryPoolsSupported, cudaMemAllocationTypePinned, cudaMemLocationTypeDevice, cudaMemPoolAttrReleaseThreshold,
+       cudaMemPoolReuseAllowInternalDependencies };
 struct cudaMemPoolProps { int allocType; struct { int type, id; } location; };
 cudaError_t cudaDeviceGetAttribute(int*, int, int);
 cudaError_t cudaMemPoolCreate(cudaMemPool_t*, const cudaMemPoolProps*);
@@ -23,7 +24,7 @@ cudaError_t cudaMalloc(void**, size_t);
 cudaError_t cudaFree(void*);
 cudaError_t cudaMallocFromPoolAsync(void**, size_t, cudaMemPool_t, cudaStream_t);
 cudaError_t cudaFreeAsync(void*, cudaStream_t);
-cudaError_t cudaStreamSynchronize(cudaStream_t);
+cudaError_t cudaDeviceSynchronize();
 cudaError_t cudaGetLastError();
 """
 RUNTIME = """
@@ -38,7 +39,11 @@ cudaError_t cudaMemPoolCreate(cudaMemPool_t* p, const cudaMemPoolProps* q) {
     *p = creates ? new int(q->location.id) : nullptr;
     return creates ? cudaSuccess : cudaErrorNotSupported;
 }
-cudaError_t cudaMemPoolSetAttribute(cudaMemPool_t, int, void* v) { std::printf("keep%llu ", *(unsigned long long*)v >> 20); return cudaSuccess; }
+cudaError_t cudaMemPoolSetAttribute(cudaMemPool_t, int a, void* v) {
+    if (a == cudaMemPoolAttrReleaseThreshold) std::printf("keep%llu ", *(unsigned long long*)v >> 20);
+    else std::printf(*(int*)v ? "tied " : "apart ");
+    return cudaSuccess;
+}
 cudaError_t cudaMemPoolDestroy(cudaMemPool_t p) { std::printf("~pool%d ", *p); return cudaSuccess; }
 cudaError_t cudaMemPoolTrimTo(cudaMemPool_t, size_t n) { std::printf("trim%zu ", n); left += idle; idle = 0; return cudaSuccess; }
 static cudaError_t take(void** out, size_t n, const char* how) {
@@ -52,7 +57,7 @@ cudaError_t cudaMalloc(void** p, size_t n) { return take(p, n, "malloc"); }
 cudaError_t cudaMallocFromPoolAsync(void** p, size_t n, cudaMemPool_t, cudaStream_t) { return take(p, n, "pooled"); }
 cudaError_t cudaFree(void* p) { std::printf("free%zu ", (size_t)p); return cudaSuccess; }
 cudaError_t cudaFreeAsync(void* p, cudaStream_t) { std::printf("async%zu ", (size_t)p); return cudaSuccess; }
-cudaError_t cudaStreamSynchronize(cudaStream_t) { std::printf("wait "); return cudaSuccess; }
+cudaError_t cudaDeviceSynchronize() { std::printf("wait "); return cudaSuccess; }
 cudaError_t cudaGetLastError() { return cudaSuccess; }
 using ptx_host::DeviceMemory;
 int main() {
@@ -78,13 +83,13 @@ def test_contexts_share_a_devices_pool(tmp_path):
     m.close(); n.close(); o.close();
     m.open(0, nullptr); m.close();
     """)
-    assert out == "pool0 keep512 pool1 keep512 pooled malloc async1 free2 ~pool0 ~pool1 pool0 keep512 ~pool0".split()
+    assert out == "pool0 keep512 apart pool1 keep512 apart pooled malloc async1 free2 ~pool0 ~pool1 pool0 keep512 apart ~pool0".split()
 
 
 def test_any_ordinal_and_no_pools(tmp_path):
     use = "m.alloc(&a, 100); m.alloc(&b, 1u << 30); m.free(a); m.free(b); m.close();"
     assert _run(tmp_path, "DeviceMemory m; m.open(71, nullptr); " + use) == \
-        "pool71 keep512 pooled malloc async1 free2 ~pool71".split()
+        "pool71 keep512 apart pooled malloc async1 free2 ~pool71".split()
     assert _run(tmp_path, "supported = false; DeviceMemory m; m.open(0, nullptr); " + use) == "malloc malloc free1 free2".split()
     assert _run(tmp_path, "creates = false; DeviceMemory m; m.open(0, nullptr); " + use) == "pool0 malloc malloc free1 free2".split()
 
@@ -116,5 +121,5 @@ def test_idle_pool_memory_does_not_refuse_a_block(tmp_path):
     std::printf("%d ", (int)m.alloc(&b, 200u << 20));
     m.free(a); m.free(b); m.close();
     """)
-    assert out == ("pool0 keep512 malloc! wait trim0 malloc 0 pooled! wait trim0 pooled! 2 "
+    assert out == ("pool0 keep512 apart malloc! wait trim0 malloc 0 pooled! wait trim0 pooled! 2 "
                    "pooled! wait trim0 pooled 0 free1 async2 ~pool0").split()
