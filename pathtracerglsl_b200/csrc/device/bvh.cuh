@@ -531,14 +531,18 @@ __device__ __forceinline__ bool flat_binary_ok(const DevScene& S, const DevBatch
 }
 
 // ---- region arms ------------------------------------------------------------------------
-// The per-scene kernels inline these arms; the library's generic kernels call them (ptx_rt.cu
-// defines PTR_ACCEL_CALL): inlined next to every other arm, the tree walks' registers spilled
-// across the region scans (fog with 256 lamps and a mesh, 512 x 384 x 8: 25.3 ms inlined, 20.7
-// called).
+// Inlined, but for the shadow queries through media (and the point classification) of the
+// library's generic kernels, which call them (ptx_rt.cu defines PTR_ACCEL_CALL): inlined next to
+// every arm of a media query, the tree walks' registers spilled across the region scans (fog with
+// 256 lamps and a mesh, 512 x 384 x 8: 25.3 ms with every arm inlined, 20.7 with every arm called).
+// The closest hits and the opaque queries lose more by the call than it saves: k_closest of a
+// 512 x 512 x 8 frame around one 320-triangle mesh takes 0.78 ms inlined and 0.99 called, around
+// one 327,680-triangle mesh at 640 x 360 x 4 1.63 and 1.97; the kernels of the lamps in fog 17.9
+// and 19.6 ms.
 #ifndef PTR_ACCEL_CALL
 #define PTR_ACCEL_CALL __forceinline__
 #endif
-__device__ PTR_ACCEL_CALL HitRec accel_closest(const DevScene& S, const ptr_region& g, int region, Ray r, HitRec h,
+__device__ __forceinline__ HitRec accel_closest(const DevScene& S, const ptr_region& g, int region, Ray r, HitRec h,
                                                Work* w = nullptr) {
     if (kHasMesh && g.shape == PTR_SHAPE_MESH) {
         const DevMesh& m = S.meshes[g.ref];
@@ -594,7 +598,7 @@ __device__ PTR_ACCEL_CALL HitRec accel_closest(const DevScene& S, const ptr_regi
     return h;
 }
 
-__device__ PTR_ACCEL_CALL bool accel_any(const DevScene& S, const ptr_region& g, Ray r, float max_dist,
+__device__ __forceinline__ bool accel_any(const DevScene& S, const ptr_region& g, Ray r, float max_dist,
                                           Work* w = nullptr) {
     if (kHasMesh && g.shape == PTR_SHAPE_MESH) return mesh_any(S, S.meshes[g.ref], r.o, r.d, max_dist, w);
     const DevBatch& b = S.batches[g.ref];
@@ -622,6 +626,14 @@ __device__ PTR_ACCEL_CALL bool accel_any(const DevScene& S, const ptr_region& g,
             if (instance(i)) return true;
         return false;
     }, w ? &w->tlas : nullptr);
+}
+
+// The same arms as calls.
+__device__ PTR_ACCEL_CALL HitRec accel_closest_call(const DevScene& S, const ptr_region& g, int region, Ray r, HitRec h, Work* w) {
+    return accel_closest(S, g, region, r, h, w);
+}
+__device__ PTR_ACCEL_CALL bool accel_any_call(const DevScene& S, const ptr_region& g, Ray r, float max_dist, Work* w) {
+    return accel_any(S, g, r, max_dist, w);
 }
 
 // Containment of an instanced SPHERE batch (the TLAS point descent of scene_region_at):

@@ -273,7 +273,9 @@ __device__ __forceinline__ int warp_append(unsigned* counter, bool pred) {
 }
 
 // ---- scene queries -------------------------------------------------------------------
-// Nearest hit over every arm; returns region (or -1), element, primitive and t.
+// Nearest hit over every arm; returns region (or -1), element, primitive and t.  CALL (here and in
+// scene_any): the library's generic kernels call the acceleration arms instead of inlining them
+// (bvh.cuh).
 
 __device__ __forceinline__ float4 int4_as_float4(int4 v) {
     return make_float4(__int_as_float(v.x), __int_as_float(v.y), __int_as_float(v.z), __int_as_float(v.w));
@@ -340,6 +342,7 @@ __device__ __forceinline__ bool for_sphere_candidates(const DevScene& S, const R
     return false;
 }
 
+template <bool CALL = true>
 __device__ __forceinline__ HitRec scene_closest(const DevScene& S, const Ray& r, Work* w = nullptr) {
     HitRec h;
     h.t = kMaxDist;
@@ -355,7 +358,7 @@ __device__ __forceinline__ HitRec scene_closest(const DevScene& S, const Ray& r,
     };
     auto arm = [&](int i, const ptr_region& g, int shape) {
         if (has_accel() && shape >= PTR_SHAPE_MESH) {
-            h = accel_closest(S, g, i, r, h, w);
+            h = CALL ? accel_closest_call(S, g, i, r, h, w) : accel_closest(S, g, i, r, h, w);
             return;
         }
         float t;
@@ -421,9 +424,10 @@ __device__ __forceinline__ HitRec scene_closest(const DevScene& S, const Ray& r,
     return h;
 }
 
+template <bool CALL = true>
 __device__ __forceinline__ bool scene_any(const DevScene& S, const Ray& r, float max_dist, Work* w = nullptr) {
     auto arm = [&](const ptr_region& g, int shape) -> bool {
-        if (has_accel() && shape >= PTR_SHAPE_MESH) return accel_any(S, g, r, max_dist, w);
+        if (has_accel() && shape >= PTR_SHAPE_MESH) return CALL ? accel_any_call(S, g, r, max_dist, w) : accel_any(S, g, r, max_dist, w);
         float t;
         return analytic_root_shape(shape, g, r, t) && t < max_dist;
     };
@@ -703,7 +707,7 @@ __device__ __forceinline__ void init_slot(const PathPool& pool, long long i, con
 
 // Camera rays for one wave.
 template <bool ADJ = false, bool SPECTRAL = false>
-__global__ void k_generate(DevScene S, PathPool pool, const FrameParams* fp, AdjParams adj = AdjParams{}) {
+__global__ void k_generate(const __grid_constant__ DevScene S, PathPool pool, const FrameParams* fp, AdjParams adj = AdjParams{}) {
     const FrameParams F = *fp;
     long long base = pool.wave[0];
     long long n = F.total - base;
@@ -892,7 +896,7 @@ __global__ void __launch_bounds__(256, PTR_TRACE_MIN_BLOCKS) k_closest(const __g
             Ray r;
             r.o = xyz(pool.ray_o[i]);
             r.d = xyz(pool.ray_d[i]);
-            HitRec h = scene_closest(S, r, COUNT ? &w : nullptr);
+            HitRec h = scene_closest<false>(S, r, COUNT ? &w : nullptr);
             hf = make_float4(h.t, h.u, h.v, 0.f);
             hi = make_int4(h.region, h.element, h.prim, 0);
             if (log && pool.hit_log_mode == 1) {
@@ -1599,7 +1603,7 @@ __device__ __forceinline__ Col shadow_visibility(const DevScene& S, const ProgPa
                                                  int crossings_left, const Wl& wl, SeedOf seed_of, bool collect, bool flag_more,
                                                  ShadowMedia& mm, Work* work) {
     constexpr bool SPECTRAL = sizeof(Col) == sizeof(s4);
-    if (!MEDIA) return scene_any(S, sr, max_dist, work) ? Col(0.0f) : Col(1.0f);
+    if (!MEDIA) return scene_any<false>(S, sr, max_dist, work) ? Col(0.0f) : Col(1.0f);
     Col T(1.0f);
     Rng srng;
     bool srng_live = false;
@@ -2228,7 +2232,7 @@ __global__ void k_film_batch_walk(BatchTables bt, WalkArgs wa) {
 
 // Raw nearest-hit queries (tests and tools): per ray (o.xyz, d.xyz) the region, the
 // element (instance), the ORIGINAL triangle index (or -1) and t (kMaxDist on a miss).
-__global__ void k_trace_rays(DevScene S, const float* rays, int n, int* region, int* element, int* prim, float* t_out) {
+__global__ void k_trace_rays(const __grid_constant__ DevScene S, const float* rays, int n, int* region, int* element, int* prim, float* t_out) {
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
         Ray r;
         r.o = f3(rays[6 * k], rays[6 * k + 1], rays[6 * k + 2]);
