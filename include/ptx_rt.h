@@ -316,8 +316,8 @@ int ptr_abi_version(void);
 
 /* Scene data upload, once per scene (Engine.registerDataTexture, Engine.ts:438;
  * sceneData.ts:27).  Builds the BVH/CWBVH of every mesh on the host and copies all
- * arrays to device memory, on a stream of its own: it returns once they are there and does not
- * wait for frames in flight on the context. */
+ * arrays to device memory, on a stream of uploads that the device's contexts share: it returns
+ * once they are there and does not wait for frames in flight. */
 int ptr_upload_scene(ptr_ctx* ctx, const ptr_scene_desc* desc, ptr_scene** out);
 int ptr_free_scene(ptr_scene* scene);
 

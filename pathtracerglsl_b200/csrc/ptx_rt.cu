@@ -61,8 +61,8 @@ struct ptr_ctx {
     // by census key
     std::map<std::string, SpecKernels> batch_spec;
     int accel_build = PTR_BUILD_HOST;   // where ptr_upload_scene builds mesh BVHs (ptr_set_accel_build)
-    // Scenes are uploaded (and their trees built) on a stream of their own, waited for before the
-    // upload returns, so an upload does not wait for frames in flight.
+    // Scenes are uploaded (and their trees built) on a stream that the device's contexts share,
+    // waited for before the upload returns, so an upload does not wait for frames in flight.
     cudaStream_t upload = nullptr;
     ptx_host::DeviceMemory memory;       // programs' and calls' blocks, ordered on stream
     ptx_host::DeviceMemory scene_memory; // scenes' and builds' blocks, ordered on upload
@@ -1984,18 +1984,14 @@ int ptr_create(int device_ordinal, ptr_ctx** out) {
         delete c;
         return PTR_E_CUDA;
     }
-    if (cudaStreamCreateWithFlags(&c->upload, cudaStreamNonBlocking) != cudaSuccess) {
-        cudaStreamDestroy(c->stream);
-        delete c;
-        return PTR_E_CUDA;
-    }
     c->memory.open(device_ordinal, c->stream);
+    c->upload = ptx_host::DevicePools::all().upload_stream(device_ordinal);
+    if (!c->upload) c->upload = c->stream;
     c->scene_memory.open(device_ordinal, c->upload);
     // the counting sort's scan stages its whole table in shared memory (above the 48 KB default)
     if (cudaFuncSetAttribute((const void*)k_sort_scan, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSortScanSmem) != cudaSuccess) {
         c->scene_memory.close();
         c->memory.close();
-        cudaStreamDestroy(c->upload);
         cudaStreamDestroy(c->stream);
         delete c;
         return PTR_E_CUDA;
@@ -2013,7 +2009,6 @@ int ptr_destroy(ptr_ctx* ctx) {
     cudaStreamSynchronize(ctx->upload);
     ctx->scene_memory.close();
     ctx->memory.close();
-    cudaStreamDestroy(ctx->upload);
     cudaStreamDestroy(ctx->stream);
     delete ctx;
     return PTR_OK;

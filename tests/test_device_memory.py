@@ -25,6 +25,9 @@ cudaError_t cudaFree(void*);
 cudaError_t cudaMallocFromPoolAsync(void**, size_t, cudaMemPool_t, cudaStream_t);
 cudaError_t cudaFreeAsync(void*, cudaStream_t);
 cudaError_t cudaDeviceSynchronize();
+enum { cudaStreamNonBlocking = 1 };
+cudaError_t cudaStreamCreateWithFlags(cudaStream_t*, unsigned);
+cudaError_t cudaStreamDestroy(cudaStream_t);
 cudaError_t cudaGetLastError();
 """
 RUNTIME = """
@@ -59,7 +62,10 @@ cudaError_t cudaFree(void* p) { std::printf("free%zu ", (size_t)p); return cudaS
 cudaError_t cudaFreeAsync(void* p, cudaStream_t) { std::printf("async%zu ", (size_t)p); return cudaSuccess; }
 cudaError_t cudaDeviceSynchronize() { std::printf("wait "); return cudaSuccess; }
 cudaError_t cudaGetLastError() { return cudaSuccess; }
+cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned) { std::printf("stream "); *s = new int(0); return cudaSuccess; }
+cudaError_t cudaStreamDestroy(cudaStream_t) { std::printf("~stream "); return cudaSuccess; }
 using ptx_host::DeviceMemory;
+using ptx_host::DevicePools;
 int main() {
     void *a, *b;
     %s
@@ -123,3 +129,16 @@ def test_idle_pool_memory_does_not_refuse_a_block(tmp_path):
     """)
     assert out == ("pool0 keep512 apart malloc! wait trim0 malloc 0 pooled! wait trim0 pooled! 2 "
                    "pooled! wait trim0 pooled 0 free1 async2 ~pool0").split()
+
+
+def test_contexts_share_a_devices_upload_stream(tmp_path):
+    out = _run(tmp_path, """
+    DeviceMemory m, n;
+    m.open(2, nullptr); n.open(2, nullptr);
+    std::printf("%s ", DevicePools::all().upload_stream(2) == DevicePools::all().upload_stream(2) ? "same" : "other");
+    m.close();
+    std::printf("| ");
+    n.close();
+    m.open(2, nullptr); m.close();
+    """)
+    assert out == "pool2 keep512 apart stream same | ~stream ~pool2 pool2 keep512 apart ~pool2".split()

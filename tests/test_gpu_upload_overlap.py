@@ -1,8 +1,10 @@
 """A scene is uploaded while a frame of another renders: the upload returns with the frame still in
-flight (its own stream carries the copies), the frame's picture is what it is alone, and the
+flight (a stream of uploads carries the copies), the frame's picture is what it is alone, and the
 uploaded scene renders as one uploaded to an idle context.  Uploads that run kernels (trees built
-on the device, rails) may have to wait for room beside the frame's; their pictures agree too."""
+on the device, rails) may have to wait for room beside the frame's; their pictures agree too.
+Contexts on several threads share that stream: each thread's scenes render as they do alone."""
 import ctypes as C
+import threading
 
 import numpy as np
 import pytest
@@ -73,3 +75,43 @@ def test_upload_beside_a_frame(scene, build):
         np.testing.assert_array_equal(picture(h), idle)
     finally:
         eng.close()
+
+
+def test_contexts_on_several_threads():
+    jobs = [_small(), _mesh(), scenes.cornell(max_depth=3), scenes.cornell_mesh_light(), _mesh(), scenes.het_fog(max_depth=3)]
+    compiled = [Compiler().compile(*j) for j in jobs]
+    want, got, errors = [None] * len(jobs), [[] for _ in jobs], []
+
+    def render(k, eng):
+        r, pk = compiled[k]
+        eng.set_accel_build("device" if k % 2 else "host")
+        eng.register_scene(pk)
+        eng.load_renderer(r)
+        eng.select_renderer(r.id)
+        eng.pin_reset_salt(7)
+        eng.reset()
+        eng.render_frame(37, 29, 2)
+        return eng.read_export("radiance").copy()
+
+    def work(k):
+        try:
+            for _ in range(4):
+                eng = CudaEngine(0)
+                got[k] += [render(k, eng) for _ in range(3)]
+                eng.close()
+        except Exception as e:   # noqa: BLE001
+            errors.append(e)
+    for k in range(len(jobs)):
+        eng = CudaEngine(0)
+        want[k] = render(k, eng)
+        eng.close()
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(len(jobs))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors
+    for w, pictures in zip(want, got, strict=True):
+        assert len(pictures) == 12
+        for p in pictures:
+            np.testing.assert_array_equal(p, w)
