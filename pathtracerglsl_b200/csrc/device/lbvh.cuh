@@ -268,9 +268,8 @@ __device__ __forceinline__ float half_area(float4 a, float4 b) {
     const float dx = b.x - a.x, dy = b.y - a.y, dz = b.z - a.z;
     return dx * dy + dy * dz + dz * dx;
 }
-// counters: [0] wide nodes allocated, [1] leaf items placed, [2] next level's tasks,
-// [3] error flag (quantization range)
-// counters: [0] nodes, [1] items, [3] error flags, [4 + l] the tasks of level l.
+// counters: [0] wide nodes allocated, [1] leaf items placed, [3] error flag (quantization range),
+// [4 + l] the tasks of level l.
 constexpr int kCollapseCounters = 32;
 __global__ void k_collapse(int n, const int* child, const int2* range, const float4* nlo, const float4* nhi,
                            const unsigned long long* keys, const int2* tasks, int2* next,

@@ -1872,10 +1872,11 @@ __global__ void __launch_bounds__(256, PTR_TRACE_MIN_BLOCKS) k_shadow(const __gr
 // sums are walk_iteration's and shadow_visibility's, so samples are bit-identical to the
 // wavefront kernels'.
 // What bounds it is instruction issue (70 % of the slots, 17.5 of 32 lanes on the Cornell box)
-// and, were its warps to run free, the instruction cache: a walk is 70 to 500 KB of code.  A block's
-// warps therefore run each part of an iteration together, so that one pass of the part's code
-// through the cache serves them all (media and spectral workload, 16.8 M paths: 128 ms with
-// free-running warps, 41 ms in step; adjoint 15.4 and 9.3; fog room in tiles 50.0 and 48.4).
+// and, were its warps to run free, the instruction cache: a walk is 70 to 220 KB of code built for
+// a scene, 150 to 710 in the library's form.  A block's warps therefore run each part of an
+// iteration together, so that one pass of the part's code through the cache serves them all
+// (media and spectral workload, 16.8 M paths: 128 ms with free-running warps, 41 ms in step;
+// adjoint 15.4 and 9.3; fog room in tiles 50.0 and 48.4).
 // 64 registers (1024 threads per SM) measured faster than 80 or 128, and two blocks of 512
 // faster than four of 256 (fewer passes through the cache; the 64-job mix 279 ms at 80
 // registers, 276 with four blocks, 267 with two; the adjoint 7.4, 7.1 and 6.5); refilling at
