@@ -379,7 +379,9 @@ int ptr_compile(ptr_ctx* ctx, const ptr_program_desc* desc, ptr_program** out);
 int ptr_free_program(ptr_program* prog);
 
 /* Render frame.spp samples per pixel into the program's film, asynchronously
- * (Engine.renderFrame, Engine.ts:190-204; one call may fold many frames). */
+ * (Engine.renderFrame, Engine.ts:190-204; one call may fold many frames).  A frame that
+ * restarts the film, or sizes it anew, and fails leaves an empty one: black pictures, and the next
+ * frame starts from zero whether it accumulates or not. */
 int ptr_render(ptr_program* prog, ptr_scene* scene, const ptr_frame* frame);
 
 /* Batched rendering: many scenes x programs x frames of uneven size in ONE wavefront —
